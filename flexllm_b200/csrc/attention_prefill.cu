@@ -12,17 +12,22 @@
 //   O[q][d]  = sum_k U[q][k] V[k][d]                        u8 x s8 -> s32   (tensor cores)
 //   out      = (float)O * a_s
 //
-// The reference quantises the FINAL normalised P and accumulates a whole row of P.V in one int32,
-// so a rescaling online softmax cannot reproduce it. The kernel therefore sweeps the keys three
-// times instead of materialising S x S scores in one pass:
+// The reference quantises the FINAL normalised P and accumulates a whole row of P.V in one int32, so a rescaling online
+// softmax cannot reproduce it. The kernel therefore sweeps the keys three times; the scores are recomputed on the tensor
+// cores each time, which are idle otherwise, and nothing is parked in memory between the sweeps:
 //   sweep 0: Q.K^T tile -> row max
-//   sweep 1: Q.K^T tile again -> e = exp(x - max), ordered partial sums; e is parked in a global
-//            scratch (128 x 64 fp32 per tile, written and read back by the same thread, L2-resident)
-//   sweep 2: e read back -> U (u8, 64-byte-swizzled shared memory) -> O += U.V
-// One thread owns one query row (TMEM lane), so every per-row fp32 chain runs in the reference's
-// order. One CTA = 128 queries of one (batch, query head) against 64-key tiles; 4 softmax warps +
-// TMA warp + MMA warp; TMEM: S (64 columns) + O (64 columns) = 128 columns, so four CTAs share an SM
-// and their 16 softmax warps hide each other's latencies.
+//   sweep 1: Q.K^T tile again -> e = exp(x - max) to the last bit, ordered partial sums
+//   sweep 2: Q.K^T tile again -> U from the hardware exponential with a proven error bound; a value so close to a rounding
+//            boundary that the bound does not decide it is worked out again as the reference does (about one in 30000 at U = 1)
+//            -> U (u8, 64-byte-swizzled shared memory) -> O += U.V
+// One thread owns one query row (TMEM lane), so every per-row fp32 chain runs in the reference's order. One CTA = 128
+// queries of one (batch, query head) against 64-key tiles; 4 softmax warps + TMA warp + MMA warp; TMEM: S (64 columns) +
+// O (64 columns) = 128 columns, so four CTAs share an SM and their 16 softmax warps hide each other's latencies. S is
+// released as soon as its last columns are in registers: the next tile's product runs under this tile's arithmetic.
+//
+// Bound: instruction issue of the softmax warps (60 % of the issue slots busy; double precision and the special-function
+// pipe 15 % each, DRAM idle). 4 prompts of 1024 tokens, 32 / 8 heads: 513 us with the exponentials of sweep 1 parked in a
+// scratch (568 MB written and read back through L2), separate fp32 operations and full divisions; 252 us now.
 #include <cstdlib>
 
 #include "attention_decode.cuh"     // layout of the paged KV cache
@@ -107,7 +112,6 @@ struct AttnArgs {
     const float* a_s;   // [HQ]
     float* out;         // [B][Sq][HQ*64]
     int32_t* oacc;      // optional, same shape
-    uint8_t* ecache;    // exp values of sweep 1 kept for sweep 2 (attn_ecache_head_bytes per (batch, head))
     int* error_flag;
 };
 
@@ -130,14 +134,21 @@ constexpr int ATT_TILE_BYTES = 64 * 64;       // one K tile [64 keys][64 B] or o
 constexpr int ATT_P_BYTES = 128 * 64;         // U tile [128 queries][64 keys] u8
 constexpr int ATT_SMEM = ATT_Q_BYTES + ATT_SLOTS * ATT_TILE_BYTES + 2 * ATT_P_BYTES + 1024 + 256;
 constexpr int ATT_TMEM_COLS = 128;
+constexpr int ATT_EXP_GROUP = 8;              // exponentials whose dependency chains interleave
 
-// Bytes of exp-cache one (batch, query head) needs: for every 128-query tile qt = q_off/128 + t (t < n_qt) its
-// 2*(qt+1) key tiles of 128 x 64 fp32.
-__host__ __device__ inline size_t attn_ecache_head_bytes(int q_off, int Sq) {
-    const size_t n_qt = (Sq + 127) / 128, qt0 = q_off / 128;
-    return n_qt * (2 * qt0 + n_qt + 1) * (size_t)(128 * ATT_KT * 4);   // sum_{t < n_qt} 2*(qt0+t+1) tiles
+// The reference's arithmetic of one probability: U = min(round((e * r * vs) / a_s), 255) with e = exp(-u). Out of line: for the
+// values that sweep 2 cannot decide, and for scales outside the range of its error bound.
+__device__ __noinline__ static uint32_t attn_u8_exact(float u, float rinv, float vs, float a_s) {
+    const float p = ref_expf(-u) * rinv;
+    const int r = round_half_away_to_int((p * vs) / a_s);
+    return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
 }
 
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_constant__ CUtensorMap tmapQ,
                                                               const __grid_constant__ CUtensorMap tmapK,
                                                               const __grid_constant__ CUtensorMap tmapV,
@@ -166,19 +177,17 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int S = args.q_off + args.Sq;                            // keys (positions 0 .. S-1)
     const int n_qt = (args.Sq + 127) >> 7;
-    const int qt_l = n_qt - 1 - (int)(blockIdx.x % n_qt);          // query tile within the call: heavy tiles (late queries) first
+    // the heaviest query tiles (most keys) of all heads first, so that the last CTAs to start are the shortest
+    const int heads = args.B * args.HQ;
+    const int qt_l = n_qt - 1 - (int)(blockIdx.x / heads);         // query tile within the call
     const int qt0 = args.q_off >> 7, qt = qt0 + qt_l;              // ... and within the sequence
-    const int hq = (int)((blockIdx.x / n_qt) % args.HQ);
-    const int b = (int)(blockIdx.x / ((long)n_qt * args.HQ));
+    const int hq = (int)(blockIdx.x % heads) % args.HQ;
+    const int b = (int)(blockIdx.x % heads) / args.HQ;
     const int hkv = hq / (args.HQ / args.HKV);
     const int n_kt_all = (S + ATT_KT - 1) / ATT_KT;
     const int n_kt = 2 * (qt + 1) < n_kt_all ? 2 * (qt + 1) : n_kt_all;   // causal: 64-key tiles 0 .. 2*qt+1 (those that hold keys)
     const bool paged = args.page_table != nullptr;
     const int32_t* pt = paged ? args.page_table + (long)b * args.max_pages : nullptr;
-    // this CTA's slice of the exp cache: [n_kt][16 float4 chunks][128 rows] float4
-    float4* ecache = reinterpret_cast<float4*>(args.ecache + ((size_t)b * args.HQ + hq) * attn_ecache_head_bytes(args.q_off, args.Sq) +
-                                               ((size_t)2 * qt_l * qt0 + (size_t)qt_l * (qt_l + 1)) * (size_t)(128 * ATT_KT * 4));
-
     if (threadIdx.x == 0) {
         mbar_init(bar_qfull, 1);
         for (int i = 0; i < ATT_SLOTS; i++) { mbar_init(bar_tfull + 8 * i, 1); mbar_init(bar_tempty + 8 * i, 1); }
@@ -197,24 +206,31 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
 
     if (warp == 4) {
         // ------------------------------------------------------------ TMA producer
-        // iterations 0 .. 2*n_kt-1: K tiles of sweeps 0 and 1; then n_kt V^T tiles for sweep 2
+        // K tiles of sweeps 0 and 1 in order; then, for sweep 2, K one tile ahead of V^T: K0, K1, V0, K2, V1, ...
         if (lane == 0) {
             tma_prefetch_desc(&tmapQ); tma_prefetch_desc(&tmapK); tma_prefetch_desc(&tmapV);
             mbar_expect_tx(bar_qfull, ATT_Q_BYTES);
             tma_load_2d(sQ, &tmapQ, bar_qfull, 0, ((b * args.HQ + hq) * args.Sq) + qt_l * 128);
             int slot = 0; uint32_t phase = 0;
-            for (int it = 0; it < 3 * n_kt; it++) {
-                const int sweep = it / n_kt, j = it - sweep * n_kt;
-                if (!mbar_wait(bar_tempty + 8 * slot, phase ^ 1u, abort_flag)) break;
+            auto load = [&](bool is_k, int j) {
+                if (!mbar_wait(bar_tempty + 8 * slot, phase ^ 1u, abort_flag)) return false;
                 const uint32_t full = bar_tfull + 8 * slot;
                 const uint32_t dst = sT + slot * ATT_TILE_BYTES;
                 mbar_expect_tx(full, ATT_TILE_BYTES);
-                if (paged) {        // one tile = one page of the cache: K rows [64 keys][64 B], V^T rows [64 dims][64 keys]
-                    const int row = (__ldg(pt + j) * args.HKV + hkv) * 64;
-                    tma_load_2d(dst, sweep < 2 ? &tmapK : &tmapV, full, 0, row);
-                } else if (sweep < 2) tma_load_2d(dst, &tmapK, full, 0, ((b * args.HKV + hkv) * args.Sk) + j * ATT_KT);
+                // paged: one tile = one page of the cache: K rows [64 keys][64 B], V^T rows [64 dims][64 keys]
+                if (paged) tma_load_2d(dst, is_k ? &tmapK : &tmapV, full, 0, (__ldg(pt + j) * args.HKV + hkv) * 64);
+                else if (is_k) tma_load_2d(dst, &tmapK, full, 0, ((b * args.HKV + hkv) * args.Sk) + j * ATT_KT);
                 else tma_load_2d(dst, &tmapV, full, j * ATT_KT, (b * args.HKV + hkv) * 64);
                 if (++slot == ATT_SLOTS) { slot = 0; phase ^= 1u; }
+                return true;
+            };
+            bool ok = true;
+            for (int sweep = 0; ok && sweep < 2; sweep++)
+                for (int j = 0; ok && j < n_kt; j++) ok = load(true, j);
+            if (ok) ok = load(true, 0);
+            for (int j = 0; ok && j < n_kt; j++) {
+                if (j + 1 < n_kt) ok = load(true, j + 1);
+                if (ok) ok = load(false, j);
             }
         }
     } else if (warp == 5) {
@@ -225,31 +241,37 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
             bool ok = mbar_wait(bar_qfull, 0, abort_flag);
             const uint64_t qdesc = umma_desc_k_sw64(sQ);
             int slot = 0; uint32_t tphase = 0;
-            for (int it = 0; ok && it < 3 * n_kt; it++) {
-                const int sweep = it / n_kt, j = it - sweep * n_kt;
-                if (!mbar_wait(bar_tfull + 8 * slot, tphase, abort_flag)) { ok = false; break; }
-                const uint32_t sTile = sT + slot * ATT_TILE_BYTES;
-                if (sweep < 2) {
-                    // S = Q.K^T for this key tile (S is single-buffered: iteration it is its phase)
-                    if (!mbar_wait(bar_sempty, (uint32_t)(it & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t kdesc = umma_desc_k_sw64(sTile);
-                    umma_i8(tmem_S, qdesc, kdesc, idesc_qk, 0u);
-                    umma_i8(tmem_S, qdesc + 2, kdesc + 2, idesc_qk, 1u);
-                    umma_commit(bar_sfull);
-                } else {
-                    // O += U.V for this key tile once the softmax warps have written U
-                    const int pb = j & 1;
-                    if (!mbar_wait(bar_pfull + 8 * pb, (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t pdesc = umma_desc_k_sw64(sP + pb * ATT_P_BYTES);
-                    const uint64_t vdesc = umma_desc_k_sw64(sTile);
-                    umma_i8(tmem_O, pdesc, vdesc, idesc_pv, j > 0 ? 1u : 0u);
-                    umma_i8(tmem_O, pdesc + 2, vdesc + 2, idesc_pv, 1u);
-                    umma_commit(bar_pempty + 8 * pb);
-                }
+            int it = 0;                                   // score tiles so far: S is single-buffered, its phase is it & 1
+            auto release_tile = [&]() {
                 umma_commit(bar_tempty + 8 * slot);
                 if (++slot == ATT_SLOTS) { slot = 0; tphase ^= 1u; }
+            };
+            auto issue_qk = [&]() {                       // S = Q.K^T of the next key tile, once the last scores are read
+                if (!mbar_wait(bar_tfull + 8 * slot, tphase, abort_flag)) return false;
+                if (!mbar_wait(bar_sempty, (uint32_t)(it & 1) ^ 1u, abort_flag)) return false;
+                tc_fence_after();
+                const uint64_t kdesc = umma_desc_k_sw64(sT + slot * ATT_TILE_BYTES);
+                umma_i8(tmem_S, qdesc, kdesc, idesc_qk, 0u);
+                umma_i8(tmem_S, qdesc + 2, kdesc + 2, idesc_qk, 1u);
+                umma_commit(bar_sfull);
+                release_tile();
+                it++;
+                return true;
+            };
+            for (int j = 0; ok && j < 2 * n_kt + 1; j++) ok = issue_qk();      // sweeps 0 and 1, and sweep 2's first tile
+            for (int j = 0; ok && j < n_kt; j++) {
+                if (j + 1 < n_kt && !issue_qk()) { ok = false; break; }
+                // O += U.V of key tile j once the softmax warps have written U
+                const int pb = j & 1;
+                if (!mbar_wait(bar_tfull + 8 * slot, tphase, abort_flag)) { ok = false; break; }
+                if (!mbar_wait(bar_pfull + 8 * pb, (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t pdesc = umma_desc_k_sw64(sP + pb * ATT_P_BYTES);
+                const uint64_t vdesc = umma_desc_k_sw64(sT + slot * ATT_TILE_BYTES);
+                umma_i8(tmem_O, pdesc, vdesc, idesc_pv, j > 0 ? 1u : 0u);
+                umma_i8(tmem_O, pdesc + 2, vdesc + 2, idesc_pv, 1u);
+                umma_commit(bar_pempty + 8 * pb);
+                release_tile();
             }
             if (ok) umma_commit(bar_ofull);
         }
@@ -258,112 +280,192 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
         const int row_in_tile = warp * 32 + lane;
         const int qpos = qt * 128 + row_in_tile;               // position of this thread's query
         const bool q_ok = qpos < S;
-        const int qlim = q_ok ? qpos : -1;                     // keys 0..qlim are visible to this row
+        const int qlim = q_ok ? qpos : S - 1;                  // keys 0..qlim are visible to this row (rows beyond S: zeros, not stored)
         const float qscale = q_ok ? args.qs[((long)b * args.HQ + hq) * args.Sq + (qpos - args.q_off)] : 0.0f;
+        const f32x2 qscale2 = pack2(qscale, qscale);
         const float* ksp = args.ks + ((long)b * args.HKV + hkv) * args.Sk;      // contiguous layout
         const float* vsp = args.vs + ((long)b * args.HKV + hkv) * args.Sk;
         const float a_s = args.a_s[hq];
-        const DivBy d_as = div_by(a_s);
         const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
-        float mx = -1e32f;
-        float ps0 = 0.f, ps1 = 0.f, ps2 = 0.f, ps3 = 0.f;
         bool ok = true;
-        // ---- sweeps 0 and 1: scores from the tensor core, 16 columns at a time
-        for (int it = 0; ok && it < 2 * n_kt; it++) {
-            const int sweep = it / n_kt, j = it - sweep * n_kt;
+        // waits for score tile number it; false when the wait ran out
+        auto scores_ready = [&](int it) {
             int got = (lane == 0) ? (mbar_wait(bar_sfull, (uint32_t)(it & 1), abort_flag) ? 1 : 0) : 1;
             got = __shfl_sync(0xffffffffu, got, 0);
-            if (!got) { ok = false; break; }
-            tc_fence_after();
-            const int k0 = j * ATT_KT;
-            const float* kst = paged ? args.ks + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : ksp + k0;   // this tile's key scales
+            if (got) tc_fence_after();
+            return got != 0;
+        };
+        auto release_scores = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_sempty);
+        };
+        // (S * qs) * ks of 16 keys starting at kc (chunk c of the tile), two values to a register pair; keys beyond S get scale 0.
+        // S is released after the tile's last chunk.
+        auto scores16 = [&](const float* kst, int kc, int c, f32x2 (&y)[8]) {
+            uint32_t v[16];
+            tmem_ld_32x16(tmem_S + lane_addr + c * 16, v);
+            float4 ks4[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                ks4[i] = (kc + 4 * i < S) ? *reinterpret_cast<const float4*>(kst + c * 16 + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            tmem_ld_wait();
+            if (c == ATT_KT / 16 - 1) release_scores();
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                y[2 * i] = mul2(mul2(pack2((float)(int)v[4 * i], (float)(int)v[4 * i + 1]), qscale2), pack2(ks4[i].x, ks4[i].y));
+                y[2 * i + 1] = mul2(mul2(pack2((float)(int)v[4 * i + 2], (float)(int)v[4 * i + 3]), qscale2), pack2(ks4[i].z, ks4[i].w));
+            }
+        };
+        const int first_masked = 2 * qt;                       // tiles before this one are visible to every row of the CTA
+
+        // ---- sweep 0: the row maximum, tracked WITHOUT the factor 0.125 (scaling by a power of two is exact and keeps the
+        // order, so max(x * 0.125) == max(x) * 0.125: applied once after the sweep)
+        float mx = -1e32f;
+        for (int j = 0; ok && j < n_kt; j++) {
+            if (!scores_ready(j)) { ok = false; break; }
+            const float* kst = paged ? args.ks + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : ksp + j * ATT_KT;   // this tile's key scales
 #pragma unroll 1
             for (int c = 0; c < ATT_KT / 16; c++) {
-                uint32_t v[16];
-                tmem_ld_32x16(tmem_S + lane_addr + c * 16, v);
-                const int kc = k0 + c * 16;
-                // key scales of these 16 keys (same addresses for the whole warp); keys beyond S are masked
-                float ksv[16];
+                const int kc = j * ATT_KT + c * 16;
+                f32x2 y[8];
+                scores16(kst, kc, c, y);
+                float x[16];
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                    const float4 t = (kc + i < S) ? *reinterpret_cast<const float4*>(kst + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    ksv[i] = t.x; ksv[i + 1] = t.y; ksv[i + 2] = t.z; ksv[i + 3] = t.w;
+                for (int i = 0; i < 8; i++) unpack2(y[i], x[2 * i], x[2 * i + 1]);
+                if (j >= first_masked) {                       // causal mask (MHA.h:262-267)
+#pragma unroll
+                    for (int i = 0; i < 16; i++) x[i] = (kc + i <= qlim) ? x[i] : -1e32f;
                 }
-                tmem_ld_wait();
-                if (sweep == 0) {
-                    // the row maximum is tracked WITHOUT the factor 0.125 (scaling by a power of two is exact and keeps
-                    // the order, so max(x * 0.125) == max(x) * 0.125: applied once after the sweep)
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
-                        float x = ((float)(int)v[i] * qscale) * ksv[i];
-                        x = (kc + i <= qlim) ? x : -1e32f;                       // causal mask (MHA.h:262-267)
-                        mx = x > mx ? x : mx;
+                for (int i = 0; i < 16; i += 2) mx = max3(mx, x[i], x[i + 1]);
+            }
+        }
+        mx = mx * 0.125f;
+        const f32x2 mx2 = pack2(mx, mx), neg8th = pack2(-0.125f, -0.125f);
+
+        // ---- sweep 1: e = exp(-u) with u = max - x, and the four ordered chains (key mod 4 == i mod 4, because a chunk starts at
+        // a multiple of 16; adding the exact zeros of masked keys leaves the sums unchanged, as in the reference). max - x is
+        // one fused step: x = y / 8 is exact, so a single rounding is left, the subtraction's.
+        f32x2 s01 = pack2(0.f, 0.f), s23 = s01;
+        const ExpTable tab = exp_table_lane();
+        for (int j = 0; ok && j < n_kt; j++) {
+            if (!scores_ready(n_kt + j)) { ok = false; break; }
+            const float* kst = paged ? args.ks + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : ksp + j * ATT_KT;
+            const bool masked = j >= first_masked;
+#pragma unroll 1
+            for (int c = 0; c < ATT_KT / 16; c++) {
+                const int kc = j * ATT_KT + c * 16;
+                float u[16], e[16];
+                {
+                    f32x2 y[8];
+                    scores16(kst, kc, c, y);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) unpack2(fma2(y[i], neg8th, mx2), u[2 * i], u[2 * i + 1]);
+                }
+                if (masked) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) u[i] = (kc + i <= qlim) ? u[i] : 0.0f;
+                }
+                float far = u[0];                              // NaN when one of them is
+#pragma unroll
+                for (int i = 1; i < 15; i += 2) far = max3_nan(far, u[i], u[i + 1]);
+                far = max3_nan(far, far, u[15]);
+                if (__all_sync(0xffffffffu, far <= kExpFastLimit)) {
+#pragma unroll
+                    for (int i0 = 0; i0 < 16; i0 += ATT_EXP_GROUP) {
+                        float uu[ATT_EXP_GROUP], ee[ATT_EXP_GROUP];
+#pragma unroll
+                        for (int i = 0; i < ATT_EXP_GROUP; i++) uu[i] = u[i0 + i];
+                        exp_neg_warp(uu, ee, tab);
+#pragma unroll
+                        for (int i = 0; i < ATT_EXP_GROUP; i++) e[i0 + i] = ee[i];
                     }
-                } else {
-                    float e[16];
+                } else {                                       // a key far below the maximum (or NaN): the general form
 #pragma unroll
-                    for (int i4 = 0; i4 < 16; i4 += 4) {          // four exponentials at a time (their chains interleave)
-                        float xx[4], ee[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const float x = (((float)(int)v[i4 + i] * qscale) * ksv[i4 + i]) * 0.125f;
-                            xx[i] = (kc + i4 + i <= qlim) ? x - mx : -1e32f;    // masked: exp(-1e32) is exactly 0
-                        }
+                    for (int i4 = 0; i4 < 16; i4 += 4) {
+                        const float xx[4] = {-u[i4], -u[i4 + 1], -u[i4 + 2], -u[i4 + 3]};
+                        float ee[4];
                         ref_expf_x4<true>(xx, ee);
 #pragma unroll
                         for (int i = 0; i < 4; i++) e[i4 + i] = ee[i];
                     }
-                    // ordered chains: key mod 4 == i mod 4 because kc is a multiple of 16; adding the
-                    // exact zeros of masked keys leaves the sums unchanged, as in the reference
-#pragma unroll
-                    for (int i = 0; i < 16; i += 4) { ps0 += e[i]; ps1 += e[i + 1]; ps2 += e[i + 2]; ps3 += e[i + 3]; }
-                    float4* dst = ecache + ((size_t)(j * 16 + c * 4) * 128 + row_in_tile);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) dst[(size_t)i * 128] = make_float4(e[4 * i], e[4 * i + 1], e[4 * i + 2], e[4 * i + 3]);
                 }
+                if (masked) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) e[i] = (kc + i <= qlim) ? e[i] : 0.0f;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) { s01 = add2(s01, pack2(e[i], e[i + 1])); s23 = add2(s23, pack2(e[i + 2], e[i + 3])); }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_sempty);
-            if (it == n_kt - 1) mx = mx * 0.125f;             // end of sweep 0: the maximum of the scaled scores
         }
-        // ---- sweep 2: U = min(round((e * r * vs) / a_s), 255) from the cached e, into shared memory
+        float ps0, ps1, ps2, ps3;
+        unpack2(s01, ps0, ps1); unpack2(s23, ps2, ps3);
         const float rinv = 1.0f / ((ps0 + ps1) + (ps2 + ps3));
+
+        // ---- sweep 2: U = min(round((e * r * vs) / a_s), 255) into shared memory.
+        // t = e * r * vs / (255.25 a_s) comes from ex2.approx: 2^(c - u log2 e) * vs with c = log2(r / (255.25 a_s)). For u <= 64,
+        // -64 <= c <= 32 and 0 <= vs <= 2^40 its relative distance from the reference's quotient is below 5e-6: roundings of
+        // the argument and its terms (2^-25 to 2^-24 of magnitudes up to 32, 64 and 92), 2^-22 of ex2.approx, and the
+        // reference's own four roundings. (For larger u the quotient is below 2^-11 and the error
+        // cannot lift it to a half.) So where 255.25 t (1 + 2^-16) and 255.25 t (1 - 2^-16) round to the same integer, that is U;
+        // the saturating product holds t at 1, that is U at 255. Otherwise the reference's arithmetic decides, as it does for
+        // scales outside these ranges.
+        const float inv_as = 1.0f / a_s;
+        const float c_row = log2f((rinv * inv_as) * (1.0f / 255.25f));
+        const bool warp_ok = __all_sync(0xffffffffu, c_row >= -64.0f && c_row <= 32.0f);
+        const f32x2 c2 = pack2(c_row, c_row), nlog2e = pack2(-1.4426950408889634f, -1.4426950408889634f);
+        const f32x2 hi2 = pack2(255.25f * (1.0f + 0x1p-16f), 255.25f * (1.0f + 0x1p-16f));
+        const f32x2 lo2 = pack2(255.25f * (1.0f - 0x1p-16f), 255.25f * (1.0f - 0x1p-16f));
+        const f32x2 magic2 = pack2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: adding it rounds to an integer, kept in the low bits
         for (int j = 0; ok && j < n_kt; j++) {
             const int pb = j & 1;
-            // fetch the first half of this tile's e values before waiting for the buffer
-            float4 ev[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) ev[i] = ecache[((size_t)(j * 16 + i) * 128 + row_in_tile)];
+            const int k0 = j * ATT_KT;
+            const float* kst = paged ? args.ks + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : ksp + k0;
+            const float* vst = paged ? args.vs + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : vsp + k0;   // this tile's value scales
+            const float va = (k0 + lane < S) ? vst[lane] : 0.0f, vb = (k0 + 32 + lane < S) ? vst[32 + lane] : 0.0f;
+            const bool fast = __all_sync(0xffffffffu, va >= 0.0f && va <= 0x1p40f && vb >= 0.0f && vb <= 0x1p40f) && warp_ok;
+            const bool masked = j >= first_masked;
             int got = (lane == 0) ? (mbar_wait(bar_pempty + 8 * pb, (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag) ? 1 : 0) : 1;
             got = __shfl_sync(0xffffffffu, got, 0);
             if (!got) { ok = false; break; }
-            const int k0 = j * ATT_KT;
-            const float* vst = paged ? args.vs + ((long)__ldg(pt + j) * args.HKV + hkv) * 64 : vsp + k0;   // this tile's value scales
+            if (!scores_ready(2 * n_kt + j)) { ok = false; break; }
             uint8_t* prow = sP_ptr + pb * ATT_P_BYTES + row_in_tile * 64;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {          // 16 keys = one 16-byte chunk of the U row
-                if (c == 2) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) ev[i] = ecache[((size_t)(j * 16 + 8 + i) * 128 + row_in_tile)];
-                }
+#pragma unroll 1
+            for (int c = 0; c < ATT_KT / 16; c++) {            // 16 keys = one 16-byte chunk of the U row
+                const int kc = k0 + c * 16;
+                f32x2 y[8];
+                scores16(kst, kc, c, y);
                 uint32_t packed[4];
 #pragma unroll
                 for (int i4 = 0; i4 < 4; i4++) {
-                    const int kk = k0 + c * 16 + i4 * 4;
-                    const float4 vs4 = (kk < S) ? *reinterpret_cast<const float4*>(vst + c * 16 + i4 * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float4 e4 = ev[(c & 1) * 4 + i4];
-                    const float ee[4] = {e4.x, e4.y, e4.z, e4.w};
+                    const float4 vs4 = (kc + 4 * i4 < S) ? *reinterpret_cast<const float4*>(vst + c * 16 + 4 * i4) : make_float4(0.f, 0.f, 0.f, 0.f);
                     const float vv[4] = {vs4.x, vs4.y, vs4.z, vs4.w};
-                    uint32_t w = 0;
+                    const f32x2 ua = fma2(y[2 * i4], neg8th, mx2), ub = fma2(y[2 * i4 + 1], neg8th, mx2);
+                    float arg[4], t[4];
+                    unpack2(fma2(ua, nlog2e, c2), arg[0], arg[1]);
+                    unpack2(fma2(ub, nlog2e, c2), arg[2], arg[3]);
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const float p = ee[i] * rinv;
-                        int r = round_half_away_to_int(div_for_rounding(p * vv[i], d_as));
-                        r = r > 255 ? 255 : r;
-                        w |= ((uint32_t)r & 0xffu) << (8 * i);
+                    for (int i = 0; i < 4; i++) t[i] = __saturatef(ex2_approx(arg[i]) * vv[i]);
+                    const f32x2 ta = pack2(t[0], t[1]), tb = pack2(t[2], t[3]);
+                    float h[4], l[4];
+                    unpack2(fma2(ta, hi2, magic2), h[0], h[1]); unpack2(fma2(tb, hi2, magic2), h[2], h[3]);
+                    unpack2(fma2(ta, lo2, magic2), l[0], l[1]); unpack2(fma2(tb, lo2, magic2), l[2], l[3]);
+                    uint32_t r[4], open = fast ? 0u : 1u;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { r[i] = __float_as_uint(h[i]); open |= r[i] ^ __float_as_uint(l[i]); }
+                    if (open) {
+                        float uu[4];
+                        unpack2(ua, uu[0], uu[1]); unpack2(ub, uu[2], uu[3]);
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            if (!fast || r[i] != __float_as_uint(l[i])) r[i] = attn_u8_exact(uu[i], rinv, vv[i], a_s);
                     }
-                    packed[i4] = w;
+                    if (masked) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) r[i] = (kc + 4 * i4 + i <= qlim) ? r[i] : 0u;
+                    }
+                    packed[i4] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
                 }
                 // 64-byte rows with 64-byte swizzle: chunk index XOR ((row >> 1) & 3)
                 const int chunk = c ^ ((row_in_tile >> 1) & 3);
@@ -428,11 +530,6 @@ constexpr int ATO_TMEM_COLS = 256;
 constexpr int ATO_SLOTS = 6;
 constexpr int ATO_SMEM = ATT_Q_BYTES + ATO_SLOTS * ATT_TILE_BYTES + 2 * ATT_P_BYTES + 1024 + 256;
 
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float lg2_approx(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -804,14 +901,12 @@ static size_t align_up_(size_t x, size_t a) { return (x + a - 1) / a * a; }
 struct PrefillWs {
     int8_t *q2, *k2, *vT, *v2;
     float *qs2, *ks2, *vsT, *vs2;
-    uint8_t* ecache;
     static size_t bytes(int B, int S, int HQ, int HKV) {
         size_t n = 0;
         n += align_up_((size_t)B * HQ * S * 64, 1024);
         n += 3 * align_up_((size_t)B * HKV * S * 64, 1024);
         n += align_up_((size_t)B * HQ * S * 4, 1024);
         n += 3 * align_up_((size_t)B * HKV * S * 4, 1024);
-        n += align_up_((size_t)B * HQ * attn_ecache_head_bytes(0, S), 1024);
         return n + 1024;
     }
     PrefillWs(void* ws, int B, int S, int HQ, int HKV) {
@@ -823,26 +918,23 @@ struct PrefillWs {
         qs2 = (float*)w; w += align_up_((size_t)B * HQ * S * 4, 1024);
         ks2 = (float*)w; w += align_up_((size_t)B * HKV * S * 4, 1024);
         vsT = (float*)w; w += align_up_((size_t)B * HKV * S * 4, 1024);
-        vs2 = (float*)w; w += align_up_((size_t)B * HKV * S * 4, 1024);
-        ecache = w;
+        vs2 = (float*)w;
     }
 };
 
-// Workspace of the model path (K and V live in the KV cache): head-major Q, token-major V scratch, exp cache.
+// Workspace of the model path (K and V live in the KV cache): head-major Q, token-major V scratch.
 struct PagedWs {
-    int8_t *q2, *v2; float *qs2, *vs2; uint8_t* ecache;
-    static size_t bytes(int B, int Sq_max, int HQ, int HKV, size_t ecache_head_bytes) {
+    int8_t *q2, *v2; float *qs2, *vs2;
+    static size_t bytes(int B, int Sq_max, int HQ, int HKV) {
         return align_up_((size_t)B * HQ * Sq_max * 64, 1024) + align_up_((size_t)B * HKV * Sq_max * 64, 1024) +
-               align_up_((size_t)B * HQ * Sq_max * 4, 1024) + align_up_((size_t)B * HKV * Sq_max * 4, 1024) +
-               align_up_((size_t)B * HQ * ecache_head_bytes, 1024) + 1024;
+               align_up_((size_t)B * HQ * Sq_max * 4, 1024) + align_up_((size_t)B * HKV * Sq_max * 4, 1024) + 1024;
     }
     PagedWs(void* ws, int B, int Sq_max, int HQ, int HKV) {
         uint8_t* w = (uint8_t*)align_up_((size_t)ws, 1024);
         q2 = (int8_t*)w; w += align_up_((size_t)B * HQ * Sq_max * 64, 1024);
         v2 = (int8_t*)w; w += align_up_((size_t)B * HKV * Sq_max * 64, 1024);
         qs2 = (float*)w; w += align_up_((size_t)B * HQ * Sq_max * 4, 1024);
-        vs2 = (float*)w; w += align_up_((size_t)B * HKV * Sq_max * 4, 1024);
-        ecache = w;
+        vs2 = (float*)w;
     }
 };
 
@@ -880,20 +972,8 @@ static int mha_prefill_core(AttnArgs a, const int8_t* q2, const int8_t* kmat, ui
     return launch_status();
 }
 
-// Exp-cache bytes per (batch, query head) that a model with these limits can need: prompts are processed in chunks of
-// max_prefill tokens starting at multiples of it.
-static size_t paged_ecache_head_bytes(int max_prefill, int max_ctx) {
-    size_t worst = 0;
-    for (long c0 = 0; c0 < max_ctx; c0 += max_prefill) {
-        const int sc = (int)(max_ctx - c0 < max_prefill ? max_ctx - c0 : max_prefill);
-        const size_t n = attn_ecache_head_bytes((int)c0, sc);
-        if (n > worst) worst = n;
-    }
-    return worst;
-}
-
 size_t mha_prefill_ws_bytes(int B, int max_prefill, int max_ctx, int HQ, int HKV) {
-    return PagedWs::bytes(B, max_prefill, HQ, HKV, paged_ecache_head_bytes(max_prefill, max_ctx));
+    return PagedWs::bytes(B, max_prefill, HQ, HKV);
 }
 
 // Model path: attention of the Sq tokens at positions q_off .. q_off + Sq - 1 of every sequence, from the fp32 output of
@@ -916,7 +996,7 @@ int mha_prefill_paged(const float* qkv, const float* cos_t, const float* sin_t, 
     AttnArgs a;
     a.B = B; a.HQ = HQ; a.HKV = HKV; a.Sq = Sq; a.q_off = q_off; a.Sk = 0;
     a.qs = ws.qs2; a.ks = ks_pool; a.vs = vs_pool; a.page_table = page_table; a.max_pages = max_pages;
-    a.a_s = a_s; a.out = out; a.oacc = nullptr; a.ecache = ws.ecache;
+    a.a_s = a_s; a.out = out; a.oacc = nullptr;
     const uint64_t rows = (uint64_t)c->n_pages * HKV * 64;
     // FLEXLLM_ATTN_ONLINE=1: the single-sweep variant (not bit-exact) in the model's prefill, for measuring what exactness costs
     static const bool online = [] { const char* e = getenv("FLEXLLM_ATTN_ONLINE"); return e && e[0] == '1'; }();
@@ -954,7 +1034,7 @@ static int mha_prefill_contiguous(bool online, const int8_t* q, const float* qs,
     AttnArgs a;
     a.B = B; a.HQ = HQ; a.HKV = HKV; a.Sq = S; a.q_off = 0; a.Sk = S;
     a.qs = ws.qs2; a.ks = ws.ks2; a.vs = ws.vsT; a.page_table = nullptr; a.max_pages = 0;
-    a.a_s = a_s; a.out = out; a.oacc = oacc; a.ecache = ws.ecache;
+    a.a_s = a_s; a.out = out; a.oacc = oacc;
     return mha_prefill_core(a, ws.q2, ws.k2, (uint64_t)B * HKV * S, ws.vT, (uint64_t)B * HKV * 64, (uint64_t)S, st, online);
 }
 

@@ -213,6 +213,41 @@ template <int N> __device__ __forceinline__ void div_rn_array(float (&r)[N], con
     }
 }
 
+// ---- pairs of floats in one 64-bit register: one instruction works on both (each rounded as its scalar form) ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// largest of three; max3 ignores NaN operands, max3_nan returns NaN if there is one
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // exp() used by SiLU and softmax. The reference calls the C library's expf, whose last-bit
 // rounding the C standard leaves open. This build evaluates the CORRECTLY ROUNDED single-precision
 // exponential, which (float)exp((double)x) reproduces bit for bit on any host with an accurate
@@ -294,6 +329,52 @@ __device__ __forceinline__ void ref_expf_x4(const float (&x)[4], float (&e)[4]) 
 #pragma unroll
         for (int i = 0; i < 4; i++)
             if (hard & (1u << i)) e[i] = ref_expf_accurate(x[i]);
+    }
+}
+
+// ---- the same function for u in [0, kExpFastLimit], e = exp(-u): the softmax inner loop -----------------------------------
+// What limits it is issue slots and the half-rate double-precision pipe, so it does with eight double-precision
+// instructions: ln2/32 as ONE constant (its representation error costs 2^-47 at u = 87), and a degree-4 polynomial, the
+// Taylor series to degree 5 economised by the Chebyshev polynomial T5 on |r| <= ln2/64 (Lanczos): the dropped term is at
+// most a^5 / (16 * 120) = 2^-43.5. The result is within 2^-43.2 of exp(-u), under 900 units of the double's last place; where
+// the 29 bits that rounding to float cuts off come within 1024 of the half (one input in 2^18), the accurate form decides. Below
+// the limit the result is a normal number, so the cut is at a fixed bit.
+// The table of 2^(j/32) lives in the warp's registers, lane j holding entry j (a shuffle instead of a load that random
+// indices make conflict). u becomes a double by integer shifts: conversions to and from double share one pipe
+// of 16 lanes a clock, and the conversion of the result keeps it half busy already.
+// Checked against the accurate form for every float in [0, 87): no difference where the test lets the fast result stand.
+// Cycles per 32 values and scheduler, 16 warps an SM: 52 in the four-wide form above, 32 here by fours, 29 by eights.
+constexpr float kExpFastLimit = 87.0f;
+
+struct ExpTable { int hi, lo; };
+__device__ __forceinline__ ExpTable exp_table_lane() {
+    const double t = g_exp2_table[threadIdx.x & 31];
+    return {__double2hiint(t), __double2loint(t)};
+}
+// Called by all 32 lanes of a warp together, every value in [0, kExpFastLimit].
+template <int NV> __device__ __forceinline__ void exp_neg_warp(const float (&u)[NV], float (&e)[NV], const ExpTable& tab) {
+    constexpr double a2 = (0x1.62e42fefa39efp-7 * 0x1.62e42fefa39efp-7);              // (ln2/64)^2
+    unsigned nearest = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const unsigned bits = __float_as_uint(u[i]);
+        const double ud = __hiloint2double((int)((bits >> 3) + 0x38000000u), (int)(bits << 29));   // 0 becomes 2^-127: exp is 1 all the same
+        const double shift = 0x1.8p52;
+        const double t = __fma_rn(ud, -FLEXLLM_EXP_INV_LN2_32, shift);
+        const int k = __double2loint(t);
+        const double r = __fma_rn(t - shift, -0x1.62e42fefa39efp-6, -ud);
+        double p = __fma_rn(r, 1.0 / 24.0, 1.0 / 6.0 + a2 / 96.0);
+        p = __fma_rn(p, r, 0.5);
+        p = __fma_rn(p, r, 1.0 - a2 * a2 / 384.0);
+        p = __fma_rn(p, r, 1.0);
+        const double res = __hiloint2double(__shfl_sync(0xffffffffu, tab.hi, k), __shfl_sync(0xffffffffu, tab.lo, k)) * p;   // lane = k mod 32
+        const unsigned lo = (unsigned)__double2loint(res);
+        nearest = min(nearest, lo * 8u + (0x80000000u + 1024u * 8u));                // distance from the half, offset by 1024, in the top 29 bits
+        e[i] = __double2float_rn(__hiloint2double(__double2hiint(res) + ((k & ~31) << 15), (int)lo));
+    }
+    if (nearest < 2048u * 8u) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) e[i] = ref_expf_accurate(-u[i]);
     }
 }
 

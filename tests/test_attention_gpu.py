@@ -72,6 +72,38 @@ def test_prefill_config3_slice(F):
     check_prefill(F, 1, 1024, 32, 8, 31)
 
 
+@pytest.mark.parametrize("what", ["peaked", "spread", "large", "saturated", "ties", "wide_scales", "tiny_scales", "zero_scales"])
+def test_prefill_quantiser_ranges(F, what):
+    """The probabilities' quantiser decides most values from the hardware exponential and an error bound, the rest as the reference
+    does; exponentials have a short form up to 87 below the maximum. Inputs on both sides of every such line, bit for bit."""
+    B, S, HQ, HKV = 1, 208, 8, 2                       # the last key tile and the last query tile are partly empty
+    q, qs, k, ks, v, vs, a_s = attn_inputs(B, S, HQ, HKV, 77)
+    if what == "peaked": qs *= 20                      # differences of scores up to thousands
+    if what == "spread": qs *= 3                       # ... on both sides of 87 and of 104
+    if what == "large": a_s[:] = 2e-6                  # U all over 0..255
+    if what == "saturated": a_s[:] = 1e-8              # most of U at 255
+    if what == "ties":                                 # equal scores: e = 1, P = 1/n; for n = 2^j quotients are k + 1/2 exactly
+        q[:] = 0
+        vs[:] = 2.0 ** g_exponents(vs.shape)
+        a_s[:] = 2.0 ** -13
+    if what == "wide_scales":                          # outside the bound's range: the reference's arithmetic throughout
+        vs *= 2.0 ** 46
+        a_s *= 2.0 ** 38
+    if what == "tiny_scales":
+        vs *= 2.0 ** -60
+    if what == "zero_scales":
+        vs[:, ::3] = 0
+    cos_t, sin_t = oracle.rope_table(S)
+    out, oacc = F.MHA_i8xi8_Prefilling(dev(q), dev(qs), dev(k), dev(ks), dev(v), dev(vs), dev(cos_t), dev(sin_t), dev(a_s), want_oacc=True)
+    ref = oracle.mha_prefill(q, qs, k, ks, v, vs, cos_t, sin_t, a_s)
+    assert_same(to_np(oacc), ref["oacc"], "int32 P.V accumulators")
+    assert_same(to_np(out), ref["out"], "fp32 output")
+
+
+def g_exponents(shape):
+    return np.random.default_rng(78).integers(-9, -3, shape).astype(np.float32)
+
+
 def test_prefill_rows_sum_property(F):
     """Size-independent property at the full config-3 size (B=4): with V == 1 and vs == a_s * 255
     every output equals sum_k U[q][k] * a_s and U rows sum to about 255 (P sums to 1)."""
