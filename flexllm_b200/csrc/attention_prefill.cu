@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
                         float uu[ATT_EXP_GROUP], ee[ATT_EXP_GROUP];
 #pragma unroll
                         for (int i = 0; i < ATT_EXP_GROUP; i++) uu[i] = u[i0 + i];
-                        exp_neg_warp(uu, ee, tab);
+                        exp_warp<true>(uu, ee, tab);
 #pragma unroll
                         for (int i = 0; i < ATT_EXP_GROUP; i++) e[i0 + i] = ee[i];
                     }

@@ -248,6 +248,33 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
     return r;
 }
 
+// ---- quantiser without divisions ----
+__device__ __noinline__ static uint32_t q8_exact(float x, float s) { return (uint32_t)round_half_away_to_int(x / s) & 0xffu; }
+// The int8 values (low byte of q[i]) of x / s, where w is 1 / s and the reference divides with up to two roundings: x w is within
+// 2^-21.9 of its quotient (four roundings at most), so where x w (1 + 2^-20) and x w (1 - 2^-20) round to the same integer, that is
+// the result; otherwise (a few values in 10^5) exact(x) decides, as it does for rows of which the caller knows that a value is
+// NaN or that a step could under- or overflow (ok false). |x w| <= 128.
+template <int NV, class Exact> __device__ __forceinline__ void q8_short(const float (&x)[NV], float w, bool ok, uint32_t (&q)[NV], Exact exact) {
+    const f32x2 whi = pack2(w * (1.0f + 0x1p-20f), w * (1.0f + 0x1p-20f)), wlo = pack2(w * (1.0f - 0x1p-20f), w * (1.0f - 0x1p-20f));
+    const f32x2 magic = pack2(12582912.0f, 12582912.0f);       // 1.5 * 2^23: adding it rounds to an integer, kept in the low bits
+    uint32_t open = ok ? 0u : 1u, l[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i += 2) {
+        float h0, h1, l0, l1;
+        const f32x2 v = pack2(x[i], x[i + 1]);
+        unpack2(fma2(v, whi, magic), h0, h1);
+        unpack2(fma2(v, wlo, magic), l0, l1);
+        q[i] = __float_as_uint(h0); q[i + 1] = __float_as_uint(h1);
+        l[i] = __float_as_uint(l0); l[i + 1] = __float_as_uint(l1);
+        open |= (q[i] ^ l[i]) | (q[i + 1] ^ l[i + 1]);
+    }
+    if (open) {
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+            if (!ok || q[i] != l[i]) q[i] = exact(x[i]);
+    }
+}
+
 // exp() used by SiLU and softmax. The reference calls the C library's expf, whose last-bit
 // rounding the C standard leaves open. This build evaluates the CORRECTLY ROUNDED single-precision
 // exponential, which (float)exp((double)x) reproduces bit for bit on any host with an accurate
@@ -332,17 +359,17 @@ __device__ __forceinline__ void ref_expf_x4(const float (&x)[4], float (&e)[4]) 
     }
 }
 
-// ---- the same function for u in [0, kExpFastLimit], e = exp(-u): the softmax inner loop -----------------------------------
+// ---- the same function for |x| <= kExpFastLimit, called by whole warps: softmax and SiLU inner loops ---------------------
 // What limits it is issue slots and the half-rate double-precision pipe, so it does with eight double-precision
-// instructions: ln2/32 as ONE constant (its representation error costs 2^-47 at u = 87), and a degree-4 polynomial, the
+// instructions: ln2/32 as ONE constant (its representation error costs 2^-47 at |x| = 87), and a degree-4 polynomial, the
 // Taylor series to degree 5 economised by the Chebyshev polynomial T5 on |r| <= ln2/64 (Lanczos): the dropped term is at
-// most a^5 / (16 * 120) = 2^-43.5. The result is within 2^-43.2 of exp(-u), under 900 units of the double's last place; where
-// the 29 bits that rounding to float cuts off come within 1024 of the half (one input in 2^18), the accurate form decides. Below
+// most a^5 / (16 * 120) = 2^-43.5. The result is within 2^-43.2 of exp(x), under 900 units of the double's last place; where
+// the 29 bits that rounding to float cuts off come within 1024 of the half (one input in 2^18), the accurate form decides. Inside
 // the limit the result is a normal number, so the cut is at a fixed bit.
 // The table of 2^(j/32) lives in the warp's registers, lane j holding entry j (a shuffle instead of a load that random
-// indices make conflict). u becomes a double by integer shifts: conversions to and from double share one pipe
-// of 16 lanes a clock, and the conversion of the result keeps it half busy already.
-// Checked against the accurate form for every float in [0, 87): no difference where the test lets the fast result stand.
+// indices make conflict). Where the sign is known (NEG: exp(-u), u >= 0) the argument becomes a double by integer shifts:
+// conversions to and from double share one pipe of 16 lanes a clock, which the conversion of the result keeps half busy.
+// Checked against the accurate form for every float in the range: no difference where the test lets the fast result stand.
 // Cycles per 32 values and scheduler, 16 warps an SM: 52 in the four-wide form above, 32 here by fours, 29 by eights.
 constexpr float kExpFastLimit = 87.0f;
 
@@ -351,18 +378,23 @@ __device__ __forceinline__ ExpTable exp_table_lane() {
     const double t = g_exp2_table[threadIdx.x & 31];
     return {__double2hiint(t), __double2loint(t)};
 }
-// Called by all 32 lanes of a warp together, every value in [0, kExpFastLimit].
-template <int NV> __device__ __forceinline__ void exp_neg_warp(const float (&u)[NV], float (&e)[NV], const ExpTable& tab) {
-    constexpr double a2 = (0x1.62e42fefa39efp-7 * 0x1.62e42fefa39efp-7);              // (ln2/64)^2
+// Called by all 32 lanes of a warp together, every |x| <= kExpFastLimit. e[i] = exp(x[i]); with NEG exp(-x[i]), x[i] >= 0.
+template <bool NEG, int NV> __device__ __forceinline__ void exp_warp(const float (&x)[NV], float (&e)[NV], const ExpTable& tab) {
+    constexpr double a2 = 0x1.62e42fefa39efp-7 * 0x1.62e42fefa39efp-7;                // (ln2/64)^2
     unsigned nearest = 0xffffffffu;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        const unsigned bits = __float_as_uint(u[i]);
-        const double ud = __hiloint2double((int)((bits >> 3) + 0x38000000u), (int)(bits << 29));   // 0 becomes 2^-127: exp is 1 all the same
+        double xd;
+        if (NEG) {                                                                    // 0 becomes -2^-127: its exponential is 1 all the same
+            const unsigned bits = __float_as_uint(x[i]);
+            xd = -__hiloint2double((int)((bits >> 3) + 0x38000000u), (int)(bits << 29));
+        } else {
+            xd = (double)x[i];
+        }
         const double shift = 0x1.8p52;
-        const double t = __fma_rn(ud, -FLEXLLM_EXP_INV_LN2_32, shift);
+        const double t = __fma_rn(xd, FLEXLLM_EXP_INV_LN2_32, shift);
         const int k = __double2loint(t);
-        const double r = __fma_rn(t - shift, -0x1.62e42fefa39efp-6, -ud);
+        const double r = __fma_rn(t - shift, -0x1.62e42fefa39efp-6, xd);
         double p = __fma_rn(r, 1.0 / 24.0, 1.0 / 6.0 + a2 / 96.0);
         p = __fma_rn(p, r, 0.5);
         p = __fma_rn(p, r, 1.0 - a2 * a2 / 384.0);
@@ -374,11 +406,12 @@ template <int NV> __device__ __forceinline__ void exp_neg_warp(const float (&u)[
     }
     if (nearest < 2048u * 8u) {
 #pragma unroll
-        for (int i = 0; i < NV; i++) e[i] = ref_expf_accurate(-u[i]);
+        for (int i = 0; i < NV; i++) e[i] = ref_expf_accurate(NEG ? -x[i] : x[i]);
     }
 }
 
 __device__ __forceinline__ float silu_f(float g) { return g / (1.0f + ref_expf(-g)); }
+__device__ __noinline__ static float silu_mul_any(float g, float u) { return silu_f(g) * u; }
 // silu(g) * u on four values (same arithmetic per value)
 __device__ __forceinline__ float4 silu_mul_x4(const float4 g, const float4 u) {
     const float x[4] = {-g.x, -g.y, -g.z, -g.w};
@@ -388,6 +421,45 @@ __device__ __forceinline__ float4 silu_mul_x4(const float4 g, const float4 u) {
     o.x = (g.x / (1.0f + e[0])) * u.x; o.y = (g.y / (1.0f + e[1])) * u.y;
     o.z = (g.z / (1.0f + e[2])) * u.z; o.w = (g.w / (1.0f + e[3])) * u.w;
     return o;
+}
+
+// The same on eight values of every lane of a warp (whole-warp call): o = (g / (1 + exp(-g))) * u, each operation rounded once.
+// The quotient: y = 1 / D from rcp.approx and one Newton step, q = RN(g y), one exact residual r = g - q D, RN(q + r y). For
+// the pairs (g, 1 + exp(-g)) that occur here this is the correctly rounded quotient: compared with the division for every
+// float g with 2^-60 <= |g| <= 80. Other values (and NaN) send the warp to the division itself.
+__device__ __forceinline__ void silu_mul_warp8(const float (&g)[8], const float (&u)[8], float (&o)[8], const ExpTable& tab) {
+    float far = fabsf(g[0]), near = far;
+#pragma unroll
+    for (int i = 1; i < 7; i += 2) {
+        far = max3_nan(far, fabsf(g[i]), fabsf(g[i + 1]));
+        near = fminf(near, fminf(fabsf(g[i]), fabsf(g[i + 1])));
+    }
+    far = max3_nan(far, far, fabsf(g[7]));
+    near = fminf(near, fabsf(g[7]));
+    if (__all_sync(0xffffffffu, far <= 80.0f && near >= 0x1p-60f)) {
+        float x[8], e[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = -g[i];
+        exp_warp<false>(x, e, tab);
+        const f32x2 one = pack2(1.0f, 1.0f);
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const f32x2 d = add2(pack2(e[i], e[i + 1]), one), gg = pack2(g[i], g[i + 1]);
+            float d0, d1, y0, y1;
+            unpack2(d, d0, d1);
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(d0));
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(d1));
+            f32x2 y = pack2(y0, y1);
+            const f32x2 nd = pack2(-d0, -d1);
+            y = fma2(fma2(nd, y, one), y, y);
+            f32x2 q = mul2(gg, y);
+            q = fma2(fma2(nd, q, gg), y, q);
+            unpack2(mul2(q, pack2(u[i], u[i + 1])), o[i], o[i + 1]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++) o[i] = silu_mul_any(g[i], u[i]);
+    }
 }
 
 }  // namespace flexllm

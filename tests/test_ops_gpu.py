@@ -123,6 +123,25 @@ def test_rope(F):
     assert_same(to_np(y), oracle.rope(x, pos, cos_t, sin_t))
 
 
+@pytest.mark.parametrize("M", [1, 111, 112, 200])        # the cluster form's last row count and the first of the other
+@pytest.mark.parametrize("what", ["plain", "wide", "small", "special"])
+def test_swiglu_fht_quant_forms(F, M, what):
+    """Both forms of the kernel, bit for bit, also outside the ranges of the short exponential, division and quantiser."""
+    g_ = rng(500 + M)
+    g = (g_.standard_normal((M, 8192)) * 2).astype(np.float32); u = g_.standard_normal((M, 8192)).astype(np.float32)
+    if what == "wide": g *= 40                               # exponentials beyond the short form's range
+    if what == "small": u *= np.float32(2.0) ** -70          # rows whose scale lies below the quantiser's range
+    if what == "special":
+        g[0, ::7] = 0.0; g[0, 1::7] = -0.0; g[0, 2::7] = 1e-30
+        u[M // 2] = 0.0                                      # a row of zeros
+        g[M - 1, 5] = 87.5; g[M - 1, 6] = -104.5
+    q, s, act = F.swiglu_fht_quant(dev(g), dev(u), want_act=True)
+    act_o = oracle.silu_mul(g, u)
+    assert_same(to_np(act), act_o, "silu(g)*u")
+    qo, so = oracle.quant_per_token(oracle.fht(act_o, 90.50966799))
+    assert_same(to_np(s), so, "scale"); assert_same(to_np(q), qo, "q")
+
+
 @pytest.mark.parametrize("T,H", [(1, 8), (100, 32), (33, 1)])
 def test_qk_prepare(F, T, H):
     g = rng(7)
