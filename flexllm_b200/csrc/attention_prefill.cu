@@ -38,43 +38,87 @@ namespace flexllm {
 using namespace tc;
 
 // ------------------------------------------------------------------ pre-pass
-// Q/K: dequant -> RoPE -> FHT-64/8 -> per-head int8 quant (same arithmetic as qk_prepare_kernel),
-// written head-major [B][H][S][64] with scales [B][H][S] so that one head's rows are contiguous.
-__global__ void __launch_bounds__(256) attn_qk_prepare_kernel(const int8_t* __restrict__ q, const float* __restrict__ s,
-                                                              const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                              int B, int S, int H, int8_t* __restrict__ q_out,
-                                                              float* __restrict__ s_out) {
-    const long w = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long total = (long)B * S * H;
-    if (w >= total) return;
-    const int h = (int)(w % H);
-    const long bt = w / H;
-    const int t = (int)(bt % S);
-    const int b = (int)(bt / S);
-    const float sc_in = s[w];
-    const float x0 = (float)q[w * 64 + lane] * sc_in;
-    const float x1 = (float)q[w * 64 + 32 + lane] * sc_in;
-    const float c = cos_t[(long)t * 32 + lane], sn = sin_t[(long)t * 32 + lane];
-    float a = x0 * c - x1 * sn;
-    float bb = x0 * sn + x1 * c;
-    auto lane_stage = [&](int bit) {
-        float pa = __shfl_xor_sync(0xffffffffu, a, 1 << bit);
-        float pb = __shfl_xor_sync(0xffffffffu, bb, 1 << bit);
-        if (lane & (1 << bit)) { a = pa - a; bb = pb - bb; }
-        else { a = a + pa; bb = bb + pb; }
-    };
-    lane_stage(1); lane_stage(2); lane_stage(3); lane_stage(4);
-    { float lo = a, hi = bb; a = lo + hi; bb = lo - hi; }
-    lane_stage(0);
-    a = a / 8.0f;
-    bb = bb / 8.0f;
-    const float mx = warp_max(fmaxf(a, bb)), mn = warp_min(fminf(a, bb));
-    const float sc = sym_scale_from(mx, mn);
+// Eight lanes share one 64-wide head: lane l of the eight holds elements 4l..4l+3 (lo) and 32+4l..32+4l+3 (hi), so that a
+// rotation pair, and index bits 0, 1 and 5 of the transform, are one lane's own and bits 2, 3, 4 take one shuffle a value.
+// (A whole warp per head, two elements a lane, spent most of its instructions on shuffles and on the divisions of the
+// quantiser: 32768 tokens of 32 + 2 x 8 heads took 269 us, 4 x 1024 tokens of 32 + 8 heads 46 us.)
+// RoPE, then the 64-point transform in the reference's stage order (index bits 1, 2, 3, 4, 5, 0), / 8
+__device__ __forceinline__ void head8_rotate_fht(float (&x)[8], const float4 c, const float4 s, const int l8) {
+    const float cc[4] = {c.x, c.y, c.z, c.w}, ss[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float x0 = x[i], x1 = x[4 + i];
+        x[i] = x0 * cc[i] - x1 * ss[i];
+        x[4 + i] = x0 * ss[i] + x1 * cc[i];
+    }
+    auto pair = [&](int i, int j) { const float a = x[i], b = x[j]; x[i] = a + b; x[j] = a - b; };
+    pair(0, 2); pair(1, 3); pair(4, 6); pair(5, 7);                    // index bit 1
+#pragma unroll
+    for (int bit = 0; bit < 3; bit++) {                                // index bits 2, 3, 4
+        const bool up = l8 & (1 << bit);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float p = __shfl_xor_sync(0xffffffffu, x[i], 1 << bit);
+            x[i] = up ? p - x[i] : x[i] + p;
+        }
+    }
+    pair(0, 4); pair(1, 5); pair(2, 6); pair(3, 7);                    // index bit 5
+    pair(0, 1); pair(2, 3); pair(4, 5); pair(6, 7);                    // index bit 0
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i] = x[i] / 8.0f;
+}
+// symmetric int8 of the head: returns the scale, the lane's eight values as two groups of four bytes
+__device__ __forceinline__ float head8_quant(const float (&x)[8], uint32_t& lo, uint32_t& hi) {
+    float amax = fabsf(x[0]), nan = amax;
+#pragma unroll
+    for (int i = 1; i < 8; i++) { amax = fmaxf(amax, fabsf(x[i])); nan = max3_nan(nan, nan, x[i]); }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float sc = sym_scale_from(amax, -amax);
+    uint32_t q[8];
+    q8_short(x, 1.0f / sc, sc >= 0x1p-60f && sc <= 0x1p60f && nan == nan, q, [&](float v) { return q8_exact(v, sc); });
+    lo = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+    hi = __byte_perm(__byte_perm(q[4], q[5], 0x0040), __byte_perm(q[6], q[7], 0x0040), 0x5410);
+    return sc;
+}
+
+// Q and K of the stand-alone operator: dequant -> RoPE -> FHT-64/8 -> per-head int8 quant (same arithmetic as
+// qk_prepare_kernel), written head-major [B][H][S][64] with scales [B][H][S] so that one head's rows are contiguous.
+// VEC: q and k are 4-byte and the tables 16-byte aligned (else the same values are fetched one by one).
+template <bool VEC>
+__global__ void __launch_bounds__(256) attn_qk_prepare_kernel(const int8_t* __restrict__ q, const float* __restrict__ qs,
+                                                              const int8_t* __restrict__ k, const float* __restrict__ ks,
+                                                              const float* __restrict__ cos_t, const float* __restrict__ sin_t, int B, int S,
+                                                              int HQ, int HKV, int8_t* __restrict__ q_out, float* __restrict__ qs_out,
+                                                              int8_t* __restrict__ k_out, float* __restrict__ ks_out) {
+    const long total = (long)B * S * (HQ + HKV);
+    long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int l8 = threadIdx.x & 7;
+    const bool live = w < total;
+    if (!live) w = total - 1;                                          // the shuffles below take whole warps
+    const long nq = (long)B * S * HQ;
+    const bool is_q = w < nq;
+    const long i = is_q ? w : w - nq;
+    const int H = is_q ? HQ : HKV;
+    const int h = (int)(i % H);
+    const long bt = i / H;
+    const int t = (int)(bt % S), b = (int)(bt / S);
+    const float sc_in = (is_q ? qs : ks)[i];
+    const int8_t* src = (is_q ? q : k) + i * 64;
+    auto four = [&](const int8_t* p) { return VEC ? *reinterpret_cast<const char4*>(p) : make_char4(p[0], p[1], p[2], p[3]); };
+    auto table = [&](const float* p) { return VEC ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]); };
+    const char4 a = four(src + 4 * l8), c = four(src + 32 + 4 * l8);
+    float x[8] = {(float)a.x * sc_in, (float)a.y * sc_in, (float)a.z * sc_in, (float)a.w * sc_in,
+                  (float)c.x * sc_in, (float)c.y * sc_in, (float)c.z * sc_in, (float)c.w * sc_in};
+    head8_rotate_fht(x, table(cos_t + (long)t * 32 + 4 * l8), table(sin_t + (long)t * 32 + 4 * l8), l8);
+    uint32_t lo, hi;
+    const float sc = head8_quant(x, lo, hi);
+    if (!live) return;
     const long o = ((long)b * H + h) * S + t;
-    if (lane == 0) s_out[o] = sc;
-    q_out[o * 64 + lane] = quant_s8(a, sc);
-    q_out[o * 64 + 32 + lane] = quant_s8(bb, sc);
+    if (l8 == 0) (is_q ? qs_out : ks_out)[o] = sc;
+    uint32_t* dst = reinterpret_cast<uint32_t*>((is_q ? q_out : k_out) + o * 64);
+    dst[l8] = lo;
+    dst[8 + l8] = hi;
 }
 
 // V [B][S][HKV][64] -> V^T [B][HKV][64][S] (keys contiguous, the K-major operand of P.V) and
@@ -821,56 +865,39 @@ __global__ void __launch_bounds__(256) attn_qkv_prepare_f32_kernel(const float* 
                                                                    int8_t* __restrict__ k_pool, float* __restrict__ ks_pool,
                                                                    const int32_t* __restrict__ page_table, int max_pages,
                                                                    int8_t* __restrict__ v2, float* __restrict__ vs2) {
-    // one CTA per token, its eight warps share the token's heads: the token's indices, rotation factors and cache row
-    // are worked out once, not per head
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads = HQ + 2 * HKV;
-    const long bt = blockIdx.x;
-    const int t = (int)(bt % Sq);
-    const int b = (int)(bt / Sq);
+    const long total = (long)B * Sq * heads;
+    long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int l8 = threadIdx.x & 7;
+    const bool live = w < total;
+    if (!live) w = total - 1;                                          // the shuffles below take whole warps
+    const long bt = w / heads;
+    const int h = (int)(w - bt * heads);
+    const int b = (int)(bt / Sq), t = (int)(bt - (long)b * Sq);
     const int pos = q_off + t;
-    const float c = cos_t[(long)pos * 32 + lane], sn = sin_t[(long)pos * 32 + lane];
-    const long krow = (long)page_table[(long)b * max_pages + pos / 64] * HKV * 64 + (pos & 63);
-    for (int h = warp; h < heads; h += 8) {
-        const float* src = qkv + bt * (long)heads * 64 + (long)h * 64;
-        const float x0 = src[lane], x1 = src[lane + 32];
-        float a, bb;
-        if (h < HQ + HKV) {
-            a = x0 * c - x1 * sn;
-            bb = x0 * sn + x1 * c;
-            auto lane_stage = [&](int bit) {
-                float pa = __shfl_xor_sync(0xffffffffu, a, 1 << bit);
-                float pb = __shfl_xor_sync(0xffffffffu, bb, 1 << bit);
-                if (lane & (1 << bit)) { a = pa - a; bb = pb - bb; }
-                else { a = a + pa; bb = bb + pb; }
-            };
-            lane_stage(1); lane_stage(2); lane_stage(3); lane_stage(4);
-            { float lo = a, hi = bb; a = lo + hi; bb = lo - hi; }
-            lane_stage(0);
-            a = a / 8.0f;
-            bb = bb / 8.0f;
-        } else {
-            a = x0; bb = x1;
-        }
-        // scale = max(|max|, |min|) / 127 = the largest magnitude / 127; one reciprocal per head, then every value is
-        // divided by the short exact sequence and rounded half away from zero (|quotient| <= 127)
-        const float amax = warp_max(fmaxf(fabsf(a), fabsf(bb)));
-        float sc = amax / 127.0f;
-        if (sc == 0.0f) sc = 1.0f;
-        const DivBy dsc = div_by(sc);
-        auto q8 = [&](float v) {
-            const float qt = div_for_rounding(v, dsc);
-            const int m = __float2int_rz(__fadd_rd(fabsf(qt), 0.5f));
-            return (int8_t)(qt < 0.0f ? -m : m);
-        };
-        int8_t* dst; float* sdst;
-        if (h < HQ) { const long o = ((long)b * HQ + h) * Sq + t; dst = q2 + o * 64; sdst = qs2 + o; }
-        else if (h < HQ + HKV) { const long row = krow + (long)(h - HQ) * 64; dst = k_pool + row * 64; sdst = ks_pool + row; }
-        else { const long o = bt * HKV + (h - HQ - HKV); dst = v2 + o * 64; sdst = vs2 + o; }
-        if (lane == 0) *sdst = sc;
-        dst[lane] = q8(a);
-        dst[lane + 32] = q8(bb);
+    const float4* src = reinterpret_cast<const float4*>(qkv + w * 64);
+    const float4 a = src[l8], c = src[8 + l8];
+    const float raw[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) x[i] = raw[i];
+    head8_rotate_fht(x, reinterpret_cast<const float4*>(cos_t + (long)pos * 32)[l8], reinterpret_cast<const float4*>(sin_t + (long)pos * 32)[l8], l8);
+    if (h >= HQ + HKV) {                                               // value heads are quantised as they are
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = raw[i];
     }
+    uint32_t lo, hi;
+    const float sc = head8_quant(x, lo, hi);
+    if (!live) return;
+    int8_t* dst; float* sdst;
+    if (h < HQ) { const long o = ((long)b * HQ + h) * Sq + t; dst = q2 + o * 64; sdst = qs2 + o; }
+    else if (h < HQ + HKV) {
+        const long row = (long)page_table[(long)b * max_pages + pos / 64] * HKV * 64 + (pos & 63) + (long)(h - HQ) * 64;
+        dst = k_pool + row * 64; sdst = ks_pool + row;
+    } else { const long o = bt * HKV + (h - HQ - HKV); dst = v2 + o * 64; sdst = vs2 + o; }
+    if (l8 == 0) *sdst = sc;
+    reinterpret_cast<uint32_t*>(dst)[l8] = lo;
+    reinterpret_cast<uint32_t*>(dst)[8 + l8] = hi;
 }
 
 // V [B][Sq][HKV][64] (token-major scratch) -> the cache's V^T pages [page][HKV][64 dims][64 tokens] and scale pages,
@@ -987,7 +1014,7 @@ int mha_prefill_paged(const float* qkv, const float* cos_t, const float* sin_t, 
     PagedWs ws(workspace, B, max_prefill, HQ, HKV);
     int8_t* k_pool = c->k + (size_t)layer * c->page_bytes; int8_t* v_pool = c->v + (size_t)layer * c->page_bytes;
     float* ks_pool = c->ks + (size_t)layer * (c->scale_bytes / 4); float* vs_pool = c->vs + (size_t)layer * (c->scale_bytes / 4);
-    attn_qkv_prepare_f32_kernel<<<(unsigned)((long)B * Sq), 256, 0, st>>>(qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2, k_pool,
+    attn_qkv_prepare_f32_kernel<<<(unsigned)(((long)B * Sq * (HQ + 2 * HKV) + 31) / 32), 256, 0, st>>>(qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2, k_pool,
                                                                             ks_pool, page_table, max_pages, ws.v2, ws.vs2);
     dim3 g((Sq + 63) / 64, HKV, B);
     attn_v_to_pages_kernel<<<g, 256, 0, st>>>(ws.v2, ws.vs2, Sq, q_off, HKV, page_table, max_pages, v_pool, vs_pool);
@@ -1024,12 +1051,11 @@ static int mha_prefill_contiguous(bool online, const int8_t* q, const float* qs,
     FLEXLLM_REQUIRE(aligned(out, 16) && (!oacc || aligned(oacc, 16)) && aligned(v, 4));
     cudaStream_t st = (cudaStream_t)stream;
     PrefillWs ws(workspace, B, S, HQ, HKV);
-    const long wq = (long)B * S * HQ, wk = (long)B * S * HKV;
-    attn_qk_prepare_kernel<<<(unsigned)((wq + 7) / 8), 256, 0, st>>>(q, qs, cos_t, sin_t, B, S, HQ, ws.q2, ws.qs2);
-    attn_qk_prepare_kernel<<<(unsigned)((wk + 7) / 8), 256, 0, st>>>(k, ks, cos_t, sin_t, B, S, HKV, ws.k2, ws.ks2);
+    auto* prepare = aligned(q, 4) && aligned(k, 4) && aligned(cos_t, 16) && aligned(sin_t, 16) ? attn_qk_prepare_kernel<true> : attn_qk_prepare_kernel<false>;
+    prepare<<<(unsigned)(((long)B * S * (HQ + HKV) + 31) / 32), 256, 0, st>>>(q, qs, k, ks, cos_t, sin_t, B, S, HQ, HKV, ws.q2, ws.qs2, ws.k2, ws.ks2);
     dim3 g((S + 63) / 64, HKV, B);
     attn_v_transpose_kernel<<<g, 256, 0, st>>>(v, vs, B, S, HKV, ws.vT, ws.vsT);
-    int rc = launch_status(3);
+    int rc = launch_status(2);
     if (rc != FLEXLLM_OK) return rc;
     AttnArgs a;
     a.B = B; a.HQ = HQ; a.HKV = HKV; a.Sq = S; a.q_off = 0; a.Sk = S;

@@ -100,6 +100,26 @@ def test_prefill_quantiser_ranges(F, what):
     assert_same(to_np(out), ref["out"], "fp32 output")
 
 
+@pytest.mark.parametrize("what", ["q", "k", "tables"])
+def test_prefill_prepare_alignment(F, what):
+    """Inputs whose address allows no wide loads take the other form of the preparation."""
+    B, S, HQ, HKV = 1, 48, 6, 3
+    q, qs, k, ks, v, vs, a_s = attn_inputs(B, S, HQ, HKV, 79)
+    cos_t, sin_t = oracle.rope_table(S)
+
+    def shifted(a):
+        buf = torch.empty(a.size + 1, dtype=torch.from_numpy(a).dtype, device="cuda")
+        buf[1:] = dev(a).reshape(-1)
+        return buf[1:].reshape(a.shape)
+
+    out, oacc = F.MHA_i8xi8_Prefilling(shifted(q) if what == "q" else dev(q), dev(qs), shifted(k) if what == "k" else dev(k), dev(ks), dev(v), dev(vs),
+                                       shifted(cos_t) if what == "tables" else dev(cos_t), shifted(sin_t) if what == "tables" else dev(sin_t), dev(a_s),
+                                       want_oacc=True)
+    ref = oracle.mha_prefill(q, qs, k, ks, v, vs, cos_t, sin_t, a_s)
+    assert_same(to_np(oacc), ref["oacc"], "int32 P.V accumulators")
+    assert_same(to_np(out), ref["out"], "fp32 output")
+
+
 def g_exponents(shape):
     return np.random.default_rng(78).integers(-9, -3, shape).astype(np.float32)
 
