@@ -139,6 +139,94 @@ template <int BN, int KCH = 1> struct GemmCfg {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + STG_BYTES;
 };
 
+// ---- epilogue of the prefill orientation, one warp, rows row0 .. row0 + 31, columns col0 .. col0 + BN - 1 ----
+// Before the accumulator is waited for: column scales of the tile into shared memory, and the residual rows into L2.
+template <int BN> __device__ __forceinline__ void staged_prefetch(const GemmArgs& args, float* stg, int row0, int col0, int lane) {
+    float* sbw = stg + 1024;
+    if (args.sB)
+        for (int i = lane; i < BN; i += 32) sbw[i] = col0 + i < args.rowsB ? args.sB[col0 + i] : 0.0f;
+    if (args.residual) {
+        for (int i = lane; i < 32 * (BN / 32); i += 32) {
+            const int rr = i / (BN / 32), seg = i - rr * (BN / 32);
+            const int row = row0 + rr, col = col0 + seg * 32;
+            if (row < args.rowsA && col < args.rowsB)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(args.residual + (long)row * args.ldo + col));
+        }
+    }
+}
+// Lane = token row of the tile. 32 columns at a time are dequantised into this warp's staging buffer (16-byte granules
+// XOR-swizzled by the row), then written out with every warp instruction covering 4 rows x 128 contiguous bytes (the direct
+// form stores 32 rows x 16 bytes per instruction and was bound by the store path).
+template <int BN>
+__device__ __forceinline__ void staged_store(const GemmArgs& args, float* stg, const uint32_t tsrc, const int row0, const int col0, const float sa,
+                                             const int lane) {
+    const float* sbw = stg + 1024;
+    const int rowA = row0 + lane;
+    const bool rowA_ok = rowA < args.rowsA;
+    __syncwarp();
+    // the TMEM load of chunk c + 1 is in flight while chunk c is processed
+    constexpr int NCH = BN / 32;
+    auto process = [&](const uint32_t (&v)[32], const int c) {
+        const int colB0 = col0 + c * 32;
+        if (args.acc && rowA_ok) {
+            const long o = (long)rowA * args.ldo + colB0;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                if (colB0 + j < args.rowsB)
+                    *reinterpret_cast<int4*>(args.acc + o + j) = make_int4((int)v[j], (int)v[j + 1], (int)v[j + 2], (int)v[j + 3]);
+        }
+        if (args.y) {
+            float* buf = stg;
+            const int g = lane & 7;
+            // this lane's share of the residual for the write-out below, requested first
+            float4 rs[8];
+            if (args.residual) {
+#pragma unroll
+                for (int it = 0; it < 8; it++) {
+                    const int row = row0 + it * 4 + (lane >> 3), col = colB0 + 4 * g;
+                    rs[it] = (row < args.rowsA && col < args.rowsB) ? *reinterpret_cast<const float4*>(args.residual + (long)row * args.ldo + col)
+                                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+#pragma unroll
+            for (int gg = 0; gg < 8; gg++) {
+                const float4 sb = *reinterpret_cast<const float4*>(sbw + c * 32 + 4 * gg);
+                float4 r;
+                r.x = ((float)(int)v[4 * gg] * sa) * sb.x;
+                r.y = ((float)(int)v[4 * gg + 1] * sa) * sb.y;
+                r.z = ((float)(int)v[4 * gg + 2] * sa) * sb.z;
+                r.w = ((float)(int)v[4 * gg + 3] * sa) * sb.w;
+                *reinterpret_cast<float4*>(buf + lane * 32 + ((gg ^ (lane & 7)) << 2)) = r;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < 8; it++) {
+                const int rr = it * 4 + (lane >> 3);
+                const int row = row0 + rr, col = colB0 + 4 * g;
+                if (row < args.rowsA && col < args.rowsB) {
+                    float4 r = *reinterpret_cast<const float4*>(buf + rr * 32 + ((g ^ (rr & 7)) << 2));
+                    if (args.residual) { r.x = rs[it].x + r.x; r.y = rs[it].y + r.y; r.z = rs[it].z + r.z; r.w = rs[it].w + r.w; }
+                    *reinterpret_cast<float4*>(args.y + (long)row * args.ldo + col) = r;
+                }
+            }
+            __syncwarp();      // the staging buffer is reused by the next chunk
+        }
+    };
+    uint32_t va[32], vb[32];
+    tmem_ld_32x32(tsrc, va);
+#pragma unroll 1
+    for (int c = 0; c < NCH; c += 2) {
+        tmem_ld_wait();
+        if (c + 1 < NCH) tmem_ld_32x32(tsrc + (c + 1) * 32, vb);
+        process(va, c);
+        if (c + 1 < NCH) {
+            tmem_ld_wait();
+            if (c + 2 < NCH) tmem_ld_32x32(tsrc + (c + 2) * 32, va);
+            process(vb, c + 1);
+        }
+    }
+}
+
 template <int BN, bool SWAP, int KCH = 1>
 __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmapA,
                                                                  const __grid_constant__ CUtensorMap tmapB,
@@ -263,97 +351,15 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
                 for (int j = 0; j < BN; j++) { const int tok = tb * BN + j; sbv[j] = tok < args.rowsB ? args.sB[tok] : 0.0f; }
             }
             float* stg = reinterpret_cast<float*>(ring_ptr + STAGES * Cfg::STAGE_BYTES + 256) + q * Cfg::STG_WARP_FLOATS;
-            if (!SWAP && BN >= 32) {
-                // column scales of this tile into shared memory, and the residual rows into L2
-                float* sbw = stg + 1024;
-                if (args.sB)
-                    for (int i = lane; i < BN; i += 32) sbw[i] = tb * BN + i < args.rowsB ? args.sB[tb * BN + i] : 0.0f;
-                if (args.residual) {
-                    for (int i = lane; i < 32 * (BN / 32); i += 32) {
-                        const int rr = i / (BN / 32), seg = i - rr * (BN / 32);
-                        const int row = ta * 128 + q * 32 + rr, col = tb * BN + seg * 32;
-                        if (row < args.rowsA && col < args.rowsB)
-                            asm volatile("prefetch.global.L2 [%0];" ::"l"(args.residual + (long)row * args.ldo + col));
-                    }
-                }
-            }
+            if constexpr (!SWAP && BN >= 32) staged_prefetch<BN>(args, stg, ta * 128 + q * 32, tb * BN, lane);
             // lane 0 polls; the verdict is broadcast so that the warp stays converged for the
             // warp-collective TMEM loads below
             int got = (lane == 0) ? (mbar_wait(bar_tfull + 8 * as, aphase, abort_flag) ? 1 : 0) : 1;
             got = __shfl_sync(0xffffffffu, got, 0);
             if (!got) { ok = false; break; }
             tc_fence_after();
-            if (!SWAP && BN >= 32) {
-                // ---- prefill orientation, staged: lane = token row of the tile. 32 columns at a time are
-                // dequantised into this warp's staging buffer (16-byte granules XOR-swizzled by the row), then
-                // written out with every warp instruction covering 4 rows x 128 contiguous bytes (the direct
-                // form stores 32 rows x 16 bytes per instruction and was bound by the store path).
-                const float* sbw = stg + 1024;
-                __syncwarp();
-                // the TMEM load of chunk c + 1 is in flight while chunk c is processed
-                constexpr int NCH = BN / 32;
-                const uint32_t tsrc = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
-                auto process = [&](const uint32_t (&v)[32], const int c) {
-                    const int colB0 = tb * BN + c * 32;
-                    if (args.acc && rowA_ok) {
-                        const long o = (long)rowA * args.ldo + colB0;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            if (colB0 + j < args.rowsB)
-                                *reinterpret_cast<int4*>(args.acc + o + j) = make_int4((int)v[j], (int)v[j + 1], (int)v[j + 2], (int)v[j + 3]);
-                    }
-                    if (args.y) {
-                        float* buf = stg;
-                        const int g = lane & 7;
-                        // this lane's share of the residual for the write-out below, requested first
-                        float4 rs[8];
-                        if (args.residual) {
-#pragma unroll
-                            for (int it = 0; it < 8; it++) {
-                                const int rr = it * 4 + (lane >> 3);
-                                const int row = ta * 128 + q * 32 + rr, col = colB0 + 4 * g;
-                                rs[it] = (row < args.rowsA && col < args.rowsB)
-                                             ? *reinterpret_cast<const float4*>(args.residual + (long)row * args.ldo + col)
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
-                            }
-                        }
-#pragma unroll
-                        for (int gg = 0; gg < 8; gg++) {
-                            const float4 sb = *reinterpret_cast<const float4*>(sbw + c * 32 + 4 * gg);
-                            float4 r;
-                            r.x = ((float)(int)v[4 * gg] * sa) * sb.x;
-                            r.y = ((float)(int)v[4 * gg + 1] * sa) * sb.y;
-                            r.z = ((float)(int)v[4 * gg + 2] * sa) * sb.z;
-                            r.w = ((float)(int)v[4 * gg + 3] * sa) * sb.w;
-                            *reinterpret_cast<float4*>(buf + lane * 32 + ((gg ^ (lane & 7)) << 2)) = r;
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int it = 0; it < 8; it++) {
-                            const int rr = it * 4 + (lane >> 3);
-                            const int row = ta * 128 + q * 32 + rr, col = colB0 + 4 * g;
-                            if (row < args.rowsA && col < args.rowsB) {
-                                float4 r = *reinterpret_cast<const float4*>(buf + rr * 32 + ((g ^ (rr & 7)) << 2));
-                                if (args.residual) { r.x = rs[it].x + r.x; r.y = rs[it].y + r.y; r.z = rs[it].z + r.z; r.w = rs[it].w + r.w; }
-                                *reinterpret_cast<float4*>(args.y + (long)row * args.ldo + col) = r;
-                            }
-                        }
-                        __syncwarp();      // the staging buffer is reused by the next chunk
-                    }
-                };
-                uint32_t va[32], vb[32];
-                tmem_ld_32x32(tsrc, va);
-#pragma unroll 1
-                for (int c = 0; c < NCH; c += 2) {
-                    tmem_ld_wait();
-                    if (c + 1 < NCH) tmem_ld_32x32(tsrc + (c + 1) * 32, vb);
-                    process(va, c);
-                    if (c + 1 < NCH) {
-                        tmem_ld_wait();
-                        if (c + 2 < NCH) tmem_ld_32x32(tsrc + (c + 2) * 32, va);
-                        process(vb, c + 1);
-                    }
-                }
+            if constexpr (!SWAP && BN >= 32) {
+                staged_store<BN>(args, stg, tmem_base + ((uint32_t)(q * 32) << 16) + as * BN, ta * 128 + q * 32, tb * BN, sa, lane);
             } else {
         #pragma unroll (SWAP ? BN / 16 : 1)
             for (int c = 0; c < BN / 16; c++) {
@@ -478,6 +484,135 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
     }
 }
 
+// ------------------------------------------------------------------ prefill form on CTA pairs
+// The same product with 256 x 256 tiles on two SMs (cta_group::2): each CTA brings in 128 rows of either side, so that per step of
+// 128 bytes of K it writes and reads 32 KB of shared memory where the single-CTA form, with 128 + 256 rows, moves 48 KB. Shared memory
+// (TMA writes and operand reads, 128 bytes a clock) is what bounds that form, together with its epilogue. Roles as
+// there, in both CTAs, but only the first CTA's warp 1 issues MMAs; its barriers count both CTAs' bytes and readers.
+// W8A8 prompt of 32 x 1024 tokens, products of 16 layers included: 78.8 -> 75.3 ms.
+constexpr int GP_STAGES = 6, GP_TILE = 128 * 128, GP_STAGE_BYTES = 2 * GP_TILE, GP_BN = 256;
+constexpr int GP_SMEM = GP_STAGES * GP_STAGE_BYTES + 1024 + 256 + GemmCfg<GP_BN>::STG_BYTES;
+__global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
+                                                              const GemmArgs args) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t ring = (raw + 1023u) & ~1023u;
+    uint8_t* ring_ptr = smem_raw + (ring - raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES);
+    const uint32_t bar_full = smem_u32(bars);                    // first CTA: bytes of both CTAs
+    const uint32_t bar_empty = bar_full + 8 * GP_STAGES;         // both CTAs, each for its own producer
+    const uint32_t bar_tfull = bar_empty + 8 * GP_STAGES;        // both CTAs
+    const uint32_t bar_tempty = bar_tfull + 16;                  // first CTA: the eight epilogue warps of both
+    uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * GP_STAGES + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    float* stg_all = reinterpret_cast<float*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES + 256);
+
+    pdl_sync();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int num_kb = (args.K + 127) >> 7;
+    const int total_tiles = args.tilesA * args.tilesB;           // tilesA: 256-row tiles
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GP_STAGES; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
+        for (int s = 0; s < 2; s++) { mbar_init(bar_tfull + 8 * s, 1); mbar_init(bar_tempty + 8 * s, 8); }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tmem_alloc_pair(smem_u32(tmem_base_slot), 2 * GP_BN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                              // the other CTA's barriers exist before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_base_slot;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer, one per CTA
+        if (lane == 0) {
+            tma_prefetch_desc(&tmapA);
+            tma_prefetch_desc(&tmapB);
+            int stage = 0; uint32_t phase = 0;
+            bool ok = true;
+            for (int t = pair; ok && t < total_tiles; t += pairs) {
+                const int rowA = (t / args.tilesB) * 256 + rank * 128, rowB = (t % args.tilesB) * GP_BN + rank * 128;
+                for (int kb = 0; kb < num_kb; kb++) {
+                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
+                    const uint32_t full = bar_full + 8 * stage, full0 = cluster_addr(full, 0);
+                    if (rank == 0) mbar_expect_tx(full, 2 * GP_STAGE_BYTES);
+                    const uint32_t dst = ring + stage * GP_STAGE_BYTES;
+                    tma_load_2d_pair(dst, &tmapA, full0, kb * 128, rowA);
+                    tma_load_2d_pair(dst + GP_TILE, &tmapB, full0, kb * 128, rowB);
+                    if (++stage == GP_STAGES) { stage = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer, first CTA
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = umma_idesc_i8(256, GP_BN, 1, 1);
+            int stage = 0; uint32_t phase = 0;
+            int it = 0;
+            bool ok = true;
+            for (int t = pair; ok && t < total_tiles; t += pairs, it++) {
+                const int as = it & 1;
+                if (!mbar_wait(bar_tempty + 8 * as, (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                for (int kb = 0; kb < num_kb; kb++) {
+                    if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sa = ring + stage * GP_STAGE_BYTES;
+                    const uint64_t adesc = umma_desc_k_sw128(sa), bdesc = umma_desc_k_sw128(sa + GP_TILE);
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        umma_i8_pair(tmem_base + as * GP_BN, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit_pair(bar_empty + 8 * stage);
+                    if (++stage == GP_STAGES) { stage = 0; phase ^= 1u; }
+                }
+                if (ok) umma_commit_pair(bar_tfull + 8 * as);
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
+        const int q = warp & 3;
+        float* stg = stg_all + q * GemmCfg<GP_BN>::STG_WARP_FLOATS;
+        int it = 0;
+        for (int t = pair; t < total_tiles; t += pairs, it++) {
+            const int row0 = (t / args.tilesB) * 256 + rank * 128 + q * 32, col0 = (t % args.tilesB) * GP_BN;
+            const int as = it & 1;
+            const float sa = (row0 + lane < args.rowsA && args.sA) ? args.sA[row0 + lane] : 0.0f;
+            staged_prefetch<GP_BN>(args, stg, row0, col0, lane);
+            int got = (lane == 0) ? (mbar_wait(bar_tfull + 8 * as, (uint32_t)((it >> 1) & 1), abort_flag) ? 1 : 0) : 1;
+            got = __shfl_sync(0xffffffffu, got, 0);
+            if (!got) break;
+            tc_fence_after();
+            staged_store<GP_BN>(args, stg, tmem_base + ((uint32_t)(q * 32) << 16) + as * GP_BN, row0, col0, sa, lane);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(bar_tempty + 8 * as, 0));
+        }
+    }
+
+    // ---------------------------------------------------------------- tear-down
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        // a wait ran out: give copies still in flight time to land before shared memory is released
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+        if (threadIdx.x == 0 && args.error_flag) atomicOr(args.error_flag, 1);
+        __syncthreads();
+    }
+    cluster_sync();                                              // both CTAs are done with each other's memory
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 2 * GP_BN);
+    }
+}
+
 // ------------------------------------------------------------------ host launcher
 struct TmapKey {
     const void* base; uint64_t rows, row_bytes; uint32_t box_rows, kch;   // kch 0: 2-D map
@@ -570,12 +705,48 @@ static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, i
     return launch_status();
 }
 
+static int launch_gemm_pair(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K, int32_t* acc, float* y,
+                            cudaStream_t st, const float* residual) {
+    CUtensorMap ta, tb;
+    int rc = cached_tmap(&ta, a, (uint64_t)M, (uint64_t)K, 128);
+    if (rc != FLEXLLM_OK) return rc;
+    rc = cached_tmap(&tb, w, (uint64_t)N, (uint64_t)K, 128);
+    if (rc != FLEXLLM_OK) return rc;
+    GemmArgs g;
+    g.rowsA = M; g.rowsB = N; g.K = K;
+    g.tilesA = (M + 255) / 256; g.tilesB = (N + GP_BN - 1) / GP_BN; g.ksplit = 1;
+    g.ldo = N; g.acc = acc; g.y = y; g.sA = s_tok; g.sB = s_ch; g.error_flag = device_error_flag();
+    g.residual = residual; g.work = nullptr; g.counters = nullptr;
+    static std::atomic<bool> attr_set[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0) return FLEXLLM_ECUDA;
+    if (!attr_set[dev].load(std::memory_order_acquire)) {
+        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(gemm_i8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
+        attr_set[dev].store(true, std::memory_order_release);
+    }
+    const int tiles = g.tilesA * g.tilesB, pairs = sm_count() / 2;
+    launch_cluster(gemm_i8_pair_kernel, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(192), 2, (size_t)GP_SMEM, st, ta, tb, g);
+    return launch_status();
+}
+
 // Prefill orientation: activations on the 128-row side. residual (optional): y = residual + dequant.
+// The tile is the one with the shortest time by a count of shared-memory traffic: per step of 128 bytes of K a CTA moves (128 + BN)
+// rows (the pair form 256 for twice the output), plus a fixed part; times the rounds of tiles that the SMs go through. (With 256
+// columns whenever there are that many, a product of 128 x 2048 x 2048 ran on 8 SMs for 15 us.)
 int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
                     int32_t* acc, float* y, cudaStream_t st, const float* residual) {
-    if (N > 128) return launch_gemm<256, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
-    if (N > 64) return launch_gemm<128, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
-    if (N > 32) return launch_gemm<64, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
+    const int sms = sm_count();
+    auto cost = [&](int rows, int cols, int units, int step) {
+        const long tiles = (long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
+        return (tiles + units - 1) / units * step;
+    };
+    const long c256 = cost(128, 256, sms, 128 + 256 + 32), c128 = cost(128, 128, sms, 128 + 128 + 32), c64 = cost(128, 64, sms, 128 + 64 + 32),
+               c32 = cost(128, 32, sms, 128 + 32 + 32), cpair = cost(256, 256, sms / 2, 256 + 48);
+    if (N > 128 && M > 128 && cpair <= c256 && cpair <= c128 && cpair <= c64 && cpair <= c32)
+        return launch_gemm_pair(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
+    if (N > 128 && c256 <= c128 && c256 <= c64 && c256 <= c32) return launch_gemm<256, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
+    if (N > 64 && c128 <= c64 && c128 <= c32) return launch_gemm<128, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
+    if (N > 32 && c64 <= c32) return launch_gemm<64, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     if (N > 16) return launch_gemm<32, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     return launch_gemm<16, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
 }

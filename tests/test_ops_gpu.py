@@ -275,6 +275,20 @@ def test_linear_prefill_tcgen05(F, M, N, K):
     assert_same(to_np(acc), acc_o, "acc"); assert_same(to_np(y), y_o, "y")
 
 
+@pytest.mark.parametrize("M,N,K", [(1990, 4104, 400),    # pairs of CTAs, all edges ragged
+                                   (2048, 2560, 144), (129, 19000, 256), (1500, 1024, 128), (640, 2048, 128)])
+def test_linear_prefill_tile_choice(F, M, N, K):
+    """Shapes on both sides of the rule that chooses the tile, with the accumulators and with a residual."""
+    a, st, w, sc = lin_inputs(M, N, K, 24)
+    acc, y = F.pref_Linear_Layer_i8xi8(dev(a), dev(st), dev(w), dev(sc), want_acc=True)
+    acc_o, y_o = oracle.linear_i8(a, st, w, sc)
+    assert_same(to_np(acc), acc_o, "acc"); assert_same(to_np(y), y_o, "y")
+    res = rng(25).standard_normal((M, N)).astype(np.float32)
+    _, yr = F.pref_Linear_Layer_i8xi8(dev(a), dev(st), dev(w), dev(sc), residual=dev(res))
+    assert_same(to_np(yr), oracle.residual(res, y_o), "residual + y")
+    assert F.lib().flexllm_device_status() == 0
+
+
 def test_linear_prefill_extremes(F):
     """Largest accumulator magnitude the path can see: |a|=|w|=128... here -128 * -128 * 8192."""
     M, N, K = 128, 128, 8192
