@@ -40,10 +40,10 @@ inline int launch_status(int n = 1) { note_launches(n); return cuda_status(cudaG
 // before it touches memory: it first lets its own dependents start launching, then waits until the
 // kernel before it has completed and flushed (so data hazards are exactly those of an ordinary stream).
 extern thread_local int g_pdl;
-__device__ __forceinline__ void pdl_sync() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+// A kernel whose weights no earlier kernel writes may ask for them between the two halves.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_sync() { pdl_launch(); pdl_wait(); }
 template <class... KArgs, class... Args>
 inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};

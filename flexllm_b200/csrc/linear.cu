@@ -131,8 +131,8 @@ extern "C" size_t flexllm_mlp_block_workspace(int M, int D, int F) {
 }
 
 // RMSNorm + quant -> fused gate|up projection -> SiLU(gate) * up, FHT-8192, quant -> down projection + residual: the four
-// launches follow one another with programmatic dependent launch, so each kernel's launch and (for the weight-streaming
-// GEMV) first weight loads overlap the tail of the one before.
+// launches follow one another with programmatic dependent launch, so each kernel's launch and, for the products, first weight
+// loads overlap the tail of the one before.
 extern "C" int flexllm_mlp_block_decode(const float* x, const float* gamma, const int8_t* w_gu, const float* s_gu, const int8_t* w_d,
                                         const float* s_d, int M, int D, int F, float eps, int order, float fht_scale, float* y,
                                         void* workspace, size_t workspace_bytes, void* stream) {
@@ -148,8 +148,10 @@ extern "C" int flexllm_mlp_block_decode(const float* x, const float* gamma, cons
     float* gu = (float*)w; w += up256((size_t)M * 2 * F * 4);
     int8_t* hq = (int8_t*)w;
     cudaStream_t st = (cudaStream_t)stream;
-    struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    // The first launch is an ordinary one: it starts when everything before it in the stream has completed, and the products, which
+    // ask for their weights without waiting, start after it. A caller's kernel may have written those weights just before.
     TRY_RC(flexllm_rmsnorm_quant(x, gamma, M, D, eps, order, nullptr, xq, xs, st));
+    struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
     TRY_RC(linear_decode(xq, xs, w_gu, s_gu, M, 2 * F, D, nullptr, gu, nullptr, st));
     TRY_RC(swiglu_fht_quant_strided(gu, gu + F, 2L * F, M, fht_scale, hq, hs, st));
     return linear_decode(hq, hs, w_d, s_d, M, D, F, nullptr, y, x, st);
