@@ -104,22 +104,34 @@ struct DecAttnSmem {
     int last;           // scratch flag for callers (e.g. "this item completed its sequence")
 };
 
-// One call by a group of NT threads per (sequence b, KV head hkv) does the whole step for its GQA group of 4 query
-// heads: Q/K/V preparation and cache append, scores, max, exp, the ordered partial sums, the u8
-// quantiser and P.V, with the score row kept in shared memory (`dsm`: 20 bytes per key, at least
-// 4096 bytes). The group's NT threads (256 or 512; `tid` = index in the group) synchronise on named
+// One call by a group of NT threads per (sequence b, KV head hkv) does the whole step for G of the four query heads of the
+// GQA group, heads hq0 .. hq0 + G - 1: Q/K/V preparation and cache append (with G = 2 both callers of a group write the same
+// bytes), scores, max, exp, the ordered partial sums, the u8 quantiser and P.V, with the score rows kept in shared
+// memory (`dsm`: dec_attn_smem_bytes<G>). The group's NT threads (256 or 512; `tid` = index in the group) synchronise on named
 // barrier `bar`.
-template <int MODE, int NT>
+// G = 2 (stand-alone operator): rows padded against bank conflicts in the ordered sums, the warp-wide exponential, and the
+// quantiser without divisions. G = 4 (persistent kernel): the forms that measured best inside that kernel.
+template <int G> constexpr size_t dec_attn_smem_bytes(int cs) {
+    const size_t n = (size_t)G * (G == 2 ? cs + 4 : cs) * 4 + (size_t)G * cs;
+    return n < 4096 ? 4096 : n;
+}
+// U = min(round((e * r * vs) / a_s), 255) as the reference forms it
+__device__ __noinline__ static uint32_t dec_u8_exact(float e, float rinv, float vs, float a_s) {
+    const int r = round_half_away_to_int(((e * rinv) * vs) / a_s);
+    return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
+}
+template <int MODE, int NT, int G = 4>
 __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const float* __restrict__ cos_t,
                                                     const float* __restrict__ sin_t, const float* __restrict__ a_s,
                                                     const KvLayer& cache, const int32_t* __restrict__ page_table, int max_pages,
                                                     const int32_t* __restrict__ ctx, int HQ, int HKV, int cs,
                                                     float* __restrict__ out, int32_t* __restrict__ oacc,
                                                     const int hkv, const int b, uint8_t* dsm, DecAttnSmem& sm, const int tid,
-                                                    const int bar) {
-    constexpr int G = 4;
-    float* sc = reinterpret_cast<float*>(dsm);                       // [G][cs]
-    uint8_t* u_sm = dsm + (size_t)G * cs * 4;                        // [G][cs]
+                                                    const int bar, const int part4 = 0) {
+    const int hq0 = hkv * 4 + part4 * G;                             // part4: which of the 4 / G parts of the group
+    const int csr = G == 2 ? cs + 4 : cs;                            // row stride of the scores
+    float* sc = reinterpret_cast<float*>(dsm);                       // [G][csr]
+    uint8_t* u_sm = dsm + (size_t)G * csr * 4;                        // [G][cs]
     int8_t (*q_sm)[64] = sm.q_sm;
     float* q_scale = sm.q_scale; float (*red)[16] = sm.red; float* row_max = sm.row_max; float* row_rinv = sm.row_rinv;
     float (*part)[4] = sm.part;
@@ -131,8 +143,8 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // MODE 2: the split-K partial sums of this warp's head do not depend on the context length, so
     // their loads go out first and overlap the context / page-table round trips below
     int a0 = 0, a1 = 0;
-    if (MODE == 2 && w < 6) {
-        const int h = w < 4 ? hkv * G + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
+    if (MODE == 2 && w < G + 2) {
+        const int h = w < G ? hq0 + w : (w == G ? HQ + hkv : HQ + HKV + hkv);
         const int32_t* src = in.qkv_acc + (long)b * heads * 64 + (long)h * 64 + lane;
 #pragma unroll 1
         for (int sl = 0; sl < in.n_slabs; sl += 4) {
@@ -156,18 +168,18 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // warm L2 with this head's V pages while the scores are computed (V is first needed in step G);
     // the persistent kernel (MODE 2) has asked for them a phase earlier
     if (MODE != 2)
-    for (int i = tid; i < npages_all * 32; i += NT) {
+    for (int i = tid + part4 * NT; i < npages_all * 32; i += NT * (4 / G)) {
         const long pg = page_table[(long)b * max_pages + (i >> 5)];
         const int8_t* line = cache.v + (pg * HKV + hkv) * (long)(64 * PAGE) + (long)(i & 31) * 128;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
     }
 
     ATT_TS(1);
-    // ---- A. prepare: warps 0..3 the query heads, warp 4 the key head, warp 5 the value head
-    if (w < 6) {
+    // ---- A. prepare: warps 0..G-1 the query heads, warp G the key head, warp G+1 the value head
+    if (w < G + 2) {
         const long pg = page_table[(long)b * max_pages + pos / PAGE];
         const int slot = pos % PAGE;
-        const int h = w < 4 ? hkv * G + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);   // index in the fused row
+        const int h = w < G ? hq0 + w : (w == G ? HQ + hkv : HQ + HKV + hkv);   // index in the fused row
         float x0, x1;
         if (MODE == 2) {
             // int32 partial sums of the fused q|k|v projection (one slab per K split), added up above
@@ -179,20 +191,20 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
             const float* src = in.qkv_f32 + (long)b * heads * 64 + (long)h * 64;
             x0 = src[lane]; x1 = src[lane + 32];
         } else {
-            const int8_t* src = w < 4 ? in.q + ((long)b * HQ + hkv * G + w) * 64 : (w == 4 ? in.k : in.v) + ((long)b * HKV + hkv) * 64;
-            const float sc_in = w < 4 ? in.qs[(long)b * HQ + hkv * G + w] : (w == 4 ? in.ks : in.vs)[(long)b * HKV + hkv];
+            const int8_t* src = w < G ? in.q + ((long)b * HQ + hq0 + w) * 64 : (w == G ? in.k : in.v) + ((long)b * HKV + hkv) * 64;
+            const float sc_in = w < G ? in.qs[(long)b * HQ + hq0 + w] : (w == G ? in.ks : in.vs)[(long)b * HKV + hkv];
             x0 = (float)src[lane]; x1 = (float)src[lane + 32];
-            if (w < 5) { x0 = x0 * sc_in; x1 = x1 * sc_in; }
-            if (w == 5) {   // int8 value head: plain copy
+            if (w < G + 1) { x0 = x0 * sc_in; x1 = x1 * sc_in; }
+            if (w == G + 1) {   // int8 value head: plain copy
                 int8_t* dst = cache.v + (pg * HKV + hkv) * (long)(64 * PAGE);
                 dst[(long)lane * PAGE + slot] = src[lane];
                 dst[(long)(lane + 32) * PAGE + slot] = src[lane + 32];
                 if (lane == 0) cache.vs[(pg * HKV + hkv) * PAGE + slot] = sc_in;
             }
         }
-        if (MODE != 0 || w < 5) {
+        if (MODE != 0 || w < G + 1) {
             float a = x0, bb = x1;
-            if (w < 5) {
+            if (w < G + 1) {
                 const float c = cos_t[(long)pos * 32 + lane], sn = sin_t[(long)pos * 32 + lane];
                 a = x0 * c - x1 * sn;
                 bb = x0 * sn + x1 * c;
@@ -211,10 +223,10 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
             const float mx = warp_max(fmaxf(a, bb)), mn = warp_min(fminf(a, bb));
             const float s2 = sym_scale_from(mx, mn);
             const int8_t qa = quant_s8(a, s2), qb = quant_s8(bb, s2);
-            if (w < 4) {
+            if (w < G) {
                 q_sm[w][lane] = qa; q_sm[w][lane + 32] = qb;
                 if (lane == 0) q_scale[w] = s2;
-            } else if (w == 4) {
+            } else if (w == G) {
                 int8_t* dst = cache.k + ((pg * HKV + hkv) * PAGE + slot) * 64L;
                 dst[lane] = qa; dst[lane + 32] = qb;
                 if (lane == 0) cache.ks[(pg * HKV + hkv) * PAGE + slot] = s2;
@@ -269,8 +281,8 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
                 const float x = (((float)acc * qsc[g]) * ksc[u]) * 0.125f;
                 if (g == l4) xg = x;
             }
-            if (key < nk) {
-                sc[l4 * cs + key] = xg;
+            if (key < nk && l4 < G) {
+                sc[l4 * csr + key] = xg;
                 mymax = xg > mymax ? xg : mymax;
             }
         }
@@ -280,7 +292,7 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, 4));
     mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, 8));
     mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, 16));
-    if (lane < 4) red[lane][w] = mymax;
+    if (lane < G) red[lane][w] = mymax;
     named_sync_id<NT>(bar);
     if (tid < G) {
         float m = red[tid][0];
@@ -302,9 +314,34 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
         }
     }
     ATT_TS(4);
-    // ---- D. e = exp(x - max), in place: the four heads of a key together (four independent evaluations in flight)
-    {
-        const float m0 = row_max[0], m1 = row_max[1], m2 = row_max[2], m3 = row_max[3];
+    // ---- D. e = exp(x - max), in place
+    if constexpr (G == 2) {
+        // eight values at a time: four keys of both heads
+        const ExpTable tab = exp_table_lane();
+        const float m0 = row_max[0], m1 = row_max[1];
+        for (int k0 = 0; k0 < nk; k0 += 4 * NT) {
+            float u[8], e[8], far = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int key = k0 + i * NT + tid;
+                const bool in = key < nk;
+                u[2 * i] = in ? m0 - sc[key] : 0.0f;
+                u[2 * i + 1] = in ? m1 - sc[csr + key] : 0.0f;
+                far = max3_nan(far, u[2 * i], u[2 * i + 1]);
+            }
+            if (__all_sync(0xffffffffu, far <= kExpFastLimit)) exp_warp<true>(u, e, tab);
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; i++) e[i] = ref_expf(-u[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int key = k0 + i * NT + tid;
+                if (key < nk) { sc[key] = e[2 * i]; sc[csr + key] = e[2 * i + 1]; }
+            }
+        }
+    } else {   // the four heads of a key together (four independent evaluations in flight)
+        const float m0 = row_max[0], m1 = row_max[1], m2 = row_max[G > 2 ? 2 : 0], m3 = row_max[G > 2 ? 3 : 0];
         for (int key = tid; key < nk; key += NT) {
             const float x0 = sc[key] - m0, x1 = sc[cs + key] - m1, x2 = sc[2 * cs + key] - m2, x3 = sc[3 * cs + key] - m3;
             const float e0 = ref_expf(x0), e1 = ref_expf(x1), e2 = ref_expf(x2), e3 = ref_expf(x3);
@@ -316,10 +353,31 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // ---- E. the four ordered chains of each row (Softmax.h:514-553): one thread per chain
     if (tid < 4 * G) {
         const int g = tid >> 2, j = tid & 3;
-        const float* e = sc + g * cs;
+        const float* e = sc + g * csr;
         float ps = 0.0f;
+        int i = j;
+        if constexpr (G == 2) {
+            // blocks of 16, the next block's loads under way while this one is added: a step costs the addition's latency
+            constexpr int UE = 16;
+            if (i + 4 * (UE - 1) < nk) {
+                float cur[UE], nxt[UE];
+#pragma unroll
+                for (int t = 0; t < UE; t++) cur[t] = e[i + 4 * t];
+                for (; i + 4 * (2 * UE - 1) < nk; i += 4 * UE) {
+#pragma unroll
+                    for (int t = 0; t < UE; t++) nxt[t] = e[i + 4 * (UE + t)];
+#pragma unroll
+                    for (int t = 0; t < UE; t++) ps += cur[t];
+#pragma unroll
+                    for (int t = 0; t < UE; t++) cur[t] = nxt[t];
+                }
+#pragma unroll
+                for (int t = 0; t < UE; t++) ps += cur[t];
+                i += 4 * UE;
+            }
+        }
 #pragma unroll 8
-        for (int i = j; i < nk; i += 4) ps += e[i];
+        for (; i < nk; i += 4) ps += e[i];
         part[g][j] = ps;
     }
     named_sync_id<NT>(bar);
@@ -331,13 +389,29 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     {
         float rinv_g[G];
         DivBy as_g[G];
+        float c_g[G];
+        bool ok_g[G];
 #pragma unroll
-        for (int g = 0; g < G; g++) { rinv_g[g] = row_rinv[g]; as_g[g] = div_by(a_s[hkv * G + g]); }
+        for (int g = 0; g < G; g++) {
+            rinv_g[g] = row_rinv[g]; as_g[g] = div_by(a_s[hq0 + g]);
+            c_g[g] = (rinv_g[g] * as_g[g].y) * (1.0f / 255.25f);
+            ok_g[g] = c_g[g] >= 0x1p-60f && c_g[g] <= 0x1p60f;
+        }
         auto quantise_key = [&](int key, float vsc) {
 #pragma unroll
             for (int g = 0; g < G; g++) {
                 uint8_t uq = 0;
-                if (key < nk) {
+                if (G == 2) {
+                    if (key < nk) {
+                        // (e c) vs with c = r / (255.25 a_s), held at 1: within 2^-21 of the reference's quotient / 255.25 (seven
+                        // roundings), so where the two sides of 2^-19 round to the same integer, that is U
+                        const float e = sc[g * csr + key], t = __saturatef((e * c_g[g]) * vsc);
+                        const float h = __fmaf_rn(t, 255.25f * (1.0f + 0x1p-19f), 12582912.0f), l = __fmaf_rn(t, 255.25f * (1.0f - 0x1p-19f), 12582912.0f);
+                        uint32_t q = __float_as_uint(h);
+                        if (!ok_g[g] || !(vsc >= 0.0f && vsc <= 0x1p40f) || q != __float_as_uint(l)) q = dec_u8_exact(e, rinv_g[g], vsc, as_g[g].s);
+                        uq = (uint8_t)q;
+                    }
+                } else if (key < nk) {
                     const float p = sc[g * cs + key] * rinv_g[g];
                     const float tt = div_for_rounding(p * vsc, as_g[g]);
                     int r = round_half_away_to_int(tt);
@@ -366,7 +440,7 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // ---- G. P.V: four lanes share one V^T row (16 keys of the page each); thread = (page slot, d, quarter)
     {
         const int d = (tid >> 2) & 63, ps = tid >> 8;     // ps: which of the NT/256 pages of an iteration
-        int acc[G] = {0, 0, 0, 0};
+        int acc[G] = {};
         const int npages = nk_pad / PAGE;
 #pragma unroll 8
         for (int p = ps; p < npages; p += NT / 256) {
@@ -393,12 +467,12 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
         // combine the NT/256 page slots through shared memory (integer adds: exact)
         int* pv_sm = reinterpret_cast<int*>(sc);          // scores are no longer needed: reuse [NT/256][G][64]
         named_sync_id<NT>(bar);
-        pv_sm[(ps * G + l4) * 64 + d] = mine;
+        if (l4 < G) pv_sm[(ps * G + l4) * 64 + d] = mine;
         named_sync_id<NT>(bar);
-        if (ps == 0) {
+        if (ps == 0 && l4 < G) {
             int tot = 0;
             for (int i = 0; i < NT / 256; i++) tot += pv_sm[(i * G + l4) * 64 + d];
-            const int hq = hkv * G + l4;
+            const int hq = hq0 + l4;
             const long o = ((long)b * HQ + hq) * 64 + d;
             out[o] = (float)tot * a_s[hq];
             if (oacc) oacc[o] = tot;

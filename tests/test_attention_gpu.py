@@ -186,7 +186,7 @@ def test_prefill_online_softmax_variant_is_close(F, B, S, HQ, HKV):
 
 
 # ------------------------------------------------------------------------------ decode (config 4)
-def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1):
+def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1, q_gain=1.0, v_gain=1.0, a_gain=1.0):
     g = np.random.default_rng(seed)
     PAGE = 64
     ctx = np.asarray(ctx, np.int32)
@@ -205,7 +205,8 @@ def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1):
     vs_pool = g.uniform(0.005, 0.05, (n_pages, HKV, PAGE)).astype(np.float32)
     max_ctx = int(ctx.max()) + steps
     cos_t, sin_t = oracle.rope_table(max_ctx + 1)
-    a_s = np.full(HQ, 0.05 / 255, np.float32)
+    a_s = np.full(HQ, 0.05 / 255 * a_gain, np.float32)
+    vs_pool *= np.float32(v_gain)
     cache = F.KVCache(1, n_pages, HKV)
     kd, ksd, vd, vsd = cache.pools(0)
     kd.copy_(dev(k_pool)); ksd.copy_(dev(ks_pool)); vsd.copy_(dev(vs_pool))
@@ -215,7 +216,8 @@ def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1):
         q = g.integers(-127, 128, (B, HQ, 64), dtype=np.int8); k = g.integers(-127, 128, (B, HKV, 64), dtype=np.int8)
         v = g.integers(-127, 128, (B, HKV, 64), dtype=np.int8)
         qs = g.uniform(0.005, 0.05, (B, HQ)).astype(np.float32); ks = g.uniform(0.005, 0.05, (B, HKV)).astype(np.float32)
-        vs = g.uniform(0.005, 0.05, (B, HKV)).astype(np.float32)
+        vs = g.uniform(0.005, 0.05, (B, HKV)).astype(np.float32) * np.float32(v_gain)
+        qs *= np.float32(q_gain)
         out, oacc = F.MHA_i8xi8_Decoding(cache, 0, dev(q), dev(qs), dev(k), dev(ks), dev(v), dev(vs), dev(cos_t), dev(sin_t),
                                          dev(a_s), dev(page_table), dev(cur), max_ctx, want_oacc=True)
         torch.cuda.synchronize()
@@ -246,6 +248,14 @@ def test_decode_config4_slice(F):
 
 def test_decode_max_context(F):
     decode_case(F, 2, [8192, 8191], seed=43)
+
+
+@pytest.mark.parametrize("what", [dict(q_gain=20.0), dict(q_gain=3.0), dict(a_gain=0.01), dict(a_gain=1e-5), dict(v_gain=2.0 ** 46, a_gain=2.0 ** 38),
+                                  dict(v_gain=2.0 ** -60)], ids=["peaked", "spread", "large", "saturated", "wide_scales", "tiny_scales"])
+def test_decode_quantiser_ranges(F, what):
+    """Both sides of every line that the exponential and the quantiser draw (as in the prompt kernel's test), with lengths on both sides
+    of a block of the ordered sums, equal lengths, and the longest sequence neither first nor last."""
+    decode_case(F, 7, [62, 126, 127, 700, 62, 0, 255], seed=46, **what)
 
 
 def test_kv_append_alone(F):
