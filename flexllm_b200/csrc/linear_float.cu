@@ -1,6 +1,8 @@
 // Linear layers of the floating-point model path apart from the tcgen05 GEMMs (gemm_bf16.cu), and the choice between the
 // forms: a weight-streaming GEMV for one or two tokens (T = bf16 or float activations, bf16 weights), its warp-MMA form for
 // more, and a tiled fp32 GEMM for the 32-bit mode.
+#include <atomic>
+
 #include "float_common.cuh"
 
 namespace flexllm {
@@ -135,62 +137,84 @@ __global__ void __launch_bounds__(128) gemv_float_kernel(const T* __restrict__ a
 }
 
 // A few tokens, bf16: weight streaming with warp-level bf16 MMAs. A CTA takes RT blocks of 16 weight rows (the MMA's row side;
-// GLU: one gate and one up block), its eight warps share K; the tokens are the column side, NT blocks of 8. Rows of both
-// operands are read straight from memory with 16-byte loads: lane % 4 holds elements 8 c .. 8 c + 7 of every 32, i.e. the inner
-// index is permuted, the same way on both sides. The warps' partial sums are added in warp order.
-template <int NT, int RT, bool GLU>
+// GLU: one gate and one up block), its eight warps share K; the tokens are the column side, NT blocks of 8. A 16-byte vector of
+// a row goes to one lane: lane % 4 holds elements 8 c .. 8 c + 7 of every 32, i.e. the inner index is permuted, the same way on
+// both sides. Every lane copies its own vectors (cp.async) into a ring of DEPTH 32-element chunks and reads them back
+// itself, so nothing but its own copies is waited for; the weights of the first DEPTH chunks are asked for before the kernels
+// in front of this one have finished. The warps' partial sums are added in warp order.
+// Bound by memory latency at these sizes: a step of the earlier form (one chunk group ahead in registers, activations fetched when
+// needed) cost a full round trip to L2 on top of the weights'. Requests of 4 x (200 + 48) tokens at the sizes of a 1B model:
+// Pibidra 49.1 -> 45.1 ms, Sabisun 49.6 -> 43.9 ms.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const bf16* src, bool live) {       // not live: 16 zero bytes, src is not read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <int NT, int RT, bool GLU, int DEPTH>
 __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict__ a, long lda, const bf16* __restrict__ w, long ldw,
                                                          const float* __restrict__ bias, int M, int N, int kv, int relu2, float* y32, bf16* y16, long ldy) {
-    constexpr int G = NT * RT >= 4 ? 2 : 4;                 // 32-element chunks per step
+    constexpr int ITEMS = RT * 2 + NT;                      // vectors of a lane per chunk
+    extern __shared__ __align__(16) uint8_t ring_raw[];     // [8 warps][DEPTH][ITEMS][32 lanes] vectors
     __shared__ float part[8][RT * 16][NT * 8 + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
     const int row0 = blockIdx.x * RT * 16;
     const int n_ch = (kv + 3) >> 2;                         // kv: 8-element vectors per row
     const int c_beg = (int)((long)warp * n_ch / 8), c_end = (int)((long)(warp + 1) * n_ch / 8);
-    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4* mine = reinterpret_cast<uint4*>(ring_raw) + (warp * DEPTH * ITEMS) * 32 + lane;
+    const uint32_t mine_u = (uint32_t)__cvta_generic_to_shared(mine);
     const bf16* wr[RT][2];
 #pragma unroll
     for (int r = 0; r < RT; r++)
 #pragma unroll
         for (int h = 0; h < 2; h++) wr[r][h] = w + (long)min(row0 + r * 16 + h * 8 + lr, N - 1) * ldw + lc * 8;
-    uint4 wv[G][RT][2], nx[G][RT][2];
-    auto load_w = [&](uint4 (&v)[G][RT][2], int c) {
+    const bf16* ar[NT];
 #pragma unroll
-        for (int g = 0; g < G; g++)
+    for (int t = 0; t < NT; t++) ar[t] = a + (long)min(t * 8 + lr, M - 1) * lda + lc * 8;
+    auto load_w = [&](int c, int slot) {
+        const bool live = c < c_end && c * 4 + lc < kv;
 #pragma unroll
-            for (int r = 0; r < RT; r++)
+        for (int r = 0; r < RT; r++)
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                    v[g][r][h] = (c + g < c_end && (c + g) * 4 + lc < kv) ? ldg_stream16(wr[r][h] + (long)(c + g) * 32) : zero;
+            for (int h = 0; h < 2; h++) cp_async16(mine_u + (slot * ITEMS + r * 2 + h) * 512, live ? wr[r][h] + (long)c * 32 : w, live);
     };
-    load_w(nx, c_beg);
+    auto load_a = [&](int c, int slot) {
+        const bool live = c < c_end && c * 4 + lc < kv;
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            const bool on = live && t * 8 + lr < M;
+            cp_async16(mine_u + (slot * ITEMS + RT * 2 + t) * 512, on ? ar[t] + (long)c * 32 : a, on);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < DEPTH; i++) load_w(c_beg + i, i);
     pdl_sync();
+#pragma unroll
+    for (int i = 0; i < DEPTH; i++) { load_a(c_beg + i, i); cp_async_commit(); }      // the first of these groups holds all the weights too
     float acc[RT][NT][4] = {};
-    for (int c = c_beg; c < c_end; c += G) {
+    int slot = 0;
+    for (int c = c_beg; c < c_end; c++) {
+        cp_async_wait<DEPTH - 1>();
+        uint4 wv[RT][2], av[NT];
 #pragma unroll
-        for (int g = 0; g < G; g++)
+        for (int r = 0; r < RT; r++)
 #pragma unroll
-            for (int r = 0; r < RT; r++)
+            for (int h = 0; h < 2; h++) wv[r][h] = mine[(slot * ITEMS + r * 2 + h) * 32];
 #pragma unroll
-                for (int h = 0; h < 2; h++) wv[g][r][h] = nx[g][r][h];
-        uint4 av[G][NT];
+        for (int t = 0; t < NT; t++) av[t] = mine[(slot * ITEMS + RT * 2 + t) * 32];
 #pragma unroll
-        for (int g = 0; g < G; g++)
+        for (int r = 0; r < RT; r++)
 #pragma unroll
-            for (int t = 0; t < NT; t++)
-                av[g][t] = (t * 8 + lr < M && c + g < c_end && (c + g) * 4 + lc < kv)
-                               ? *reinterpret_cast<const uint4*>(a + (long)(t * 8 + lr) * lda + (long)(c + g) * 32 + lc * 8) : zero;
-        load_w(nx, c + G);
-#pragma unroll
-        for (int g = 0; g < G; g++)
-#pragma unroll
-            for (int r = 0; r < RT; r++)
-#pragma unroll
-                for (int t = 0; t < NT; t++) {
-                    mma_bf16(acc[r][t], wv[g][r][0].x, wv[g][r][1].x, wv[g][r][0].y, wv[g][r][1].y, av[g][t].x, av[g][t].y);
-                    mma_bf16(acc[r][t], wv[g][r][0].z, wv[g][r][1].z, wv[g][r][0].w, wv[g][r][1].w, av[g][t].z, av[g][t].w);
-                }
+            for (int t = 0; t < NT; t++) {
+                mma_bf16(acc[r][t], wv[r][0].x, wv[r][1].x, wv[r][0].y, wv[r][1].y, av[t].x, av[t].y);
+                mma_bf16(acc[r][t], wv[r][0].z, wv[r][1].z, wv[r][0].w, wv[r][1].w, av[t].z, av[t].w);
+            }
+        load_w(c + DEPTH, slot);                            // the vectors above are in registers: their slot is free
+        load_a(c + DEPTH, slot);
+        cp_async_commit();
+        if (++slot == DEPTH) slot = 0;
     }
+    cp_async_wait<0>();
 #pragma unroll
     for (int r = 0; r < RT; r++)
 #pragma unroll
@@ -217,13 +241,29 @@ __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict_
     }
 }
 
+template <int NT, int RT, bool GLU, int DEPTH>
+int launch_skinny(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int kv, int relu2, LinearOut y, cudaStream_t st) {
+    auto kern = skinny_mma_kernel<NT, RT, GLU, DEPTH>;
+    constexpr int smem = 8 * DEPTH * (RT * 2 + NT) * 512;
+    static std::atomic<bool> attr_set[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0) return FLEXLLM_ECUDA;
+    if (!attr_set[dev].load(std::memory_order_acquire)) {
+        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_set[dev].store(true, std::memory_order_release);
+    }
+    launch_k(kern, dim3((N + RT * 16 - 1) / (RT * 16)), dim3(256), smem, st, a, lda, w, ldw, bias, M, N, kv, relu2, y.f32, (bf16*)y.t, y.ld);
+    return launch_status();
+}
+// Depth of the ring: about 74 KB a CTA, so that three share an SM; twice that where the grid leaves one CTA an SM at most.
 template <int NT>
 int skinny_nt(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     const int kv = (K + 7) / 8, r2 = act == kActRelu2;
-    if (act == kActGeluGate) launch_k(skinny_mma_kernel<NT, 2, true>, dim3((N + 31) / 32), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
-    else if (N >= 148 * 4 * 16) launch_k(skinny_mma_kernel<NT, 2, false>, dim3((N + 31) / 32), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
-    else launch_k(skinny_mma_kernel<NT, 1, false>, dim3((N + 15) / 16), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
-    return launch_status();
+    constexpr int D1 = 18 / (2 + NT), D2 = NT == 4 ? 2 : 3;
+    if (act == kActGeluGate) return launch_skinny<NT, 2, true, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
+    if (N >= 148 * 4 * 16) return launch_skinny<NT, 2, false, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
+    if ((N + 15) / 16 <= 148) return launch_skinny<NT, 1, false, 2 * D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
+    return launch_skinny<NT, 1, false, D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
 }
 int skinny_mma(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     if (M <= 8) return skinny_nt<1>(a, lda, w, ldw, bias, M, N, K, act, y, st);

@@ -56,6 +56,21 @@ def test_linear(F, dtype, N, K):
         assert np.abs(got - (want - b)).max() < tol * np.abs(want).max(), M
 
 
+@pytest.mark.parametrize("N,K", [(2368, 3000), (2384, 3000), (9456, 520), (9472, 264), (40, 8), (2048, 8200)])
+def test_linear_few_tokens_ring(F, N, K):
+    """A few tokens on both sides of the rules that choose the ring's depth and the rows of a CTA, with fewer chunks than the ring holds
+    and with many more, and a ragged last chunk. Bounds as in test_linear."""
+    g = np.random.default_rng(K)
+    w = bf16_round(g.standard_normal((N, K)) * K ** -0.5)
+    b = g.standard_normal(N).astype(np.float32)
+    wd, bd = padded(w, up(K, 8), torch.bfloat16), torch.from_numpy(b).cuda()
+    for M in (2, 8, 9, 16, 17, 32):
+        a = bf16_round(g.standard_normal((M, K)))
+        want = P.linear(w.astype(np.float64), a.astype(np.float64), b)
+        got = F.linear_float(padded(a, up(K, 8), torch.bfloat16), wd, bd, K=K, out_f32=True).cpu().numpy()
+        assert np.abs(got - want).max() < 2e-5 * np.abs(want).max(), (M, np.abs(got - want).max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("ff,K", [(16, 64), (80, 90), (368, 512), (4096, 1024)])
 def test_gated_gelu_linear(F, dtype, ff, K):
