@@ -14,8 +14,10 @@
 //   prefill : A = activations [M][K], B = weights [N][K]            out[rowA][rowB]
 //   decode  : A = weights [N][K],     B = activations [M<=64][K]     out[rowB][rowA]   (SWAP)
 // so that a handful of tokens still fills the 128-row dimension of the tensor core with weight
-// rows and the weight matrix is streamed exactly once. With split-K (decode) partial sums are added
-// into a zeroed int32 buffer with red.global.add (integer addition is exact and order-free).
+// rows and the weight matrix is streamed exactly once. With split-K (decode) the splits of a tile form a thread-block
+// cluster: each CTA leaves its int32 partial tile in shared memory and the cluster's CTAs add them, a share of the tokens
+// each, over distributed shared memory. (Adding into a buffer in global memory, with the last arriver reading it back, took
+// 26 us for 64 tokens of 2048 x 8192.) The allocation-free entry point keeps the form that adds into a zeroed buffer.
 //
 // Replaces pref_Linear_Layer_i4xi4 / dec_Linear_Layer_i4xi4 + the dequant layers
 // (Modules/Linear_Layer.h:293-341, :862-923; Modules/quant.h:115-164, :434-524) at 8-bit precision.
@@ -108,16 +110,14 @@ struct GemmArgs {
     int rowsA, rowsB, K;     // A side (128-row tiles), B side (BN-row tiles), reduction length
     int tilesA, tilesB, ksplit;
     int ldo;                 // leading dimension of the outputs
-    int32_t* acc;            // optional int32 output (required when ksplit > 1: added atomically)
-    float* y;                // optional fp32 output (ignored when ksplit > 1)
+    int32_t* acc;            // optional int32 output (required when ksplit > 1 without a cluster: added atomically)
+    float* y;                // optional fp32 output (ignored in that case)
     const float* sA;         // per-row scale of the A side
     const float* sB;         // per-row scale of the B side
     int* error_flag;         // set to 1 if a device-side wait ran out
     // fused epilogue extras
     const float* residual;   // optional: y = residual + dequant (same layout as y)
-    int32_t* work;           // split-K: zeroed int32 partial-sum buffer [rowsB][ldo]; the last arriver
-                             // turns it into the outputs and leaves it zeroed again
-    int* counters;           // split-K: zeroed arrival counters, one per (A tile, warp quarter)
+    int cluster;             // split-K: the splits of a tile are a thread-block cluster (else they add into acc)
 };
 
 // KCH = 128-byte K chunks per pipeline stage (1 for prefill; > 1 for the weight-streaming decode
@@ -413,13 +413,19 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
                     }
                 } else {
                     // out[colB0 + j][rowA]: token = colB, channel = rowA; a warp store covers 32 channels
+                    if (args.cluster) {
+                        int* part = reinterpret_cast<int*>(ring_ptr);        // the MMAs have finished reading the ring
+#pragma unroll
+                        for (int j = 0; j < 16; j++) part[(c * 16 + j) * 128 + q * 32 + lane] = (int)v[j];
+                        continue;
+                    }
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
                         const int tok = colB0 + j;
                         if (rowA_ok && tok < args.rowsB) {
                             const long o = (long)tok * args.ldo + rowA;
                             if (args.ksplit > 1) {
-                                atomicAdd((args.work ? args.work : args.acc) + o, (int)v[j]);
+                                atomicAdd(args.acc + o, (int)v[j]);
                             } else {
                                 if (args.acc) args.acc[o] = (int)v[j];
                                 if (args.y) {
@@ -436,53 +442,36 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_tempty + 8 * as);
-            if (SWAP && args.ksplit > 1 && args.work) {
-                // split-K with fused finalisation: the warp that arrives last on this (tile, quarter)
-                // reads the complete integer sums, writes the outputs and re-zeroes the work buffer
-                __threadfence();
-                int last = 0;
-                if (lane == 0) last = (atomicAdd(args.counters + ta * 4 + q, 1) == args.ksplit - 1);
-                last = __shfl_sync(0xffffffffu, last, 0);
-                if (last) {
-                    __threadfence();
-                    if (rowA_ok) {
-                        // batches of 16 tokens: the loads of a batch are independent, so their
-                        // L2 latencies overlap
-                        for (int t0 = 0; t0 < args.rowsB; t0 += 16) {
-                            int vv[16];
+        }
+    }
+
+    if (SWAP && args.cluster) {
+        // one tile per CTA, the same for the CTAs of a cluster; CTA r adds up tokens r, r + ksplit, ...
+        tc_fence_before();
+        cluster_sync();
+        if (warp >= 2 && !*abort_flag) {
+            const int q = warp & 3, ta = blockIdx.x / args.ksplit, r = blockIdx.x % args.ksplit;
+            const int rowA = ta * 128 + q * 32 + lane;
+            if (rowA < args.rowsA) {
+                const float sa = args.sA ? args.sA[rowA] : 0.0f;
+                for (int tok = r; tok < args.rowsB; tok += args.ksplit) {
+                    const long o = (long)tok * args.ldo + rowA;
+                    const float rs = args.residual ? args.residual[o] : 0.0f;
+                    int p[8];
 #pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const int tok = t0 + j;
-                                vv[j] = tok < args.rowsB ? __ldcg(args.work + (long)tok * args.ldo + rowA) : 0;
-                            }
-                            float rs[16];
-                            if (args.residual) {
-#pragma unroll
-                                for (int j = 0; j < 16; j++) {
-                                    const int tok = t0 + j;
-                                    rs[j] = tok < args.rowsB ? args.residual[(long)tok * args.ldo + rowA] : 0.0f;
-                                }
-                            }
-#pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const int tok = t0 + j;
-                                if (tok < args.rowsB) {
-                                    const long o = (long)tok * args.ldo + rowA;
-                                    args.work[o] = 0;
-                                    if (args.acc) args.acc[o] = vv[j];
-                                    if (args.y) {
-                                        float r = ((float)vv[j] * args.sB[tok]) * sa;   // L1/L2 hit: fetched before the wait
-                                        if (args.residual) r = rs[j] + r;
-                                        args.y[o] = r;
-                                    }
-                                }
-                            }
-                        }
+                    for (int k = 0; k < 8; k++)
+                        p[k] = k < args.ksplit ? __float_as_int(ld_cluster_f32(cluster_addr(ring + (uint32_t)(tok * 128 + q * 32 + lane) * 4u, k))) : 0;
+                    const int t = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+                    if (args.acc) args.acc[o] = t;
+                    if (args.y) {
+                        float v = ((float)t * args.sB[tok]) * sa;
+                        if (args.residual) v = rs + v;
+                        args.y[o] = v;
                     }
-                    if (lane == 0) args.counters[ta * 4 + q] = 0;
                 }
             }
         }
+        cluster_sync();                      // nobody leaves while its partial tile may still be read
     }
 
     // ---------------------------------------------------------------- tear-down
@@ -695,7 +684,7 @@ static int sm_count() {
 template <int BN, bool SWAP, int KCH = 1>
 static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, int K, int ksplit, int ldo,
                        int32_t* acc, float* y, const float* sA, const float* sB, cudaStream_t st,
-                       const float* residual = nullptr, int32_t* work = nullptr, int* counters = nullptr) {
+                       const float* residual = nullptr) {
     using Cfg = GemmCfg<BN, KCH>;
     CUtensorMap ta, tb;
     int rc = cached_tmap(&ta, A, (uint64_t)rowsA, (uint64_t)K, 128, KCH > 1 ? KCH : 0);
@@ -706,7 +695,7 @@ static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, i
     g.rowsA = rowsA; g.rowsB = rowsB; g.K = K;
     g.tilesA = (rowsA + 127) / 128; g.tilesB = (rowsB + BN - 1) / BN; g.ksplit = ksplit;
     g.ldo = ldo; g.acc = acc; g.y = y; g.sA = sA; g.sB = sB; g.error_flag = device_error_flag();
-    g.residual = residual; g.work = work; g.counters = counters;
+    g.residual = residual; g.cluster = SWAP && ksplit > 1;
     auto kern = gemm_i8_tcgen05_kernel<BN, SWAP, KCH>;
     // the attribute belongs to (function, device): once per device, not once per process
     static std::atomic<bool> attr_set[kMaxDevices];
@@ -717,6 +706,10 @@ static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, i
         attr_set[dev].store(true, std::memory_order_release);
     }
     const int total = g.tilesA * g.tilesB * g.ksplit;
+    if (g.cluster) {                       // one tile per CTA (tilesB is 1)
+        launch_cluster(kern, dim3(total), dim3(192), ksplit, (size_t)Cfg::SMEM_BYTES, st, ta, tb, g);
+        return launch_status();
+    }
     const int grid = total < sm_count() ? total : sm_count();
     launch_k(kern, dim3(grid), dim3(192), (size_t)Cfg::SMEM_BYTES, st, ta, tb, g);
     return launch_status();
@@ -733,7 +726,7 @@ static int launch_gemm_pair(const int8_t* a, const float* s_tok, const int8_t* w
     g.rowsA = M; g.rowsB = N; g.K = K;
     g.tilesA = (M + 255) / 256; g.tilesB = (N + GP_BN - 1) / GP_BN; g.ksplit = 1;
     g.ldo = N; g.acc = acc; g.y = y; g.sA = s_tok; g.sB = s_ch; g.error_flag = device_error_flag();
-    g.residual = residual; g.work = nullptr; g.counters = nullptr;
+    g.residual = residual; g.cluster = 0;
     static std::atomic<bool> attr_set[kMaxDevices];
     const int dev = current_device();
     if (dev < 0) return FLEXLLM_ECUDA;
@@ -768,22 +761,20 @@ int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const 
     return launch_gemm<16, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
 }
 
-// Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side, optional split-K.
-// With ksplit > 1 the partial sums go through `work` (zeroed int32 [M][N]) and `counters` (zeroed,
-// 4 per 128-channel tile); the last-arriving warp writes acc / y (+ residual) and re-zeroes both.
+// Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side. K is split over clusters of up to eight CTAs as
+// long as the tiles leave half the SMs idle and every split keeps two 128-byte blocks.
 int gemm_i8_decode(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
-                   int ksplit, int32_t* acc, float* y, cudaStream_t st, const float* residual, int32_t* work, int* counters) {
+                   int32_t* acc, float* y, cudaStream_t st, const float* residual) {
     if (M > 64) return FLEXLLM_ENOTSUP;
-    // chunks of K per pipeline stage: KCH*128 contiguous bytes per weight row and TMA request
+    const int tiles = (N + 127) / 128, kb = (K + 127) / 128;
+    int ksplit = 1;
+    while (ksplit < 8 && tiles * ksplit * 2 <= sm_count() && kb >= 4 * ksplit) ksplit *= 2;
+    // chunks of K per pipeline stage: KCH*128 contiguous bytes per weight row and TMA request, two steps per split
     int kch = 1;
-    if (K % 512 == 0) kch = 4;
-    else if (K % 256 == 0) kch = 2;
-    const int steps = (K + 127) / 128 / kch;
-    if (ksplit > steps) ksplit = steps;
-    if (ksplit < 1) ksplit = 1;
-    if (ksplit > 1 && !(work && counters)) return FLEXLLM_EINVAL;
+    if (K % 512 == 0 && kb / 4 >= 2 * ksplit) kch = 4;
+    else if (K % 256 == 0 && kb / 2 >= 2 * ksplit) kch = 2;
 #define FLEXLLM_DEC(BN_, KCH_) \
-    return launch_gemm<BN_, true, KCH_>(w, N, a, M, K, ksplit, N, acc, y, s_ch, s_tok, st, residual, work, counters)
+    return launch_gemm<BN_, true, KCH_>(w, N, a, M, K, ksplit, N, acc, y, s_ch, s_tok, st, residual)
     if (M > 32) { if (kch == 4) FLEXLLM_DEC(64, 4); if (kch == 2) FLEXLLM_DEC(64, 2); FLEXLLM_DEC(64, 1); }
     if (M > 16) { if (kch == 4) FLEXLLM_DEC(32, 4); if (kch == 2) FLEXLLM_DEC(32, 2); FLEXLLM_DEC(32, 1); }
     if (kch == 4) FLEXLLM_DEC(16, 4);
@@ -831,7 +822,7 @@ static int launch_gemm_noalloc(const int8_t* w, int N, const int8_t* a, int M, i
     g.rowsA = N; g.rowsB = M; g.K = K;
     g.tilesA = (N + 127) / 128; g.tilesB = 1; g.ksplit = ksplit;
     g.ldo = N; g.acc = acc; g.y = nullptr; g.sA = nullptr; g.sB = nullptr; g.error_flag = flag;
-    g.residual = nullptr; g.work = nullptr; g.counters = nullptr;
+    g.residual = nullptr; g.cluster = 0;
     auto kern = gemm_i8_tcgen05_kernel<BN, true>;
     static std::atomic<bool> attr_set[kMaxDevices];
     const int dev = current_device();

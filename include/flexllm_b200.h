@@ -82,10 +82,7 @@ FLEXLLM_API int flexllm_linear_prefill_i8(const int8_t* a, const float* s_tok, c
                               int M, int N, int K, int32_t* acc, float* y, void* stream);
 FLEXLLM_API int flexllm_linear_decode_i8(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch,
                              int M, int N, int K, int32_t* acc, float* y, void* stream);
-/* Library-owned state of the decode layer (9..64 tokens): its split-K partial sums go through ONE scratch
- * buffer per device (32 MiB, allocated by the first such call on the device and kept until the process
- * exits -- make that call outside any stream capture). Calls on one stream share it safely; calls that can
- * overlap on the GPU (different streams of one device) would mix their partial sums: serialise them. */
+/* The decode layer keeps no state between calls: split-K partial sums are added inside a thread-block cluster. */
 
 /* The same two layers fused with the residual add that follows them in the model
  * (pref_Residual_Layer / dec_Residual_Layer, Residual_Layer.h:46-87): y = residual + dequant(acc).
