@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
         const bool in = row0 + w < M;
         const float4* src = reinterpret_cast<const float4*>(x + (row0 + w) * D);
         float4* dst = reinterpret_cast<float4*>(rows_sm + w * ld);
+#pragma unroll 8
         for (int c = lane; c < nv; c += 32) dst[c] = in ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
@@ -213,8 +214,26 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
         const int rr = lane >> 2, j = lane & 3;      // chain (row rr, residue j)
         const float* src = rows_sm + rr * ld + j;
         float ss = 0.0f;
-#pragma unroll 8
-        for (int k = 0; k < nv; k++) { const float v = src[4 * k]; ss += v * v; }
+        // blocks of 16 elements, the next block's loads under way while this one is added: a step then costs the
+        // addition's latency alone
+        constexpr int UB = 16;
+        float cur[UB], nxt[UB];
+        const int blocks = nv / UB;
+        if (blocks > 0) {
+#pragma unroll
+            for (int i = 0; i < UB; i++) cur[i] = src[4 * i];
+        }
+#pragma unroll 2
+        for (int bk = 0; bk < blocks; bk++) {
+            const float* at = src + 4 * UB * (bk + 1 < blocks ? bk + 1 : bk);
+#pragma unroll
+            for (int i = 0; i < UB; i++) nxt[i] = at[4 * i];
+#pragma unroll
+            for (int i = 0; i < UB; i++) ss += cur[i] * cur[i];
+#pragma unroll
+            for (int i = 0; i < UB; i++) cur[i] = nxt[i];
+        }
+        for (int k = blocks * UB; k < nv; k++) { const float v = src[4 * k]; ss += v * v; }
         // (p0+p1)+(p2+p3) inside each group of four lanes
         const int base = lane & ~3;
         const float p0 = __shfl_sync(0xffffffffu, ss, base), p1 = __shfl_sync(0xffffffffu, ss, base + 1);
@@ -231,33 +250,35 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
     float4* yr = y ? reinterpret_cast<float4*>(y + row * D) : nullptr;
     // first pass: the normalised row's largest magnitude (max(|max|, |min|) of the row = max of |.|), fp32 output if asked for;
     // second pass: the same products again (same bits) and the quantiser -- nothing of the row is held in registers
-    float amax = 0.0f;
+    float amax = 0.0f, nan = 0.0f;
+    const f32x2 r2 = pack2(r, r);
+    auto normed = [&](int c, float (&o)[4]) {
+        const float4 v = xr[c], g = g4[c];
+        unpack2(mul2(mul2(pack2(v.x, v.y), r2), pack2(g.x, g.y)), o[0], o[1]);
+        unpack2(mul2(mul2(pack2(v.z, v.w), r2), pack2(g.z, g.w)), o[2], o[3]);
+    };
 #pragma unroll 4
     for (int c = lane; c < nv; c += 32) {
-        const float4 v = xr[c], g = g4[c];
-        float4 o;
-        o.x = (v.x * r) * g.x; o.y = (v.y * r) * g.y; o.z = (v.z * r) * g.z; o.w = (v.w * r) * g.w;
-        if (yr) yr[c] = o;
-        amax = fmaxf(fmaxf(amax, fabsf(o.x)), fmaxf(fabsf(o.y), fmaxf(fabsf(o.z), fabsf(o.w))));
+        float o[4];
+        normed(c, o);
+        if (yr) yr[c] = make_float4(o[0], o[1], o[2], o[3]);
+        amax = max3(max3(amax, fabsf(o[0]), fabsf(o[1])), fabsf(o[2]), fabsf(o[3]));
+        nan = max3_nan(max3_nan(nan, o[0], o[1]), o[2], o[3]);
     }
     if (q) {
         amax = warp_max(amax);
-        float sc = amax / 127.0f;
-        if (sc == 0.0f) sc = 1.0f;
-        const DivBy dsc = div_by(sc);       // one reciprocal per row: every element is then quantised without a full division
+        const float sc = sym_scale_from(amax, -amax);
+        const bool ok = __all_sync(0xffffffffu, nan == nan) && sc >= 0x1p-60f && sc <= 0x1p60f;
+        const float w8 = 1.0f / sc;         // one reciprocal per row
         if (lane == 0) s[row] = sc;
-        char4* qr = reinterpret_cast<char4*>(q + row * D);
-        auto q8 = [&](float t) {            // round half away from zero of the correctly rounded quotient; |quotient| <= 127
-            const float qt = div_for_rounding(t, dsc);
-            const int m = __float2int_rz(__fadd_rd(fabsf(qt), 0.5f));
-            return (int8_t)(qt < 0.0f ? -m : m);
-        };
+        uint32_t* qr = reinterpret_cast<uint32_t*>(q + row * D);
 #pragma unroll 4
         for (int c = lane; c < nv; c += 32) {
-            const float4 v = xr[c], g = g4[c];
-            char4 v4;
-            v4.x = q8((v.x * r) * g.x); v4.y = q8((v.y * r) * g.y); v4.z = q8((v.z * r) * g.z); v4.w = q8((v.w * r) * g.w);
-            qr[c] = v4;
+            float o[4];
+            uint32_t b[4];
+            normed(c, o);
+            q8_short(o, w8, ok, b, [&](float t) { return q8_exact(t, sc); });
+            qr[c] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
         }
     }
 }
@@ -287,6 +308,81 @@ __global__ void __launch_bounds__(RMS_WARPS * 32) rmsnorm_decode_kernel(const fl
     rmsnorm_decode_row<MAXV, KEEP_G>(v, g, gamma, D, eps, lanes, buf, lane, y ? y + row * D : nullptr, q ? q + row * D : nullptr,
                                      s ? s + row : nullptr);
 }
+
+// The same for few rows: one CTA per row, so that the loads, the normalised values and the quantiser are spread over eight warps
+// and only the ordered sums stay on one (a warp that does everything takes 64 values a lane one after another).
+template <int MAXV>
+__global__ void __launch_bounds__(256) rmsnorm_decode_cta_kernel(const float* __restrict__ x, const float* __restrict__ gamma, int D, float eps,
+                                                                 int lanes, float* __restrict__ y, int8_t* __restrict__ q, float* __restrict__ s) {
+    extern __shared__ __align__(16) float rowbuf[];          // D + 4*lanes
+    __shared__ float rinv_sm, red[8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const long row = blockIdx.x;
+    const int nv = D >> 2, C = D / lanes;
+    const float4* gr = reinterpret_cast<const float4*>(gamma);
+    float4 v[MAXV], g[MAXV];
+    pdl_wait();            // before the kernels after this one may start: they ask for weights at once (see the MLP block)
+    pdl_launch();
+#pragma unroll
+    for (int i = 0; i < MAXV; i++) {
+        const int c = tid + i * 256;
+        v[i] = g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < nv) {
+            v[i] = reinterpret_cast<const float4*>(x + row * D)[c];
+            g[i] = gr[c];
+            *reinterpret_cast<float4*>(rowbuf + c * 4 + 4 * (c * 4 / C)) = v[i];      // element e at e + 4*(e / C)
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int chunk = lane >> 2, j = lane & 3;
+        float ss = 0.0f;
+        if (chunk < lanes) {
+            const float* bc = rowbuf + chunk * (C + 4) + j;
+            const int n = C >> 2;
+#pragma unroll 16
+            for (int k = 0; k < n; k++) { const float t = bc[4 * k]; ss += t * t; }
+        }
+        float tot = 0.0f;
+        for (int c = 0; c < lanes; c++) {
+            const float p0 = __shfl_sync(0xffffffffu, ss, c * 4 + 0), p1 = __shfl_sync(0xffffffffu, ss, c * 4 + 1);
+            const float p2 = __shfl_sync(0xffffffffu, ss, c * 4 + 2), p3 = __shfl_sync(0xffffffffu, ss, c * 4 + 3);
+            tot += (p0 + p1) + (p2 + p3);
+        }
+        if (lane == 0) rinv_sm = 1.0f / sqrtf(tot / (float)D + eps);
+    }
+    __syncthreads();
+    const float r = rinv_sm;
+    float o[4 * MAXV], mx = 0.0f, nan = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MAXV; i++) {
+        const int c = tid + i * 256;
+        const bool in = c < nv;
+        o[4 * i] = in ? (v[i].x * r) * g[i].x : 0.0f; o[4 * i + 1] = in ? (v[i].y * r) * g[i].y : 0.0f;
+        o[4 * i + 2] = in ? (v[i].z * r) * g[i].z : 0.0f; o[4 * i + 3] = in ? (v[i].w * r) * g[i].w : 0.0f;
+        if (in && y) reinterpret_cast<float4*>(y + row * D)[c] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) { mx = fmaxf(mx, fabsf(o[4 * i + k])); nan = max3_nan(nan, nan, o[4 * i + k]); }
+    }
+    if (!q) return;
+    mx = warp_max(mx);
+    if (lane == 0) red[warp] = mx;
+    const int bad = __syncthreads_or(!(nan == nan));
+#pragma unroll
+    for (int w = 0; w < 8; w++) mx = fmaxf(mx, red[w]);
+    const float sc = sym_scale_from(mx, -mx);
+    if (tid == 0) s[row] = sc;
+    uint32_t b[4 * MAXV];
+    q8_short(o, 1.0f / sc, !bad && sc >= 0x1p-60f && sc <= 0x1p60f, b, [&](float t) { return q8_exact(t, sc); });
+#pragma unroll
+    for (int i = 0; i < MAXV; i++) {
+        const int c = tid + i * 256;
+        if (c < nv)
+            reinterpret_cast<uint32_t*>(q + row * D)[c] =
+                __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
+    }
+}
+constexpr int RMS_CTA_ROWS = 4 * 148;      // up to four CTAs an SM
 
 // ---------------------------------------------------------------------------------------------
 // SiLU / gate / residual (Swish.h:19, Linear_Layer.h:626, Residual_Layer.h:61)
@@ -535,6 +631,9 @@ extern "C" int flexllm_rmsnorm_quant(const float* x, const float* gamma, int M, 
             attr_done[dev].store(1, std::memory_order_release);
         }
         rmsnorm_prefill_kernel<<<grid, RMSP_ROWS * 32, smem, st>>>(x, gamma, M, D, eps, y, q, s);
+    } else if (M <= RMS_CTA_ROWS) {
+        const size_t smem = (size_t)(D + 4 * order) * sizeof(float);
+        launch_k(D <= 2048 ? rmsnorm_decode_cta_kernel<2> : rmsnorm_decode_cta_kernel<4>, dim3(M), dim3(256), smem, st, x, gamma, D, eps, order, y, q, s);
     } else {
         const int grid = (M + RMS_WARPS - 1) / RMS_WARPS;
         const size_t smem = (size_t)RMS_WARPS * (D + 4 * order) * sizeof(float);

@@ -94,10 +94,10 @@ extern "C" int flexllm_mlp_block_decode(const float* x, const float* gamma, cons
     float* gu = (float*)w; w += up256((size_t)M * 2 * F * 4);
     int8_t* hq = (int8_t*)w;
     cudaStream_t st = (cudaStream_t)stream;
-    // The first launch is an ordinary one: it starts when everything before it in the stream has completed, and the products, which
-    // ask for their weights without waiting, start after it. A caller's kernel may have written those weights just before.
-    TRY_RC(flexllm_rmsnorm_quant(x, gamma, M, D, eps, order, nullptr, xq, xs, st));
+    // The products ask for their weights without waiting, and a caller's kernel may have written those just before: the first
+    // kernel therefore lets the others start only when everything before it in the stream has completed.
     struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    TRY_RC(flexllm_rmsnorm_quant(x, gamma, M, D, eps, order, nullptr, xq, xs, st));
     TRY_RC(linear_decode(xq, xs, w_gu, s_gu, M, 2 * F, D, nullptr, gu, nullptr, st));
     TRY_RC(swiglu_fht_quant_strided(gu, gu + F, 2L * F, M, fht_scale, hq, hs, st));
     return linear_decode(hq, hs, w_d, s_d, M, D, F, nullptr, y, x, st);

@@ -181,6 +181,18 @@ def test_softmax_summation_order_is_the_reference(F):
 
 
 # ------------------------------------------------------------------------------ RMSNorm
+@pytest.mark.parametrize("order,M,D", [(8, 1, 2048), (4, 592, 512), (8, 593, 512), (8, 3, 4096), (4, 5, 96), (0, 9, 2048), (0, 5, 3968), (0, 3, 128)])
+def test_rmsnorm_forms(F, order, M, D):
+    """Row counts on both sides of the rule between the decode forms, widths that do not fill the last block of the sums."""
+    g = rng(90)
+    x = (g.standard_normal((M, D)) * 3).astype(np.float32); gamma = (1 + 0.1 * g.standard_normal(D)).astype(np.float32)
+    x[0] *= np.float32(2.0) ** -62                            # normalised values far below the others
+    y, q, s = F.pref_Layer_Norm(dev(x), dev(gamma), 1e-5, order, quant=True)
+    yo = oracle.rmsnorm(x, gamma, 1e-5, order)
+    qo, so = oracle.quant_per_token(yo)
+    assert_same(to_np(y), yo, "y"); assert_same(to_np(s), so, "scale"); assert_same(to_np(q), qo, "q")
+
+
 @pytest.mark.parametrize("order", [0, 4, 8])
 @pytest.mark.parametrize("M", [1, 64, 130])
 def test_rmsnorm_quant(F, order, M):
