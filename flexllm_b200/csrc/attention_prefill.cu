@@ -27,7 +27,8 @@
 //
 // Bound: instruction issue of the softmax warps (60 % of the issue slots busy; double precision and the special-function
 // pipe 15 % each, DRAM idle). 4 prompts of 1024 tokens, 32 / 8 heads: 513 us with the exponentials of sweep 1 parked in a
-// scratch (568 MB written and read back through L2), separate fp32 operations and full divisions; 252 us now.
+// scratch (568 MB written and read back through L2), separate fp32 operations and full divisions; 240 us now (252 us with one
+// test per four values in sweep 2, and the rare forms inline).
 #include <cstdlib>
 
 #include "attention_decode.cuh"     // layout of the paged KV cache
@@ -180,19 +181,35 @@ constexpr int ATT_SMEM = ATT_Q_BYTES + ATT_SLOTS * ATT_TILE_BYTES + 2 * ATT_P_BY
 constexpr int ATT_TMEM_COLS = 128;
 constexpr int ATT_EXP_GROUP = 8;              // exponentials whose dependency chains interleave
 
-// The reference's arithmetic of one probability: U = min(round((e * r * vs) / a_s), 255) with e = exp(-u). Out of line: for the
-// values that sweep 2 cannot decide, and for scales outside the range of its error bound.
-__device__ __noinline__ static uint32_t attn_u8_exact(float u, float rinv, float vs, float a_s) {
-    const float p = ref_expf(-u) * rinv;
-    const int r = round_half_away_to_int((p * vs) / a_s);
-    return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
-}
-
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+
+// Sweep 2's decision on one probability (see there): the two sides of 255.25 t as rounded integers in the low bits, t the
+// approximate quotient / 255.25.
+constexpr float ATT_U8_HI = 255.25f * (1.0f + 0x1p-16f), ATT_U8_LO = 255.25f * (1.0f - 0x1p-16f), ATT_MAGIC = 12582912.0f;
+// One value of a group with an undecided one, or of a row or tile outside the range of the bound (fast false): the same
+// decision again, and where it does not hold the reference's arithmetic, U = min(round((e * r * vs) / a_s), 255), e = exp(-u).
+__device__ __noinline__ static uint32_t attn_u8_resolve(float u, float c_row, float rinv, float vs, float a_s, bool fast) {
+    if (fast) {
+        const float t = __saturatef(ex2_approx(__fmaf_rn(u, -1.4426950408889634f, c_row)) * vs);
+        const uint32_t h = __float_as_uint(__fmaf_rn(t, ATT_U8_HI, ATT_MAGIC));
+        if (h == __float_as_uint(__fmaf_rn(t, ATT_U8_LO, ATT_MAGIC))) return h;
+    }
+    const float p = ref_expf(-u) * rinv;
+    const int r = round_half_away_to_int((p * vs) / a_s);
+    return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
+}
+// Four exponentials exp(-u), any u >= 0 or NaN: out of line, for chunks with a key far below the row's maximum
+__device__ __noinline__ static float4 attn_exp_any(float4 u) {
+    const float x[4] = {-u.x, -u.y, -u.z, -u.w};
+    float e[4];
+    ref_expf_x4<true>(x, e);
+    return make_float4(e[0], e[1], e[2], e[3]);
+}
+
 __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_constant__ CUtensorMap tmapQ,
                                                               const __grid_constant__ CUtensorMap tmapK,
                                                               const __grid_constant__ CUtensorMap tmapV,
@@ -426,13 +443,14 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
                         for (int i = 0; i < ATT_EXP_GROUP; i++) e[i0 + i] = ee[i];
                     }
                 } else {                                       // a key far below the maximum (or NaN): the general form
+                    float near = u[0];
+#pragma unroll
+                    for (int i = 1; i < 16; i++) near = fminf(near, u[i]);
+                    const bool zero = __all_sync(0xffffffffu, near > 104.0f && far == far);     // exp(-104) rounds to 0
 #pragma unroll
                     for (int i4 = 0; i4 < 16; i4 += 4) {
-                        const float xx[4] = {-u[i4], -u[i4 + 1], -u[i4 + 2], -u[i4 + 3]};
-                        float ee[4];
-                        ref_expf_x4<true>(xx, ee);
-#pragma unroll
-                        for (int i = 0; i < 4; i++) e[i4 + i] = ee[i];
+                        const float4 ee = zero ? make_float4(0.f, 0.f, 0.f, 0.f) : attn_exp_any(make_float4(u[i4], u[i4 + 1], u[i4 + 2], u[i4 + 3]));
+                        e[i4] = ee.x; e[i4 + 1] = ee.y; e[i4 + 2] = ee.z; e[i4 + 3] = ee.w;
                     }
                 }
                 if (masked) {
@@ -459,9 +477,8 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
         const float c_row = log2f((rinv * inv_as) * (1.0f / 255.25f));
         const bool warp_ok = __all_sync(0xffffffffu, c_row >= -64.0f && c_row <= 32.0f);
         const f32x2 c2 = pack2(c_row, c_row), nlog2e = pack2(-1.4426950408889634f, -1.4426950408889634f);
-        const f32x2 hi2 = pack2(255.25f * (1.0f + 0x1p-16f), 255.25f * (1.0f + 0x1p-16f));
-        const f32x2 lo2 = pack2(255.25f * (1.0f - 0x1p-16f), 255.25f * (1.0f - 0x1p-16f));
-        const f32x2 magic2 = pack2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: adding it rounds to an integer, kept in the low bits
+        const f32x2 hi2 = pack2(ATT_U8_HI, ATT_U8_HI), lo2 = pack2(ATT_U8_LO, ATT_U8_LO);
+        const f32x2 magic2 = pack2(ATT_MAGIC, ATT_MAGIC);      // 1.5 * 2^23: adding it rounds to an integer, kept in the low bits
         for (int j = 0; ok && j < n_kt; j++) {
             const int pb = j & 1;
             const int k0 = j * ATT_KT;
@@ -480,37 +497,43 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
                 const int kc = k0 + c * 16;
                 f32x2 y[8];
                 scores16(kst, kc, c, y);
-                uint32_t packed[4];
+                uint32_t r[16], open = fast ? 0u : 1u;
+                float4 vs4[4];
 #pragma unroll
                 for (int i4 = 0; i4 < 4; i4++) {
-                    const float4 vs4 = (kc + 4 * i4 < S) ? *reinterpret_cast<const float4*>(vst + c * 16 + 4 * i4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const float vv[4] = {vs4.x, vs4.y, vs4.z, vs4.w};
-                    const f32x2 ua = fma2(y[2 * i4], neg8th, mx2), ub = fma2(y[2 * i4 + 1], neg8th, mx2);
-                    float arg[4], t[4];
-                    unpack2(fma2(ua, nlog2e, c2), arg[0], arg[1]);
-                    unpack2(fma2(ub, nlog2e, c2), arg[2], arg[3]);
+                    vs4[i4] = (kc + 4 * i4 < S) ? *reinterpret_cast<const float4*>(vst + c * 16 + 4 * i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float vv[4] = {vs4[i4].x, vs4[i4].y, vs4[i4].z, vs4[i4].w};
 #pragma unroll
-                    for (int i = 0; i < 4; i++) t[i] = __saturatef(ex2_approx(arg[i]) * vv[i]);
-                    const f32x2 ta = pack2(t[0], t[1]), tb = pack2(t[2], t[3]);
-                    float h[4], l[4];
-                    unpack2(fma2(ta, hi2, magic2), h[0], h[1]); unpack2(fma2(tb, hi2, magic2), h[2], h[3]);
-                    unpack2(fma2(ta, lo2, magic2), l[0], l[1]); unpack2(fma2(tb, lo2, magic2), l[2], l[3]);
-                    uint32_t r[4], open = fast ? 0u : 1u;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) { r[i] = __float_as_uint(h[i]); open |= r[i] ^ __float_as_uint(l[i]); }
-                    if (open) {
-                        float uu[4];
-                        unpack2(ua, uu[0], uu[1]); unpack2(ub, uu[2], uu[3]);
-#pragma unroll
-                        for (int i = 0; i < 4; i++)
-                            if (!fast || r[i] != __float_as_uint(l[i])) r[i] = attn_u8_exact(uu[i], rinv, vv[i], a_s);
+                    for (int i = 0; i < 4; i += 2) {
+                        float a0, a1, h0, h1, l0, l1;
+                        f32x2& yy = y[2 * i4 + (i >> 1)];
+                        yy = fma2(yy, neg8th, mx2);            // u = max - x
+                        unpack2(fma2(yy, nlog2e, c2), a0, a1);
+                        const f32x2 t = pack2(__saturatef(ex2_approx(a0) * vv[i]), __saturatef(ex2_approx(a1) * vv[i + 1]));
+                        unpack2(fma2(t, hi2, magic2), h0, h1);
+                        unpack2(fma2(t, lo2, magic2), l0, l1);
+                        r[4 * i4 + i] = __float_as_uint(h0); r[4 * i4 + i + 1] = __float_as_uint(h1);
+                        open |= (__float_as_uint(h0) ^ __float_as_uint(l0)) | (__float_as_uint(h1) ^ __float_as_uint(l1));
                     }
-                    if (masked) {
-#pragma unroll
-                        for (int i = 0; i < 4; i++) r[i] = (kc + 4 * i4 + i <= qlim) ? r[i] : 0u;
-                    }
-                    packed[i4] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
                 }
+                if (open) {
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        float u0, u1;
+                        unpack2(y[i >> 1], u0, u1);
+                        const float4 q = vs4[i >> 2];
+                        r[i] = attn_u8_resolve(u0, c_row, rinv, (i & 3) ? q.z : q.x, a_s, fast);
+                        r[i + 1] = attn_u8_resolve(u1, c_row, rinv, (i & 3) ? q.w : q.y, a_s, fast);
+                    }
+                }
+                if (masked) {
+#pragma unroll
+                    for (int i = 0; i < 16; i++) r[i] = (kc + i <= qlim) ? r[i] : 0u;
+                }
+                uint32_t packed[4];
+#pragma unroll
+                for (int i4 = 0; i4 < 4; i4++)
+                    packed[i4] = __byte_perm(__byte_perm(r[4 * i4], r[4 * i4 + 1], 0x0040), __byte_perm(r[4 * i4 + 2], r[4 * i4 + 3], 0x0040), 0x5410);
                 // 64-byte rows with 64-byte swizzle: chunk index XOR ((row >> 1) & 3)
                 const int chunk = c ^ ((row_in_tile >> 1) & 3);
                 *reinterpret_cast<uint4*>(prow + chunk * 16) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
