@@ -109,8 +109,8 @@ struct DecAttnSmem {
 // bytes), scores, max, exp, the ordered partial sums, the u8 quantiser and P.V, with the score rows kept in shared
 // memory (`dsm`: dec_attn_smem_bytes<G>). The group's NT threads (256 or 512; `tid` = index in the group) synchronise on named
 // barrier `bar`.
-// G = 2 (stand-alone operator): rows padded against bank conflicts in the ordered sums, the warp-wide exponential, and the
-// quantiser without divisions. G = 4 (persistent kernel): the forms that measured best inside that kernel.
+// G = 2 (stand-alone operator): rows padded against bank conflicts in the ordered sums, which fetch ahead, and the warp-wide
+// exponential. G = 4: the persistent kernel's form for contexts beyond its staging area.
 template <int G> constexpr size_t dec_attn_smem_bytes(int cs) {
     const size_t n = (size_t)G * (G == 2 ? cs + 4 : cs) * 4 + (size_t)G * cs;
     return n < 4096 ? 4096 : n;
@@ -119,6 +119,20 @@ template <int G> constexpr size_t dec_attn_smem_bytes(int cs) {
 __device__ __noinline__ static uint32_t dec_u8_exact(float e, float rinv, float vs, float a_s) {
     const int r = round_half_away_to_int(((e * rinv) * vs) / a_s);
     return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
+}
+// The same without divisions: (e c) vs with c = r / (255.25 a_s) (dec_u8_factor), held at 1, is within 2^-21 of the reference's
+// quotient / 255.25 (seven roundings), so where the two sides of 2^-19 round to the same integer, that is U; otherwise, and outside
+// the range of the bound, the reference's arithmetic decides.
+__device__ __forceinline__ float dec_u8_factor(float rinv, float a_s, bool& ok) {
+    const float c = (rinv * (1.0f / a_s)) * (1.0f / 255.25f);
+    ok = c >= 0x1p-60f && c <= 0x1p60f;
+    return c;
+}
+__device__ __forceinline__ uint32_t dec_u8(float e, float c, bool ok, float rinv, float vs, float a_s) {
+    const float t = __saturatef((e * c) * vs);
+    const uint32_t h = __float_as_uint(__fmaf_rn(t, 255.25f * (1.0f + 0x1p-19f), 12582912.0f));
+    const uint32_t l = __float_as_uint(__fmaf_rn(t, 255.25f * (1.0f - 0x1p-19f), 12582912.0f));
+    return ok && vs >= 0.0f && vs <= 0x1p40f && h == l ? h & 0xffu : dec_u8_exact(e, rinv, vs, a_s);
 }
 template <int MODE, int NT, int G = 4>
 __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const float* __restrict__ cos_t,
@@ -242,6 +256,7 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     ATT_TS(2);
 
     // ---- B. scores: four lanes share one key (16 bytes of its row each), NT/4 keys per iteration
+    const ExpTable tab = exp_table_lane();     // for step D: asked for now
     const int l4 = tid & 3, slot = tid >> 2;
     int qreg[G][4];
     float qsc[G];
@@ -317,7 +332,6 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // ---- D. e = exp(x - max), in place
     if constexpr (G == 2) {
         // eight values at a time: four keys of both heads
-        const ExpTable tab = exp_table_lane();
         const float m0 = row_max[0], m1 = row_max[1];
         for (int k0 = 0; k0 < nk; k0 += 4 * NT) {
             float u[8], e[8], far = 0.0f;
@@ -388,36 +402,18 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     const int nk_pad = (nk + PAGE - 1) / PAGE * PAGE;
     {
         float rinv_g[G];
-        DivBy as_g[G];
-        float c_g[G];
+        float as_g[G], c_g[G];
         bool ok_g[G];
 #pragma unroll
         for (int g = 0; g < G; g++) {
-            rinv_g[g] = row_rinv[g]; as_g[g] = div_by(a_s[hq0 + g]);
-            c_g[g] = (rinv_g[g] * as_g[g].y) * (1.0f / 255.25f);
-            ok_g[g] = c_g[g] >= 0x1p-60f && c_g[g] <= 0x1p60f;
+            rinv_g[g] = row_rinv[g]; as_g[g] = a_s[hq0 + g];
+            c_g[g] = dec_u8_factor(rinv_g[g], as_g[g], ok_g[g]);
         }
         auto quantise_key = [&](int key, float vsc) {
 #pragma unroll
             for (int g = 0; g < G; g++) {
                 uint8_t uq = 0;
-                if (G == 2) {
-                    if (key < nk) {
-                        // (e c) vs with c = r / (255.25 a_s), held at 1: within 2^-21 of the reference's quotient / 255.25 (seven
-                        // roundings), so where the two sides of 2^-19 round to the same integer, that is U
-                        const float e = sc[g * csr + key], t = __saturatef((e * c_g[g]) * vsc);
-                        const float h = __fmaf_rn(t, 255.25f * (1.0f + 0x1p-19f), 12582912.0f), l = __fmaf_rn(t, 255.25f * (1.0f - 0x1p-19f), 12582912.0f);
-                        uint32_t q = __float_as_uint(h);
-                        if (!ok_g[g] || !(vsc >= 0.0f && vsc <= 0x1p40f) || q != __float_as_uint(l)) q = dec_u8_exact(e, rinv_g[g], vsc, as_g[g].s);
-                        uq = (uint8_t)q;
-                    }
-                } else if (key < nk) {
-                    const float p = sc[g * cs + key] * rinv_g[g];
-                    const float tt = div_for_rounding(p * vsc, as_g[g]);
-                    int r = round_half_away_to_int(tt);
-                    r = r > 255 ? 255 : r;
-                    uq = (uint8_t)r;
-                }
+                if (key < nk) uq = (uint8_t)dec_u8(sc[g * csr + key], c_g[g], ok_g[g], rinv_g[g], vsc, as_g[g]);
                 u_sm[g * cs + key] = uq;
             }
         };
@@ -646,6 +642,7 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     if (!sm.last) return false;
     ATT_TS(2);
 
+    const ExpTable tab = exp_table_lane();      // for step D: asked for now
     // ---- B. scores on the tensor cores: a warp takes blocks of 16 keys; A = 16 key rows x 32 dims from the staging area,
     //         B = 32 dims x the 4 query heads (columns 4..7 are zero), two steps for the 64 dims
     const int gi = lane >> 2, ti = lane & 3;
@@ -723,11 +720,25 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     ATT_TS(4);
     // ---- D. e = exp(x - max), in place: the four heads of a key together (four independent evaluations in flight)
     {
-        const float m0 = row_max[0], m1 = row_max[1], m2 = row_max[2], m3 = row_max[3];
-        for (int key = tid; key < nk; key += NT) {
-            const float x0 = sc[key] - m0, x1 = sc[cs + key] - m1, x2 = sc[2 * cs + key] - m2, x3 = sc[3 * cs + key] - m3;
-            const float e0 = ref_expf(x0), e1 = ref_expf(x1), e2 = ref_expf(x2), e3 = ref_expf(x3);
-            sc[key] = e0; sc[cs + key] = e1; sc[2 * cs + key] = e2; sc[3 * cs + key] = e3;
+        // (the warp-wide form when no key of the warp lies far below its row's maximum)
+        const float m[4] = {row_max[0], row_max[1], row_max[2], row_max[3]};
+        for (int k0 = 0; k0 < nk; k0 += NT) {
+            const int key = k0 + tid;
+            float u[4], e[4], far = 0.0f;
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                u[g] = key < nk ? m[g] - sc[g * cs + key] : 0.0f;
+                far = max3_nan(far, far, u[g]);
+            }
+            if (__all_sync(0xffffffffu, far <= kExpFastLimit)) exp_warp<true>(u, e, tab);
+            else {
+#pragma unroll
+                for (int g = 0; g < 4; g++) e[g] = ref_expf(-u[g]);
+            }
+            if (key < nk) {
+#pragma unroll
+                for (int g = 0; g < 4; g++) sc[g * cs + key] = e[g];
+            }
         }
     }
     named_sync_id<NT>(bar);
@@ -762,23 +773,21 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     // ---- F. u8 probabilities (zero beyond the last key up to the page boundary)
     const int nk_pad = npages * PAGE;
     {
-        float rinv_g[G];
-        DivBy as_g[G];
+        float rinv_g[G], as_g[G], c_g[G];
+        bool ok_g[G];
 #pragma unroll
-        for (int g = 0; g < G; g++) { rinv_g[g] = row_rinv[g]; as_g[g] = div_by(a_s[hkv * G + g]); }
+        for (int g = 0; g < G; g++) {
+            rinv_g[g] = row_rinv[g]; as_g[g] = a_s[hkv * G + g];
+            c_g[g] = dec_u8_factor(rinv_g[g], as_g[g], ok_g[g]);
+        }
 #pragma unroll
         for (int u = 0; u < UF; u++) {
             const int key = tid + u * NT;
             if (key < nk_pad) {
 #pragma unroll
                 for (int g = 0; g < G; g++) {
-                    int r = 0;
-                    if (key < nk) {
-                        const float p = sc[g * cs + key] * rinv_g[g];
-                        r = round_half_away_to_int(div_for_rounding(p * vsc_pre[u], as_g[g]));
-                        r = r > 255 ? 255 : r;
-                    }
-                    u_sm[g * cs + key] = (uint8_t)r;
+                    u_sm[g * cs + key] =
+                        key < nk ? (uint8_t)dec_u8(sc[g * cs + key], c_g[g], ok_g[g], rinv_g[g], vsc_pre[u], as_g[g]) : (uint8_t)0;
                 }
             }
         }

@@ -423,27 +423,27 @@ __device__ __forceinline__ float4 silu_mul_x4(const float4 g, const float4 u) {
     return o;
 }
 
-// The same on eight values of every lane of a warp (whole-warp call): o = (g / (1 + exp(-g))) * u, each operation rounded once.
+// The same on NV (4 or 8) values of every lane of a warp (whole-warp call): o = (g / (1 + exp(-g))) * u, each operation rounded once.
 // The quotient: y = 1 / D from rcp.approx and one Newton step, q = RN(g y), one exact residual r = g - q D, RN(q + r y). For
 // the pairs (g, 1 + exp(-g)) that occur here this is the correctly rounded quotient: compared with the division for every
 // float g with 2^-60 <= |g| <= 80. Other values (and NaN) send the warp to the division itself.
-__device__ __forceinline__ void silu_mul_warp8(const float (&g)[8], const float (&u)[8], float (&o)[8], const ExpTable& tab) {
+template <int NV> __device__ __forceinline__ void silu_mul_warp(const float (&g)[NV], const float (&u)[NV], float (&o)[NV], const ExpTable& tab) {
     float far = fabsf(g[0]), near = far;
 #pragma unroll
-    for (int i = 1; i < 7; i += 2) {
+    for (int i = 1; i < NV - 1; i += 2) {
         far = max3_nan(far, fabsf(g[i]), fabsf(g[i + 1]));
         near = fminf(near, fminf(fabsf(g[i]), fabsf(g[i + 1])));
     }
-    far = max3_nan(far, far, fabsf(g[7]));
-    near = fminf(near, fabsf(g[7]));
+    far = max3_nan(far, far, fabsf(g[NV - 1]));
+    near = fminf(near, fabsf(g[NV - 1]));
     if (__all_sync(0xffffffffu, far <= 80.0f && near >= 0x1p-60f)) {
-        float x[8], e[8];
+        float x[NV], e[NV];
 #pragma unroll
-        for (int i = 0; i < 8; i++) x[i] = -g[i];
+        for (int i = 0; i < NV; i++) x[i] = -g[i];
         exp_warp<false>(x, e, tab);
         const f32x2 one = pack2(1.0f, 1.0f);
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
+        for (int i = 0; i < NV; i += 2) {
             const f32x2 d = add2(pack2(e[i], e[i + 1]), one), gg = pack2(g[i], g[i + 1]);
             float d0, d1, y0, y1;
             unpack2(d, d0, d1);
@@ -458,7 +458,7 @@ __device__ __forceinline__ void silu_mul_warp8(const float (&g)[8], const float 
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) o[i] = silu_mul_any(g[i], u[i]);
+        for (int i = 0; i < NV; i++) o[i] = silu_mul_any(g[i], u[i]);
     }
 }
 

@@ -179,6 +179,24 @@ __device__ __forceinline__ bool mega_grid_sync(unsigned long long* ctr, unsigned
     return *go_flag != 0;
 }
 
+// Largest value over the NT threads of a group (named barrier BAR), every thread's v >= 0. red: NT / 32 floats.
+template <int BAR, int NT> __device__ __forceinline__ float group_max(float v, float* red, int tid) {
+    v = warp_max(v);
+    if ((tid & 31) == 0) red[tid >> 5] = v;
+    named_sync<BAR, NT>();
+    const int l = tid & 31;
+    return warp_max(l < NT / 32 ? red[l] : 0.0f);
+}
+// Four values -> int8, w = 1 / sc (all of the caller's threads need not take part)
+__device__ __forceinline__ uint32_t mega_q8x4(const float (&x)[4], float sc) {
+    uint32_t q[4];
+    float nan = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) nan = max3_nan(nan, nan, x[i]);
+    q8_short(x, 1.0f / sc, sc >= 0x1p-60f && sc <= 0x1p60f && nan == nan, q, [&](float v) { return q8_exact(v, sc); });
+    return __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+}
+
 // ---- row phases (all 512 threads of the CTA that owns the row; one float4 per thread) -------------
 // x[row] (+)= dequantised projection sums (or the embedding row), then RMSNorm in the reference's
 // decode summation order (Modules/LayerNorm.h:210-370: 8 chunks of 4 interleaved chains; the same
@@ -231,10 +249,11 @@ __device__ __forceinline__ void mega_row_norm(const MegaArgs& a, int row, const 
         {
             const float* bc = buf + chunk * (C + 4);
             const int n = C >> 2;
-#pragma unroll 8
+#pragma unroll 32
             for (int k = 0; k < n; k++) { const float t = bc[4 * k + j]; ss += t * t; }
         }
         float tot = 0.0f;
+#pragma unroll
         for (int cc = 0; cc < LANES; cc++) {
             const float p0 = __shfl_sync(0xffffffffu, ss, cc * 4 + 0), p1 = __shfl_sync(0xffffffffu, ss, cc * 4 + 1);
             const float p2 = __shfl_sync(0xffffffffu, ss, cc * 4 + 2), p3 = __shfl_sync(0xffffffffu, ss, cc * 4 + 3);
@@ -244,21 +263,13 @@ __device__ __forceinline__ void mega_row_norm(const MegaArgs& a, int row, const 
     }
     named_sync<MG_BAR_WORK, NT>();
     const float r = red[64];
-    float mx = -1e32f, mn = 1e32f;
-    if (active) {
-        float4 o;
-        o.x = (v.x * r) * g.x; o.y = (v.y * r) * g.y; o.z = (v.z * r) * g.z; o.w = (v.w * r) * g.w;
-        v = o;
-        mx = fmaxf(fmaxf(o.x, o.y), fmaxf(o.z, o.w));
-        mn = fminf(fminf(o.x, o.y), fminf(o.z, o.w));
-    }
-    group_max_min<MG_BAR_WORK, NT>(mx, mn, red, tid);
-    const float sc = sym_scale_from(mx, mn);
+    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (active) { o[0] = (v.x * r) * g.x; o[1] = (v.y * r) * g.y; o[2] = (v.z * r) * g.z; o[3] = (v.w * r) * g.w; }
+    const float mx = group_max<MG_BAR_WORK, NT>(max3(max3(fabsf(o[0]), fabsf(o[1]), fabsf(o[2])), fabsf(o[3]), 0.0f), red, tid);
+    const float sc = sym_scale_from(mx, -mx);
     if (tid == 0) a.xs[row] = sc;
     if (active) {
-        char4 o;
-        o.x = quant_s8(v.x, sc); o.y = quant_s8(v.y, sc); o.z = quant_s8(v.z, sc); o.w = quant_s8(v.w, sc);
-        reinterpret_cast<char4*>(a.xq + (long)row * D)[c] = o;
+        reinterpret_cast<uint32_t*>(a.xq + (long)row * D)[c] = mega_q8x4(o, sc);
         asm volatile("fence.proxy.async.global;" ::: "memory");   // xq is read by other CTAs' TMA (async proxy)
     }
 }
@@ -297,14 +308,13 @@ __device__ __forceinline__ void mega_att_row_quant(const MegaArgs& a, int b, Dec
     for (int w = 0; w < 8; w++) { mx = fmaxf(mx, sm.red[0][w]); mn = fminf(mn, sm.red[1][w]); }
     const float sc = sym_scale_from(mx, mn);
     if (t == 0) a.xs[b] = sc;
-    char4* qr = reinterpret_cast<char4*>(a.xq + (long)b * D);
+    uint32_t* qr = reinterpret_cast<uint32_t*>(a.xq + (long)b * D);
 #pragma unroll
     for (int i = 0; i < 2; i++) {
         const int c = t + i * 256;
         if (c < nv) {
-            char4 o;
-            o.x = quant_s8(v[i].x, sc); o.y = quant_s8(v[i].y, sc); o.z = quant_s8(v[i].z, sc); o.w = quant_s8(v[i].w, sc);
-            qr[c] = o;
+            const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+            qr[c] = mega_q8x4(x, sc);
         }
     }
     asm volatile("fence.proxy.async.global;" ::: "memory");   // xq is read by other CTAs' TMA (async proxy)
@@ -319,6 +329,7 @@ __device__ __forceinline__ void mega_row_fht(const MegaArgs& a, const MegaLayer&
     const int4* ur = gr + N / 4;
     const float4* sg = reinterpret_cast<const float4*>(L.sgu);
     const float4* su = sg + N / 4;
+    const ExpTable tab = exp_table_lane();
     {
         int4 ga[4], ua[4];
         float4 s1[4], s2[4];
@@ -335,12 +346,14 @@ __device__ __forceinline__ void mega_row_fht(const MegaArgs& a, const MegaLayer&
             const int4 u4 = it == 0 ? ua[0] : it == 1 ? ua[1] : it == 2 ? ua[2] : ua[3];
             const float4 a1 = it == 0 ? s1[0] : it == 1 ? s1[1] : it == 2 ? s1[2] : s1[3];
             const float4 a2 = it == 0 ? s2[0] : it == 1 ? s2[1] : it == 2 ? s2[2] : s2[3];
-            float4 g, u, v;
+            float4 g, u;
             g.x = ((float)g4.x * st) * a1.x; g.y = ((float)g4.y * st) * a1.y; g.z = ((float)g4.z * st) * a1.z; g.w = ((float)g4.w * st) * a1.w;
             u.x = ((float)u4.x * st) * a2.x; u.y = ((float)u4.y * st) * a2.y; u.z = ((float)u4.z * st) * a2.z; u.w = ((float)u4.w * st) * a2.w;
-            v.x = silu_f(g.x) * u.x; v.y = silu_f(g.y) * u.y; v.z = silu_f(g.z) * u.z; v.w = silu_f(g.w) * u.w;
+            const float gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
+            float v[4];
+            silu_mul_warp(gg, uu, v, tab);
             const int p = pad32(c * 4);
-            buf[p] = v.x; buf[p + 1] = v.y; buf[p + 2] = v.z; buf[p + 3] = v.w;
+            buf[p] = v[0]; buf[p + 1] = v[1]; buf[p + 2] = v[2]; buf[p + 3] = v[3];
         }
     }
     named_sync<MG_BAR_WORK, MG_WORKERS>();
@@ -389,8 +402,11 @@ __device__ __forceinline__ void mega_row_fht4(const MegaArgs& a, const MegaLayer
         float4 g, u;
         g.x = ((float)g4.x * st) * a1.x; g.y = ((float)g4.y * st) * a1.y; g.z = ((float)g4.z * st) * a1.z; g.w = ((float)g4.w * st) * a1.w;
         u.x = ((float)u4.x * st) * a2.x; u.y = ((float)u4.y * st) * a2.y; u.z = ((float)u4.z * st) * a2.z; u.w = ((float)u4.w * st) * a2.w;
+        const float gg[4] = {g.x, g.y, g.z, g.w}, uu[4] = {u.x, u.y, u.z, u.w};
+        float v[4];
+        silu_mul_warp(gg, uu, v, exp_table_lane());
         const int p = pad32(tid * 4);
-        buf[p] = silu_f(g.x) * u.x; buf[p + 1] = silu_f(g.y) * u.y; buf[p + 2] = silu_f(g.z) * u.z; buf[p + 3] = silu_f(g.w) * u.w;
+        buf[p] = v[0]; buf[p + 1] = v[1]; buf[p + 2] = v[2]; buf[p + 3] = v[3];
     }
     named_sync<MG_BAR_WORK, MG_WORKERS>();
     if (tid < 256) {   // 2. stages on bits 1..10: four passes over groups of three index bits, 8 values per thread
@@ -438,25 +454,26 @@ __device__ __forceinline__ void mega_row_fht4(const MegaArgs& a, const MegaLayer
         const float4 m = part == 0 ? w[0] : part == 1 ? w[1] : part == 2 ? w[2] : w[3];
         x[0] = m.x + m.y; x[1] = m.x - m.y; x[2] = m.z + m.w; x[3] = m.z - m.w;             // bit 0
     }
-    div_rn_array(x, div_by(a.fht_scale));
-    float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), mn = fminf(fminf(x[0], x[1]), fminf(x[2], x[3]));
-    group_max_min<MG_BAR_WORK, MG_WORKERS>(mx, mn, red, tid);
+    // the largest magnitude before the division by fht_scale, which keeps the order
+    float nan = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) nan = max3_nan(nan, nan, x[i]);
+    const float mx = group_max<MG_BAR_WORK, MG_WORKERS>(max3(max3(fabsf(x[0]), fabsf(x[1]), fabsf(x[2])), fabsf(x[3]), 0.0f), red, tid);
     if (tid == 0) {   // 5. the row's largest magnitude over the four parts
-        const float am = fmaxf(fabsf(mx), fabsf(mn));
-        atomicMax(amax_bits, __float_as_uint(am));
+        atomicMax(amax_bits, __float_as_uint(mx));
         asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(flag_b), "r"(1) : "memory");
         mega_wait_flag(flag_b, 4, abort_flag, a.error_flag, a.wait_limit_ns);
     }
     named_sync<MG_BAR_WORK, MG_WORKERS>();
     if (*abort_flag) return;
-    float sc = __uint_as_float(__ldcg(amax_bits)) / 127.0f;          // sym_scale_from on the merged maximum
-    if (sc == 0.0f) sc = 1.0f;
-    const DivBy dsc = div_by(sc);
+    const float all = __uint_as_float(__ldcg(amax_bits)), top = all / a.fht_scale;
+    const float sc = sym_scale_from(top, -top);
     if (part == 0 && tid == 0) a.xs[row] = sc;
-    char4 o;
-    o.x = (int8_t)round_half_away_to_int(div_for_rounding(x[0], dsc)); o.y = (int8_t)round_half_away_to_int(div_for_rounding(x[1], dsc));
-    o.z = (int8_t)round_half_away_to_int(div_for_rounding(x[2], dsc)); o.w = (int8_t)round_half_away_to_int(div_for_rounding(x[3], dsc));
-    reinterpret_cast<char4*>(a.hq + (long)row * N + part * NP)[tid] = o;
+    uint32_t q[4];
+    const float fs = a.fht_scale;
+    q8_short(x, 1.0f / (fs * sc), fht_q8_in_range(all, fs) && nan == nan, q, [&](float v) { return fht_q8_exact(v, fs, sc); });
+    reinterpret_cast<uint32_t*>(a.hq + (long)row * N + part * NP)[tid] =
+        __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
     asm volatile("fence.proxy.async.global;" ::: "memory");   // hq is read by other CTAs' TMA (async proxy)
 }
 

@@ -23,17 +23,6 @@ using namespace tc;
 // for the column window [win.col0, win.col0 + win.cols) written compactly (tensor-parallel down_proj).
 struct FhtWindow { int g; long rows; int col0, cols; };
 
-// x / scale / sc rounded to an integer as the reference does: two correctly rounded divisions, halves away from zero.
-// Out of line: for the values that q8_short cannot decide, and for rows outside its range.
-__device__ __noinline__ static uint32_t fht_q8_exact(float x, float scale, float sc) {
-    return (uint32_t)round_half_away_to_int((x / scale) / sc) & 0xffu;
-}
-// May q8_short be used on a row whose largest transformed magnitude is mx? (Values far below mx give a quotient far below a half
-// either way.)
-__device__ __forceinline__ bool fht_q8_in_range(float mx, float scale) {
-    return (mx == 0.0f || (mx >= 0x1p-40f && mx <= 0x1p60f)) && scale >= 0x1p-20f && scale <= 0x1p20f;
-}
-
 // One CTA of 128 threads per row, 64 elements a thread. Bound by issue slots and by shared-memory bandwidth (128 bytes a
 // clock), so the row passes through shared memory twice and not three times: index bit 1 is done on the float4 as it comes
 // from memory, bits 2..7 with 64 values in registers, bits 8..12 and then 0 likewise. Element i lives at i + 4 * (i >> 8): the
@@ -78,7 +67,7 @@ __global__ void __launch_bounds__(128, 4) fht8192_kernel(const float* __restrict
             if (FUSED == 1) {
                 const float w[8] = {uv[i].x, uv[i].y, uv[i].z, uv[i].w, uv[i + 1].x, uv[i + 1].y, uv[i + 1].z, uv[i + 1].w};
                 float o[8];
-                silu_mul_warp8(v, w, o, tab);
+                silu_mul_warp(v, w, o, tab);
 #pragma unroll
                 for (int j = 0; j < 8; j++) v[j] = o[j];
             }
@@ -173,7 +162,7 @@ __global__ void __launch_bounds__(128) fht8192_cluster_kernel(const float* __res
     const ExpTable tab = exp_table_lane();
     const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w}, uu[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
     float r[8];
-    silu_mul_warp8(gg, uu, r, tab);
+    silu_mul_warp(gg, uu, r, tab);
     if (act) {
         float4* ao = reinterpret_cast<float4*>(act + row * N + part * L);
         ao[tid] = make_float4(r[0], r[1], r[2], r[3]);

@@ -20,6 +20,17 @@ __device__ __forceinline__ void reg_butterfly(float (&r)[N]) {
     }
 }
 
+// x / scale / sc rounded to an integer as the reference does: two correctly rounded divisions, halves away from zero.
+// Out of line: for the values that q8_short cannot decide, and for rows outside its range.
+__device__ __noinline__ static uint32_t fht_q8_exact(float x, float scale, float sc) {
+    return (uint32_t)round_half_away_to_int((x / scale) / sc) & 0xffu;
+}
+// May q8_short be used on a row whose largest transformed magnitude is mx? (Values far below mx give a quotient far below a half
+// either way.)
+__device__ __forceinline__ bool fht_q8_in_range(float mx, float scale) {
+    return (mx == 0.0f || (mx >= 0x1p-40f && mx <= 0x1p60f)) && scale >= 0x1p-20f && scale <= 0x1p20f;
+}
+
 // `buf` holds the row at pad32(i); on return thread `tid` of the 256 holds the transformed
 // (unscaled) elements i = hi*2048 + tid*8 + c in r[hi*8 + c], hi < 4, c < 8. Synchronises the 256
 // threads on named barrier BAR (first thing, so the caller's writes to `buf` need no barrier).
