@@ -44,6 +44,93 @@ template <int BN, int KCH> struct GemmBfCfg {
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + STG_BYTES;
 };
 
+// Epilogue of the prompt form: one warp, rows row0 .. row0 + 31 (lane = row), columns col0 .. col0 + BN - 1 of the accumulator at tsrc;
+// the columns' biases are at stg + 1024.
+template <int BN>
+__device__ __forceinline__ void staged_store_bf(const GemmBfArgs& args, float* stg, const uint32_t tsrc, const int row0, const int col0, const int lane) {
+    const float* bw = stg + 1024;
+    __syncwarp();
+    // 32 columns at a time go through this warp's staging buffer (16-byte granules XOR-swizzled by the
+    // row), so that the global stores of a warp cover whole sectors of few rows
+    auto process = [&](const uint32_t (&v)[32], const int c) {
+        const int c0 = col0 + c * 32;
+        if (c0 >= args.rowsB) return;
+        const int s7 = lane & 7;
+        if (args.glu) {
+#pragma unroll
+            for (int g = 0; g < 4; g++) {
+                float r[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float gt = __uint_as_float(v[4 * g + i]) + bw[c * 32 + 4 * g + i];
+                    const float up = __uint_as_float(v[16 + 4 * g + i]) + bw[c * 32 + 16 + 4 * g + i];
+                    r[i] = gelu_tanh_f<true>(gt) * up;
+                }
+                *reinterpret_cast<float4*>(stg + lane * 32 + ((g ^ s7) << 2)) = make_float4(r[0], r[1], r[2], r[3]);
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < 8; g++) {
+                const float4 b4 = *reinterpret_cast<const float4*>(bw + c * 32 + 4 * g);
+                float4 o4 = make_float4(__uint_as_float(v[4 * g]) + b4.x, __uint_as_float(v[4 * g + 1]) + b4.y,
+                                        __uint_as_float(v[4 * g + 2]) + b4.z, __uint_as_float(v[4 * g + 3]) + b4.w);
+                if (args.relu2) o4 = make_float4(relu2_f(o4.x), relu2_f(o4.y), relu2_f(o4.z), relu2_f(o4.w));
+                *reinterpret_cast<float4*>(stg + lane * 32 + ((g ^ s7) << 2)) = o4;
+            }
+        }
+        __syncwarp();
+        const int ocol0 = args.glu ? c0 >> 1 : c0;            // first output column of the chunk
+        const int n_out = args.glu ? args.rowsB >> 1 : args.rowsB;
+        const int width = args.glu ? 16 : 32;
+        if (args.vec && args.y16) {
+            const int lpr = width >> 3;                            // lanes per row, 8 columns each
+            const int rstep = 32 / lpr, g2 = (lane % lpr) * 2, r0 = lane / lpr;
+            for (int rr = r0; rr < 32; rr += rstep) {
+                const int row = row0 + rr, col = ocol0 + g2 * 4;
+                if (row < args.rowsA && col < n_out) {
+                    const float4 x = *reinterpret_cast<const float4*>(stg + rr * 32 + ((g2 ^ (rr & 7)) << 2));
+                    const float4 z = *reinterpret_cast<const float4*>(stg + rr * 32 + (((g2 + 1) ^ (rr & 7)) << 2));
+                    *reinterpret_cast<uint4*>(args.y16 + (long)row * args.ldo + col) =
+                        make_uint4(bf_pack(x.x, x.y), bf_pack(x.z, x.w), bf_pack(z.x, z.y), bf_pack(z.z, z.w));
+                }
+            }
+        } else if (args.vec) {
+            const int lpr = width >> 2, rstep = 32 / lpr, g1 = lane % lpr, r0 = lane / lpr;
+            for (int rr = r0; rr < 32; rr += rstep) {
+                const int row = row0 + rr, col = ocol0 + g1 * 4;
+                if (row < args.rowsA && col < n_out)
+                    *reinterpret_cast<float4*>(args.y32 + (long)row * args.ldo + col) =
+                        *reinterpret_cast<const float4*>(stg + rr * 32 + ((g1 ^ (rr & 7)) << 2));
+            }
+        } else {
+            for (int i = lane; i < 32 * width; i += 32) {
+                const int rr = i / width, cc = i - rr * width;
+                const int row = row0 + rr, col = ocol0 + cc;
+                if (row < args.rowsA && col < n_out) {
+                    const float x = stg[rr * 32 + (((cc >> 2) ^ (rr & 7)) << 2) + (cc & 3)];
+                    if (args.y16) args.y16[(long)row * args.ldo + col] = __float2bfloat16_rn(x);
+                    else args.y32[(long)row * args.ldo + col] = x;
+                }
+            }
+        }
+        __syncwarp();
+    };
+    constexpr int NCH = BN / 32;
+    uint32_t va[32], vb[32];
+    tmem_ld_32x32(tsrc, va);
+#pragma unroll 1
+    for (int c = 0; c < NCH; c += 2) {
+        tmem_ld_wait();
+        if (c + 1 < NCH) tmem_ld_32x32(tsrc + (c + 1) * 32, vb);
+        process(va, c);
+        if (c + 1 < NCH) {
+            tmem_ld_wait();
+            if (c + 2 < NCH) tmem_ld_32x32(tsrc + (c + 2) * 32, va);
+            process(vb, c + 1);
+        }
+    }
+}
+
 template <int BN, bool SWAP, int KCH>
 __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmapA,
                                                                    const __grid_constant__ CUtensorMap tmapB, const GemmBfArgs args) {
@@ -195,86 +282,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
             tc_fence_after();
             const uint32_t tsrc = tmem_base + ((uint32_t)(q * 32) << 16) + as * BN;
             if constexpr (!SWAP) {
-                __syncwarp();
-                // 32 columns at a time go through this warp's staging buffer (16-byte granules XOR-swizzled by the
-                // row), so that the global stores of a warp cover whole sectors of few rows
-                auto process = [&](const uint32_t (&v)[32], const int c) {
-                    const int col0 = tb * BN + c * 32;
-                    if (col0 >= args.rowsB) return;
-                    const int s7 = lane & 7;
-                    if (args.glu) {
-#pragma unroll
-                        for (int g = 0; g < 4; g++) {
-                            float r[4];
-#pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const float gt = __uint_as_float(v[4 * g + i]) + bw[c * 32 + 4 * g + i];
-                                const float up = __uint_as_float(v[16 + 4 * g + i]) + bw[c * 32 + 16 + 4 * g + i];
-                                r[i] = gelu_tanh_f<true>(gt) * up;
-                            }
-                            *reinterpret_cast<float4*>(stg + lane * 32 + ((g ^ s7) << 2)) = make_float4(r[0], r[1], r[2], r[3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int g = 0; g < 8; g++) {
-                            const float4 b4 = *reinterpret_cast<const float4*>(bw + c * 32 + 4 * g);
-                            float4 o4 = make_float4(__uint_as_float(v[4 * g]) + b4.x, __uint_as_float(v[4 * g + 1]) + b4.y,
-                                                    __uint_as_float(v[4 * g + 2]) + b4.z, __uint_as_float(v[4 * g + 3]) + b4.w);
-                            if (args.relu2) o4 = make_float4(relu2_f(o4.x), relu2_f(o4.y), relu2_f(o4.z), relu2_f(o4.w));
-                            *reinterpret_cast<float4*>(stg + lane * 32 + ((g ^ s7) << 2)) = o4;
-                        }
-                    }
-                    __syncwarp();
-                    const int ocol0 = args.glu ? col0 >> 1 : col0;            // first output column of the chunk
-                    const int n_out = args.glu ? args.rowsB >> 1 : args.rowsB;
-                    const int width = args.glu ? 16 : 32;
-                    if (args.vec && args.y16) {
-                        const int lpr = width >> 3;                            // lanes per row, 8 columns each
-                        const int rstep = 32 / lpr, g2 = (lane % lpr) * 2, r0 = lane / lpr;
-                        for (int rr = r0; rr < 32; rr += rstep) {
-                            const int row = row0 + rr, col = ocol0 + g2 * 4;
-                            if (row < args.rowsA && col < n_out) {
-                                const float4 x = *reinterpret_cast<const float4*>(stg + rr * 32 + ((g2 ^ (rr & 7)) << 2));
-                                const float4 z = *reinterpret_cast<const float4*>(stg + rr * 32 + (((g2 + 1) ^ (rr & 7)) << 2));
-                                *reinterpret_cast<uint4*>(args.y16 + (long)row * args.ldo + col) =
-                                    make_uint4(bf_pack(x.x, x.y), bf_pack(x.z, x.w), bf_pack(z.x, z.y), bf_pack(z.z, z.w));
-                            }
-                        }
-                    } else if (args.vec) {
-                        const int lpr = width >> 2, rstep = 32 / lpr, g1 = lane % lpr, r0 = lane / lpr;
-                        for (int rr = r0; rr < 32; rr += rstep) {
-                            const int row = row0 + rr, col = ocol0 + g1 * 4;
-                            if (row < args.rowsA && col < n_out)
-                                *reinterpret_cast<float4*>(args.y32 + (long)row * args.ldo + col) =
-                                    *reinterpret_cast<const float4*>(stg + rr * 32 + ((g1 ^ (rr & 7)) << 2));
-                        }
-                    } else {
-                        for (int i = lane; i < 32 * width; i += 32) {
-                            const int rr = i / width, cc = i - rr * width;
-                            const int row = row0 + rr, col = ocol0 + cc;
-                            if (row < args.rowsA && col < n_out) {
-                                const float x = stg[rr * 32 + (((cc >> 2) ^ (rr & 7)) << 2) + (cc & 3)];
-                                if (args.y16) args.y16[(long)row * args.ldo + col] = __float2bfloat16_rn(x);
-                                else args.y32[(long)row * args.ldo + col] = x;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                };
-                constexpr int NCH = BN / 32;
-                uint32_t va[32], vb[32];
-                tmem_ld_32x32(tsrc, va);
-#pragma unroll 1
-                for (int c = 0; c < NCH; c += 2) {
-                    tmem_ld_wait();
-                    if (c + 1 < NCH) tmem_ld_32x32(tsrc + (c + 1) * 32, vb);
-                    process(va, c);
-                    if (c + 1 < NCH) {
-                        tmem_ld_wait();
-                        if (c + 2 < NCH) tmem_ld_32x32(tsrc + (c + 2) * 32, va);
-                        process(vb, c + 1);
-                    }
-                }
+                staged_store_bf<BN>(args, stg, tsrc, row0, tb * BN, lane);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_tempty + 8 * as);
@@ -334,6 +342,145 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, Cfg::TMEM_COLS); }
 }
 
+// The prompt form on CTA pairs (cta_group::2): 256 x 256 tiles on two SMs, as gemm_i8_pair_kernel: a third less shared-memory and L2
+// traffic per multiply-add than 128 x 256 on one, and in the power-limited regime of a long prompt that is clock. Prompts of 4 x 1000
+// tokens at the sizes of a 1B model, all layers: Pibidra 11.2 -> 10.2 ms, Sabisun 10.6 -> 10.1 ms.
+constexpr int GP_STAGES = 6, GP_TILE = 128 * 128, GP_STAGE_BYTES = 2 * GP_TILE, GP_BN = 256;
+constexpr int GP_SMEM = GP_STAGES * GP_STAGE_BYTES + 1024 + 256 + GemmBfCfg<GP_BN, 1>::STG_BYTES;
+__global__ void __launch_bounds__(192, 1) gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
+                                                                const GemmBfArgs args) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t ring = (raw + 1023u) & ~1023u;
+    uint8_t* ring_ptr = smem_raw + (ring - raw);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES);
+    const uint32_t bar_full = smem_u32(bars);                    // first CTA: bytes of both CTAs
+    const uint32_t bar_empty = bar_full + 8 * GP_STAGES;         // both CTAs, each for its own producer
+    const uint32_t bar_tfull = bar_empty + 8 * GP_STAGES;        // both CTAs
+    const uint32_t bar_tempty = bar_tfull + 16;                  // first CTA: the eight epilogue warps of both
+    uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * GP_STAGES + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
+    float* stg_all = reinterpret_cast<float*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES + 256);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int total_tiles = args.tilesA * args.tilesB;           // tilesA: 256-row tiles
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GP_STAGES; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
+        for (int s = 0; s < 2; s++) { mbar_init(bar_tfull + 8 * s, 1); mbar_init(bar_tempty + 8 * s, 8); }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tmem_alloc_pair(smem_u32(tmem_base_slot), 2 * GP_BN);
+        tmem_relinquish_pair();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                              // the other CTA's barriers exist before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            tma_prefetch_desc(&tmapA);
+            tma_prefetch_desc(&tmapB);
+            int stage = 0; uint32_t phase = 0;
+            bool ok = true;
+            for (int t = pair; ok && t < total_tiles; t += pairs) {
+                const int rowA = (t / args.tilesB) * 256 + rank * 128, rowB = (t % args.tilesB) * GP_BN + rank * 128;
+                for (int kb = 0; kb < args.num_kb; kb++) {
+                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
+                    const uint32_t full = bar_full + 8 * stage, full0 = cluster_addr(full, 0);
+                    if (rank == 0) mbar_expect_tx(full, 2 * GP_STAGE_BYTES);
+                    const uint32_t dst = ring + stage * GP_STAGE_BYTES;
+                    tma_load_2d_pair(dst, &tmapA, full0, kb * 128, rowA);
+                    tma_load_2d_pair(dst + GP_TILE, &tmapB, full0, kb * 128, rowB);
+                    if (++stage == GP_STAGES) { stage = 0; phase ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = umma_idesc_bf16(256, GP_BN);
+            int stage = 0; uint32_t phase = 0;
+            int it = 0;
+            bool ok = true;
+            for (int t = pair; ok && t < total_tiles; t += pairs, it++) {
+                const int as = it & 1;
+                if (!mbar_wait(bar_tempty + 8 * as, (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                for (int kb = 0; kb < args.num_kb; kb++) {
+                    if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t sa = ring + stage * GP_STAGE_BYTES;
+                    const uint64_t adesc = umma_desc_k_sw128(sa), bdesc = umma_desc_k_sw128(sa + GP_TILE);
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        umma_bf16_pair(tmem_base + as * GP_BN, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit_pair(bar_empty + 8 * stage);
+                    if (++stage == GP_STAGES) { stage = 0; phase ^= 1u; }
+                }
+                if (ok) umma_commit_pair(bar_tfull + 8 * as);
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        float* stg = stg_all + q * GemmBfCfg<GP_BN, 1>::STG_WARP_FLOATS;
+        int it = 0;
+        for (int t = pair; t < total_tiles; t += pairs, it++) {
+            const int row0 = (t / args.tilesB) * 256 + rank * 128 + q * 32, col0 = (t % args.tilesB) * GP_BN;
+            const int as = it & 1;
+            for (int i = lane; i < GP_BN; i += 32) stg[1024 + i] = (args.bias && col0 + i < args.rowsB) ? args.bias[col0 + i] : 0.0f;
+            int got = (lane == 0) ? (mbar_wait(bar_tfull + 8 * as, (uint32_t)((it >> 1) & 1), abort_flag) ? 1 : 0) : 1;
+            got = __shfl_sync(0xffffffffu, got, 0);
+            if (!got) break;
+            tc_fence_after();
+            staged_store_bf<GP_BN>(args, stg, tmem_base + ((uint32_t)(q * 32) << 16) + as * GP_BN, row0, col0, lane);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(bar_tempty + 8 * as, 0));
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        // a wait ran out: give copies still in flight time to land before shared memory is released
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+        if (threadIdx.x == 0 && args.error_flag) atomicOr(args.error_flag, 1);
+        __syncthreads();
+    }
+    cluster_sync();                                              // both CTAs are done with each other's memory
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, 2 * GP_BN);
+    }
+}
+
+int launch_pair(const bf16* A, int rowsA, long ldA, const bf16* B, int rowsB, long ldB, int K, GemmBfArgs g, cudaStream_t st) {
+    CUtensorMap ta, tb;
+    TRY_RC(cached_tmap_u8(&ta, A, (uint64_t)rowsA, (uint64_t)ldA * 2, 128, 0));
+    TRY_RC(cached_tmap_u8(&tb, B, (uint64_t)rowsB, (uint64_t)ldB * 2, 128, 0));
+    g.rowsA = rowsA; g.rowsB = rowsB; g.num_kb = (K + 63) / 64;
+    g.tilesA = (rowsA + 255) / 256; g.tilesB = (rowsB + GP_BN - 1) / GP_BN;
+    g.error_flag = device_error_flag();
+    static std::atomic<bool> attr_set[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0) return FLEXLLM_ECUDA;
+    if (!attr_set[dev].load(std::memory_order_acquire)) {
+        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
+        attr_set[dev].store(true, std::memory_order_release);
+    }
+    const int tiles = g.tilesA * g.tilesB, pairs = gemm_sm_count() / 2;
+    launch_cluster(gemm_bf16_pair_kernel, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(192), 2, (size_t)GP_SMEM, st, ta, tb, g);
+    return launch_status();
+}
+
 template <int BN, bool SWAP, int KCH>
 int launch(const bf16* A, int rowsA, long ldA, const bf16* B, int rowsB, long ldB, int K, GemmBfArgs g, cudaStream_t st) {
     using Cfg = GemmBfCfg<BN, KCH>;
@@ -376,8 +523,11 @@ int gemm_bf16_prefill(const bf16* a, long lda, const bf16* w, long ldw, const fl
     GemmBfArgs g = base_args(bias, act, y);
     const int n_out = g.glu ? N / 2 : N;
     g.vec = y.t ? (y.ld % 8 == 0 && n_out % 8 == 0 && aligned(y.t, 16)) : (y.ld % 4 == 0 && n_out % 4 == 0 && aligned(y.f32, 16));
-    // the widest tile that still gives every SM work
-    const long tiles256 = (long)((M + 127) / 128) * ((N + 255) / 256);
+    // the widest tile that still gives every SM work; pairs of CTAs unless their larger tiles need more rounds
+    const long tiles256 = (long)((M + 127) / 128) * ((N + 255) / 256), tiles_pair = (long)((M + 255) / 256) * ((N + 255) / 256);
+    const int sms = gemm_sm_count();
+    if (N > 128 && tiles256 >= sms && (tiles_pair + sms / 2 - 1) / (sms / 2) <= (tiles256 + sms - 1) / sms)
+        return launch_pair(a, M, lda, w, N, ldw, K, g, st);
     if (N > 128 && tiles256 >= gemm_sm_count()) return launch<256, false, 1>(a, M, lda, w, N, ldw, K, g, st);
     if (N > 64 && tiles256 * 2 >= gemm_sm_count()) return launch<128, false, 1>(a, M, lda, w, N, ldw, K, g, st);
     return launch<64, false, 1>(a, M, lda, w, N, ldw, K, g, st);

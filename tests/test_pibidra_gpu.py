@@ -71,6 +71,28 @@ def test_linear_few_tokens_ring(F, N, K):
         assert np.abs(got - want).max() < 2e-5 * np.abs(want).max(), (M, np.abs(got - want).max())
 
 
+@pytest.mark.parametrize("M,N,K,gated", [(1300, 4108, 90, False),      # pairs of CTAs: ragged rows, columns and K
+                                         (1100, 4160, 264, True),
+                                         (2300, 2048, 64, False)])      # as many rounds of pairs as of single tiles, and one more tile
+def test_linear_cta_pairs(F, M, N, K, gated):
+    """Prompt products whose tiles go to pairs of CTAs, fp32 and bf16 output. Bounds as in the tests around."""
+    g = np.random.default_rng(M)
+    a = bf16_round(g.standard_normal((M, K)))
+    ad = padded(a, up(K, 8), torch.bfloat16)
+    if gated:
+        gate, upw = (bf16_round(g.standard_normal((N // 2, K)) * 2 * K ** -0.5) for _ in range(2))
+        w = np.stack([gate.reshape(-1, 16, K), upw.reshape(-1, 16, K)], 1).reshape(N, K)
+        want = P.gelu_tanh(P.linear(gate.astype(np.float64), a)) * P.linear(upw.astype(np.float64), a)
+    else:
+        w = bf16_round(g.standard_normal((N, K)) * K ** -0.5)
+        want = P.linear(w.astype(np.float64), a.astype(np.float64))
+    wd = padded(w, up(K, 8), torch.bfloat16)
+    got = F.linear_float(ad, wd, None, K=K, gelu_gate=gated, out_f32=True).cpu().numpy()
+    assert np.abs(got - want).max() < 3e-5 * np.abs(want).max()
+    got = F.linear_float(ad, wd, None, K=K, gelu_gate=gated).float().cpu().numpy()
+    assert np.abs(got - want).max() < 5e-3 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("ff,K", [(16, 64), (80, 90), (368, 512), (4096, 1024)])
 def test_gated_gelu_linear(F, dtype, ff, K):
