@@ -17,11 +17,12 @@ def _ptr(t):
     if t is None:
         return None
     assert t.is_cuda and t.is_contiguous(), "flexllm_b200 takes contiguous CUDA tensors"
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()             # the argument types of the library's functions make it a pointer
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle alone: torch.cuda.current_stream() builds a stream object on every call
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _call(name, *args):
