@@ -15,8 +15,8 @@
 //   decode  : A = weights [N][K],     B = activations [M<=64][K]     out[rowB][rowA]   (SWAP)
 // so that a handful of tokens still fills the 128-row dimension of the tensor core with weight
 // rows and the weight matrix is streamed exactly once. With split-K (decode) the splits of a tile form a thread-block
-// cluster: each CTA leaves its int32 partial tile in shared memory and the cluster's CTAs add them, a share of the tokens
-// each, over distributed shared memory. (Adding into a buffer in global memory, with the last arriver reading it back, took
+// cluster of up to four: each CTA leaves its int32 partial tile in shared memory and the cluster's CTAs add them, a share of
+// the tokens each, over distributed shared memory. (Adding into a buffer in global memory, with the last arriver reading it back, took
 // 26 us for 64 tokens of 2048 x 8192.) The allocation-free entry point keeps the form that adds into a zeroed buffer.
 //
 // Replaces pref_Linear_Layer_i4xi4 / dec_Linear_Layer_i4xi4 + the dequant layers
@@ -457,11 +457,11 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
                 for (int tok = r; tok < args.rowsB; tok += args.ksplit) {
                     const long o = (long)tok * args.ldo + rowA;
                     const float rs = args.residual ? args.residual[o] : 0.0f;
-                    int p[8];
+                    int p[4];
 #pragma unroll
-                    for (int k = 0; k < 8; k++)
+                    for (int k = 0; k < 4; k++)
                         p[k] = k < args.ksplit ? __float_as_int(ld_cluster_f32(cluster_addr(ring + (uint32_t)(tok * 128 + q * 32 + lane) * 4u, k))) : 0;
-                    const int t = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+                    const int t = (p[0] + p[1]) + (p[2] + p[3]);
                     if (args.acc) args.acc[o] = t;
                     if (args.y) {
                         float v = ((float)t * args.sB[tok]) * sa;
@@ -761,14 +761,15 @@ int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const 
     return launch_gemm<16, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
 }
 
-// Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side. K is split over clusters of up to eight CTAs as
-// long as the tiles leave half the SMs idle and every split keeps two 128-byte blocks.
+// Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side. K is split over clusters of up to four CTAs as
+// long as the tiles leave half the SMs idle and every split keeps two 128-byte blocks. (64 tokens of 2048 x 8192: 23.5 / 19.8 /
+// 14.0 / 18.3 us with clusters of 1 / 2 / 4 / 8, of 2048 x 2048: 13.3 / 14.4 / 10.4 / 15.4 us: larger clusters start and meet later.)
 int gemm_i8_decode(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
                    int32_t* acc, float* y, cudaStream_t st, const float* residual) {
     if (M > 64) return FLEXLLM_ENOTSUP;
     const int tiles = (N + 127) / 128, kb = (K + 127) / 128;
     int ksplit = 1;
-    while (ksplit < 8 && tiles * ksplit * 2 <= sm_count() && kb >= 4 * ksplit) ksplit *= 2;
+    while (ksplit < 4 && tiles * ksplit * 2 <= sm_count() && kb >= 4 * ksplit) ksplit *= 2;
     // chunks of K per pipeline stage: KCH*128 contiguous bytes per weight row and TMA request, two steps per split
     int kch = 1;
     if (K % 512 == 0 && kb / 4 >= 2 * ksplit) kch = 4;
