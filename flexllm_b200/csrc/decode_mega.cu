@@ -26,8 +26,8 @@
 // TMA thread has issued the last loads of one projection it starts streaming the WEIGHT tiles of
 // the next one into the ring -- weights do not depend on the phases in between -- and only the
 // small activation tiles wait for the grid barrier. Arithmetic is the same device code the
-// stand-alone kernels use (attention_decode.cuh, fht_core.cuh, sampling.cuh; the RMSNorm statements of
-// rmsnorm_core.cuh spread over a CTA), hence bit-identical.
+// stand-alone kernels use (attention_decode.cuh, fht_core.cuh, sampling.cuh) or the same arithmetic in the same order, hence
+// bit-identical.
 //
 // Every wait (mbarrier, grid barrier) is bounded; on a timeout the CTA raises the global error
 // flag, all CTAs leave through the tear-down and the host sees FLEXLLM_ETIMEDOUT.
@@ -40,7 +40,6 @@
 #include "attention_decode.cuh"
 #include "common.cuh"
 #include "fht_core.cuh"
-#include "rmsnorm_core.cuh"
 #include "sampling.cuh"
 #include "tc_common.cuh"
 
@@ -200,7 +199,7 @@ __device__ __forceinline__ uint32_t mega_q8x4(const float (&x)[4], float sc) {
 // ---- row phases (all 512 threads of the CTA that owns the row; one float4 per thread) -------------
 // x[row] (+)= dequantised projection sums (or the embedding row), then RMSNorm in the reference's
 // decode summation order (Modules/LayerNorm.h:210-370: 8 chunks of 4 interleaved chains; the same
-// statements as rmsnorm_decode_row, with the row spread over the CTA instead of one warp) and the
+// arithmetic as rmsnorm_decode_kernel) and the
 // per-token quantiser. acc: `ks` slabs [max_batch][D] of split-K partial sums (integer adds: exact in
 // any order), nullptr for the embedding. buf: D + 32 floats, red: 65 floats of shared memory.
 __device__ __forceinline__ void mega_row_norm(const MegaArgs& a, int row, const int32_t* acc, int ks, const float* s_ch,

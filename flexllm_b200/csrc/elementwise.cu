@@ -4,7 +4,6 @@
 #include <atomic>
 
 #include "common.cuh"
-#include "rmsnorm_core.cuh"
 
 namespace flexllm {
 
@@ -146,12 +145,10 @@ __global__ void static_quant_kernel(const float* __restrict__ x, long rows, int 
 //                                  added from 0 in chunk order.
 // A chain is a strictly sequential fp32 accumulation, so one thread owns it. To keep all 32 lanes
 // busy a warp runs 32 chains at once: in the prefill order the 4 chains of 8 different rows, in the
-// decode order the (up to) 32 chains of one row. The rows sit in shared memory (prefill) or in
-// registers (decode) between the sum and the output pass: each is read from global memory once.
+// decode order the (up to) 32 chains of one row. The rows sit on chip between the sum and the output
+// pass: each is read from global memory once.
 // ---------------------------------------------------------------------------------------------
-constexpr int RMS_WARPS = 4;
 constexpr int RMS_PIECE = 128;           // floats per row per staging step
-constexpr int RMS_PSTRIDE = RMS_PIECE + 4;   // padded: rows land in different banks
 
 template <int MAXV>  // float4 per lane kept in registers for the output pass (D <= MAXV*128)
 __device__ __forceinline__ void rmsnorm_output_row(const float* __restrict__ xr, const float* __restrict__ gamma, int D, float r,
@@ -283,36 +280,12 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
     }
 }
 
-// Decode order with `lanes` (4 or 8) chunks: one warp per row, lane = chunk*4 + j. The row and gamma
-// are fetched with one batch of independent 128-bit loads and stay in registers for the output pass
-// (a decode step is latency-bound: one global round trip instead of one per loop iteration).
+// Decode order with `lanes` (4 or 8) chunks, Modules/LayerNorm.h:210-370: one CTA per row, so that the loads, the normalised values
+// and the quantiser are spread over eight warps and only the ordered sums stay on one: lane = chunk*4 + j sums the squares of the chunk's
+// elements k with k mod 4 == j in increasing k; the chunks' totals are added from 0 in chunk order. Latency-bound at a decode step's
+// row counts. Rows of 2048, 1 / 592 / 4736 of them: 4.3 / 6.3 / 18.7 us; one warp per row, four rows a CTA, took 8.4 / 8.4 / 24.6 us.
 template <int MAXV>
-__global__ void __launch_bounds__(RMS_WARPS * 32) rmsnorm_decode_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                                                        int M, int D, float eps, int lanes, float* __restrict__ y,
-                                                                        int8_t* __restrict__ q, float* __restrict__ s) {
-    extern __shared__ __align__(16) float rowbuf[];          // RMS_WARPS x (D + 4*lanes)
-    pdl_sync();
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long row = (long)blockIdx.x * RMS_WARPS + w;
-    if (row >= M) return;
-    const int nv = D >> 2;
-    float* buf = rowbuf + (size_t)w * (D + 4 * lanes);
-    const float* xr = x + row * D;
-    constexpr bool KEEP_G = MAXV <= 16;                       // gamma in registers too when it fits
-    float4 v[MAXV], g[KEEP_G ? MAXV : 1];
-#pragma unroll
-    for (int i = 0; i < MAXV; i++) {
-        const int c = lane + i * 32;
-        if (c < nv) { v[i] = reinterpret_cast<const float4*>(xr)[c]; if (KEEP_G) g[i] = reinterpret_cast<const float4*>(gamma)[c]; }
-    }
-    rmsnorm_decode_row<MAXV, KEEP_G>(v, g, gamma, D, eps, lanes, buf, lane, y ? y + row * D : nullptr, q ? q + row * D : nullptr,
-                                     s ? s + row : nullptr);
-}
-
-// The same for few rows: one CTA per row, so that the loads, the normalised values and the quantiser are spread over eight warps
-// and only the ordered sums stay on one (a warp that does everything takes 64 values a lane one after another).
-template <int MAXV>
-__global__ void __launch_bounds__(256) rmsnorm_decode_cta_kernel(const float* __restrict__ x, const float* __restrict__ gamma, int D, float eps,
+__global__ void __launch_bounds__(256) rmsnorm_decode_kernel(const float* __restrict__ x, const float* __restrict__ gamma, int D, float eps,
                                                                  int lanes, float* __restrict__ y, int8_t* __restrict__ q, float* __restrict__ s) {
     extern __shared__ __align__(16) float rowbuf[];          // D + 4*lanes
     __shared__ float rinv_sm, red[8];
@@ -382,7 +355,6 @@ __global__ void __launch_bounds__(256) rmsnorm_decode_cta_kernel(const float* __
                 __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
     }
 }
-constexpr int RMS_CTA_ROWS = 4 * 148;      // up to four CTAs an SM
 
 // ---------------------------------------------------------------------------------------------
 // SiLU / gate / residual (Swish.h:19, Linear_Layer.h:626, Residual_Layer.h:61)
@@ -631,17 +603,9 @@ extern "C" int flexllm_rmsnorm_quant(const float* x, const float* gamma, int M, 
             attr_done[dev].store(1, std::memory_order_release);
         }
         rmsnorm_prefill_kernel<<<grid, RMSP_ROWS * 32, smem, st>>>(x, gamma, M, D, eps, y, q, s);
-    } else if (M <= RMS_CTA_ROWS) {
-        const size_t smem = (size_t)(D + 4 * order) * sizeof(float);
-        launch_k(D <= 2048 ? rmsnorm_decode_cta_kernel<2> : rmsnorm_decode_cta_kernel<4>, dim3(M), dim3(256), smem, st, x, gamma, D, eps, order, y, q, s);
     } else {
-        const int grid = (M + RMS_WARPS - 1) / RMS_WARPS;
-        const size_t smem = (size_t)RMS_WARPS * (D + 4 * order) * sizeof(float);
-        if (D <= 2048) launch_k(rmsnorm_decode_kernel<16>, dim3(grid), dim3(RMS_WARPS * 32), smem, st, x, gamma, M, D, eps, order, y, q, s);
-        else {
-            FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_decode_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            rmsnorm_decode_kernel<32><<<grid, RMS_WARPS * 32, smem, st>>>(x, gamma, M, D, eps, order, y, q, s);
-        }
+        const size_t smem = (size_t)(D + 4 * order) * sizeof(float);
+        launch_k(D <= 2048 ? rmsnorm_decode_kernel<2> : rmsnorm_decode_kernel<4>, dim3(M), dim3(256), smem, st, x, gamma, D, eps, order, y, q, s);
     }
     return launch_status();
 }
