@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(64 * G) dec_pv_kernel(KvLayer cache, const int
 // Grid (2 HKV, B): two CTAs per (sequence, KV head), two query heads each, so that 10 bytes of shared memory a key hold a CTA's
 // rows and two CTAs share an SM: one's loads run under the other's softmax. The second reading of the pages comes from L2. Sequences go
 // longest first (the last CTAs to start are the shortest): CTA row y takes the sequence with the y-th largest context.
-// 64 sequences of 512 to 8192 keys, 8 KV heads: 198 us a call with four heads to a CTA (one CTA an SM) in batch order, 145 us now.
+// 64 sequences of 512 to 8192 keys, 8 KV heads: 198 us a call with four heads to a CTA (one CTA an SM) in batch order, 135 to 143 us now.
 constexpr int DEC_RANK_MAX = 1024;         // batches up to this are ordered by length
 template <bool IN_F32, int NT>
 __global__ void __launch_bounds__(NT, 2) dec_attn_fused_kernel(const int8_t* __restrict__ q, const float* __restrict__ qs,

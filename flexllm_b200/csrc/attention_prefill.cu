@@ -25,10 +25,10 @@
 // O (64 columns) = 128 columns, so four CTAs share an SM and their 16 softmax warps hide each other's latencies. S is
 // released as soon as its last columns are in registers: the next tile's product runs under this tile's arithmetic.
 //
-// Bound: instruction issue of the softmax warps (60 % of the issue slots busy; double precision and the special-function
+// Bound: instruction issue of the softmax warps (59 % of the issue slots busy; double precision and the special-function
 // pipe 15 % each, DRAM idle). 4 prompts of 1024 tokens, 32 / 8 heads: 513 us with the exponentials of sweep 1 parked in a
-// scratch (568 MB written and read back through L2), separate fp32 operations and full divisions; 240 us now (252 us with one
-// test per four values in sweep 2, and the rare forms inline).
+// scratch (568 MB written and read back through L2), separate fp32 operations and full divisions; 230 us now (252 us with one
+// test per four values in sweep 2 and the rare forms inline, 243 us with barrier waits that polled).
 #include <cstdlib>
 
 #include "attention_decode.cuh"     // layout of the paged KV cache
