@@ -1,6 +1,6 @@
 // Linear layers of the floating-point model path apart from the tcgen05 GEMMs (gemm_bf16.cu), and the choice between the
-// forms: a weight-streaming GEMV for one token (float activations: up to four), its warp-MMA form for more, and a tiled fp32 GEMM
-// for the 32-bit mode.
+// forms: a weight-streaming GEMV for one or two tokens (T = bf16 or float activations, bf16 weights), its warp-MMA form for
+// more, and a tiled fp32 GEMM for the 32-bit mode.
 #include <atomic>
 
 #include "float_common.cuh"
@@ -291,17 +291,13 @@ int gemv_bt(const T* a, long lda, const bf16* w, long ldw, const float* bias, in
     return launch_gemv<T, BT, 2, 1, GLU>(a, lda, w, ldw, bias, M, N, K, relu2, y, st);
 }
 
-template <class T>               // M <= 4 (bf16: one token, more goes to the MMA forms)
+template <class T>               // M <= 4 (bf16: M <= 2, more goes to the MMA forms)
 int gemv_any(const T* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
 #define FLEXLLM_GEMV(BT_) return act == kActGeluGate ? gemv_bt<T, BT_, true>(a, lda, w, ldw, bias, M, N, K, 0, y, st) \
                                                      : gemv_bt<T, BT_, false>(a, lda, w, ldw, bias, M, N, K, act == kActRelu2, y, st)
-    if constexpr (sizeof(T) == 2) {
-        FLEXLLM_GEMV(1);
-    } else {
-        if (M <= 1) FLEXLLM_GEMV(1);
-        if (M <= 2) FLEXLLM_GEMV(2);
-        FLEXLLM_GEMV(4);
-    }
+    if (M <= 1) FLEXLLM_GEMV(1);
+    if (sizeof(T) == 2 || M <= 2) FLEXLLM_GEMV(2);
+    FLEXLLM_GEMV(sizeof(T) == 2 ? 2 : 4);
 #undef FLEXLLM_GEMV
 }
 
@@ -376,16 +372,17 @@ int linear_bf16(const bf16* a, long lda, const bf16* w, long ldw, const float* b
     TRY_RC(check(a, lda, w, ldw, M, N, K, act, y));
     if (M == 0) return FLEXLLM_OK;
     // Measured on the layer shapes of 1B to 8B models (us; GEMV / warp-MMA / tensor-core form):
-    //   1 token : 5120x2048 5.8 / 7.1 / 9.5, 16384x2048 13.7 / 14.7 / 14.5; long rows 2048x8192 9.6 / 7.6 / 18.6, 4096x14336 29 / 21 / 23
-    //   2 to 8  : 5120x2048 8.0 / 7.1 / 9.5, 16384x2048 15.5 / 14.7 / 14.6, 28672x4096 47 / 39 / 44, head 128256x2048 92 / 77 / 80
-    //   16      : 5120x2048 - / 7.3 / 11.4, 28672x4096 - / 42 / 46; but 4096x14336 - / 31 / 25 and the head - / 95 / 83
-    if (M == 1 && K < 4096) {
+    //   1 token : 5120x2048 5.8 / 7.1 / 9.5, 16384x2048 13.7 / 14.7 / 14.5; long rows 2048x8192 9.6 / 7.6 / 18.6
+    //   2 to 8  : 5120x2048 8.0 / 7.1 / 9.5, 16384x2048 15.5 / 14.7 / 14.6, head 128256x2048 92 / 77 / 80
+    //   16      : 5120x2048 - / 7.3 / 11.4; but 4096x14336 - / 31 / 25 and the head - / 95 / 83
+    // One token, and two of a wide matrix, stay with the GEMV where an MMA form is faster too: its fp32 sums round, 1e-7 of the
+    // result from 64 bits at any length, those of the tensor cores cut bits off and are 2.4e-7 (2048 long) to 1e-6 (8192) away.
+    const bool wide = (N + 127) / 128 >= 100;
+    if ((M == 1 && K <= 12288) || (M == 2 && wide)) {
         const int rc = gemv_any<bf16>(a, lda, w, ldw, bias, M, N, K, act, y, st);
         if (rc != FLEXLLM_ENOTSUP) return rc;
     }
-    const bool wide = (N + 127) / 128 >= 100;
-    if (M <= 8 || (M <= 16 && K <= 8192 && N <= 32768) || (M <= 32 && !wide && (long)N * K <= (17L << 20)))
-        return skinny_mma(a, lda, w, ldw, bias, M, N, K, act, y, st);
+    if (M <= 16 ? !wide : M <= 32 && !wide && (long)N * K <= (17L << 20)) return skinny_mma(a, lda, w, ldw, bias, M, N, K, act, y, st);
     if (M <= 64) return gemm_bf16_decode(a, lda, w, ldw, bias, M, N, K, act, y, st);
     return gemm_bf16_prefill(a, lda, w, ldw, bias, M, N, K, act, y, st);
 }

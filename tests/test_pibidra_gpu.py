@@ -56,6 +56,18 @@ def test_linear(F, dtype, N, K):
         assert np.abs(got - (want - b)).max() < tol * np.abs(want).max(), M
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 4096), (1, 2048, 8192), (1, 4096, 12288), (1, 16384, 4096), (2, 16384, 2048), (2, 28672, 4096)])
+def test_linear_rounded_sums(F, M, N, K):
+    """One token, or two of a wide matrix: sums in fp32 that round after every step, in chains of at most K / 32 terms and a tree. Their
+    distance from 64 bits was measured as 0.8e-7 to 1e-7 of the result at all lengths; sums on the tensor cores, which cut bits off,
+    are from 2.4e-7 up."""
+    g = torch.Generator(device="cuda").manual_seed(K + M)
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    a = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    got, want = F.linear_float(a, w, out_f32=True).double(), a.double() @ w.double().T
+    assert (got - want).norm() < 1.5e-7 * want.norm()
+
+
 @pytest.mark.parametrize("N,K", [(2368, 3000), (2384, 3000), (9456, 520), (9472, 264), (40, 8), (2048, 8200)])
 def test_linear_few_tokens_ring(F, N, K):
     """A few tokens on both sides of the rules that choose the ring's depth and the rows of a CTA, with fewer chunks than the ring holds
