@@ -4,9 +4,10 @@
 // producer warp (128-byte-swizzled K-major tiles), one MMA-issuing thread, four epilogue warps on a
 // double-buffered TMEM accumulator.
 //   prompts: A = activations (128-row side), B = weights (BN rows)
-//   decode : A = weights, B = activations (M <= 64), split over K within a thread-block cluster: each CTA leaves its
-//            fp32 partial tile in shared memory and the cluster's CTAs add them, a share of the tokens each, over
-//            distributed shared memory and in rank order, so the result does not depend on timing
+//   decode : A = weights, B = activations (M <= 64), K split into up to eight parts within a thread-block cluster of up to four
+//            CTAs: a CTA with two parts accumulates them side by side in its two TMEM buffers, leaves its fp32 partial
+//            tiles in shared memory, and the cluster's CTAs add them, a share of the tokens each, over
+//            distributed shared memory and in the order of the parts, so the result does not depend on timing
 // Epilogue: optional bias, optional gated GELU (weight rows alternating in blocks of 16 gate / 16 up rows) or squared ReLU,
 // fp32 or bf16 output.
 #include <atomic>
@@ -23,6 +24,7 @@ namespace {
 struct GemmBfArgs {
     int rowsA, rowsB, num_kb;          // rows of the two sides, K in 128-byte blocks
     int tilesA, tilesB, ksplit;
+    int parts;                         // consecutive K parts of a tile that one CTA takes (1 or 2; the cluster is ksplit / parts CTAs)
     long ldo;
     float* y32; bf16* y16;
     const float* bias;                 // per output channel (row of the weights)
@@ -151,6 +153,10 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = args.num_kb / KCH;
     const int total_tiles = args.tilesA * args.tilesB * args.ksplit;
+    // this CTA's (tile, part) pairs: `parts` neighbours where K is split, else every gridDim.x-th
+    const bool split_k = SWAP && args.ksplit > 1;
+    const int t_first = split_k ? blockIdx.x * args.parts : blockIdx.x, t_end = split_k ? t_first + args.parts : total_tiles;
+    const int t_step = split_k ? 1 : gridDim.x;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
@@ -195,9 +201,9 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
             // decode form: the A side are weights, which no earlier kernel writes. The ring is filled with the first tile's
             // while the kernels before this one still run.
             int ahead = 0;
-            if (SWAP && blockIdx.x < total_tiles) {
-                const int split = blockIdx.x % args.ksplit, ta = blockIdx.x / (args.ksplit * args.tilesB);
-                const int kb0 = (int)((long)split * num_kb / args.ksplit), kb1 = (int)((long)(split + 1) * num_kb / args.ksplit);
+            if (SWAP && t_first < total_tiles) {
+                const int split = t_first % args.ksplit, ta = t_first / (args.ksplit * args.tilesB);
+                const int kb0 = (int)((long)split * num_kb / args.ksplit), kb1 = (int)((long)(split + args.parts) * num_kb / args.ksplit);
                 for (; ahead < STAGES && kb0 + ahead < kb1; ahead++) {
                     mbar_expect_tx(bar_full + 8 * ahead, Cfg::STAGE_BYTES);
                     load_a(ahead, ta, kb0 + ahead);
@@ -206,7 +212,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
             }
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
-            for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
+            for (int t = t_first; ok && t < t_end; t += t_step) {
                 const int split = t % args.ksplit;
                 const int tb = (t / args.ksplit) % args.tilesB;
                 const int ta = t / (args.ksplit * args.tilesB);
@@ -232,7 +238,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
             int stage = 0; uint32_t phase = 0;
             int it = 0;
             bool ok = true;
-            for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, it++) {
+            for (int t = t_first; ok && t < t_end; t += t_step, it++) {
                 const int split = t % args.ksplit;
                 const int kb0 = (int)((long)split * num_kb / args.ksplit), kb1 = (int)((long)(split + 1) * num_kb / args.ksplit);
                 const int as = it & 1;
@@ -263,7 +269,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
         int it = 0;
         bool ok = true;
         float* stg = reinterpret_cast<float*>(ring_ptr + STAGES * Cfg::STAGE_BYTES + 256) + q * Cfg::STG_WARP_FLOATS;
-        for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, it++) {
+        for (int t = t_first; ok && t < t_end; t += t_step, it++) {
             const int split = t % args.ksplit;
             const int tb = (t / args.ksplit) % args.tilesB;
             const int ta = t / (args.ksplit * args.tilesB);
@@ -277,6 +283,8 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
                 for (int i = lane; i < BN; i += 32) bw[i] = (args.bias && tb * BN + i < args.rowsB) ? args.bias[tb * BN + i] : 0.0f;
             const float bA = (SWAP && args.bias && rowA_ok) ? args.bias[rowA] : 0.0f;
             int got = (lane == 0) ? (mbar_wait(bar_tfull + 8 * as, aphase, abort_flag) ? 1 : 0) : 1;
+            // the partial tiles go to the ring: every part's MMAs must have read it
+            if (split_k && it == 0 && args.parts == 2 && lane == 0 && got) got = mbar_wait(bar_tfull + 8, 0, abort_flag) ? 1 : 0;
             got = __shfl_sync(0xffffffffu, got, 0);
             if (!got) { ok = false; break; }
             tc_fence_after();
@@ -297,7 +305,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
 #pragma unroll
                     for (int j = 0; j < 16; j++) {
                         const int tok = tb * BN + c * 16 + j;
-                        if (args.ksplit > 1) part[(c * 16 + j) * 128 + q * 32 + lane] = __uint_as_float(v[j]);
+                        if (split_k) part[(as * BN + c * 16 + j) * 128 + q * 32 + lane] = __uint_as_float(v[j]);
                         else if (tok < args.rowsB) emit(__uint_as_float(v[j]), tok, rowA, row0, bA);
                     }
                 }
@@ -308,23 +316,24 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tcgen05_kernel(const __grid_
         }
     }
 
-    if (SWAP && args.ksplit > 1) {
-        // every CTA of the cluster has one tile, the same for all of them: the partial tiles are in the rings (their MMAs
-        // have finished reading), and CTA r adds up tokens r, r + ksplit, ...
+    if (split_k) {
+        // every CTA of the cluster has the same tile: the partial tiles are in the rings (their MMAs
+        // have finished reading), and CTA r adds up tokens r, r + (CTAs), ...
         tc_fence_before();
         cluster_sync();
         if (warp >= 2 && !*abort_flag) {
-            const int q = warp & 3, ta = blockIdx.x / args.ksplit, r = blockIdx.x % args.ksplit;
+            const int ctas = args.ksplit / args.parts, two = args.parts - 1;
+            const int q = warp & 3, ta = blockIdx.x / ctas, r = blockIdx.x % ctas;
             const int row0 = ta * 128 + q * 32, rowA = row0 + lane;
             const float bA = (args.bias && rowA < args.rowsA) ? args.bias[rowA] : 0.0f;
-            for (int tok = r; tok < args.rowsB; tok += args.ksplit) {
-                float p[4];
+            for (int tok = r; tok < args.rowsB; tok += ctas) {
+                float p[8];
 #pragma unroll
-                for (int k = 0; k < 4; k++)
-                    p[k] = k < args.ksplit ? ld_cluster_f32(cluster_addr(ring + (uint32_t)(tok * 128 + q * 32 + lane) * 4u, k)) : 0.0f;
+                for (int k = 0; k < 8; k++)
+                    p[k] = k < args.ksplit ? ld_cluster_f32(cluster_addr(ring + (uint32_t)(((k & two) * BN + tok) * 128 + q * 32 + lane) * 4u, k >> two)) : 0.0f;
                 float s = p[0];
 #pragma unroll
-                for (int k = 1; k < 4; k++) s += p[k];
+                for (int k = 1; k < 8; k++) s += p[k];
                 emit(s, tok, rowA, row0, bA);
             }
         }
@@ -500,8 +509,8 @@ int launch(const bf16* A, int rowsA, long ldA, const bf16* B, int rowsB, long ld
     }
     const int total = g.tilesA * g.tilesB * g.ksplit;
     if (SWAP && g.ksplit > 1) {
-        // one tile per CTA, the splits of a tile form a cluster
-        launch_cluster(kern, dim3(total), dim3(192), g.ksplit, (size_t)Cfg::SMEM_BYTES, st, ta, tb, g);
+        // the CTAs with the parts of a tile (tilesB is 1) form a cluster
+        launch_cluster(kern, dim3(total / g.parts), dim3(192), g.ksplit / g.parts, (size_t)Cfg::SMEM_BYTES, st, ta, tb, g);
         return launch_status();
     }
     const int grid = total < gemm_sm_count() ? total : gemm_sm_count();
@@ -511,7 +520,7 @@ int launch(const bf16* A, int rowsA, long ldA, const bf16* B, int rowsB, long ld
 
 GemmBfArgs base_args(const float* bias, int act, const LinearOut& y) {
     GemmBfArgs g = {};
-    g.ksplit = 1; g.ldo = y.ld; g.y32 = y.f32; g.y16 = (bf16*)y.t; g.bias = bias;
+    g.ksplit = 1; g.parts = 1; g.ldo = y.ld; g.y32 = y.f32; g.y16 = (bf16*)y.t; g.bias = bias;
     g.glu = act == kActGeluGate; g.relu2 = act == kActRelu2;
     return g;
 }
@@ -537,17 +546,21 @@ int gemm_bf16_decode(const bf16* a, long lda, const bf16* w, long ldw, const flo
                      cudaStream_t st) {
     if (M > 64) return FLEXLLM_ENOTSUP;
     GemmBfArgs g = base_args(bias, act, y);
-    // K blocks per pipeline stage: longer contiguous runs per weight row and TMA request
-    // ... as long as the splits that give every SM work keep two steps each
-    // (clusters of at most four: with eight, 64 tokens of 2048 x 2048 took 21.1 us instead of 13.4, of 2048 x 8192 28.7 instead of 19.5)
+    // Parts of K: as many, up to eight, as leave no SM with two tiles and keep two steps each. A tensor-core sum cuts bits off at
+    // every step, so its distance from 64 bits grows with its length (64 tokens of 2048 x 2048, of 2048 x 8192: 2.3e-7 and 1.0e-6 of the
+    // result with eight parts, 4.7e-7 and 2.1e-6 with four), which is why there are eight also in clusters of four.
+    // Clusters of at most four CTAs: 64 tokens of 2048 x 2048 take 12.3 us, of 2048 x 8192 18.3 us; with eight CTAs 22.6 and
+    // 29.2 us (large clusters start and meet later).
     const int kb = (K + 63) / 64, tiles = (N + 127) / 128;
     int ks = 1;
-    while (ks < 4 && tiles * ks * 2 <= gemm_sm_count() && kb >= 4 * ks) ks *= 2;
+    while (ks < 8 && tiles * ks * 2 <= gemm_sm_count() && kb >= 4 * ks) ks *= 2;
+    // K blocks per pipeline stage: longer contiguous runs per weight row and TMA request
     int kch = 1;
     if (lda % 64 == 0 && ldw % 64 == 0) {
         if (kb % 4 == 0 && kb / 4 >= 2 * ks) kch = 4;
         else if (kb % 2 == 0 && kb / 2 >= 2 * ks) kch = 2;
     }
+    g.parts = ks > 4 ? 2 : 1;
     g.ksplit = ks;
 #define FLEXLLM_DEC(BN_, KCH_) return launch<BN_, true, KCH_>(w, N, ldw, a, M, lda, K, g, st)
     if (M > 32) { if (kch == 4) FLEXLLM_DEC(64, 4); if (kch == 2) FLEXLLM_DEC(64, 2); FLEXLLM_DEC(64, 1); }
