@@ -312,7 +312,7 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     if (tid < G) {
         float m = red[tid][0];
         for (int i = 1; i < NT / 32; i++) m = fmaxf(m, red[tid][i]);
-        row_max[tid] = m;
+        row_max[tid] = m + 0.0f;               // a zero without a sign: max - x is then never -0 (exp_warp)
     }
     named_sync_id<NT>(bar);
     // the V scales of this thread's first UF keys (step F) are requested now: their latency hides behind

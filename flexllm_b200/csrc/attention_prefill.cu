@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
         };
         const int first_masked = 2 * qt;                       // tiles before this one are visible to every row of the CTA
 
-        // ---- sweep 0: the row maximum, tracked WITHOUT the factor 0.125 (scaling by a power of two is exact and keeps the
-        // order, so max(x * 0.125) == max(x) * 0.125: applied once after the sweep)
+        // ---- sweep 0: the row maximum, tracked WITHOUT the factor 0.125 (scaling by a power of two keeps the order: applied
+        // once after the sweep)
         float mx = -1e32f;
         for (int j = 0; ok && j < n_kt; j++) {
             if (!scores_ready(j)) { ok = false; break; }
@@ -402,12 +402,15 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
                 for (int i = 0; i < 16; i += 2) mx = max3(mx, x[i], x[i + 1]);
             }
         }
-        mx = mx * 0.125f;
+        // Rounded up and without a sign if it is zero: max - x below is then never negative and never -0, which exp_warp does not take.
+        // (The product is exact unless |max| < 2^-123; there the last bit of a subnormal makes no difference to the exponentials.)
+        mx = __fmul_ru(mx, 0.125f) + 0.0f;
         const f32x2 mx2 = pack2(mx, mx), neg8th = pack2(-0.125f, -0.125f);
 
         // ---- sweep 1: e = exp(-u) with u = max - x, and the four ordered chains (key mod 4 == i mod 4, because a chunk starts at
         // a multiple of 16; adding the exact zeros of masked keys leaves the sums unchanged, as in the reference). max - x is
-        // one fused step: x = y / 8 is exact, so a single rounding is left, the subtraction's.
+        // one fused step: x = y / 8 is exact, so a single rounding is left, the subtraction's. (Only for |y| < 2^-123 does y / 8 round in
+        // the reference and not here; u can then differ where it is below 2^-100, and its exponential is 1 on both sides.)
         f32x2 s01 = pack2(0.f, 0.f), s23 = s01;
         const ExpTable tab = exp_table_lane();
         for (int j = 0; ok && j < n_kt; j++) {

@@ -100,6 +100,19 @@ def test_prefill_quantiser_ranges(F, what):
     assert_same(to_np(out), ref["out"], "fp32 output")
 
 
+@pytest.mark.parametrize("e", [-62, -64, -66, -70, -80])
+def test_prefill_scores_below_the_normal_range(F, e):
+    """Scores, or their eighths, that are subnormal or round to a zero of either sign: every exponential is 1. One visible key and many."""
+    B, S, HQ, HKV = 1, 208, 8, 2
+    q, qs, k, ks, v, vs, a_s = attn_inputs(B, S, HQ, HKV, 81)
+    qs *= np.float32(2.0) ** e; ks *= np.float32(2.0) ** e
+    cos_t, sin_t = oracle.rope_table(S)
+    out, oacc = F.MHA_i8xi8_Prefilling(dev(q), dev(qs), dev(k), dev(ks), dev(v), dev(vs), dev(cos_t), dev(sin_t), dev(a_s), want_oacc=True)
+    ref = oracle.mha_prefill(q, qs, k, ks, v, vs, cos_t, sin_t, a_s)
+    assert_same(to_np(oacc), ref["oacc"], "int32 P.V accumulators")
+    assert_same(to_np(out), ref["out"], "fp32 output")
+
+
 @pytest.mark.parametrize("what", ["q", "k", "tables"])
 def test_prefill_prepare_alignment(F, what):
     """Inputs whose address allows no wide loads take the other form of the preparation."""
@@ -186,7 +199,8 @@ def test_prefill_online_softmax_variant_is_close(F, B, S, HQ, HKV):
 
 
 # ------------------------------------------------------------------------------ decode (config 4)
-def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1, q_gain=1.0, v_gain=1.0, a_gain=1.0):
+def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1, q_gain=1.0, v_gain=1.0, a_gain=1.0, k_gain=1.0, signed_from=None):
+    """signed_from n: keys before position n point against the first query head of their group, the others along it."""
     g = np.random.default_rng(seed)
     PAGE = 64
     ctx = np.asarray(ctx, np.int32)
@@ -206,10 +220,10 @@ def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1, q_gain=1.0, v_gain=1.
     max_ctx = int(ctx.max()) + steps
     cos_t, sin_t = oracle.rope_table(max_ctx + 1)
     a_s = np.full(HQ, 0.05 / 255 * a_gain, np.float32)
-    vs_pool *= np.float32(v_gain)
+    vs_pool *= np.float32(v_gain); ks_pool *= np.float32(k_gain)
     cache = F.KVCache(1, n_pages, HKV)
     kd, ksd, vd, vsd = cache.pools(0)
-    kd.copy_(dev(k_pool)); ksd.copy_(dev(ks_pool)); vsd.copy_(dev(vs_pool))
+    ksd.copy_(dev(ks_pool)); vsd.copy_(dev(vs_pool))
     vd.copy_(dev(np.ascontiguousarray(v_pool.transpose(0, 1, 3, 2))))
     cur = ctx.copy()
     for step in range(steps):
@@ -217,7 +231,13 @@ def decode_case(F, B, ctx, HQ=32, HKV=8, seed=40, steps=1, q_gain=1.0, v_gain=1.
         v = g.integers(-127, 128, (B, HKV, 64), dtype=np.int8)
         qs = g.uniform(0.005, 0.05, (B, HQ)).astype(np.float32); ks = g.uniform(0.005, 0.05, (B, HKV)).astype(np.float32)
         vs = g.uniform(0.005, 0.05, (B, HKV)).astype(np.float32) * np.float32(v_gain)
-        qs *= np.float32(q_gain)
+        qs *= np.float32(q_gain); ks *= np.float32(k_gain)
+        if signed_from is not None:
+            prepared = oracle.qk_prepare(q.reshape(B, HQ, 64), qs, cur, cos_t, sin_t)[0]
+            for b in range(B):
+                along = np.where(prepared[b, ::HQ // HKV] < 0, -100, 100).astype(np.int8)
+                for t in range(cur[b]): k_pool[page_table[b, t // PAGE], :, t % PAGE] = -along if t < signed_from else along
+        if step == 0: kd.copy_(dev(k_pool))
         out, oacc = F.MHA_i8xi8_Decoding(cache, 0, dev(q), dev(qs), dev(k), dev(ks), dev(v), dev(vs), dev(cos_t), dev(sin_t),
                                          dev(a_s), dev(page_table), dev(cur), max_ctx, want_oacc=True)
         torch.cuda.synchronize()
@@ -256,6 +276,17 @@ def test_decode_quantiser_ranges(F, what):
     """Both sides of every line that the exponential and the quantiser draw (as in the prompt kernel's test), with lengths on both sides
     of a block of the ordered sums, equal lengths, and the longest sequence neither first nor last."""
     decode_case(F, 7, [62, 126, 127, 700, 62, 0, 255], seed=46, **what)
+
+
+@pytest.mark.parametrize("e", [-62, -66, -70, -80])
+def test_decode_scores_below_the_normal_range(F, e):
+    """As in the prompt kernel's test; at 2^-80 every score is a zero, of the sign of the integer it comes from."""
+    decode_case(F, 7, [62, 126, 127, 700, 62, 0, 255], seed=47, q_gain=2.0 ** e, k_gain=2.0 ** e)
+
+
+def test_decode_maximum_of_either_zero(F):
+    """Scores that underflow to -0 in the keys that every thread sees first and to +0 in later ones."""
+    decode_case(F, 2, [300, 700], seed=48, q_gain=2.0 ** -80, k_gain=2.0 ** -80, signed_from=128)
 
 
 def test_kv_append_alone(F):
