@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256) rmsnorm_decode_kernel(const float* __rest
     }
     __syncthreads();
     const float r = rinv_sm;
-    float o[4 * MAXV], mx = 0.0f, nan = 0.0f;
+    float o[4 * MAXV], mx = -1.0f, nan = 0.0f;           // mx stays below zero if every value is NaN
 #pragma unroll
     for (int i = 0; i < MAXV; i++) {
         const int c = tid + i * 256;
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(256) rmsnorm_decode_kernel(const float* __rest
         o[4 * i + 2] = in ? (v[i].z * r) * g[i].z : 0.0f; o[4 * i + 3] = in ? (v[i].w * r) * g[i].w : 0.0f;
         if (in && y) reinterpret_cast<float4*>(y + row * D)[c] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
 #pragma unroll
-        for (int k = 0; k < 4; k++) { mx = fmaxf(mx, fabsf(o[4 * i + k])); nan = max3_nan(nan, nan, o[4 * i + k]); }
+        for (int k = 0; k < 4; k++) { if (in) mx = fmaxf(mx, fabsf(o[4 * i + k])); nan = max3_nan(nan, nan, o[4 * i + k]); }
     }
     if (!q) return;
     mx = warp_max(mx);
@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(256) rmsnorm_decode_kernel(const float* __rest
     const int bad = __syncthreads_or(!(nan == nan));
 #pragma unroll
     for (int w = 0; w < 8; w++) mx = fmaxf(mx, red[w]);
+    if (mx < 0.0f) mx = 1e32f;                            // the reference's starting values
     const float sc = sym_scale_from(mx, -mx);
     if (tid == 0) s[row] = sc;
     uint32_t b[4 * MAXV];

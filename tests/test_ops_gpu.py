@@ -193,6 +193,19 @@ def test_rmsnorm_forms(F, order, M, D):
     assert_same(to_np(y), yo, "y"); assert_same(to_np(s), so, "scale"); assert_same(to_np(q), qo, "q")
 
 
+@pytest.mark.parametrize("order", [4, 8])
+@pytest.mark.parametrize("D", [512, 2048, 2080])
+def test_rmsnorm_row_of_nan(F, order, D):
+    """A NaN makes the whole row NaN: the quantiser's scale is then that of its starting values, as the reference's loop leaves them."""
+    x = rng(91).standard_normal((3, D)).astype(np.float32); gamma = np.ones(D, np.float32)
+    x[1, 7] = np.nan
+    y, q, s = F.pref_Layer_Norm(dev(x), dev(gamma), 1e-5, order, quant=True)
+    yo = oracle.rmsnorm(x, gamma, 1e-5, order)
+    assert np.isnan(to_np(y)[1]).all() and np.isnan(yo[1]).all()
+    _, so = oracle.quant_per_token(yo)
+    assert_same(to_np(s), so, "scale"); assert not to_np(q)[1].any()
+
+
 @pytest.mark.parametrize("order", [0, 4, 8])
 @pytest.mark.parametrize("M", [1, 64, 130])
 def test_rmsnorm_quant(F, order, M):
