@@ -465,8 +465,8 @@ __device__ __forceinline__ void mega_row_fht4(const MegaArgs& a, const MegaLayer
     }
     named_sync<MG_BAR_WORK, MG_WORKERS>();
     if (*abort_flag) return;
-    const float all = __uint_as_float(__ldcg(amax_bits)), top = all / a.fht_scale;
-    const float sc = sym_scale_from(top, -top);
+    const float all = __uint_as_float(__ldcg(amax_bits));
+    const float sc = fht_row_scale(all, a.fht_scale);
     if (part == 0 && tid == 0) a.xs[row] = sc;
     uint32_t q[4];
     const float fs = a.fht_scale;

@@ -118,8 +118,7 @@ __global__ void __launch_bounds__(128, 4) fht8192_kernel(const float* __restrict
     __syncthreads();
     mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
     const bool ok = fht_q8_in_range(mx, scale) && (red_nan[0] + red_nan[1]) + (red_nan[2] + red_nan[3]) == 0.0f;
-    const float top = mx / scale;
-    const float sc = sym_scale_from(top, -top);
+    const float sc = fht_row_scale(mx, scale);
     if (tid == 0) s[row] = sc;
 #pragma unroll
     for (int h0 = 0; h0 < 32; h0 += 4) {
@@ -211,8 +210,7 @@ __global__ void __launch_bounds__(128) fht8192_cluster_kernel(const float* __res
     mx = 0.0f;
 #pragma unroll
     for (int v = 0; v < FHT_CL; v++) { mx = fmaxf(mx, peer_mx[v]); any_bad |= peer_bad[v]; }
-    const float top = mx / scale;
-    const float sc = sym_scale_from(top, -top);
+    const float sc = fht_row_scale(mx, scale);
     if (part == 0 && tid == 0) s[row] = sc;
     uint32_t b[8];
     q8_short(r, 1.0f / (scale * sc), fht_q8_in_range(mx, scale) && !any_bad, b, [&](float v) { return fht_q8_exact(v, scale, sc); });

@@ -25,6 +25,12 @@ __device__ __forceinline__ void reg_butterfly(float (&r)[N]) {
 __device__ __noinline__ static uint32_t fht_q8_exact(float x, float scale, float sc) {
     return (uint32_t)round_half_away_to_int((x / scale) / sc) & 0xffu;
 }
+// The quantiser's scale of a row whose largest transformed magnitude is mx, divided by `scale`: the largest quotient is the quotient of
+// the largest. Quotients that are NaN (a divisor of 0, infinity or NaN) do not count.
+__device__ __forceinline__ float fht_row_scale(float mx, float scale) {
+    const float top = fmaxf(fabsf(mx / scale), 0.0f);
+    return sym_scale_from(top, -top);
+}
 // May q8_short be used on a row whose largest transformed magnitude is mx? (Values far below mx give a quotient far below a half
 // either way.)
 __device__ __forceinline__ bool fht_q8_in_range(float mx, float scale) {

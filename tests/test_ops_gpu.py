@@ -142,6 +142,21 @@ def test_swiglu_fht_quant_forms(F, M, what):
     assert_same(to_np(s), so, "scale"); assert_same(to_np(q), qo, "q")
 
 
+@pytest.mark.parametrize("M", [2, 400])                    # either form
+def test_swiglu_fht_quant_degenerate_divisor(F, M):
+    """A divisor that makes every quotient NaN counts as a row without values: scale 1. Infinite and negative ones as any other."""
+    g = (rng(503).standard_normal((M, 8192)) * 2).astype(np.float32); u = rng(504).standard_normal((M, 8192)).astype(np.float32)
+    u[M - 1] = 0
+    for d in (0.0, np.nan, np.inf, -90.5):
+        _, s, act = F.swiglu_fht_quant(dev(g), dev(u), want_act=True, scale=d)
+        h = oracle.fht(to_np(act), 1.0)
+        with np.errstate(all="ignore"):
+            top = np.fmax.reduce(np.abs(h / np.float32(d)), axis=1, initial=0.0)
+            want = (top / np.float32(127)).astype(np.float32)
+        want[want == 0] = 1
+        assert_same(to_np(s), want, f"scale of rows divided by {d}")
+
+
 @pytest.mark.parametrize("T,H", [(1, 8), (100, 32), (33, 1)])
 def test_qk_prepare(F, T, H):
     g = rng(7)
