@@ -217,9 +217,10 @@ __global__ void __launch_bounds__(128) fht8192_cluster_kernel(const float* __res
 #pragma unroll
     for (int v = 0; v < 8; v++) q[row * N + v * L + part * 128 + tid] = (int8_t)b[v];
 }
-// Rows up to which the cluster form is taken: 1 / 64 / 148 / 296 rows take it 6.1 / 8.0 / 11.5 / 16.5 us, the other form
-// 8.3 / 9.2 / 10.8 / 12.4 us (one CTA of 256 threads per row, in three exchanges, took 10.3 us for 1 row, 10.9 us for 64).
-constexpr int FHT_CLUSTER_ROWS = 148;
+// Rows up to which the cluster form is taken: 1 / 64 / 128 / 142 / 143 / 148 / 296 rows take it 3.5 / 6.0 / 7.5 / 8.3 / 9.3 / 9.8 / 15.0 us, the
+// other form 6.8 / 8.1 / 8.5 / 9.1 / 9.1 / 9.2 / 10.7 us (launches of a graph, inputs from memory; with 143 clusters a second wave begins). One
+// CTA of 256 threads per row, in three exchanges, took 7.7 us for 1 row, 9.5 us for 64, 10 us for 148.
+constexpr int FHT_CLUSTER_ROWS = 142;
 
 static int swiglu_fht_quant(const float* g, const float* u, long ld, int M, float scale, int8_t* q, float* s, float* act, cudaStream_t st) {
     if (M == 0) return FLEXLLM_OK;
