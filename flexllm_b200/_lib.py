@@ -109,6 +109,7 @@ SIGNATURES = {
     "flexllm_model_buffer": [_P, _I, _P],
     "flexllm_model_limits": [_P, _P, _P, _P],
     "flexllm_debug_hook": [_I, C.c_longlong],
+    "flexllm_exp_probe": [_P, _L, _I, _P, _P],
     "flexllm_gemm_i8_mainloop_probe": [_P, _P, _I, _I, _I, _P],
 }
 

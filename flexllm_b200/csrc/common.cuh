@@ -369,7 +369,7 @@ __device__ __forceinline__ void ref_expf_x4(const float (&x)[4], float (&e)[4]) 
 // The table of 2^(j/32) lives in the warp's registers, lane j holding entry j (a shuffle instead of a load that random
 // indices make conflict). Where the sign is known (NEG: exp(-u), u >= 0) the argument becomes a double by integer shifts:
 // conversions to and from double share one pipe of 16 lanes a clock, which the conversion of the result keeps half busy.
-// Checked against the accurate form for every float in the range: no difference where the test lets the fast result stand.
+// tests/test_ops_gpu.py compares every float in the range, either sign and both forms, with (float)exp((double)x): no difference.
 // Cycles per 32 values and scheduler, 16 warps an SM: 52 in the four-wide form above, 32 here by fours, 29 by eights.
 constexpr float kExpFastLimit = 87.0f;
 
@@ -425,8 +425,9 @@ __device__ __forceinline__ float4 silu_mul_x4(const float4 g, const float4 u) {
 }
 
 // The same on NV (4 or 8) values of every lane of a warp (whole-warp call): o = (g / (1 + exp(-g))) * u, each operation rounded once.
-// The quotient: y = 1 / D from rcp.approx and one Newton step, q = RN(g y), one exact residual r = g - q D, RN(q + r y). For
-// the pairs (g, 1 + exp(-g)) that occur here this is the correctly rounded quotient: compared with the division for every
+// The quotient: y = 1 / D from rcp.approx and one Newton step, q = RN(g y), one exact residual r = g - q D, RN(q + r y) (Markstein's
+// last step, but from a y that need not be correctly rounded). There is no proof for all pairs; for the pairs (g, 1 + exp(-g)) that
+// occur here it is the correctly rounded quotient: tests/test_ops_gpu.py compares it with the division for every
 // float g with 2^-60 <= |g| <= 80. Other values (and NaN) send the warp to the division itself.
 template <int NV> __device__ __forceinline__ void silu_mul_warp(const float (&g)[NV], const float (&u)[NV], float (&o)[NV], const ExpTable& tab) {
     float far = fabsf(g[0]), near = far;

@@ -611,6 +611,30 @@ extern "C" int flexllm_rmsnorm_quant(const float* x, const float* gamma, int M, 
     return launch_status();
 }
 
+// See include/flexllm_b200.h: both forms of exp_warp, eight values of every lane, as the kernels call them.
+static __global__ void __launch_bounds__(256) exp_probe_kernel(const float* __restrict__ x, long n, int negated, float* __restrict__ y) {
+    const ExpTable tab = exp_table_lane();
+    const long base = ((long)blockIdx.x * 256 + threadIdx.x) * 8;
+    float v[8], e[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        v[i] = base + i < n ? x[base + i] : 0.0f;
+        if (!(fabsf(v[i]) <= kExpFastLimit)) v[i] = 0.0f;
+    }
+    if (negated) exp_warp<true>(v, e, tab);
+    else exp_warp<false>(v, e, tab);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        if (base + i < n) y[base + i] = e[i];
+}
+
+extern "C" int flexllm_exp_probe(const float* x, long n, int negated, float* y, void* stream) {
+    FLEXLLM_REQUIRE(x && y && n >= 0 && n <= (1L << 31) && (negated == 0 || negated == 1));
+    if (n == 0) return FLEXLLM_OK;
+    exp_probe_kernel<<<(unsigned)((n + 2047) / 2048), 256, 0, (cudaStream_t)stream>>>(x, n, negated, y);
+    return launch_status();
+}
+
 extern "C" int flexllm_swish(const float* g, long n, float* y, void* stream) {
     FLEXLLM_REQUIRE(g && y && n >= 0 && aligned(g, 16) && aligned(y, 16));
     if (n == 0) return FLEXLLM_OK;

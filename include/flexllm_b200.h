@@ -488,6 +488,10 @@ FLEXLLM_API int flexllm_model_set_sampling_host(flexllm_model* m, int lanes, int
  * the int8 tensor-core ceiling this library's main loop reaches on the device (N > 128). */
 FLEXLLM_API int flexllm_gemm_i8_mainloop_probe(const int8_t* a, const int8_t* w, int M, int N, int K, void* stream);
 
+/* Test aid: y[i] = exp(x[i]) (negated: exp(-x[i]), x[i] >= 0 and not -0) for |x[i]| <= 87 by the short exponential of the attention
+ * and SiLU kernels, which is to be the correctly rounded one; any other x[i] counts as 0. n <= 2^31. */
+FLEXLLM_API int flexllm_exp_probe(const float* x, long n, int negated, float* y, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * The reference's on-disk model (its demo's parameters/ directory; host code, HOST buffers):
  *   <proj>_L%02d.bin int8 [out][in]; w_<proj>_s_sum.h with w_<proj>_s / w_<proj>_sum [layers][out]; w_rmsnorm.h with

@@ -157,6 +157,41 @@ def test_swiglu_fht_quant_degenerate_divisor(F, M):
         assert_same(to_np(s), want, f"scale of rows divided by {d}")
 
 
+def float_patterns(first, last, chunk):
+    """All floats whose bits lie in [first, last), `chunk` at a time (the last chunk filled up with ones)."""
+    for at in range(first, last, chunk):
+        v = torch.arange(at, at + chunk, dtype=torch.int64, device="cuda").to(torch.int32).view(torch.float32)
+        v[max(0, last - at):] = 1.0
+        yield v
+
+
+def same_bits(a, b):
+    return torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("negated,first", [(0, 0), (0, 1 << 31), (1, 0)], ids=["positive", "negative", "negated"])
+def test_short_exponential_every_float(F, negated, first):
+    """The short exponential on every float up to 87 in magnitude, zeros and subnormals among them, is (float)exp((double)x)."""
+    limit = int(np.float32(87.0).view(np.uint32))
+    for x in float_patterns(first, first + limit + 1, 1 << 26):
+        y = torch.empty_like(x)
+        assert F.lib().flexllm_exp_probe(x.data_ptr(), x.numel(), negated, y.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        want = torch.exp(-x.double() if negated else x.double()).float()
+        assert same_bits(y, want), x[y != want][:5]
+
+
+@pytest.mark.parametrize("first", [0, 1 << 31], ids=["positive", "negative"])
+def test_silu_every_float(F, first):
+    """silu(g) * 1 as the fused kernel forms it, for every float g up to 81 in magnitude: the short quotient (2^-60 to 80, where a whole warp
+    lies in that range) is the division's."""
+    M = 4096
+    one = torch.ones((M, 8192), device="cuda")
+    for g in float_patterns(first, first + int(np.float32(81.0).view(np.uint32)) + 1, M * 8192):
+        act = F.swiglu_fht_quant(g.view(M, 8192), one, want_act=True)[2].view(-1)
+        want = g / (1 + torch.exp(-g.double()).float())
+        assert same_bits(act, want), g[act != want][:5]
+
+
 @pytest.mark.parametrize("T,H", [(1, 8), (100, 32), (33, 1)])
 def test_qk_prepare(F, T, H):
     g = rng(7)
