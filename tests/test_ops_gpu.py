@@ -385,6 +385,52 @@ def test_linear_decode_tcgen05(F, M, N, K):
     assert_same(to_np(y2), y_o, "y (scratch)")
 
 
+def test_linear_decode_streams_at_once(F):
+    """The layer keeps nothing between calls: launches that overlap on several streams do not touch one another's sums."""
+    M, N, K = 40, 2048, 8192
+    work = []
+    for i in range(4):
+        a, st, w, sc = lin_inputs(M, N, K, 60 + i)
+        work.append(([dev(x) for x in (a, st, w, sc)], oracle.linear_i8(a, st, w, sc)[1], torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    got = [[] for _ in work]
+    for _ in range(8):
+        for i, (t, _, stream) in enumerate(work):
+            with torch.cuda.stream(stream):
+                got[i].append(F.dec_Linear_Layer_i8xi8(*t)[1])
+    torch.cuda.synchronize()
+    for i, (_, want, _) in enumerate(work):
+        for y in got[i]:
+            assert_same(to_np(y), want, f"stream {i}")
+
+
+FIRST_CALL = """
+import sys; sys.path.insert(0, %r)
+import torch, flexllm_b200 as F
+torch.manual_seed(0)
+M, N, K = 40, 2048, 2048
+a = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda"); w = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda")
+s = torch.rand(M, device="cuda"); c = torch.rand(N, device="cuda")
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = F.dec_Linear_Layer_i8xi8(a, s, w, c)[1]
+g.replay(); torch.cuda.synchronize()
+want = ((a.double() @ w.double().T).float() * s[:, None]) * c[None]
+assert torch.equal(y, want)
+print("same")
+"""
+
+
+def test_linear_decode_first_call_in_a_capture():
+    """A process whose first call of the layer is captured into a graph."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL % root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stdout[-500:] + r.stderr[-1500:]
+
+
 @pytest.mark.parametrize("M,N,K,decode", [(200, 2048, 2048, False), (130, 264, 144, False), (1, 2048, 2048, True), (5, 512, 2048, True),
                                             (32, 2048, 2048, True), (64, 2048, 8192, True), (20, 3072, 2048, True)])
 def test_linear_fused_residual(F, M, N, K, decode):
