@@ -150,42 +150,6 @@ __global__ void static_quant_kernel(const float* __restrict__ x, long rows, int 
 // ---------------------------------------------------------------------------------------------
 constexpr int RMS_PIECE = 128;           // floats per row per staging step
 
-template <int MAXV>  // float4 per lane kept in registers for the output pass (D <= MAXV*128)
-__device__ __forceinline__ void rmsnorm_output_row(const float* __restrict__ xr, const float* __restrict__ gamma, int D, float r,
-                                                   float* __restrict__ yr, int8_t* __restrict__ qr8, float* __restrict__ srow, int lane) {
-    const int nv = D >> 2;
-    float4 o[MAXV];
-    float mx = -1e32f, mn = 1e32f;
-#pragma unroll
-    for (int i = 0; i < MAXV; i++) {
-        int c = lane + i * 32;
-        if (c < nv) {
-            float4 v = reinterpret_cast<const float4*>(xr)[c];
-            float4 g = reinterpret_cast<const float4*>(gamma)[c];
-            o[i].x = (v.x * r) * g.x; o[i].y = (v.y * r) * g.y; o[i].z = (v.z * r) * g.z; o[i].w = (v.w * r) * g.w;
-            if (yr) reinterpret_cast<float4*>(yr)[c] = o[i];
-            mx = fmaxf(mx, fmaxf(fmaxf(o[i].x, o[i].y), fmaxf(o[i].z, o[i].w)));
-            mn = fminf(mn, fminf(fminf(o[i].x, o[i].y), fminf(o[i].z, o[i].w)));
-        }
-    }
-    if (qr8) {
-        mx = warp_max(mx); mn = warp_min(mn);
-        const float sc = sym_scale_from(mx, mn);
-    const DivBy dsc = div_by(sc);       // one reciprocal per row: every element is then quantised without a full division
-        if (lane == 0) *srow = sc;
-        char4* qr = reinterpret_cast<char4*>(qr8);
-#pragma unroll
-        for (int i = 0; i < MAXV; i++) {
-            int c = lane + i * 32;
-            if (c < nv) {
-                char4 w;
-                w.x = (int8_t)round_half_away_to_int(div_for_rounding(o[i].x, dsc)); w.y = (int8_t)round_half_away_to_int(div_for_rounding(o[i].y, dsc)); w.z = (int8_t)round_half_away_to_int(div_for_rounding(o[i].z, dsc)); w.w = (int8_t)round_half_away_to_int(div_for_rounding(o[i].w, dsc));
-                qr[c] = w;
-            }
-        }
-    }
-}
-
 // Prefill order: a CTA of 8 warps takes 8 consecutive rows. All threads bring the rows into shared memory (coalesced
 // 128-bit loads, all in flight at once); warp 0 then runs the 32 chains (4 per row) over them; afterwards every warp
 // normalises and quantises one row straight from shared memory -- each row is read from global memory once. Row stride

@@ -231,9 +231,10 @@ def test_softmax_summation_order_is_the_reference(F):
 
 
 # ------------------------------------------------------------------------------ RMSNorm
-@pytest.mark.parametrize("order,M,D", [(8, 1, 2048), (4, 592, 512), (8, 593, 512), (8, 3, 4096), (4, 5, 96), (0, 9, 2048), (0, 5, 3968), (0, 3, 128)])
+@pytest.mark.parametrize("order,M,D", [(8, 1, 2048), (4, 592, 512), (8, 593, 512), (8, 3, 4096), (4, 5, 96), (4, 2, 2048), (4, 2, 2064), (8, 2, 2080), (0, 9, 2048), (0, 5, 3968), (0, 3, 128)])
 def test_rmsnorm_forms(F, order, M, D):
-    """Row counts on both sides of the rule between the decode forms, widths that do not fill the last block of the sums."""
+    """Few rows and many, widths on both sides of the decode form's line between two and four vectors a thread (2048), and widths that do
+    not fill the last block of the sums."""
     g = rng(90)
     x = (g.standard_normal((M, D)) * 3).astype(np.float32); gamma = (1 + 0.1 * g.standard_normal(D)).astype(np.float32)
     x[0] *= np.float32(2.0) ** -62                            # normalised values far below the others
