@@ -120,9 +120,10 @@ __device__ __noinline__ static uint32_t dec_u8_exact(float e, float rinv, float 
     const int r = round_half_away_to_int(((e * rinv) * vs) / a_s);
     return (uint32_t)(r > 255 ? 255 : r) & 0xffu;
 }
-// The same without divisions: (e c) vs with c = r / (255.25 a_s) (dec_u8_factor), held at 1, is within 2^-21 of the reference's
-// quotient / 255.25 (seven roundings), so where the two sides of 2^-19 round to the same integer, that is U; otherwise, and outside
-// the range of the bound, the reference's arithmetic decides.
+// The same without divisions: (e c) vs with c = r / (255.25 a_s) (dec_u8_factor), held at 1, times 255.25 is within 2^-20.5 of the
+// reference's quotient: three roundings there (e r, vs, / a_s), seven here (1 / a_s, r times it, the constant 1 / 255.25, the product with it,
+// e c, vs, the constant 255.25 (1 +- 2^-19)), each 2^-24. So where the two sides of 2^-19 round to the same integer, that is U;
+// otherwise, and outside the range of the bound, the reference's arithmetic decides.
 __device__ __forceinline__ float dec_u8_factor(float rinv, float a_s, bool& ok) {
     const float c = (rinv * (1.0f / a_s)) * (1.0f / 255.25f);
     ok = c >= 0x1p-60f && c <= 0x1p60f;
