@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_launch();
-    if (!SWAP || warp != 0) pdl_wait();                  // (the decode form's producer asks for weights first)
+    if (!SWAP || warp != 0) pdl_wait();                  // (the decode form's producer has its own wait below)
     const int num_kb = ((args.K + 127) >> 7) / KCH;      // pipeline steps of KCH chunks (K % (128*KCH) == 0 when KCH > 1)
     const int total_tiles = args.tilesA * args.tilesB * args.ksplit;
 
@@ -278,8 +278,9 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
                 if (KCH == 1) tma_load_2d(dst, &tmapA, bar_full + 8 * st, kb * 128, ta * 128);
                 else tma_load_3d(dst, &tmapA, bar_full + 8 * st, 0, ta * 128, kb * KCH);
             };
-            // decode form: the A side are weights, which no earlier kernel writes. The ring is filled with the first tile's
-            // while the kernels before this one still run.
+            // decode form: the A side are weights, which no earlier kernel writes. The ring is filled with the first tile's before the
+            // activations are asked for. (Not while the kernels before this one still run: the other warps have waited for those ahead
+            // of the barrier above.)
             int ahead = 0;
             if (SWAP && blockIdx.x < total_tiles) {
                 const int split = blockIdx.x % args.ksplit, ta = blockIdx.x / (args.ksplit * args.tilesB);
