@@ -255,14 +255,16 @@ int launch_skinny(const bf16* a, long lda, const bf16* w, long ldw, const float*
     launch_k(kern, dim3((N + RT * 16 - 1) / (RT * 16)), dim3(256), smem, st, a, lda, w, ldw, bias, M, N, kv, relu2, y.f32, (bf16*)y.t, y.ld);
     return launch_status();
 }
-// Depth of the ring: about 74 KB a CTA, so that three share an SM; twice that where the grid leaves one CTA an SM at most.
+// Two blocks of 16 rows a CTA where that still gives every SM two CTAs. Depth of the ring: about 74 KB a CTA, so that three share an SM;
+// twice that where the grid leaves one CTA an SM at most.
 template <int NT>
 int skinny_nt(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     const int kv = (K + 7) / 8, r2 = act == kActRelu2;
     constexpr int D1 = 18 / (2 + NT), D2 = NT == 4 ? 2 : 3;
     if (act == kActGeluGate) return launch_skinny<NT, 2, true, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
-    if (N >= 148 * 4 * 16) return launch_skinny<NT, 2, false, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
-    if ((N + 15) / 16 <= 148) return launch_skinny<NT, 1, false, 2 * D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
+    const int sms = gemm_sm_count();
+    if (N >= sms * 4 * 16) return launch_skinny<NT, 2, false, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
+    if ((N + 15) / 16 <= sms) return launch_skinny<NT, 1, false, 2 * D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
     return launch_skinny<NT, 1, false, D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
 }
 int skinny_mma(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
