@@ -327,7 +327,7 @@ def unit_configs(F, torch, peaks, with_cpu=True):
     ops, nbytes = 2.0 * M * N * K, 262144 + 4194304 + 512 + 8192 + 1048576
     c1 = {"ms": round(ms, 5), "tops": round(ops / ms / 1e9, 2), "GB/s": round(nbytes / ms / 1e6, 1),
           "frac_hbm": round(nbytes / ms / 1e6 / hbm, 4), "frac_int8_proxy": round(ops / ms / 1e9 / i8_proxy, 4),
-          "bound": "hbm + launch latency (16 output tiles on 148 SMs)", "algorithmic_bytes": nbytes, "ops": int(ops)}
+          "bound": "hbm + launch latency (64 output tiles on 148 SMs)", "algorithmic_bytes": nbytes, "ops": int(ops)}
     if with_cpu:
         import oracle
         an, wn = a.cpu().numpy(), ws[0].cpu().numpy(); sn, cn = st_.cpu().numpy(), sc.cpu().numpy()
@@ -409,7 +409,7 @@ def unit_configs(F, torch, peaks, with_cpu=True):
     c3 = {"ms": round(ms, 4), "tops": round(ops / ms / 1e9, 2), "frac_int8_proxy": round(ops / ms / 1e9 / i8_proxy, 4),
           "GB/s": round(nbytes / ms / 1e6, 1), "frac_hbm": round(nbytes / ms / 1e6 / hbm, 4),
           "bound": "CUDA-core softmax arithmetic (exact ordered sums, correctly rounded exp)", "algorithmic_bytes": nbytes, "ops": int(ops),
-          "l2": "working set 47 MB < L2: the operands of consecutive runs may hit L2 (the exp scratch is written and re-read each run)"}
+          "l2": "working set 47 MB < L2: the operands of consecutive runs may hit L2"}
     if with_cpu:
         import oracle
         an = [t.cpu().numpy() for t in (q[:1], qs[:1], k[:1], ks[:1], v[:1], vs[:1])]
