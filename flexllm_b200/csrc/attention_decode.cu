@@ -27,6 +27,7 @@
 namespace flexllm {
 
 int* device_error_flag();
+int gemm_sm_count();
 
 static inline KvLayer kv_layer(const flexllm_kv_cache* c, int layer) {
     KvLayer l;
@@ -300,12 +301,11 @@ __global__ void __launch_bounds__(64 * G) dec_pv_kernel(KvLayer cache, const int
 }
 
 // ---- fused single-kernel path (body in attention_decode.cuh) ----------------------------------------
-// Grid (2 HKV, B): two CTAs per (sequence, KV head), two query heads each, so that 10 bytes of shared memory a key hold a CTA's
-// rows and two CTAs share an SM: one's loads run under the other's softmax. The second reading of the pages comes from L2. Sequences go
-// longest first (the last CTAs to start are the shortest): CTA row y takes the sequence with the y-th largest context.
-// 64 sequences of 512 to 8192 keys, 8 KV heads: 198 us a call with four heads to a CTA (one CTA an SM) in batch order, 135 to 143 us now.
+// Grid (4 / G HKV, B): a CTA per (sequence, KV head) with the four query heads of the group, or two CTAs with two heads each, which halves
+// the shared memory of a CTA's rows and its chain of phases, for a second reading of the pages from L2. Two CTAs share an SM.
+// RANK: CTA row y takes the sequence with the y-th largest context, so that the last CTAs to start are the shortest.
 constexpr int DEC_RANK_MAX = 1024;         // batches up to this are ordered by length
-template <bool IN_F32, int NT>
+template <bool IN_F32, int NT, int G, bool RANK>
 __global__ void __launch_bounds__(NT, 2) dec_attn_fused_kernel(const int8_t* __restrict__ q, const float* __restrict__ qs,
                                                              const int8_t* __restrict__ k, const float* __restrict__ ks,
                                                              const int8_t* __restrict__ v, const float* __restrict__ vs,
@@ -322,21 +322,38 @@ __global__ void __launch_bounds__(NT, 2) dec_attn_fused_kernel(const int8_t* __r
     in.q = q; in.qs = qs; in.k = k; in.ks = ks; in.v = v; in.vs = vs; in.qkv_f32 = qkv_f32;
     in.qkv_acc = nullptr; in.tok_scale = nullptr; in.ch_scale = nullptr; in.n_slabs = 0; in.slab_stride = 0;
     in.max_pos = max_pos; in.error_flag = error_flag;
-    __shared__ int b_sm;
-    const int B = gridDim.y;
-    if (threadIdx.x == 0) b_sm = blockIdx.y;
-    __syncthreads();
-    if (B <= DEC_RANK_MAX) {
-        for (int t = threadIdx.x; t < B; t += NT) {
+    int b = blockIdx.y;
+    if constexpr (RANK) {
+        // the rank of a sequence is the number of longer ones (equal ones in order): a warp counts for one sequence at a time
+        __shared__ int b_sm;
+        const int B = gridDim.y, lane = threadIdx.x & 31;
+        for (int t = threadIdx.x >> 5; t < B; t += NT / 32) {
             const int mine = ctx[t];
             int rank = 0;
-            for (int u = 0; u < B; u++) { const int c = ctx[u]; rank += c > mine || (c == mine && u < t); }
-            if (rank == (int)blockIdx.y) b_sm = t;
+            for (int u0 = 0; u0 < B; u0 += 32) {
+                const int u = u0 + lane, c = u < B ? ctx[u] : 0;
+                rank += __popc(__ballot_sync(0xffffffffu, u < B && (c > mine || (c == mine && u < t))));
+            }
+            if (lane == 0 && rank == (int)blockIdx.y) b_sm = t;
         }
         __syncthreads();
+        b = b_sm;
     }
-    dec_attn_fused_body<IN_F32 ? 1 : 0, NT, 2>(in, cos_t, sin_t, a_s, cache, page_table, max_pages, ctx, HQ, HKV, cs, out, oacc,
-                                                  (int)blockIdx.x >> 1, b_sm, dsm, sm, (int)threadIdx.x, 0, (int)blockIdx.x & 1);
+    dec_attn_fused_body<IN_F32 ? 1 : 0, NT, G>(in, cos_t, sin_t, a_s, cache, page_table, max_pages, ctx, HQ, HKV, cs, out, oacc,
+                                               (int)blockIdx.x / (4 / G), b, dsm, sm, (int)threadIdx.x, 0, (int)blockIdx.x % (4 / G));
+}
+
+template <int G, bool RANK>
+static int launch_dec_fused(bool in_f32, const int8_t* q, const float* qs, const int8_t* k, const float* ks, const int8_t* v, const float* vs,
+                            const float* qkv_f32, const float* cos_t, const float* sin_t, const float* a_s, const KvLayer& L, const int32_t* page_table,
+                            int max_pages, const int32_t* ctx, int B, int HQ, int HKV, int cs, float* out, int32_t* oacc, int max_ctx, int* err,
+                            cudaStream_t st) {
+    const size_t smem = dec_attn_smem_bytes<G>(cs);
+    auto kern = in_f32 ? dec_attn_fused_kernel<true, 512, G, RANK> : dec_attn_fused_kernel<false, 512, G, RANK>;
+    if (smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_k(kern, dim3(4 / G * HKV, B), dim3(512), smem, st, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx,
+             HQ, HKV, cs, out, oacc, max_ctx, err);
+    return launch_status(1);
 }
 
 // ---- 5. out ------------------------------------------------------------------------------------
@@ -534,21 +551,22 @@ int flexllm::mha_decode_run(flexllm_kv_cache* c, int layer, const int8_t* q, con
     int* err = device_error_flag();     // raised (and the length clamped) when a ctx[] entry lies beyond max_ctx
 
     // enough (sequence, head) pairs, or short rows: one fused kernel; otherwise the split kernels
-    const size_t fused_smem = dec_attn_smem_bytes<2>(ctx_stride);
     if (ctx_stride <= 10240 && (B * HKV >= 64 || max_ctx <= 2048)) {
-        dim3 fg(2 * HKV, B);
-        if (qkv_f32) {
-            auto kern = dec_attn_fused_kernel<true, 512>;
-            if (fused_smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem));
-            launch_k(kern, fg, dim3(512), fused_smem, st, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx,
-                     HQ, HKV, ctx_stride, out, oacc, max_ctx, err);
-        } else {
-            auto kern = dec_attn_fused_kernel<false, 512>;
-            if (fused_smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fused_smem));
-            launch_k(kern, fg, dim3(512), fused_smem, st, q, qs, k, ks, v, vs, (const float*)nullptr, cos_t, sin_t, a_s, L, page_table,
-                     max_pages, ctx, HQ, HKV, ctx_stride, out, oacc, max_ctx, err);
-        }
-        return launch_status(1);
+        const int sms = gemm_sm_count();
+        // Four heads to a CTA while two CTAs' rows fit an SM (contexts up to about 5700): less work in all. Two heads beyond that, where the
+        // four-head form leaves one CTA an SM, and where the CTAs are few: every SM at most one, or at most two and long contexts.
+        // Sequences by length where CTAs follow one another on an SM and contexts are long enough to pay for the ranking, and among two-head
+        // CTAs where they share an SM.
+        // us, four heads / two heads / two heads by length, 8 KV heads: 8 x 2000 keys 20.4 / 14.7 / 14.7; 16 x 510 11.6 / 12.1 / 12.4, 16 x 2000
+        // 20.7 / 19.4 / 19.8; 64 x 30 15.9 / 25.4 / 28.0, 64 x 4096 121 / 135 / 139, 64 x 6000 244 / 189 / 189; 64 of 512 to 8192
+        // 175 / 141 / 125. Four heads, in order / by length: 64 x 30 15.9 / 19.3, 64 x 2000 61.5 / 63.7, 64 x 4096 121 / 121.
+        const bool room4 = 2 * (dec_attn_smem_bytes<4>(ctx_stride) + 3072) <= 228 * 1024;
+        const int ctas2 = 2 * HKV * B;
+        const bool two = !room4 || ctas2 <= sms || (ctas2 <= 2 * sms && max_ctx > 1536);
+        const bool rank = B <= DEC_RANK_MAX && (two ? ctas2 > sms : HKV * B > 2 * sms && max_ctx > 2048);
+        auto launch = two ? (rank ? launch_dec_fused<2, true> : launch_dec_fused<2, false>) : (rank ? launch_dec_fused<4, true> : launch_dec_fused<4, false>);
+        return launch(qkv_f32 != nullptr, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx, B, HQ, HKV, ctx_stride, out, oacc,
+                      max_ctx, err, st);
     }
     const int warps = B * (HQ + 2 * HKV);
     if (qkv_f32)

@@ -402,19 +402,29 @@ __device__ __forceinline__ void dec_attn_fused_body(const DecAttnIn& in, const f
     // ---- F. u8 probabilities (zero beyond the last key up to the page boundary)
     const int nk_pad = (nk + PAGE - 1) / PAGE * PAGE;
     {
+        // (four heads: the division's short form, which needs fewer registers)
         float rinv_g[G];
         float as_g[G], c_g[G];
         bool ok_g[G];
+        DivBy div_g[G];
 #pragma unroll
         for (int g = 0; g < G; g++) {
             rinv_g[g] = row_rinv[g]; as_g[g] = a_s[hq0 + g];
-            c_g[g] = dec_u8_factor(rinv_g[g], as_g[g], ok_g[g]);
+            if constexpr (G == 2) c_g[g] = dec_u8_factor(rinv_g[g], as_g[g], ok_g[g]);
+            else div_g[g] = div_by(as_g[g]);
         }
         auto quantise_key = [&](int key, float vsc) {
 #pragma unroll
             for (int g = 0; g < G; g++) {
                 uint8_t uq = 0;
-                if (key < nk) uq = (uint8_t)dec_u8(sc[g * csr + key], c_g[g], ok_g[g], rinv_g[g], vsc, as_g[g]);
+                if (key < nk) {
+                    if constexpr (G == 2) {
+                        uq = (uint8_t)dec_u8(sc[g * csr + key], c_g[g], ok_g[g], rinv_g[g], vsc, as_g[g]);
+                    } else {
+                        const int r = round_half_away_to_int(div_for_rounding((sc[g * csr + key] * rinv_g[g]) * vsc, div_g[g]));
+                        uq = (uint8_t)(r > 255 ? 255 : r);
+                    }
+                }
                 u_sm[g * cs + key] = uq;
             }
         };

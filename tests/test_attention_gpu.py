@@ -289,6 +289,15 @@ def test_decode_maximum_of_either_zero(F):
     decode_case(F, 2, [300, 700], seed=48, q_gain=2.0 ** -80, k_gain=2.0 ** -80, signed_from=128)
 
 
+@pytest.mark.parametrize("B,lo,hi,what", [(9, 1, 300, {}), (10, 1, 300, {}), (20, 0, 130, dict(q_gain=3.0)), (20, 60, 130, dict(a_gain=0.01)),
+                                          (37, 0, 2100, {}), (38, 0, 100, {}), (38, 0, 2100, {}), (40, 126, 126, {}), (12, 1400, 1530, {}), (12, 100, 1600, dict(q_gain=20.0)),
+                                          (8, 100, 5800, {}), (10, 100, 5800, {}), (10, 100, 5600, {})])
+def test_decode_forms(F, B, lo, hi, what):
+    """Numbers of sequences and contexts on both sides of the lines between the forms: four query heads or two to a CTA, sequences in
+    their order or by length."""
+    decode_case(F, B, np.append(np.random.default_rng(B).integers(lo, hi + 1, B - 1), hi), seed=50 + B, **what)
+
+
 def test_kv_append_alone(F):
     """The cache managers' append on its own: the new token's K row, transposed V column and both scales land at
     position ctx[b] of the right page; everything else in the pools is untouched."""
