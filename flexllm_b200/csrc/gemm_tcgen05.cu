@@ -248,8 +248,7 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_launch();
-    if (!SWAP || warp != 0) pdl_wait();                  // (the decode form's producer has its own wait below)
+    pdl_sync();
     const int num_kb = ((args.K + 127) >> 7) / KCH;      // pipeline steps of KCH chunks (K % (128*KCH) == 0 when KCH > 1)
     const int total_tiles = args.tilesA * args.tilesB * args.ksplit;
 
@@ -273,24 +272,6 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
         if (lane == 0) {
             tma_prefetch_desc(&tmapA);
             tma_prefetch_desc(&tmapB);
-            auto load_a = [&](int st, int ta, int kb) {
-                const uint32_t dst = ring + st * Cfg::STAGE_BYTES;
-                if (KCH == 1) tma_load_2d(dst, &tmapA, bar_full + 8 * st, kb * 128, ta * 128);
-                else tma_load_3d(dst, &tmapA, bar_full + 8 * st, 0, ta * 128, kb * KCH);
-            };
-            // decode form: the A side are weights, which no earlier kernel writes. The ring is filled with the first tile's before the
-            // activations are asked for. (Not while the kernels before this one still run: the other warps have waited for those ahead
-            // of the barrier above.)
-            int ahead = 0;
-            if (SWAP && blockIdx.x < total_tiles) {
-                const int split = blockIdx.x % args.ksplit, ta = blockIdx.x / (args.ksplit * args.tilesB);
-                const int kb0 = (int)((long)split * num_kb / args.ksplit), kb1 = (int)((long)(split + 1) * num_kb / args.ksplit);
-                for (; ahead < STAGES && kb0 + ahead < kb1; ahead++) {
-                    mbar_expect_tx(bar_full + 8 * ahead, Cfg::STAGE_BYTES);
-                    load_a(ahead, ta, kb0 + ahead);
-                }
-                pdl_wait();
-            }
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
@@ -300,16 +281,17 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
                 const int kb0 = (int)((long)split * num_kb / args.ksplit);
                 const int kb1 = (int)((long)(split + 1) * num_kb / args.ksplit);
                 for (int kb = kb0; kb < kb1; kb++) {
+                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
                     const uint32_t full = bar_full + 8 * stage;
-                    if (ahead > 0) ahead--;
-                    else {
-                        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
-                        mbar_expect_tx(full, Cfg::STAGE_BYTES);
-                        load_a(stage, ta, kb);
+                    mbar_expect_tx(full, Cfg::STAGE_BYTES);
+                    const uint32_t dstA = ring + stage * Cfg::STAGE_BYTES, dstB = dstA + Cfg::A_BYTES;
+                    if (KCH == 1) {
+                        tma_load_2d(dstA, &tmapA, full, kb * 128, ta * 128);
+                        tma_load_2d(dstB, &tmapB, full, kb * 128, tb * BN);
+                    } else {
+                        tma_load_3d(dstA, &tmapA, full, 0, ta * 128, kb * KCH);
+                        tma_load_3d(dstB, &tmapB, full, 0, tb * BN, kb * KCH);
                     }
-                    const uint32_t dstB = ring + stage * Cfg::STAGE_BYTES + Cfg::A_BYTES;
-                    if (KCH == 1) tma_load_2d(dstB, &tmapB, full, kb * 128, tb * BN);
-                    else tma_load_3d(dstB, &tmapB, full, 0, tb * BN, kb * KCH);
                     if (++stage == STAGES) { stage = 0; phase ^= 1u; }
                 }
             }
