@@ -151,6 +151,38 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const bf16* src, bool l
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// The end of both forms: the warps' partial sums, added in warp order, and the epilogue.
+template <int NT, int RT, bool GLU>
+__device__ __forceinline__ void skinny_finish(const float (&acc)[RT][NT][4], float (&part)[8][RT * 16][NT * 8 + 1], const float* __restrict__ bias, int M, int N,
+                                              int relu2, float* y32, bf16* y16, long ldy) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    const int row0 = blockIdx.x * RT * 16;
+#pragma unroll
+    for (int r = 0; r < RT; r++)
+#pragma unroll
+        for (int t = 0; t < NT; t++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) part[warp][r * 16 + lr + 8 * (i >> 1)][t * 8 + lc * 2 + (i & 1)] = acc[r][t][i];
+    __syncthreads();
+    auto total = [&](int row, int tok) {
+        float v = part[0][row][tok];
+#pragma unroll
+        for (int k = 1; k < 8; k++) v += part[k][row][tok];
+        const int n = row0 + row;
+        return v + (bias && n < N ? bias[n] : 0.0f);
+    };
+    constexpr int OUT = GLU ? 16 : RT * 16;                 // output columns of the CTA
+    const int n0 = GLU ? row0 >> 1 : row0, n_out = GLU ? N >> 1 : N;
+    for (int i = threadIdx.x; i < OUT * M; i += 256) {
+        const int tok = i / OUT, o = i - tok * OUT;
+        if (n0 + o >= n_out) continue;
+        float v = GLU ? gelu_tanh_f<true>(total(o, tok)) * total(RT * 16 - 16 + o, tok) : total(o, tok);
+        if (!GLU && relu2) v = relu2_f(v);
+        if (y32) y32[(long)tok * ldy + n0 + o] = v;
+        else y16[(long)tok * ldy + n0 + o] = __float2bfloat16_rn(v);
+    }
+}
+
 template <int NT, int RT, bool GLU, int DEPTH>
 __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict__ a, long lda, const bf16* __restrict__ w, long ldw,
                                                          const float* __restrict__ bias, int M, int N, int kv, int relu2, float* y32, bf16* y16, long ldy) {
@@ -215,30 +247,65 @@ __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict_
         if (++slot == DEPTH) slot = 0;
     }
     cp_async_wait<0>();
+    skinny_finish<NT, RT, GLU>(acc, part, bias, M, N, relu2, y32, y16, ldy);
+}
+
+// The form without a ring, where that is the better one (skinny_nt): weights one group of chunks ahead in registers, activations read where
+// they are used. The same sums in the same order.
+template <int NT, int RT, bool GLU>
+__global__ void __launch_bounds__(256) skinny_short_kernel(const bf16* __restrict__ a, long lda, const bf16* __restrict__ w, long ldw,
+                                                           const float* __restrict__ bias, int M, int N, int kv, int relu2, float* y32, bf16* y16, long ldy) {
+    constexpr int G = NT * RT >= 4 ? 2 : 4;                 // 32-element chunks per step
+    __shared__ float part[8][RT * 16][NT * 8 + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    const int row0 = blockIdx.x * RT * 16;
+    const int n_ch = (kv + 3) >> 2;                         // kv: 8-element vectors per row
+    const int c_beg = (int)((long)warp * n_ch / 8), c_end = (int)((long)(warp + 1) * n_ch / 8);
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const bf16* wr[RT][2];
 #pragma unroll
     for (int r = 0; r < RT; r++)
 #pragma unroll
-        for (int t = 0; t < NT; t++)
+        for (int h = 0; h < 2; h++) wr[r][h] = w + (long)min(row0 + r * 16 + h * 8 + lr, N - 1) * ldw + lc * 8;
+    uint4 wv[G][RT][2], nx[G][RT][2];
+    auto load_w = [&](uint4 (&v)[G][RT][2], int c) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) part[warp][r * 16 + lr + 8 * (i >> 1)][t * 8 + lc * 2 + (i & 1)] = acc[r][t][i];
-    __syncthreads();
-    auto total = [&](int row, int tok) {
-        float v = part[0][row][tok];
+        for (int g = 0; g < G; g++)
 #pragma unroll
-        for (int k = 1; k < 8; k++) v += part[k][row][tok];
-        const int n = row0 + row;
-        return v + (bias && n < N ? bias[n] : 0.0f);
+            for (int r = 0; r < RT; r++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    v[g][r][h] = (c + g < c_end && (c + g) * 4 + lc < kv) ? ldg_stream16(wr[r][h] + (long)(c + g) * 32) : zero;
     };
-    constexpr int OUT = GLU ? 16 : RT * 16;                 // output columns of the CTA
-    const int n0 = GLU ? row0 >> 1 : row0, n_out = GLU ? N >> 1 : N;
-    for (int i = threadIdx.x; i < OUT * M; i += 256) {
-        const int tok = i / OUT, o = i - tok * OUT;
-        if (n0 + o >= n_out) continue;
-        float v = GLU ? gelu_tanh_f<true>(total(o, tok)) * total(RT * 16 - 16 + o, tok) : total(o, tok);
-        if (!GLU && relu2) v = relu2_f(v);
-        if (y32) y32[(long)tok * ldy + n0 + o] = v;
-        else y16[(long)tok * ldy + n0 + o] = __float2bfloat16_rn(v);
+    load_w(nx, c_beg);
+    pdl_sync();
+    float acc[RT][NT][4] = {};
+    for (int c = c_beg; c < c_end; c += G) {
+#pragma unroll
+        for (int g = 0; g < G; g++)
+#pragma unroll
+            for (int r = 0; r < RT; r++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) wv[g][r][h] = nx[g][r][h];
+        uint4 av[G][NT];
+#pragma unroll
+        for (int g = 0; g < G; g++)
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+                av[g][t] = (t * 8 + lr < M && c + g < c_end && (c + g) * 4 + lc < kv)
+                               ? *reinterpret_cast<const uint4*>(a + (long)(t * 8 + lr) * lda + (long)(c + g) * 32 + lc * 8) : zero;
+        load_w(nx, c + G);
+#pragma unroll
+        for (int g = 0; g < G; g++)
+#pragma unroll
+            for (int r = 0; r < RT; r++)
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    mma_bf16(acc[r][t], wv[g][r][0].x, wv[g][r][1].x, wv[g][r][0].y, wv[g][r][1].y, av[g][t].x, av[g][t].y);
+                    mma_bf16(acc[r][t], wv[g][r][0].z, wv[g][r][1].z, wv[g][r][0].w, wv[g][r][1].w, av[g][t].z, av[g][t].w);
+                }
     }
+    skinny_finish<NT, RT, GLU>(acc, part, bias, M, N, relu2, y32, y16, ldy);
 }
 
 template <int NT, int RT, bool GLU, int DEPTH>
@@ -261,8 +328,19 @@ template <int NT>
 int skinny_nt(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     const int kv = (K + 7) / 8, r2 = act == kActRelu2;
     constexpr int D1 = 18 / (2 + NT), D2 = NT == 4 ? 2 : 3;
-    if (act == kActGeluGate) return launch_skinny<NT, 2, true, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
     const int sms = gemm_sm_count();
+    // The ring pays where a warp has more than a few chunks. With rows of up to 1024 (four chunks) setting it up costs more than it hides
+    // (us, without / with it, 4 tokens: 1024x1024 2.45 / 3.08, 2560x1024 3.4 / 4.2, 8192x1024 6.5 / 7.5; 1024x4096 6.3 / 5.6, 2048x8192 13.1 / 10.9,
+    // 10240x4096 24.3 / 19.5). One or two tokens go without it also where both sides are large or the rows are few: other products of such a
+    // step are GEMVs, which start their weights early only if the kernel in front leaves them shared memory (decode steps of 2 sequences
+    // without / with it: width 4096 1116 / 1143 and 1038 / 1051 us, width 1024 331 / 342; width 2048 888 / 867 and 906 / 835).
+    if (K <= 1024 || (M <= 2 && (N < 2048 || (K > 2048 && N > 2048)))) {
+        if (act == kActGeluGate) launch_k(skinny_short_kernel<NT, 2, true>, dim3((N + 31) / 32), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
+        else if (N >= sms * 4 * 16) launch_k(skinny_short_kernel<NT, 2, false>, dim3((N + 31) / 32), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
+        else launch_k(skinny_short_kernel<NT, 1, false>, dim3((N + 15) / 16), dim3(256), 0, st, a, lda, w, ldw, bias, M, N, kv, r2, y.f32, (bf16*)y.t, y.ld);
+        return launch_status();
+    }
+    if (act == kActGeluGate) return launch_skinny<NT, 2, true, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
     if (N >= sms * 4 * 16) return launch_skinny<NT, 2, false, D2>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
     if ((N + 15) / 16 <= sms) return launch_skinny<NT, 1, false, 2 * D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);
     return launch_skinny<NT, 1, false, D1>(a, lda, w, ldw, bias, M, N, kv, r2, y, st);

@@ -86,10 +86,11 @@ def test_linear_split_sums(F, M, N, K):
     assert (got - want - bias.double()).norm() < (1.25e-9 * K / parts + 1.2e-7) * got.norm()
 
 
-@pytest.mark.parametrize("N,K", [(2368, 3000), (2384, 3000), (9456, 520), (9472, 264), (40, 8), (2048, 8200)])
+@pytest.mark.parametrize("N,K", [(2368, 3000), (2384, 3000), (9456, 520), (9472, 264), (40, 8), (2048, 8200), (2368, 1024), (2368, 1032), (9480, 1000),
+                                 (4096, 6144), (4104, 6144)])
 def test_linear_few_tokens_ring(F, N, K):
-    """A few tokens on both sides of the rules that choose the ring's depth and the rows of a CTA, with fewer chunks than the ring holds
-    and with many more, and a ragged last chunk. Bounds as in test_linear."""
+    """A few tokens on both sides of the rules that choose the ring or the form without it, the ring's depth and the rows of a CTA, with fewer
+    chunks than the ring holds and with many more, and a ragged last chunk. Bounds as in test_linear."""
     g = np.random.default_rng(K)
     w = bf16_round(g.standard_normal((N, K)) * K ** -0.5)
     b = g.standard_normal(N).astype(np.float32)
