@@ -109,8 +109,9 @@ struct DecAttnSmem {
 // bytes), scores, max, exp, the ordered partial sums, the u8 quantiser and P.V, with the score rows kept in shared
 // memory (`dsm`: dec_attn_smem_bytes<G>). The group's NT threads (256 or 512; `tid` = index in the group) synchronise on named
 // barrier `bar`.
-// G = 2 (stand-alone operator): rows padded against bank conflicts in the ordered sums, which fetch ahead, and the warp-wide
-// exponential. G = 4: the persistent kernel's form for contexts beyond its staging area.
+// G = 2 (stand-alone operator, long contexts or few sequences): rows padded against bank conflicts in the ordered sums, which fetch ahead, the
+// warp-wide exponential and a quantiser without divisions. G = 4: the stand-alone operator otherwise, and the persistent kernel's form for
+// contexts beyond its staging area.
 template <int G> constexpr size_t dec_attn_smem_bytes(int cs) {
     const size_t n = (size_t)G * (G == 2 ? cs + 4 : cs) * 4 + (size_t)G * cs;
     return n < 4096 ? 4096 : n;
