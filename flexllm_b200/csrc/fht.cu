@@ -140,6 +140,66 @@ __global__ void __launch_bounds__(128, 4) fht8192_kernel(const float* __restrict
     }
 }
 
+// The rest of the fused form behind a product that has done silu(gate) * up and index bits 1..4 itself (gemm_i8_prefill_swiglu): bits 5..10 with the
+// values as they come from memory (a lane's values 32 apart, so that a warp reads 128 bytes at a time), bits 11, 12 and 0 after the only exchange
+// through shared memory, then the quantiser. Bound by memory: 254 us for 32768 rows (1.34 GB, 205 us at the copy rate). Element i lives at i with its 16-byte granule exchanged by index bits 5 and 6: both sides of the
+// exchange touch every bank once.
+__device__ __forceinline__ int fht_rest_at(int i) { return i ^ (((i >> 5) & 3) << 2); }
+__global__ void __launch_bounds__(128, 4) fht8192_rest_kernel(const float* __restrict__ x, float scale, int8_t* __restrict__ q, float* __restrict__ s) {
+    constexpr int N = 8192;
+    __shared__ __align__(16) float buf[N];
+    __shared__ float red[4], red_nan[4];
+    pdl_sync();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long row = blockIdx.x;
+    float r[64];
+    {
+        const float* xr = x + row * N + warp * 2048 + lane;
+#pragma unroll
+        for (int v = 0; v < 64; v++) r[v] = xr[v * 32];
+        reg_butterfly<0>(r); reg_butterfly<1>(r); reg_butterfly<2>(r); reg_butterfly<3>(r); reg_butterfly<4>(r); reg_butterfly<5>(r);
+#pragma unroll
+        for (int v = 0; v < 64; v++) buf[fht_rest_at(warp * 2048 + v * 32 + lane)] = r[v];
+    }
+    __syncthreads();
+    // register bits 0..3: index bits 0..3, bits 4 and 5: index bits 11 and 12; index bits 4..10 are the thread's
+#pragma unroll
+    for (int h = 0; h < 4; h++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const float4 t = *reinterpret_cast<const float4*>(buf + fht_rest_at(h * 2048 + tid * 16 + c * 4));
+            r[h * 16 + c * 4] = t.x; r[h * 16 + c * 4 + 1] = t.y; r[h * 16 + c * 4 + 2] = t.z; r[h * 16 + c * 4 + 3] = t.w;
+        }
+    reg_butterfly<4>(r); reg_butterfly<5>(r); reg_butterfly<0>(r);
+    float mx = 0.0f, mn = 0.0f;                                            // mn: NaN when a value is
+#pragma unroll
+    for (int v = 0; v < 64; v += 2) { mx = max3(mx, fabsf(r[v]), fabsf(r[v + 1])); mn = max3_nan(mn, fabsf(r[v]), fabsf(r[v + 1])); }
+    mx = warp_max(mx);
+    const bool bad = __any_sync(0xffffffffu, !(mn <= mx));
+    if (lane == 0) { red[warp] = mx; red_nan[warp] = bad ? 1.0f : 0.0f; }
+    __syncthreads();
+    mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+    const bool ok = fht_q8_in_range(mx, scale) && (red_nan[0] + red_nan[1]) + (red_nan[2] + red_nan[3]) == 0.0f;
+    const float sc = fht_row_scale(mx, scale);
+    if (tid == 0) s[row] = sc;
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        uint32_t o[4];
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+            float t[8];
+            uint32_t b[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) t[i] = r[h * 16 + c * 4 + i];
+            q8_short(t, 1.0f / (scale * sc), ok, b, [&](float v) { return fht_q8_exact(v, scale, sc); });
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                o[c + i] = __byte_perm(__byte_perm(b[4 * i], b[4 * i + 1], 0x0040), __byte_perm(b[4 * i + 2], b[4 * i + 3], 0x0040), 0x5410);
+        }
+        *reinterpret_cast<uint4*>(q + row * N + h * 2048 + tid * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 // The same for few rows (decoding): a cluster of eight CTAs per row, 1024 elements a CTA, eight a thread, so that SiLU's
 // arithmetic and the loads, which one SM does one after another, are spread over eight. Index bits 1 and 9 are a thread's
 // own, 2..6 the lane's (shuffles), 7 and 8 the warp's: bit 1 in registers, 2..6 by shuffle, 7..9 after an exchange through
@@ -286,6 +346,11 @@ __global__ void __launch_bounds__(256) qk_prepare_kernel(const int8_t* __restric
 }
 
 // gate and up halves of one fused projection output: rows of `ld` floats, gate at g, up at u
+int fht8192_rest(const float* h, int M, float scale, int8_t* q, float* s, cudaStream_t st) {
+    if (M == 0) return FLEXLLM_OK;
+    launch_k(fht8192_rest_kernel, dim3(M), dim3(128), 0, st, h, scale, q, s);
+    return launch_status();
+}
 int swiglu_fht_quant_strided(const float* g, const float* u, long ld, int M, float scale, int8_t* q, float* s, cudaStream_t st) {
     return swiglu_fht_quant(g, u, ld, M, scale, q, s, nullptr, st);
 }

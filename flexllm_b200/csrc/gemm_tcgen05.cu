@@ -27,6 +27,7 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "fht_core.cuh"
 #include "tc_common.cuh"
 
 namespace flexllm {
@@ -224,6 +225,58 @@ __device__ __forceinline__ void staged_store(const GemmArgs& args, float* stg, c
             if (c + 2 < NCH) tmem_ld_32x32(tsrc + (c + 2) * 32, va);
             process(vb, c + 1);
         }
+    }
+}
+
+// The same for the fused gate | up product of the feed-forward block: columns 0..127 of the tile are gate channels f0 .. f0 + 127, columns 128..255
+// the up channels of the same numbers, and what is stored is silu(gate) * up (each operation rounded as in the kernels that do it apart) after
+// the first four stages of the 8192-point transform that follows, index bits 1..4 (Modules/FHT.h:31-53): a lane has 32 channels of its row at a time.
+__device__ __forceinline__ void staged_store_swiglu(const GemmArgs& args, float* stg, const uint32_t tsrc, const int row0, const int f0, const float sa,
+                                                    const int lane, const int c0) {
+    const float* sbw = stg + 1024;                             // scales of the warp's 64 gate and 64 up channels
+    const bool row_ok = row0 + lane < args.rowsA;
+    const ExpTable tab = exp_table_lane();
+    __syncwarp();
+#pragma unroll 1
+    for (int c = c0; c < c0 + 2; c++) {
+        float h[32];
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            uint32_t vg[16], vu[16];
+            tmem_ld_32x16(tsrc + c * 32 + half * 16, vg);
+            tmem_ld_32x16(tsrc + 128 + c * 32 + half * 16, vu);
+            tmem_ld_wait();
+            const f32x2 sa2 = pack2(sa, sa);
+#pragma unroll
+            for (int j0 = 0; j0 < 16; j0 += 8) {
+                float g[8], u[8], o[8];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    const int col = (c - c0) * 32 + half * 16 + j0 + j;
+                    const float2 sg = *reinterpret_cast<const float2*>(sbw + col), su = *reinterpret_cast<const float2*>(sbw + 64 + col);
+                    unpack2(mul2(mul2(pack2((float)(int)vg[j0 + j], (float)(int)vg[j0 + j + 1]), sa2), pack2(sg.x, sg.y)), g[j], g[j + 1]);
+                    unpack2(mul2(mul2(pack2((float)(int)vu[j0 + j], (float)(int)vu[j0 + j + 1]), sa2), pack2(su.x, su.y)), u[j], u[j + 1]);
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) if (!row_ok) g[j] = 1.0f;             // rows past the last keep the warp on the short form
+                silu_mul_warp(g, u, o, tab);
+#pragma unroll
+                for (int j = 0; j < 8; j++) h[half * 16 + j0 + j] = o[j];
+            }
+        }
+        reg_butterfly<1>(h); reg_butterfly<2>(h); reg_butterfly<3>(h); reg_butterfly<4>(h);
+#pragma unroll
+        for (int gg = 0; gg < 8; gg++)
+            *reinterpret_cast<float4*>(stg + lane * 32 + ((gg ^ (lane & 7)) << 2)) = make_float4(h[4 * gg], h[4 * gg + 1], h[4 * gg + 2], h[4 * gg + 3]);
+        __syncwarp();
+        const int g = lane & 7;
+#pragma unroll
+        for (int it = 0; it < 8; it++) {
+            const int rr = it * 4 + (lane >> 3), row = row0 + rr;
+            if (row < args.rowsA)
+                *reinterpret_cast<float4*>(args.y + (long)row * args.ldo + f0 + c * 32 + 4 * g) = *reinterpret_cast<const float4*>(stg + rr * 32 + ((g ^ (rr & 7)) << 2));
+        }
+        __syncwarp();          // the staging buffer is reused by the next chunk
     }
 }
 
@@ -479,10 +532,18 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_tcgen05_kernel(const __grid_co
 // (TMA writes and operand reads, 128 bytes a clock) is what bounds that form, together with its epilogue. Roles as
 // there, in both CTAs, but only the first CTA's warp 1 issues MMAs; its barriers count both CTAs' bytes and readers.
 // W8A8 prompt of 32 x 1024 tokens, products of 16 layers included: 78.8 -> 75.3 ms.
-constexpr int GP_STAGES = 6, GP_TILE = 128 * 128, GP_STAGE_BYTES = 2 * GP_TILE, GP_BN = 256;
-constexpr int GP_SMEM = GP_STAGES * GP_STAGE_BYTES + 1024 + 256 + GemmCfg<GP_BN>::STG_BYTES;
-__global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
+constexpr int GP_STAGES_MAX = 6, GP_TILE = 128 * 128, GP_STAGE_BYTES = 2 * GP_TILE, GP_BN = 256;
+// SWIGLU: eight epilogue warps, two to a quarter of the tile's rows with half of the columns each (32768 rows of 16384 x 2048: 1343 us with four,
+// whose arithmetic took longer than the product, 1240 with eight), and a shorter ring to make room for their staging.
+template <bool SWIGLU> struct GpCfg {
+    static constexpr int STAGES = SWIGLU ? 5 : GP_STAGES_MAX, EPI_WARPS = SWIGLU ? 8 : 4, THREADS = 64 + 32 * EPI_WARPS;
+    static constexpr int STG_FLOATS = SWIGLU ? 1024 + 128 : GemmCfg<GP_BN>::STG_WARP_FLOATS;
+    static constexpr int SMEM = STAGES * GP_STAGE_BYTES + 1024 + 256 + EPI_WARPS * STG_FLOATS * 4;
+};
+template <bool SWIGLU>
+__global__ void __launch_bounds__(GpCfg<SWIGLU>::THREADS, 1) gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB,
                                                               const GemmArgs args) {
+    constexpr int GP_STAGES = GpCfg<SWIGLU>::STAGES, EPI_WARPS = GpCfg<SWIGLU>::EPI_WARPS;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -491,7 +552,7 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_const
     const uint32_t bar_full = smem_u32(bars);                    // first CTA: bytes of both CTAs
     const uint32_t bar_empty = bar_full + 8 * GP_STAGES;         // both CTAs, each for its own producer
     const uint32_t bar_tfull = bar_empty + 8 * GP_STAGES;        // both CTAs
-    const uint32_t bar_tempty = bar_tfull + 16;                  // first CTA: the eight epilogue warps of both
+    const uint32_t bar_tempty = bar_tfull + 16;                  // first CTA: the epilogue warps of both
     uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + 2 * GP_STAGES + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
     float* stg_all = reinterpret_cast<float*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES + 256);
@@ -504,7 +565,7 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_const
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < GP_STAGES; s++) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(bar_tfull + 8 * s, 1); mbar_init(bar_tempty + 8 * s, 8); }
+        for (int s = 0; s < 2; s++) { mbar_init(bar_tfull + 8 * s, 1); mbar_init(bar_tempty + 8 * s, 2 * EPI_WARPS); }
         *abort_flag = 0;
         fence_barrier_init();
     }
@@ -527,7 +588,7 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_const
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             for (int t = pair; ok && t < total_tiles; t += pairs) {
-                const int rowA = (t / args.tilesB) * 256 + rank * 128, rowB = (t % args.tilesB) * GP_BN + rank * 128;
+                const int rowA = (t / args.tilesB) * 256 + rank * 128, rowB = SWIGLU ? (t % args.tilesB) * 128 + rank * (args.rowsB >> 1) : (t % args.tilesB) * GP_BN + rank * 128;
                 for (int kb = 0; kb < num_kb; kb++) {
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
                     const uint32_t full = bar_full + 8 * stage, full0 = cluster_addr(full, 0);
@@ -565,20 +626,29 @@ __global__ void __launch_bounds__(192, 1) gemm_i8_pair_kernel(const __grid_const
             }
         }
     } else {
-        // ------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
-        const int q = warp & 3;
-        float* stg = stg_all + q * GemmCfg<GP_BN>::STG_WARP_FLOATS;
+        // ------------------------------------------------------------ epilogue (warps 2.. of both CTAs)
+        const int q = warp & 3, half = (warp - 2) >> 2;          // TMEM lanes 32 q ..; SWIGLU: columns 64 half ..
+        float* stg = stg_all + (warp - 2) * GpCfg<SWIGLU>::STG_FLOATS;
         int it = 0;
         for (int t = pair; t < total_tiles; t += pairs, it++) {
             const int row0 = (t / args.tilesB) * 256 + rank * 128 + q * 32, col0 = (t % args.tilesB) * GP_BN;
             const int as = it & 1;
             const float sa = (row0 + lane < args.rowsA && args.sA) ? args.sA[row0 + lane] : 0.0f;
-            staged_prefetch<GP_BN>(args, stg, row0, col0, lane);
+            if (SWIGLU) {
+                for (int i = lane; i < 64; i += 32) {
+                    stg[1024 + i] = args.sB[col0 / 2 + half * 64 + i];
+                    stg[1024 + 64 + i] = args.sB[(args.rowsB >> 1) + col0 / 2 + half * 64 + i];
+                }
+            } else {
+                staged_prefetch<GP_BN>(args, stg, row0, col0, lane);
+            }
             int got = (lane == 0) ? (mbar_wait(bar_tfull + 8 * as, (uint32_t)((it >> 1) & 1), abort_flag) ? 1 : 0) : 1;
             got = __shfl_sync(0xffffffffu, got, 0);
             if (!got) break;
             tc_fence_after();
-            staged_store<GP_BN>(args, stg, tmem_base + ((uint32_t)(q * 32) << 16) + as * GP_BN, row0, col0, sa, lane);
+            const uint32_t tsrc = tmem_base + ((uint32_t)(q * 32) << 16) + as * GP_BN;
+            if (SWIGLU) staged_store_swiglu(args, stg, tsrc, row0, col0 / 2, sa, lane, half * 2);
+            else staged_store<GP_BN>(args, stg, tsrc, row0, col0, sa, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(cluster_addr(bar_tempty + 8 * as, 0));
@@ -698,6 +768,8 @@ static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, i
     return launch_status();
 }
 
+// SWIGLU: w holds N / 2 gate and N / 2 up rows, y is [M][N / 2].
+template <bool SWIGLU = false>
 static int launch_gemm_pair(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K, int32_t* acc, float* y,
                             cudaStream_t st, const float* residual) {
     CUtensorMap ta, tb;
@@ -708,17 +780,18 @@ static int launch_gemm_pair(const int8_t* a, const float* s_tok, const int8_t* w
     GemmArgs g;
     g.rowsA = M; g.rowsB = N; g.K = K;
     g.tilesA = (M + 255) / 256; g.tilesB = (N + GP_BN - 1) / GP_BN; g.ksplit = 1;
-    g.ldo = N; g.acc = acc; g.y = y; g.sA = s_tok; g.sB = s_ch; g.error_flag = device_error_flag();
+    g.ldo = SWIGLU ? N / 2 : N; g.acc = acc; g.y = y; g.sA = s_tok; g.sB = s_ch; g.error_flag = device_error_flag();
     g.residual = residual; g.cluster = 0;
+    auto kern = gemm_i8_pair_kernel<SWIGLU>;
     static std::atomic<bool> attr_set[kMaxDevices];
     const int dev = current_device();
     if (dev < 0) return FLEXLLM_ECUDA;
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(gemm_i8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
+        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GpCfg<SWIGLU>::SMEM));
         attr_set[dev].store(true, std::memory_order_release);
     }
     const int tiles = g.tilesA * g.tilesB, pairs = sm_count() / 2;
-    launch_cluster(gemm_i8_pair_kernel, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(192), 2, (size_t)GP_SMEM, st, ta, tb, g);
+    launch_cluster(kern, dim3(2 * (tiles < pairs ? tiles : pairs)), dim3(GpCfg<SWIGLU>::THREADS), 2, (size_t)GpCfg<SWIGLU>::SMEM, st, ta, tb, g);
     return launch_status();
 }
 
@@ -726,22 +799,39 @@ static int launch_gemm_pair(const int8_t* a, const float* s_tok, const int8_t* w
 // The tile is the one with the shortest time by a count of shared-memory traffic: per step of 128 bytes of K a CTA moves (128 + BN)
 // rows (the pair form 256 for twice the output), plus a fixed part; times the rounds of tiles that the SMs go through. (With 256
 // columns whenever there are that many, a product of 128 x 2048 x 2048 ran on 8 SMs for 15 us.)
-int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
-                    int32_t* acc, float* y, cudaStream_t st, const float* residual) {
+struct TileCosts { long c256, c128, c64, c32; bool pair; };
+static TileCosts tile_costs(int M, int N) {
     const int sms = sm_count();
     auto cost = [&](int rows, int cols, int units, int step) {
         const long tiles = (long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
         return (tiles + units - 1) / units * step;
     };
-    const long c256 = cost(128, 256, sms, 128 + 256 + 32), c128 = cost(128, 128, sms, 128 + 128 + 32), c64 = cost(128, 64, sms, 128 + 64 + 32),
-               c32 = cost(128, 32, sms, 128 + 32 + 32), cpair = cost(256, 256, sms / 2, 256 + 48);
-    if (N > 128 && M > 128 && cpair <= c256 && cpair <= c128 && cpair <= c64 && cpair <= c32)
-        return launch_gemm_pair(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
+    TileCosts c = {cost(128, 256, sms, 128 + 256 + 32), cost(128, 128, sms, 128 + 128 + 32), cost(128, 64, sms, 128 + 64 + 32),
+                   cost(128, 32, sms, 128 + 32 + 32), false};
+    const long cpair = cost(256, 256, sms / 2, 256 + 48);
+    c.pair = N > 128 && M > 128 && cpair <= c.c256 && cpair <= c.c128 && cpair <= c.c64 && cpair <= c.c32;
+    return c;
+}
+int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
+                    int32_t* acc, float* y, cudaStream_t st, const float* residual) {
+    const TileCosts t = tile_costs(M, N);
+    const long c256 = t.c256, c128 = t.c128, c64 = t.c64, c32 = t.c32;
+    if (t.pair) return launch_gemm_pair(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
     if (N > 128 && c256 <= c128 && c256 <= c64 && c256 <= c32) return launch_gemm<256, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     if (N > 64 && c128 <= c64 && c128 <= c32) return launch_gemm<128, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     if (N > 32 && c64 <= c32) return launch_gemm<64, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     if (N > 16) return launch_gemm<32, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
     return launch_gemm<16, false>(a, M, w, N, K, 1, N, acc, y, s_tok, s_ch, st, residual);
+}
+
+// The fused gate | up product (w: F gate rows, then F up rows) with silu(gate) * up and the transform's index bits 1..4 in its epilogue: h [M][F],
+// for fht8192_rest. It writes half of what the plain product writes and the transform then reads, and the transform loses its first passes. 32768
+// rows, 8192 channels: product 1006 + SiLU, transform and quantiser 692 us apart, 1240 + 254 us this way (2 x 1.07 GB less through memory);
+// a prompt of 32 x 1024 tokens 74.9 -> 71.4 ms, 32 x 256 15.8 -> 15.0, 1 x 256 2.58 -> 2.48. Taken where the product runs on CTA pairs
+// anyway (more than 128 rows); elsewhere FLEXLLM_ENOTSUP and nothing is launched.
+int gemm_i8_prefill_swiglu(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int F, int K, float* h, cudaStream_t st) {
+    if (F % 128 != 0 || !tile_costs(M, 2 * F).pair) return FLEXLLM_ENOTSUP;
+    return launch_gemm_pair<true>(a, s_tok, w, s_ch, M, 2 * F, K, nullptr, h, st, nullptr);
 }
 
 // Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side. K is split over clusters of up to four CTAs as

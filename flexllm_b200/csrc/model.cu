@@ -28,6 +28,8 @@
 namespace flexllm {
 int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
                     int32_t* acc, float* y, cudaStream_t st, const float* residual);
+int fht8192_rest(const float* h, int M, float scale, int8_t* q, float* s, cudaStream_t st);
+int gemm_i8_prefill_swiglu(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int F, int K, float* h, cudaStream_t st);
 int swiglu_fht_quant_strided(const float* g, const float* u, long ld, int M, float scale, int8_t* q, float* s, cudaStream_t st);
 size_t mha_prefill_ws_bytes(int B, int max_prefill, int max_ctx, int HQ, int HKV);
 int mha_prefill_paged(const float* qkv, const float* cos_t, const float* sin_t, const float* a_s, int B, int Sq, int q_off, int HQ, int HKV,
@@ -460,8 +462,14 @@ static int prefill_chunk(flexllm_model* m, const int32_t* tokens, const float* e
             TRY(flexllm_quant_per_token(m->att, M, D, m->xq, m->xs, st));
             TRY(gemm_i8_prefill(m->xq, m->xs, L.wo, L.so, M, D, D, nullptr, m->x, st, m->x));       // x += o_proj
             TRY(flexllm_rmsnorm_quant(m->x, L.g1, M, D, m->cfg.eps, FLEXLLM_NORM_PREFILL, nullptr, m->xq, m->xs, st));
-            TRY(gemm_i8_prefill(m->xq, m->xs, L.wgu, L.sgu, M, 2 * F, D, nullptr, m->gu, st, nullptr));
-            TRY(swiglu_fht_quant_strided(m->gu, m->gu + F, 2L * F, M, m->cfg.fht_scale, m->hq, m->xs, st));
+            const int fused = gemm_i8_prefill_swiglu(m->xq, m->xs, L.wgu, L.sgu, M, F, D, m->gu, st);
+            if (fused == FLEXLLM_ENOTSUP) {
+                TRY(gemm_i8_prefill(m->xq, m->xs, L.wgu, L.sgu, M, 2 * F, D, nullptr, m->gu, st, nullptr));
+                TRY(swiglu_fht_quant_strided(m->gu, m->gu + F, 2L * F, M, m->cfg.fht_scale, m->hq, m->xs, st));
+            } else {
+                TRY(fused);
+                TRY(fht8192_rest(m->gu, M, m->cfg.fht_scale, m->hq, m->xs, st));
+            }
             TRY(gemm_i8_prefill(m->hq, m->xs, L.wd, L.sd, M, D, F, nullptr, m->x, st, m->x));       // x += down_proj
         } else {
             // heads are local: gather the attention output, quantise whole rows, keep this rank's columns

@@ -74,6 +74,13 @@ def test_model_full_width(F):
     run_case(F, layers=2, hidden=2048, hq=32, hkv=8, vocab=128256, B=2, S=64, n_new=3, seed=52, use_graph=True)
 
 
+@pytest.mark.parametrize("B,S", [(1, 128), (1, 144), (2, 192), (3, 112), (5, 128)])
+def test_model_swiglu_in_the_product(F, B, S):
+    """Prompts on both sides of the row count from which silu(gate) * up is formed in the product's epilogue, with full tiles of 256 rows, a rest
+    in the first half of the last tile and one in the second."""
+    run_case(F, 1, 256, 4, 1, 512, B, S, 1, seed=70 + S, use_graph=False)
+
+
 def test_model_batch_over_8(F):
     """More than 8 sequences sends the decode linear layers down the tensor-core split-K path."""
     run_case(F, layers=2, hidden=512, hq=8, hkv=2, vocab=1000, B=12, S=16, n_new=4, seed=53, use_graph=True)
