@@ -300,12 +300,10 @@ __global__ void __launch_bounds__(64 * G) dec_pv_kernel(KvLayer cache, const int
     atomicAdd(oacc + ((long)b * HQ + hq) * 64 + t, acc);
 }
 
-// ---- fused single-kernel path (body in attention_decode.cuh) ----------------------------------------
+// ---- fused single-kernel path (body in attention_decode.cuh): short contexts ------------------------------------------------------
 // Grid (4 / G HKV, B): a CTA per (sequence, KV head) with the four query heads of the group, or two CTAs with two heads each, which halves
-// the shared memory of a CTA's rows and its chain of phases, for a second reading of the pages from L2. Two CTAs share an SM.
-// RANK: CTA row y takes the sequence with the y-th largest context, so that the last CTAs to start are the shortest.
-constexpr int DEC_RANK_MAX = 1024;         // batches up to this are ordered by length
-template <bool IN_F32, int NT, int G, bool RANK>
+// a CTA's chain of phases for a second reading of the pages from L2. Two CTAs share an SM.
+template <bool IN_F32, int NT, int G>
 __global__ void __launch_bounds__(NT, 2) dec_attn_fused_kernel(const int8_t* __restrict__ q, const float* __restrict__ qs,
                                                              const int8_t* __restrict__ k, const float* __restrict__ ks,
                                                              const int8_t* __restrict__ v, const float* __restrict__ vs,
@@ -322,37 +320,344 @@ __global__ void __launch_bounds__(NT, 2) dec_attn_fused_kernel(const int8_t* __r
     in.q = q; in.qs = qs; in.k = k; in.ks = ks; in.v = v; in.vs = vs; in.qkv_f32 = qkv_f32;
     in.qkv_acc = nullptr; in.tok_scale = nullptr; in.ch_scale = nullptr; in.n_slabs = 0; in.slab_stride = 0;
     in.max_pos = max_pos; in.error_flag = error_flag;
-    int b = blockIdx.y;
-    if constexpr (RANK) {
-        // the rank of a sequence is the number of longer ones (equal ones in order): a warp counts for one sequence at a time
-        __shared__ int b_sm;
-        const int B = gridDim.y, lane = threadIdx.x & 31;
-        for (int t = threadIdx.x >> 5; t < B; t += NT / 32) {
-            const int mine = ctx[t];
-            int rank = 0;
-            for (int u0 = 0; u0 < B; u0 += 32) {
-                const int u = u0 + lane, c = u < B ? ctx[u] : 0;
-                rank += __popc(__ballot_sync(0xffffffffu, u < B && (c > mine || (c == mine && u < t))));
-            }
-            if (lane == 0 && rank == (int)blockIdx.y) b_sm = t;
-        }
-        __syncthreads();
-        b = b_sm;
-    }
     dec_attn_fused_body<IN_F32 ? 1 : 0, NT, G>(in, cos_t, sin_t, a_s, cache, page_table, max_pages, ctx, HQ, HKV, cs, out, oacc,
-                                               (int)blockIdx.x / (4 / G), b, dsm, sm, (int)threadIdx.x, 0, (int)blockIdx.x % (4 / G));
+                                               (int)blockIdx.x / (4 / G), (int)blockIdx.y, dsm, sm, (int)threadIdx.x, 0, (int)blockIdx.x % (4 / G));
 }
 
-template <int G, bool RANK>
+template <int G>
 static int launch_dec_fused(bool in_f32, const int8_t* q, const float* qs, const int8_t* k, const float* ks, const int8_t* v, const float* vs,
                             const float* qkv_f32, const float* cos_t, const float* sin_t, const float* a_s, const KvLayer& L, const int32_t* page_table,
                             int max_pages, const int32_t* ctx, int B, int HQ, int HKV, int cs, float* out, int32_t* oacc, int max_ctx, int* err,
                             cudaStream_t st) {
     const size_t smem = dec_attn_smem_bytes<G>(cs);
-    auto kern = in_f32 ? dec_attn_fused_kernel<true, 512, G, RANK> : dec_attn_fused_kernel<false, 512, G, RANK>;
-    if (smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    auto kern = in_f32 ? dec_attn_fused_kernel<true, 512, G> : dec_attn_fused_kernel<false, 512, G>;
+    if (smem > 40 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));   // 48 KB with the static part
     launch_k(kern, dim3(4 / G * HKV, B), dim3(512), smem, st, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx,
              HQ, HKV, cs, out, oacc, max_ctx, err);
+    return launch_status(1);
+}
+
+// ---- the same step by a cluster of four CTAs per (sequence, KV head) ------------------------------------------------------------------
+// Grid (4 HKV, B). CTA r takes the r-th quarter of the item's pages for the two products, so every page is read by one SM only, and the softmax of
+// the group's query head r over all keys, so the ordered sums run for the four heads at once. Scores go straight into the shared memory of the
+// CTA of their head, the 8-bit probabilities from there to the CTA that has the key's page; three cluster barriers in all. Both
+// products are warp-level integer MMAs whose inner index is permuted the same way on both sides, so that a lane's 16 consecutive
+// bytes of a row are its four operand words. A CTA needs 5 bytes per key, so four share an SM (64 registers a thread): while one waits for its
+// pages, its peers or the ordered sums, the others have work.
+// Bound by that chain of phases (64 x 8100 keys, one generation of CTAs: 46 us, of which the scores 11, ordered sums 8, P.V 5) and by memory:
+// 64 sequences of 512 to 8192 keys (47 us at the copy rate) 98 us, 125 before with every page read by two SMs.
+constexpr int DEC_FUSED_KEYS = 10240;      // most keys of the forms with an item per CTA
+constexpr int DEC_CL = 4, DEC_CL_NT = 256, DEC_CL_PAGES = 512;       // CTAs of a cluster (one per query head), threads, most pages of a sequence
+struct DecClusterSmem {
+    __align__(16) int8_t q_sm[4][64];
+    __align__(16) int8_t new_k[64];
+    float q_scale[4], new_ks, wmax[32], rinv;
+    int pv[4][64], tot[64];
+    int pt[DEC_CL_PAGES];
+    int b;
+};
+// dynamic shared memory: one score row over all pages, then four rows of 8-bit probabilities over a CTA's pages
+__host__ __device__ constexpr int dec_cluster_own(int pages) { return (pages + DEC_CL - 1) / DEC_CL; }
+constexpr size_t dec_cluster_smem_bytes(int pages) { return (size_t)pages * PAGE * 4 + (size_t)DEC_CL * dec_cluster_own(pages) * PAGE; }
+
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+template <bool IN_F32>
+__global__ void __launch_bounds__(DEC_CL_NT, 4) dec_attn_cluster_kernel(const DecAttnIn in, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                                                        const float* __restrict__ a_s, KvLayer cache,
+                                                                        const int32_t* __restrict__ page_table, int max_pages,
+                                                                        const int32_t* __restrict__ ctx, int HQ, int HKV, int pages, int rank_b,
+                                                                        float* __restrict__ out, int32_t* __restrict__ oacc) {
+    constexpr int NW = DEC_CL_NT / 32, CL = DEC_CL;
+    extern __shared__ __align__(16) uint8_t dsm[];
+    __shared__ DecClusterSmem sm;
+    float* row = reinterpret_cast<float*>(dsm);                      // [pages * PAGE]: scores, then exponentials, of head r
+    uint8_t* u_sm = dsm + (size_t)pages * PAGE * 4;                  // [4][own * PAGE]
+    const int ur = dec_cluster_own(pages) * PAGE;                    // row length of u_sm
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, gi = lane >> 2, ti = lane & 3;
+    const int r = blockIdx.x % CL, hkv = blockIdx.x / CL;
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");    // the peers may write here once all have arrived (waited for below)
+    sm.pv[tid >> 6][tid & 63] = 0;
+    if (tid < 64) sm.tot[tid] = 0;
+    pdl_sync();
+    int b = blockIdx.y;
+    if (rank_b) {
+        // grid row y takes the sequence with the y-th largest context (equal ones in order): the last clusters to start are the shortest
+        const int B = gridDim.y;
+        int* len = reinterpret_cast<int*>(u_sm);                     // (no peer writes here before the second cluster barrier)
+        for (int t = tid; t < B; t += DEC_CL_NT) len[t] = ctx[t];
+        __syncthreads();
+        for (int t0 = 0; t0 < B; t0 += DEC_CL_NT / 4) {              // four lanes count for one sequence
+            const int t = t0 + (tid >> 2), mine = t < B ? len[t] : 0;
+            int rank = 0;
+#pragma unroll 4
+            for (int u = ti; u < B; u += 4) rank += len[u] > mine || (len[u] == mine && u < t);
+            rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+            rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+            if (t < B && rank == (int)blockIdx.y) sm.b = t;
+        }
+        __syncthreads();
+        b = sm.b;
+    }
+    const int heads = HQ + 2 * HKV;
+    const int pos = dec_guarded_pos(ctx, b, in.max_pos, in.error_flag);
+    const int nk = pos + 1, np_all = (nk + PAGE - 1) / PAGE;
+    auto first_page = [&](int c) { return np_all * c / CL; };        // of CTA c
+    const int p0 = first_page(r), np = first_page(r + 1) - p0;       // this CTA's pages (none in short contexts)
+    const bool has_new = r == CL - 1;                                // the new token is in the last page
+    for (int p = tid; p < np_all; p += DEC_CL_NT) sm.pt[p] = page_table[(long)b * max_pages + p];
+    // ---- A. prepare: warps 0..3 the query heads (every CTA), warp 4 the key head and warp 5 the value head (the CTA that has the new token)
+    if (w < 4 || (w < 6 && has_new)) {
+        const int h = w < 4 ? hkv * 4 + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
+        float a, bb;
+        int8_t c0 = 0, c1 = 0;
+        float sc_in = 0.0f;
+        if (IN_F32) {
+            const float* src = in.qkv_f32 + (long)b * heads * 64 + (long)h * 64;
+            a = src[lane]; bb = src[lane + 32];
+        } else {
+            const int8_t* src = w < 4 ? in.q + ((long)b * HQ + hkv * 4 + w) * 64 : (w == 4 ? in.k : in.v) + ((long)b * HKV + hkv) * 64;
+            sc_in = w < 4 ? in.qs[(long)b * HQ + hkv * 4 + w] : (w == 4 ? in.ks : in.vs)[(long)b * HKV + hkv];
+            c0 = src[lane]; c1 = src[lane + 32];
+            a = (float)c0 * sc_in; bb = (float)c1 * sc_in;
+        }
+        const int slot = pos % PAGE;
+        const long pg = w >= 4 ? page_table[(long)b * max_pages + pos / PAGE] : 0;
+        float s2 = sc_in;
+        int8_t qa = c0, qb = c1;                                     // an int8 value head is copied
+        if (IN_F32 || w < 5) {
+            if (w < 5) {
+                const float c = cos_t[(long)pos * 32 + lane], sn = sin_t[(long)pos * 32 + lane];
+                const float x0 = a, x1 = bb;
+                a = x0 * c - x1 * sn;
+                bb = x0 * sn + x1 * c;
+                auto lane_stage = [&](int bit) {
+                    float pa = __shfl_xor_sync(0xffffffffu, a, 1 << bit);
+                    float pb = __shfl_xor_sync(0xffffffffu, bb, 1 << bit);
+                    if (lane & (1 << bit)) { a = pa - a; bb = pb - bb; }
+                    else { a = a + pa; bb = bb + pb; }
+                };
+                lane_stage(1); lane_stage(2); lane_stage(3); lane_stage(4);
+                { float lo = a, hi = bb; a = lo + hi; bb = lo - hi; }
+                lane_stage(0);
+                a = a / 8.0f;
+                bb = bb / 8.0f;
+            }
+            const float mx = warp_max(fmaxf(a, bb)), mn = warp_min(fminf(a, bb));
+            s2 = sym_scale_from(mx, mn);
+            qa = quant_s8(a, s2); qb = quant_s8(bb, s2);
+        }
+        if (w < 4) {
+            sm.q_sm[w][lane] = qa; sm.q_sm[w][lane + 32] = qb;
+            if (lane == 0) sm.q_scale[w] = s2;
+        } else if (w == 4) {                                         // into the cache, and beside it for this step's product
+            int8_t* dst = cache.k + ((pg * HKV + hkv) * PAGE + slot) * 64L;
+            dst[lane] = qa; dst[lane + 32] = qb;
+            sm.new_k[lane] = qa; sm.new_k[lane + 32] = qb;
+            if (lane == 0) { cache.ks[(pg * HKV + hkv) * PAGE + slot] = s2; sm.new_ks = s2; }
+        } else {
+            int8_t* dst = cache.v + (pg * HKV + hkv) * (long)(64 * PAGE);
+            dst[(long)lane * PAGE + slot] = qa;
+            dst[(long)(lane + 32) * PAGE + slot] = qb;
+            if (lane == 0) cache.vs[(pg * HKV + hkv) * PAGE + slot] = s2;
+        }
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");      // every peer has started
+    // ---- B. scores: a warp takes a page at a time; A = 16 key rows, B = the four query heads (columns 4..7 zero). Lanes with ti = 2, 3 take over
+    //         the sums of key rows 8..15 from lanes ti - 2: every lane then has one key of two heads.
+    {
+        int bq[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) bq[i] = gi < 4 ? *reinterpret_cast<const int*>(&sm.q_sm[gi & 3][ti * 16 + i * 4]) : 0;
+        const int h0 = (ti & 1) * 2, kl = gi + 8 * (ti >> 1);
+        const float qs0 = sm.q_scale[h0], qs1 = sm.q_scale[h0 + 1];
+        const uint32_t row0 = tc::cluster_addr(tc::smem_u32(row), h0), row1 = tc::cluster_addr(tc::smem_u32(row), h0 + 1);
+        float mx0 = -1e32f, mx1 = -1e32f;
+        for (int p = w; p < np; p += NW) {
+            const long base = (long)sm.pt[p0 + p] * HKV + hkv;
+            const int8_t* rows = cache.k + base * (long)(64 * PAGE) + gi * 64 + ti * 16;
+            int4 k4[8];
+            float ks[4];
+#pragma unroll
+            for (int i = 0; i < 8; i++) k4[i] = *reinterpret_cast<const int4*>(rows + i * 512);
+#pragma unroll
+            for (int i = 0; i < 4; i++) ks[i] = cache.ks[base * PAGE + i * 16 + kl];
+            // the page of V is asked into L2 meanwhile, with its scales
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(cache.v + base * (long)(64 * PAGE) + lane * 128));
+            if (lane < 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(cache.vs + base * PAGE + lane * 32));
+            if (has_new && p == np - 1) {                            // the new token's row, which the loads may or may not have seen
+                const int slot = pos % PAGE;
+#pragma unroll
+                for (int i = 0; i < 8; i++) if (i * 8 + gi == slot) k4[i] = *reinterpret_cast<const int4*>(sm.new_k + ti * 16);
+#pragma unroll
+                for (int i = 0; i < 4; i++) if (i * 16 + kl == slot) ks[i] = sm.new_ks;
+            }
+            const int key0 = (p0 + p) * PAGE + kl;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                int d[4] = {0, 0, 0, 0};
+                const int a0[4] = {k4[2 * i].x, k4[2 * i + 1].x, k4[2 * i].y, k4[2 * i + 1].y}, b0[2] = {bq[0], bq[1]};
+                const int a1[4] = {k4[2 * i].z, k4[2 * i + 1].z, k4[2 * i].w, k4[2 * i + 1].w}, b1[2] = {bq[2], bq[3]};
+                mma_s8s8(d, a0, b0);
+                mma_s8s8(d, a1, b1);
+                const int o2 = __shfl_sync(0xffffffffu, d[2], lane & ~2), o3 = __shfl_sync(0xffffffffu, d[3], lane & ~2);
+                const float x0 = (((float)(ti < 2 ? d[0] : o2) * qs0) * ks[i]) * 0.125f, x1 = (((float)(ti < 2 ? d[1] : o3) * qs1) * ks[i]) * 0.125f;
+                const int key = key0 + i * 16;
+                st_cluster_f32(row0 + key * 4, x0);
+                st_cluster_f32(row1 + key * 4, x1);
+                if (key < nk) { mx0 = x0 > mx0 ? x0 : mx0; mx1 = x1 > mx1 ? x1 : mx1; }
+            }
+        }
+        // maximum over the lanes with the same ti & 1 (xor 2, 4, 8, 16)
+#pragma unroll
+        for (int o = 2; o < 32; o <<= 1) {
+            mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
+            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+        }
+        // lanes 0 and 2 hold heads 0 and 1, lanes 1 and 3 heads 2 and 3
+        if (lane < 4) st_cluster_f32(tc::cluster_addr(tc::smem_u32(&sm.wmax[r * NW + w]), ((lane & 1) << 1) | (lane >> 1)), lane >> 1 ? mx1 : mx0);
+    }
+    const ExpTable tab = exp_table_lane();
+    tc::cluster_sync();
+    // ---- D. e = exp(x - max) in place, zero beyond the last key: eight values at a time
+    const int npk = np_all * PAGE;
+    {
+        const float m = warp_max(sm.wmax[lane]) + 0.0f;              // a zero without a sign: max - x is then never -0 (exp_warp)
+        for (int k0 = w * 256; k0 < npk; k0 += DEC_CL_NT * 8) {      // a warp takes 256 keys, a lane eight of them
+            float u[8], e[8], far = 0.0f;
+            float4* at[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int key = k0 + i * 128 + lane * 4;
+                at[i] = reinterpret_cast<float4*>(row + key);
+                const float4 x = key < npk ? *at[i] : make_float4(m, m, m, m);
+                u[4 * i] = key < nk ? m - x.x : 0.0f; u[4 * i + 1] = key + 1 < nk ? m - x.y : 0.0f;
+                u[4 * i + 2] = key + 2 < nk ? m - x.z : 0.0f; u[4 * i + 3] = key + 3 < nk ? m - x.w : 0.0f;
+                far = max3_nan(max3_nan(far, u[4 * i], u[4 * i + 1]), u[4 * i + 2], u[4 * i + 3]);
+            }
+            if (__all_sync(0xffffffffu, far <= kExpFastLimit)) exp_warp<true>(u, e, tab);
+            else {
+#pragma unroll
+                for (int i = 0; i < 8; i++) e[i] = ref_expf(-u[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int key = k0 + i * 128 + lane * 4;
+                if (key < npk) *at[i] = make_float4(key < nk ? e[4 * i] : 0.0f, key + 1 < nk ? e[4 * i + 1] : 0.0f, key + 2 < nk ? e[4 * i + 2] : 0.0f,
+                                                    key + 3 < nk ? e[4 * i + 3] : 0.0f);
+            }
+        }
+    }
+    __syncthreads();
+    // ---- E. the four ordered chains of the head, key = j mod 4 (Softmax.h:514-553): one lane per chain, the 16 terms of a page at a time, the next page's
+    //         loads under way while this one is added: a step costs the addition's latency. (The zeros of the last page change nothing.)
+    //         Meanwhile the other warps, which quantise, fetch their keys' V scales.
+    constexpr int FV = 8, F_KEYS = (DEC_CL_NT - 32) * 4;             // vectors of four scales held by a thread, keys of one pass over its warps
+    float4 vs4[FV];
+    auto v_scales = [&](int k) { return *reinterpret_cast<const float4*>(cache.vs + ((long)sm.pt[k / PAGE] * HKV + hkv) * PAGE + k % PAGE); };
+    if (w == 0) {
+        float ps = 0.0f, c0[16], c1[16];
+        auto load = [&](float (&c)[16], int p) {
+#pragma unroll
+            for (int t = 0; t < 16; t++) c[t] = row[p * PAGE + 4 * t + ti];
+        };
+        auto add = [&](const float (&c)[16]) {
+#pragma unroll
+            for (int t = 0; t < 16; t++) ps += c[t];
+        };
+        load(c0, 0);
+        int p = 0;
+        for (; p + 2 < np_all; p += 2) { load(c1, p + 1); add(c0); load(c0, p + 2); add(c1); }
+        if (p + 1 < np_all) { load(c1, p + 1); add(c0); add(c1); }
+        else add(c0);
+        const float q0 = __shfl_sync(0xffffffffu, ps, 0), q1 = __shfl_sync(0xffffffffu, ps, 1);
+        const float q2 = __shfl_sync(0xffffffffu, ps, 2), q3 = __shfl_sync(0xffffffffu, ps, 3);
+        if (lane == 0) sm.rinv = 1.0f / ((q0 + q1) + (q2 + q3));
+    } else {
+#pragma unroll
+        for (int i = 0; i < FV; i++) {
+            const int k = i * F_KEYS + (tid - 32) * 4;
+            if (k < npk) vs4[i] = v_scales(k);
+        }
+    }
+    __syncthreads();
+    // ---- F. probabilities to u8 (zero beyond the last key), four keys a thread, into the CTA that has their page
+    if (w > 0) {
+        const float rinv = sm.rinv, as = a_s[hkv * 4 + r];
+        bool ok;
+        const float c = dec_u8_factor(rinv, as, ok);
+        const uint32_t u_at = tc::smem_u32(u_sm) + r * ur;
+        const int f1 = first_page(1), f2 = first_page(2), f3 = first_page(3);
+        auto quantise = [&](int k, const float4& s4) {
+            const int p = k / PAGE, own = (p >= f1) + (p >= f2) + (p >= f3), fp = own == 0 ? 0 : own == 1 ? f1 : own == 2 ? f2 : f3;
+            const float4 e4 = *reinterpret_cast<const float4*>(row + k);
+            const float e[4] = {e4.x, e4.y, e4.z, e4.w}, vs[4] = {s4.x, s4.y, s4.z, s4.w};
+            uint32_t v = 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) v |= (k + i < nk ? dec_u8(e[i], c, ok, rinv, vs[i], as) : 0u) << (8 * i);
+            st_cluster_u32(tc::cluster_addr(u_at + (p - fp) * PAGE + k % PAGE, own), v);
+        };
+#pragma unroll
+        for (int i = 0; i < FV; i++) {
+            const int k = i * F_KEYS + (tid - 32) * 4;
+            if (k < npk) quantise(k, vs4[i]);
+        }
+        for (int k = FV * F_KEYS + (tid - 32) * 4; k < npk; k += F_KEYS) quantise(k, v_scales(k));
+    }
+    tc::cluster_sync();
+    // ---- G. P.V, a page per warp at a time: A = 16 dims x keys of the V^T page, B = keys x the four heads
+    {
+        int acc[4][4] = {};
+        for (int p = w; p < np; p += NW) {
+            const long base = (long)sm.pt[p0 + p] * HKV + hkv;
+            const int8_t* rows = cache.v + base * (long)(64 * PAGE) + gi * PAGE + ti * 16;
+            int4 v4[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v4[i] = *reinterpret_cast<const int4*>(rows + i * 8 * PAGE);
+            const int4 u4 = gi < 4 ? *reinterpret_cast<const int4*>(u_sm + gi * ur + p * PAGE + ti * 16) : make_int4(0, 0, 0, 0);
+            const int b0[2] = {u4.x, u4.y}, b1[2] = {u4.z, u4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int a0[4] = {v4[2 * i].x, v4[2 * i + 1].x, v4[2 * i].y, v4[2 * i + 1].y};
+                const int a1[4] = {v4[2 * i].z, v4[2 * i + 1].z, v4[2 * i].w, v4[2 * i + 1].w};
+                mma_s8u8(acc[i], a0, b0);
+                mma_s8u8(acc[i], a1, b1);
+            }
+        }
+        if (ti < 2 && w < np) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) atomicAdd(&sm.pv[2 * ti + (j & 1)][i * 16 + gi + (j >> 1) * 8], acc[i][j]);
+        }
+    }
+    __syncthreads();
+    if (np > 0)                                                      // whole numbers: exact in any order
+        asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;"
+                     ::"r"(tc::cluster_addr(tc::smem_u32(&sm.tot[tid & 63]), tid >> 6)), "r"(sm.pv[tid >> 6][tid & 63]) : "memory");
+    tc::cluster_sync();
+    if (tid < 64) {
+        const int hq = hkv * 4 + r, tot = sm.tot[tid];
+        const long o = ((long)b * HQ + hq) * 64 + tid;
+        out[o] = (float)tot * a_s[hq];
+        if (oacc) oacc[o] = tot;
+    }
+}
+
+static int launch_dec_cluster(bool in_f32, const DecAttnIn& in, const float* cos_t, const float* sin_t, const float* a_s, const KvLayer& L,
+                              const int32_t* page_table, int max_pages, const int32_t* ctx, int B, int HQ, int HKV, int pages, bool rank, float* out,
+                              int32_t* oacc, cudaStream_t st) {
+    const size_t smem = dec_cluster_smem_bytes(pages);
+    auto kern = in_f32 ? dec_attn_cluster_kernel<true> : dec_attn_cluster_kernel<false>;
+    FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_cluster(kern, dim3(DEC_CL * HKV, B), dim3(DEC_CL_NT), DEC_CL, smem, st, in, cos_t, sin_t, a_s, L, page_table, max_pages, ctx, HQ, HKV,
+                   pages, rank ? 1 : 0, out, oacc);
     return launch_status(1);
 }
 
@@ -550,21 +855,23 @@ int flexllm::mha_decode_run(flexllm_kv_cache* c, int layer, const int8_t* q, con
     KvLayer L = kv_layer(c, layer);
     int* err = device_error_flag();     // raised (and the length clamped) when a ctx[] entry lies beyond max_ctx
 
-    // enough (sequence, head) pairs, or short rows: one fused kernel; otherwise the split kernels
-    if (ctx_stride <= 10240 && (B * HKV >= 64 || max_ctx <= 2048)) {
-        const int sms = gemm_sm_count();
-        // Four heads to a CTA while two CTAs' rows fit an SM (contexts up to about 5700): less work in all. Two heads beyond that, where the
-        // four-head form leaves one CTA an SM, and where the CTAs are few: every SM at most one, or at most two and long contexts.
-        // Sequences by length where CTAs follow one another on an SM and contexts are long enough to pay for the ranking, and among two-head
-        // CTAs where they share an SM.
-        // us, four heads / two heads / two heads by length, 8 KV heads: 8 x 2000 keys 20.4 / 14.7 / 14.7; 16 x 510 11.6 / 12.1 / 12.4, 16 x 2000
-        // 20.7 / 19.4 / 19.8; 64 x 30 15.9 / 25.4 / 28.0, 64 x 4096 121 / 135 / 139, 64 x 6000 244 / 189 / 189; 64 of 512 to 8192
-        // 175 / 141 / 125. Four heads, in order / by length: 64 x 30 15.9 / 19.3, 64 x 2000 61.5 / 63.7, 64 x 4096 121 / 121.
-        const bool room4 = 2 * (dec_attn_smem_bytes<4>(ctx_stride) + 3072) <= 228 * 1024;
-        const int ctas2 = 2 * HKV * B;
-        const bool two = !room4 || ctas2 <= sms || (ctas2 <= 2 * sms && max_ctx > 1536);
-        const bool rank = B <= DEC_RANK_MAX && (two ? ctas2 > sms : HKV * B > 2 * sms && max_ctx > 2048);
-        auto launch = two ? (rank ? launch_dec_fused<2, true> : launch_dec_fused<2, false>) : (rank ? launch_dec_fused<4, true> : launch_dec_fused<4, false>);
+    // Three forms. us, 8 KV heads: one or two CTAs per (sequence, head) / a cluster of four: 1 x 400 keys 8.0 / 8.2, 1 x 513 9.0 / 7.9,
+    // 1 x 2000 13.3 / 9.6; 16 x 400 9.4 / 10.3, 16 x 513 11.6 / 10.6, 16 x 8100 66.6 / 43.2; 18 x 2000 20.3 / 21.7; 32 x 1400 22.8 / 25.5,
+    // 32 x 1700 27.6 / 27.2, 32 x 8100 132 / 93.5; 64 x 300 19.2 / 33.3, 64 x 1700 57.7 / 56.1, 64 x 4096 120 / 102, 64 x 8100 245 / 170, 64 of 512 to
+    // 8192 125 / 98. So clusters from 513 keys where they all run at once (25 for every 24 SMs do not: their CTAs share a part of the
+    // chip), from 1665 where they follow one another, and where the second wave would be nearly empty not at all.
+    // Kernel per phase / cluster, the only choices for longer contexts: 1 x 10500 65 / 25, 16 x 32000 449 / 346, 64 x 14000 535 / 335.
+    const int sms = gemm_sm_count(), items = B * HKV;
+    const bool at_once = items * 25 <= sms * 24;
+    if (max_ctx > (at_once ? 512 : 1664) && ctx_stride <= DEC_CL_PAGES * PAGE && (at_once || items > sms || ctx_stride > DEC_FUSED_KEYS)) {
+        DecAttnIn in = {};
+        in.q = q; in.qs = qs; in.k = k; in.ks = ks; in.v = v; in.vs = vs; in.qkv_f32 = qkv_f32; in.max_pos = max_ctx; in.error_flag = err;
+        return launch_dec_cluster(qkv_f32 != nullptr, in, cos_t, sin_t, a_s, L, page_table, max_pages, ctx, B, HQ, HKV, ctx_stride / PAGE,
+                                  !at_once && B <= dec_cluster_own(ctx_stride / PAGE) * PAGE, out, oacc, st);
+    }
+    if (ctx_stride <= DEC_FUSED_KEYS) {
+        // Four heads to a CTA, or two where the CTAs are few: every SM at most one, or at most two and long contexts.
+        const auto launch = 2 * items <= sms || (items <= sms && max_ctx > 1536) ? launch_dec_fused<2> : launch_dec_fused<4>;
         return launch(qkv_f32 != nullptr, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx, B, HQ, HKV, ctx_stride, out, oacc,
                       max_ctx, err, st);
     }

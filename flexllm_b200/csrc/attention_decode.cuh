@@ -109,7 +109,7 @@ struct DecAttnSmem {
 // bytes), scores, max, exp, the ordered partial sums, the u8 quantiser and P.V, with the score rows kept in shared
 // memory (`dsm`: dec_attn_smem_bytes<G>). The group's NT threads (256 or 512; `tid` = index in the group) synchronise on named
 // barrier `bar`.
-// G = 2 (stand-alone operator, long contexts or few sequences): rows padded against bank conflicts in the ordered sums, which fetch ahead, the
+// G = 2 (stand-alone operator, few sequences): rows padded against bank conflicts in the ordered sums, which fetch ahead, the
 // warp-wide exponential and a quantiser without divisions. G = 4: the stand-alone operator otherwise, and the persistent kernel's form for
 // contexts beyond its staging area.
 template <int G> constexpr size_t dec_attn_smem_bytes(int cs) {

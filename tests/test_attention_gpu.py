@@ -328,3 +328,16 @@ def test_kv_append_alone(F):
     k0 = cache.pools(0)[0]
     assert int(k0.abs().max()) == 0          # the other layer was not touched
     cache.close()
+
+
+@pytest.mark.parametrize("ctx,HKV,what", [
+    ([512, 0, 63, 64, 65, 127, 128, 191, 192, 256], 8, {}), ([511, 510, 100], 8, {}),                # one side and the other of the first length
+    ([3000, 0, 63, 64, 255, 256, 257, 3000, 1023, 1024], 2, {}), ([3000, 2999, 31], 1, dict(q_gain=20.0)),
+    ([1700] + [130] * 9 + [1700] * 9 + [0], 8, {}), ([1662] + [40] * 18, 8, {}), ([1664, 1663] + [40] * 17, 8, dict(a_gain=0.01)),       # by length, with equal ones
+    ([2000] + [300] * 16, 8, {}), ([2000] + [300] * 17, 8, {}),                                      # all clusters at once, and not quite
+    ([10238], 8, {}), ([10239, 5], 8, {}), ([32766, 700], 1, {}), ([32767, 700], 1, {})],            # longest rows of either form
+    ids=lambda v: "%d_of_%d" % (len(v), v[0]) if isinstance(v, list) else None)
+def test_decode_cluster(F, ctx, HKV, what):
+    """The form with a cluster of four CTAs per item: lengths around its lines, sequences of fewer pages than CTAs, page and quarter
+    edges, few and many KV heads, two steps (the second reads what the first appended)."""
+    decode_case(F, len(ctx), ctx, HQ=4 * HKV, HKV=HKV, seed=70 + len(ctx), steps=2 if ctx[0] < 5000 else 1, **what)
