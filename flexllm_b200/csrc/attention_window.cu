@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ float red[16];
     __shared__ int last_sm;
+    __shared__ __align__(16) bf16 knew_sm[256];
     const AttnCall& c = a.c;
     const AttnShape& s = c.s;
     const int R = s.H / s.G;
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
     float* o_sm = mx_sm + 128;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = lane & 3;
     const int split = blockIdx.x, n_split = gridDim.x, g = blockIdx.y, b = blockIdx.z;
-    pdl_sync();
+    pdl_launch();
     const int pos = start_pos(c, b, a.error_flag);
     const KeyPages pages(s, pos, pos);
     const int n_pg = pages.n, n_tiles = (n_pg + 1) / 2;
@@ -438,34 +439,14 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
     const long kh = (long)PG * s.dkp, vh = (long)PG * s.dv;
     for (int i = tid; i < 2 * (t_end - t_beg); i += 256) pt_sm[i] = 2 * t_beg + i < n_pg ? pt[pages.at(2 * t_beg + i)] : -1;
     const int nv = s.dkp >> 3;
-    const float2 rms = qk_rms(c, prow, tid, red);
-    const float rq = rms.x, rk = rms.y;
-    for (int i = tid; i < 8 * nv; i += 256) {
-        const int r = i / nv, e0 = (i - r * nv) * 8;
-        float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (r < R) normed8(prow + s.q_off, c.q_gain, (g * R + r) * s.dk, e0, s.dk, rq, f);
-        store8(q_sm + r * (s.dkp + 8) + e0, f);
-    }
-    if (s.k_off >= 0 && split == n_split - 1) {
-        const long page = pt[pages.at(n_pg - 1)];
-        const int slot = pos & (PG - 1);
-        bf16* kp = (bf16*)c.k_pool + (page * s.G + g) * kh + (long)slot * s.dkp;
-        for (int i = tid; i < nv; i += 256) {
-            float f[8];
-            normed8(prow + s.k_off, c.k_gain, g * s.dk, i * 8, s.dk, rk, f);
-            store8(kp + i * 8, f);
-        }
-        bf16* vp = (bf16*)c.v_pool + (page * s.G + g) * vh + slot;
-        for (int d = tid; d < s.dv; d += 256) vp[(long)d * PG] = prow[s.v_off + g * s.dv + d];
-    }
     __syncthreads();
-
-    uint4 qb[DKC];
-#pragma unroll
-    for (int ch = 0; ch < DKC; ch++) {
-        const int e = ch * 32 + lc * 8;
-        qb[ch] = e < s.dkp ? *reinterpret_cast<const uint4*>(q_sm + lr * (s.dkp + 8) + e) : make_uint4(0, 0, 0, 0);
-    }
+    // Ahead of the wait for the kernel in front, all from memory: gains, the first tile's keys (but the new token's row, which is put in
+    // place below), its biases, and its values into L2.
+    const int qr = tid / nv, qe = (tid - qr * nv) * 8, qj = (g * R + qr) * s.dk + qe, kj = g * s.dk + tid * 8;        // 8 nv <= 256: a thread has 8 elements of q at most
+    float4 qg0 = make_float4(1.f, 1.f, 1.f, 1.f), qg1 = qg0, kg0 = qg0, kg1 = qg0;
+    const bool ahead = c.q_gain && (s.dk & 7) == 0;
+    if (ahead && qr < R && qe < s.dk) { qg0 = load4(c.q_gain + qj); qg1 = load4(c.q_gain + qj + 4); }
+    if (ahead && tid * 8 < s.dk && s.k_off >= 0) { kg0 = load4(c.k_gain + kj); kg1 = load4(c.k_gain + kj + 4); }
     uint4 kr[DKC][2];
     auto load_k = [&](int t) {
         const int page = pt_sm[2 * (t - t_beg) + (warp >> 2)];
@@ -478,13 +459,86 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
                 kr[ch][h] = in ? *reinterpret_cast<const uint4*>(kp + (long)h * 8 * s.dkp + ch * 32) : make_uint4(0, 0, 0, 0);
         }
     };
+    // biases of this thread's two keys and two heads (-inf: no such head; the table has -inf where a key is masked)
+    const float* bias_g = ONLINE ? nullptr : c.bias + (long)g * (2 * kBiasPad + s.window) * R;
+    auto distance = [&](int t) { return pos - (pages.at(2 * t + (warp >> 2)) * PG + (warp & 3) * 16 + lr); };       // of this thread's first key
+    float bi[2][2];
+    auto load_bias = [&](int t) {
+        const int d0 = distance(t);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                bi[h][u] = lc * 2 + u < R ? bias_g[(long)(d0 - 8 * h + kBiasPad) * R + lc * 2 + u] : -INFINITY;
+    };
+    if (t_beg < t_end) {
+        load_k(t_beg);
+        if (!ONLINE) load_bias(t_beg);
+        for (int i = tid * 64; i < 2 * (int)vh; i += 256 * 64) {                  // 128 bytes a request
+            const int page = pt_sm[i >= vh];
+            if (page >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"((const bf16*)c.v_pool + ((long)page * s.G + g) * vh + (i >= vh ? i - vh : i)));
+        }
+    }
+    pdl_wait();
+    float gate = 0.0f;                                                           // of this thread's first output
+    if (s.g_off >= 0 && tid < R * s.dv) gate = to_f(prow[s.g_off + (long)g * R * s.dv + tid]);
+    const float2 rms = qk_rms(c, prow, tid, red);
+    const float rq = rms.x, rk = rms.y;
+    auto scaled = [&](float (&f)[8], const float4& x, const float4& y, float r) {
+        f[0] = (f[0] * r) * x.x; f[1] = (f[1] * r) * x.y; f[2] = (f[2] * r) * x.z; f[3] = (f[3] * r) * x.w;
+        f[4] = (f[4] * r) * y.x; f[5] = (f[5] * r) * y.y; f[6] = (f[6] * r) * y.z; f[7] = (f[7] * r) * y.w;
+    };
+    if (qr < 8) {
+        float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (qr < R) {
+            if (ahead && qe < s.dk) { load8(prow + s.q_off + qj, f); scaled(f, qg0, qg1, rq); }
+            else if (!ahead) normed8(prow + s.q_off, c.q_gain, (g * R + qr) * s.dk, qe, s.dk, rq, f);
+        }
+        store8(q_sm + qr * (s.dkp + 8) + qe, f);
+    }
+    const bool has_new = split == n_split - 1;
+    if (s.k_off >= 0 && has_new) {
+        const long page = pt[pages.at(n_pg - 1)];
+        const int slot = pos & (PG - 1);
+        bf16* kp = (bf16*)c.k_pool + (page * s.G + g) * kh + (long)slot * s.dkp;
+        if (tid < nv) {
+            float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (ahead && tid * 8 < s.dk) { load8(prow + s.k_off + kj, f); scaled(f, kg0, kg1, rk); }
+            else if (!ahead) normed8(prow + s.k_off, c.k_gain, g * s.dk, tid * 8, s.dk, rk, f);
+            store8(kp + tid * 8, f);
+            store8(knew_sm + tid * 8, f);
+        }
+        bf16* vp = (bf16*)c.v_pool + (page * s.G + g) * vh + slot;
+        for (int d = tid; d < s.dv; d += 256) vp[(long)d * PG] = prow[s.v_off + g * s.dv + d];
+    }
+    __syncthreads();
+
+    uint4 qb[DKC];
+#pragma unroll
+    for (int ch = 0; ch < DKC; ch++) {
+        const int e = ch * 32 + lc * 8;
+        qb[ch] = e < s.dkp ? *reinterpret_cast<const uint4*>(q_sm + lr * (s.dkp + 8) + e) : make_uint4(0, 0, 0, 0);
+    }
+    // the new token's key row, where the first tile has it (a later tile is loaded after it is in memory): this layer's own, or that of the layer
+    // whose keys are used, written by an earlier kernel of this step
+    if (has_new && t_beg == n_tiles - 1 && (warp >> 2) == ((n_pg - 1) & 1)) {
+        const int slot = pos & (PG - 1), page = pt_sm[(n_pg - 1) & 1];
+        const bf16* krow = (const bf16*)c.k_pool + ((long)page * s.G + g) * kh + (long)slot * s.dkp;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if ((warp & 3) * 16 + lr + 8 * h == slot) {
+#pragma unroll
+                for (int ch = 0; ch < DKC; ch++)
+                    if (ch * 32 + lc * 8 < s.dkp)            // (past L1, which has the row as it was before)
+                        kr[ch][h] = s.k_off >= 0 ? *reinterpret_cast<const uint4*>(knew_sm + ch * 32 + lc * 8)
+                                                 : __ldcg(reinterpret_cast<const uint4*>(krow + ch * 32 + lc * 8));
+            }
+    }
     const int mt = warp % MTP, slice = warp / MTP;
     const bool pv_on = slice < KS;
     float acc[MPW][4] = {};
     float lsum[2] = {0.0f, 0.0f}, m_run[2] = {kNoScore, kNoScore};
-    const float* bias_g = ONLINE ? nullptr : c.bias + (long)g * (2 * kBiasPad + s.window) * R;
     const float badd = s.softcap * kLog2e - a.shift2;
-    if (t_beg < t_end) load_k(t_beg);
     for (int t = t_beg; t < t_end; t++) {
         uint4 vr[MPW][NCH][2];
         if (pv_on) {
@@ -502,15 +556,13 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
                     }
             }
         }
-        // biases of this thread's two keys and two heads (-inf: masked, or no such head)
-        const int d0 = pos - (pages.at(2 * t + (warp >> 2)) * PG + (warp & 3) * 16 + lr);        // distance of this thread's first key
-        float bi[2][2];
-        if (!ONLINE)
+        const int d0 = distance(t);
+        float bt[2][2];
+        if (!ONLINE) {
 #pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-                bi[h][u] = lc * 2 + u < R ? bias_g[(long)(d0 - 8 * h + kBiasPad) * R + lc * 2 + u] : -INFINITY;
+            for (int h = 0; h < 2; h++) { bt[h][0] = bi[h][0]; bt[h][1] = bi[h][1]; }
+            if (t + 1 < t_end) load_bias(t + 1);
+        }
         float sc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (int ch = 0; ch < DKC; ch++) {
@@ -555,7 +607,7 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 const float s2 = ONLINE ? sc[2 * h + u] - m_run[u]
-                                        : __fmaf_rn(a.b2, rcp_fast(1.0f + ex2_fast(sc[2 * h + u] * a.a2)), __fmaf_rn(bi[h][u], kLog2e, badd));
+                                        : __fmaf_rn(a.b2, rcp_fast(1.0f + ex2_fast(sc[2 * h + u] * a.a2)), __fmaf_rn(bt[h][u], kLog2e, badd));
                 const float p = ex2_fast(s2);
                 lsum[u] += p;
                 pb[(lc * 2 + u) * DT_PS + 8 * h] = __float2bfloat16_rn(p);
@@ -639,7 +691,7 @@ __global__ void __launch_bounds__(256, DKC == 8 || MPW == 2 ? 1 : 2) attn_decode
             l += head_l(r); v = head_o(r, i - r * s.dv);
         }
         v /= l;
-        if (s.g_off >= 0) v *= sigmoid_f<true>(to_f(prow[s.g_off + (long)g * R * s.dv + i]));
+        if (s.g_off >= 0) v *= sigmoid_f<true>(i == tid ? gate : to_f(prow[s.g_off + (long)g * R * s.dv + i]));
         out[i] = __float2bfloat16_rn(v);
     }
 }

@@ -39,8 +39,10 @@ inline int launch_status(int n = 1) { note_launches(n); return cuda_status(cudaG
 // scheduling overlap the tail of the previous one. Every kernel launched this way calls pdl_sync()
 // before it touches memory: it first lets its own dependents start launching, then waits until the
 // kernel before it has completed and flushed (so data hazards are exactly those of an ordinary stream).
+// g_pdl = 2: the next kernel is launched without the attribute and sets g_pdl to 1. It starts when everything before it in the stream has
+// completed, and the kernels behind it start after it: between the two halves (pdl_launch, pdl_wait) these may read whatever no kernel
+// of the same sequence of launches writes. Weights may be read there in any case.
 extern thread_local int g_pdl;
-// A kernel whose weights no earlier kernel writes may ask for them between the two halves.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { pdl_launch(); pdl_wait(); }
@@ -49,11 +51,12 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[1];
-    if (g_pdl) {
+    if (g_pdl == 1) {
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
     }
+    if (g_pdl) g_pdl = 1;
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
@@ -66,11 +69,12 @@ inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cl
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    if (g_pdl) {
+    if (g_pdl == 1) {
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
+    if (g_pdl) g_pdl = 1;
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 

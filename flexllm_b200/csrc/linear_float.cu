@@ -45,7 +45,15 @@ __global__ void __launch_bounds__(128) gemv_float_kernel(const T* __restrict__ a
     for (int r = 0; r < R; r++)
 #pragma unroll
         for (int u = 0; u < 2; u++) { const int c = kbeg + lane + 32 * u; nx[r][u] = (active && c < kend) ? ldg_stream16(wr[r] + (long)c * 8) : zero; }
-    pdl_sync();
+    pdl_launch();
+    float bs[OUT][2];                                    // biases: from memory as well
+#pragma unroll
+    for (int o = 0; o < OUT; o++) {
+        const int n = min(n0 + o, n_out - 1);
+        bs[o][0] = bias && active ? bias[weight_row<GLU>(n, 0, n_out)] : 0.0f;
+        bs[o][1] = GLU && bias && active ? bias[weight_row<true>(n, 1, n_out)] : 0.0f;
+    }
+    pdl_wait();
     for (int i = threadIdx.x; i < BT * kv; i += 128) {
         const int b = i / kv, c = i - b * kv;
         float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -123,11 +131,10 @@ __global__ void __launch_bounds__(128) gemv_float_kernel(const T* __restrict__ a
             if (b >= M) continue;
             float v;
             if (GLU) {
-                const long rg = weight_row<true>(n, 0, n_out), ru = weight_row<true>(n, 1, n_out);
-                const float gt = acc[2 * o < R ? 2 * o : 0][b] + (bias ? bias[rg] : 0.0f), up = acc[2 * o + 1 < R ? 2 * o + 1 : 0][b] + (bias ? bias[ru] : 0.0f);
+                const float gt = acc[2 * o < R ? 2 * o : 0][b] + bs[o][0], up = acc[2 * o + 1 < R ? 2 * o + 1 : 0][b] + bs[o][1];
                 v = gelu_tanh_f<FAST>(gt) * up;
             } else {
-                v = acc[o][b] + (bias ? bias[n] : 0.0f);
+                v = acc[o][b] + bs[o][0];
                 if (relu2) v = relu2_f(v);
             }
             if (y32) y32[(long)b * ldy + n] = v;
@@ -151,9 +158,16 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const bf16* src, bool l
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Biases of the output that thread t of a CTA writes (for every token: 256 is a multiple of the CTA's outputs); GLU: of its gate and its up row.
+// Asked for before the kernels in front have finished.
+struct SkinnyBias { float b0, b1; };
+template <int RT, bool GLU> __device__ __forceinline__ SkinnyBias skinny_bias(const float* __restrict__ bias, int N) {
+    const int n = blockIdx.x * RT * 16 + (int)threadIdx.x % (GLU ? 16 : RT * 16);
+    return {bias && n < N ? bias[n] : 0.0f, GLU && bias && n + RT * 16 - 16 < N ? bias[n + RT * 16 - 16] : 0.0f};
+}
 // The end of both forms: the warps' partial sums, added in warp order, and the epilogue.
 template <int NT, int RT, bool GLU>
-__device__ __forceinline__ void skinny_finish(const float (&acc)[RT][NT][4], float (&part)[8][RT * 16][NT * 8 + 1], const float* __restrict__ bias, int M, int N,
+__device__ __forceinline__ void skinny_finish(const float (&acc)[RT][NT][4], float (&part)[8][RT * 16][NT * 8 + 1], const SkinnyBias& bias, int M, int N,
                                               int relu2, float* y32, bf16* y16, long ldy) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
     const int row0 = blockIdx.x * RT * 16;
@@ -164,19 +178,18 @@ __device__ __forceinline__ void skinny_finish(const float (&acc)[RT][NT][4], flo
 #pragma unroll
             for (int i = 0; i < 4; i++) part[warp][r * 16 + lr + 8 * (i >> 1)][t * 8 + lc * 2 + (i & 1)] = acc[r][t][i];
     __syncthreads();
-    auto total = [&](int row, int tok) {
+    auto total = [&](int row, int tok, float b) {
         float v = part[0][row][tok];
 #pragma unroll
         for (int k = 1; k < 8; k++) v += part[k][row][tok];
-        const int n = row0 + row;
-        return v + (bias && n < N ? bias[n] : 0.0f);
+        return v + b;
     };
     constexpr int OUT = GLU ? 16 : RT * 16;                 // output columns of the CTA
     const int n0 = GLU ? row0 >> 1 : row0, n_out = GLU ? N >> 1 : N;
     for (int i = threadIdx.x; i < OUT * M; i += 256) {
         const int tok = i / OUT, o = i - tok * OUT;
         if (n0 + o >= n_out) continue;
-        float v = GLU ? gelu_tanh_f<true>(total(o, tok)) * total(RT * 16 - 16 + o, tok) : total(o, tok);
+        float v = GLU ? gelu_tanh_f<true>(total(o, tok, bias.b0)) * total(RT * 16 - 16 + o, tok, bias.b1) : total(o, tok, bias.b0);
         if (!GLU && relu2) v = relu2_f(v);
         if (y32) y32[(long)tok * ldy + n0 + o] = v;
         else y16[(long)tok * ldy + n0 + o] = __float2bfloat16_rn(v);
@@ -218,9 +231,11 @@ __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict_
             cp_async16(mine_u + (slot * ITEMS + RT * 2 + t) * 512, on ? ar[t] + (long)c * 32 : a, on);
         }
     };
+    pdl_launch();
 #pragma unroll
     for (int i = 0; i < DEPTH; i++) load_w(c_beg + i, i);
-    pdl_sync();
+    const SkinnyBias sb = skinny_bias<RT, GLU>(bias, N);
+    pdl_wait();
 #pragma unroll
     for (int i = 0; i < DEPTH; i++) { load_a(c_beg + i, i); cp_async_commit(); }      // the first of these groups holds all the weights too
     float acc[RT][NT][4] = {};
@@ -247,7 +262,7 @@ __global__ void __launch_bounds__(256) skinny_mma_kernel(const bf16* __restrict_
         if (++slot == DEPTH) slot = 0;
     }
     cp_async_wait<0>();
-    skinny_finish<NT, RT, GLU>(acc, part, bias, M, N, relu2, y32, y16, ldy);
+    skinny_finish<NT, RT, GLU>(acc, part, sb, M, N, relu2, y32, y16, ldy);
 }
 
 // The form without a ring, where that is the better one (skinny_nt): weights one group of chunks ahead in registers, activations read where
@@ -277,8 +292,10 @@ __global__ void __launch_bounds__(256) skinny_short_kernel(const bf16* __restric
                 for (int h = 0; h < 2; h++)
                     v[g][r][h] = (c + g < c_end && (c + g) * 4 + lc < kv) ? ldg_stream16(wr[r][h] + (long)(c + g) * 32) : zero;
     };
+    pdl_launch();
     load_w(nx, c_beg);
-    pdl_sync();
+    const SkinnyBias sb = skinny_bias<RT, GLU>(bias, N);
+    pdl_wait();
     float acc[RT][NT][4] = {};
     for (int c = c_beg; c < c_end; c += G) {
 #pragma unroll
@@ -305,7 +322,7 @@ __global__ void __launch_bounds__(256) skinny_short_kernel(const bf16* __restric
                     mma_bf16(acc[r][t], wv[g][r][0].z, wv[g][r][1].z, wv[g][r][0].w, wv[g][r][1].w, av[g][t].z, av[g][t].w);
                 }
     }
-    skinny_finish<NT, RT, GLU>(acc, part, bias, M, N, relu2, y32, y16, ldy);
+    skinny_finish<NT, RT, GLU>(acc, part, sb, M, N, relu2, y32, y16, ldy);
 }
 
 template <int NT, int RT, bool GLU, int DEPTH>

@@ -682,7 +682,7 @@ static int decode_step(flexllm_model* m, cudaStream_t st) {
     if (m->mega_state == 1) return mega_launch(m->mega, m->B, m->mega_variant, st);
     static int use_pdl = -1;
     if (use_pdl < 0) { const char* e = getenv("FLEXLLM_PDL"); use_pdl = e ? atoi(e) : 1; }
-    g_pdl = use_pdl;
+    g_pdl = use_pdl ? 2 : 0;             // the kernels of a step read the contexts, page tables and older cache entries ahead of their wait
     const int rc = decode_step_body(m, st);
     g_pdl = 0;
     return rc;

@@ -9,12 +9,28 @@ namespace {
 
 // One CTA of NT threads per row, VPT float4 of the row per thread. All sums and the residual are fp32. The columns from D
 // up to the next multiple of 4 are zero in x, the gains, y and the embedding table.
-template <class T, int NT, int VPT>
+// AHEAD (decoding: few rows, and gains that come from memory): the gains are asked for before the kernel in front has finished. Each took a
+// round trip to memory of its own in a chain of kernels that are all latency: steps of 4 sequences at the sizes of a 1B model, the same
+// done in products (biases), attention and state-space mixers, Pibidra 869 -> 761 us, Sabisun 846 -> 751 us. With the many rows of a prompt
+// it costs registers and a barrier for nothing.
+constexpr int kAheadRows = 64;
+template <class T, int NT, int VPT, bool AHEAD>
 __global__ void __launch_bounds__(NT) res_norm_kernel(const ResNormArgs a) {
     __shared__ float red[2 * NT / 32];
-    pdl_sync();
     const int r = blockIdx.x, tid = threadIdx.x;
     const int nv = (a.D + 3) >> 2;
+    pdl_launch();
+    float4 gp[AHEAD ? VPT : 1], gn[AHEAD ? VPT : 1];
+    if (AHEAD) {
+#pragma unroll
+        for (int i = 0; i < VPT; i++) {
+            const int c = tid + i * NT;
+            gp[i] = gn[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < nv && a.gain_post) gp[i] = load4(a.gain_post + 4 * c);
+            if (c < nv && a.gain_pre) gn[i] = load4(a.gain_pre + 4 * c);
+        }
+    }
+    pdl_wait();
     const long row = a.rows ? a.rows[r] : r;
     float* xr = a.x + row * a.ldx;
     const bf16* er = nullptr;
@@ -53,7 +69,7 @@ __global__ void __launch_bounds__(NT) res_norm_kernel(const ResNormArgs a) {
         for (int i = 0; i < VPT; i++) {
             const int c = tid + i * NT;
             if (c < nv) {
-                const float4 g = load4(a.gain_post + 4 * c);
+                const float4 g = AHEAD ? gp[AHEAD ? i : 0] : load4(a.gain_post + 4 * c);
                 v[i].x += (y[i].x * rinv) * g.x; v[i].y += (y[i].y * rinv) * g.y;
                 v[i].z += (y[i].z * rinv) * g.z; v[i].w += (y[i].w * rinv) * g.w;
             }
@@ -88,19 +104,35 @@ __global__ void __launch_bounds__(NT) res_norm_kernel(const ResNormArgs a) {
     for (int i = 0; i < VPT; i++) {
         const int c = tid + i * NT;
         if (c < nv) {
-            const float4 g = load4(a.gain_pre + 4 * c);
+            const float4 g = AHEAD ? gn[AHEAD ? i : 0] : load4(a.gain_pre + 4 * c);
             store4(hr + 4 * c, make_float4((v[i].x * rinv) * g.x, (v[i].y * rinv) * g.y, (v[i].z * rinv) * g.z, (v[i].w * rinv) * g.w));
         }
     }
 }
 
 // One CTA per row, all streams of VPT float4 per thread in registers.
-template <class T, int NS, int NT, int VPT>
+template <class T, int NS, int NT, int VPT, bool AHEAD>
 __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
-    __shared__ float red[2 * NT / 32];
-    pdl_sync();
+    __shared__ float red[2 * NT / 32], coef[AHEAD ? NS * NS + 2 * NS : 1];
     const int r = blockIdx.x, tid = threadIdx.x, n = a.n;
     const int nv = (a.D + 3) >> 2;
+    // AHEAD: mixing matrix, output and input coefficients, gains (see res_norm_kernel)
+    pdl_launch();
+    const float *mix = a.mix, *out = a.out, *in = a.in;
+    float4 gn[AHEAD ? VPT : 1];
+    if (AHEAD) {
+        if (tid < n * n && a.y) coef[tid] = a.mix[tid];
+        if (tid < n && a.y) coef[NS * NS + tid] = a.out[tid];
+        if (tid < n && a.gain) coef[NS * NS + NS + tid] = a.in[tid];
+        mix = coef; out = coef + NS * NS; in = out + NS;
+#pragma unroll
+        for (int i = 0; i < VPT; i++) {
+            gn[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid + i * NT < nv && a.gain) gn[i] = load4(a.gain + 4 * (tid + i * NT));
+        }
+        __syncthreads();
+    }
+    pdl_wait();
     const long row = a.rows ? a.rows[r] : r;
     float* xr = a.x + row * n * a.lds;
     float4 v[NS][VPT];
@@ -140,12 +172,12 @@ __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
             for (int t = 0; t < NS; t++) {
                 w[t] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (t >= n) continue;
-                const float o = a.out[t];
+                const float o = out[t];
                 w[t] = make_float4(o * y.x, o * y.y, o * y.z, o * y.w);
 #pragma unroll
                 for (int s = 0; s < NS; s++) {
                     if (s >= n) continue;
-                    const float k = a.mix[s * n + t];
+                    const float k = mix[s * n + t];
                     w[t].x = __fmaf_rn(k, v[s][i].x, w[t].x); w[t].y = __fmaf_rn(k, v[s][i].y, w[t].y);
                     w[t].z = __fmaf_rn(k, v[s][i].z, w[t].z); w[t].w = __fmaf_rn(k, v[s][i].w, w[t].w);
                 }
@@ -184,7 +216,7 @@ __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
 #pragma unroll
         for (int s = 0; s < NS; s++) {
             if (s >= n) continue;
-            const float k = a.in[s];
+            const float k = in[s];
             u[i].x = __fmaf_rn(k, v[s][i].x, u[i].x); u[i].y = __fmaf_rn(k, v[s][i].y, u[i].y);
             u[i].z = __fmaf_rn(k, v[s][i].z, u[i].z); u[i].w = __fmaf_rn(k, v[s][i].w, u[i].w);
         }
@@ -197,7 +229,7 @@ __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
     for (int i = 0; i < VPT; i++) {
         const int c = tid + i * NT;
         if (c < nv) {
-            const float4 g = load4(a.gain + 4 * c);
+            const float4 g = AHEAD ? gn[AHEAD ? i : 0] : load4(a.gain + 4 * c);
             store4(hr + 4 * c, make_float4((u[i].x * rinv) * g.x, (u[i].y * rinv) * g.y, (u[i].z * rinv) * g.z, (u[i].w * rinv) * g.w));
         }
     }
@@ -205,12 +237,15 @@ __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
 
 template <class T, int NS> int launch_hyper(const HyperNormArgs& a, int rows, cudaStream_t st) {
     const int nv = (a.D + 3) / 4;
-    if (nv <= 128) launch_k(hyper_norm_kernel<T, NS, 128, 1>, dim3(rows), dim3(128), 0, st, a);
-    else if (nv <= 256) launch_k(hyper_norm_kernel<T, NS, 256, 1>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 512) launch_k(hyper_norm_kernel<T, NS, 256, 2>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 1024) launch_k(hyper_norm_kernel<T, NS, 256, 4>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 4096) launch_k(hyper_norm_kernel<T, NS, 512, 8>, dim3(rows), dim3(512), 0, st, a);
+    const bool ahead = rows <= kAheadRows;
+#define FLEXLLM_HYPER(NT_, VPT_) launch_k(ahead ? hyper_norm_kernel<T, NS, NT_, VPT_, true> : hyper_norm_kernel<T, NS, NT_, VPT_, false>, dim3(rows), dim3(NT_), 0, st, a)
+    if (nv <= 128) FLEXLLM_HYPER(128, 1);
+    else if (nv <= 256) FLEXLLM_HYPER(256, 1);
+    else if (nv <= 512) FLEXLLM_HYPER(256, 2);
+    else if (nv <= 1024) FLEXLLM_HYPER(256, 4);
+    else if (nv <= 4096) launch_k(hyper_norm_kernel<T, NS, 512, 8, false>, dim3(rows), dim3(512), 0, st, a);
     else return FLEXLLM_ENOTSUP;
+#undef FLEXLLM_HYPER
     return launch_status();
 }
 
@@ -233,12 +268,15 @@ template <class T> int res_norm(const ResNormArgs& a, int rows, cudaStream_t st)
     FLEXLLM_REQUIRE(a.D > 0 && rows >= 0 && a.ldx % 4 == 0 && a.ldx >= up_to(a.D, 4));
     if (rows == 0) return FLEXLLM_OK;
     const int nv = (a.D + 3) / 4;
-    if (nv <= 128) launch_k(res_norm_kernel<T, 128, 1>, dim3(rows), dim3(128), 0, st, a);
-    else if (nv <= 256) launch_k(res_norm_kernel<T, 256, 1>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 512) launch_k(res_norm_kernel<T, 256, 2>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 1024) launch_k(res_norm_kernel<T, 256, 4>, dim3(rows), dim3(256), 0, st, a);
-    else if (nv <= 4096) launch_k(res_norm_kernel<T, 1024, 4>, dim3(rows), dim3(1024), 0, st, a);
+    const bool ahead = rows <= kAheadRows;
+#define FLEXLLM_RES(NT_, VPT_) launch_k(ahead ? res_norm_kernel<T, NT_, VPT_, true> : res_norm_kernel<T, NT_, VPT_, false>, dim3(rows), dim3(NT_), 0, st, a)
+    if (nv <= 128) FLEXLLM_RES(128, 1);
+    else if (nv <= 256) FLEXLLM_RES(256, 1);
+    else if (nv <= 512) FLEXLLM_RES(256, 2);
+    else if (nv <= 1024) FLEXLLM_RES(256, 4);
+    else if (nv <= 4096) launch_k(res_norm_kernel<T, 1024, 4, false>, dim3(rows), dim3(1024), 0, st, a);
     else return FLEXLLM_ENOTSUP;
+#undef FLEXLLM_RES
     return launch_status();
 }
 template int res_norm<float>(const ResNormArgs&, int, cudaStream_t);

@@ -62,12 +62,15 @@ template <> struct Vec8<float> {
     __device__ __forceinline__ void zero() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
     __device__ __forceinline__ void get(float (&f)[8]) const { f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w; }
 };
-template <class T, int TAPS>
+// AHEAD (one token): weights and the inputs of earlier calls are asked for before the kernel in front has finished (see res_norm_kernel; in prompts
+// the second set of loads costs more than it hides: 4000 rows 24.9 -> 43.8 us).
+template <class T, int TAPS, bool AHEAD>
 __global__ void __launch_bounds__(128) ssm_conv_kernel(const SsmCall k) {
     constexpr bool FAST = sizeof(T) == 2;
-    pdl_sync();
     const SsmShape& s = k.s;
     const int c = (blockIdx.x * 128 + threadIdx.x) * 8, t0 = blockIdx.y * kConvTokens, b = blockIdx.z;
+    pdl_launch();
+    if (!AHEAD) pdl_wait();
     if (c >= s.ch) return;
     const int p0 = first_pos(k, b), t1 = min(t0 + kConvTokens, k.Sc), taps = TAPS ? TAPS : s.taps;
     auto load = [&](int at, float (&f)[8]) {
@@ -89,10 +92,14 @@ __global__ void __launch_bounds__(128) ssm_conv_kernel(const SsmCall k) {
 #pragma unroll
         for (int j = 0; j < TAPS - 1 + kConvTokens; j++) {
             const int at = p0 + t0 - (TAPS - 1) + j;
-            if (at >= 0 && at < p0 + t1) in[j].load(conv_row<T>(k, b, p0, at) + c); else in[j].zero();
+            if (at >= 0 && at < (AHEAD ? p0 : p0 + t1)) in[j].load(conv_row<T>(k, b, p0, at) + c); else in[j].zero();
         }
 #pragma unroll
         for (int j = 0; j < TAPS; j++) load8(k.conv_w + (long)j * s.ch + c, w[j]);
+        if (AHEAD) {
+            pdl_wait();
+            in[TAPS - 1].load(conv_row<T>(k, b, p0, p0) + c);                  // the token's own
+        }
 #pragma unroll
         for (int t = 0; t < kConvTokens; t++) {
             if (t0 + t >= t1) break;
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const SsmCall k) {
     const int tid = threadIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (s.H / s.G);
     const int pb = blockIdx.x * 32, pr = tid >> 3, p = pb + pr, ns = tid & 7;
     const bool on = p < s.P;
-    pdl_sync();
+    pdl_launch();
     const int p0 = first_pos(k, b);
     float* st = k.state + (((long)b * s.H + h) * s.P + (on ? p : 0)) * s.Np;
     float4 S[NV];
@@ -149,6 +156,7 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const SsmCall k) {
     }
     const float A = k.A[h], Dh = k.D[h], dtb = k.dt_bias[h];
     const int xc = h * s.P8 + pb, bc = s.inner + g * s.N8, cc = bc + s.G * s.N8;       // first channels of x, B and C
+    pdl_wait();                                              // the state is this kernel's own: asked for before the kernel in front has finished
     for (int t0 = 0; t0 < k.Sc; t0 += TT) {
         const int nt = min(TT, k.Sc - t0);
         if (t0) __syncthreads();
@@ -198,13 +206,24 @@ __global__ void __launch_bounds__(256) ssm_scan_kernel(const SsmCall k) {
 // ---------------------------------------------------------------------------------------------------------------
 // RMS norm of a row in `parts` equal parts of its H * P true columns (a part may begin and end inside a head). One CTA per row;
 // a part's sum is formed by its own warps, or a warp takes several parts.
-template <class T>
+template <class T, bool AHEAD>
 __global__ void __launch_bounds__(256) ssm_norm_kernel(const SsmCall k) {
     extern __shared__ float rinv[];                          // [parts], then [8] partial sums
-    pdl_sync();
     const SsmShape& s = k.s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long row = blockIdx.x;
+    pdl_launch();
+    // AHEAD (decoding): the gains of the first 2 x 256 vectors before the kernel in front has finished (see res_norm_kernel)
+    float4 ga[2], gb[2];
+    if (AHEAD) {
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int i = tid + j * 256;
+            ga[j] = gb[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < s.inner >> 3) { ga[j] = load4(k.gain + 8 * i); gb[j] = load4(k.gain + 8 * i + 4); }
+        }
+    }
+    pdl_wait();
     const T* y = (const T*)k.y + row * s.inner;
     T* out = (T*)k.out + row * s.inner;
     const int len = s.H * s.P / s.parts;
@@ -251,7 +270,8 @@ __global__ void __launch_bounds__(256) ssm_norm_kernel(const SsmCall k) {
     for (int i = tid; i < s.inner >> 3; i += 256) {
         float f[8];
         load8(y + 8 * i, f);
-        const float4 a = load4(k.gain + 8 * i), b = load4(k.gain + 8 * i + 4);
+        const float4 a = AHEAD && i == tid ? ga[0] : AHEAD && i == tid + 256 ? ga[1] : load4(k.gain + 8 * i);
+        const float4 b = AHEAD && i == tid ? gb[0] : AHEAD && i == tid + 256 ? gb[1] : load4(k.gain + 8 * i + 4);
         const float gn[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
         if (vec) {
             const float r = rinv[8 * i / len];
@@ -562,11 +582,12 @@ template <> int run_chunks<bf16>(const SsmCall& c, cudaStream_t st) {
 
 template <class T> int run_conv(const SsmCall& c, cudaStream_t st) {
     const dim3 grid((c.s.ch + 1023) / 1024, (c.Sc + kConvTokens - 1) / kConvTokens, c.B);
+    const bool one = c.Sc == 1;
     switch (c.s.taps) {
-        case 2: launch_k(ssm_conv_kernel<T, 2>, grid, dim3(128), 0, st, c); break;
-        case 3: launch_k(ssm_conv_kernel<T, 3>, grid, dim3(128), 0, st, c); break;
-        case 4: launch_k(ssm_conv_kernel<T, 4>, grid, dim3(128), 0, st, c); break;
-        default: launch_k(ssm_conv_kernel<T, 0>, grid, dim3(128), 0, st, c);
+        case 2: launch_k(one ? ssm_conv_kernel<T, 2, true> : ssm_conv_kernel<T, 2, false>, grid, dim3(128), 0, st, c); break;
+        case 3: launch_k(one ? ssm_conv_kernel<T, 3, true> : ssm_conv_kernel<T, 3, false>, grid, dim3(128), 0, st, c); break;
+        case 4: launch_k(one ? ssm_conv_kernel<T, 4, true> : ssm_conv_kernel<T, 4, false>, grid, dim3(128), 0, st, c); break;
+        default: launch_k(ssm_conv_kernel<T, 0, false>, grid, dim3(128), 0, st, c);
     }
     return launch_status();
 }
@@ -593,7 +614,7 @@ template <class T> int ssm_mixer(const SsmCall& c, cudaStream_t st) {
     int rc = c.Sc == 1 ? run_scan<T, 1>(c, st) : run_chunks<T>(c, st);
     if (rc == FLEXLLM_ENOTSUP) rc = run_scan<T, kScanTile>(c, st);
     TRY_RC(rc);
-    launch_k(ssm_norm_kernel<T>, dim3(c.B * c.Sc), dim3(256), (size_t)(s.parts + 8) * 4, st, c);
+    launch_k(c.B * c.Sc <= 64 ? ssm_norm_kernel<T, true> : ssm_norm_kernel<T, false>, dim3(c.B * c.Sc), dim3(256), (size_t)(s.parts + 8) * 4, st, c);
     return launch_status();
 }
 template int ssm_mixer<float>(const SsmCall&, cudaStream_t);
