@@ -526,15 +526,18 @@ __device__ __forceinline__ void mma_s8u8(int (&d)[4], const int (&a)[4], const i
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Returns false when a bounded wait ran out (the same verdict for all NT threads).
-template <int NT>
+// G query heads of the group, hq0 .. hq0 + G - 1: all four, or one, with one caller per head (few items: the exponentials and the quantiser of a
+// head then have all threads. All callers write the new token into the cache, the
+// same bytes.) Returns false when a bounded wait ran out (the same verdict for all NT threads).
+template <int NT, int G>
 __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const float* __restrict__ cos_t,
                                                      const float* __restrict__ sin_t, const float* __restrict__ a_s,
                                                      const KvLayer& cache, const int32_t* __restrict__ page_table, int max_pages,
                                                      int HQ, int HKV, int cs, float* __restrict__ out, const int hkv, const int b,
                                                      const int pos, uint8_t* dsm, DecAttnSmem& sm, const DecAttnStage& st,
-                                                     const int tid, const int bar) {
-    constexpr int G = 4;
+                                                     const int tid, const int bar, const int hq0) {
+    constexpr bool ONE = G == 1;
+    static_assert(G == 1 || G == 4, "one head or the whole group");
     float* sc = reinterpret_cast<float*>(dsm);                       // [G][cs]
     uint8_t* u_sm = dsm + (size_t)G * cs * 4;                        // [G][cs]
     int8_t (*q_sm)[64] = sm.q_sm;
@@ -559,20 +562,20 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     }
     // split-K partial sums of this warp's head (independent of the context): loads first
     int a0 = 0, a1 = 0;
-    if (w < 6) {
-        const int h = w < 4 ? hkv * G + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
+    if (w < G || w == 4 || w == 5) {
+        const int h = w < 4 ? hq0 + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
         const int32_t* src = in.qkv_acc + (long)b * heads * 64 + (long)h * 64 + lane;
 #pragma unroll 1
-        for (int sl = 0; sl < in.n_slabs; sl += 4) {
-            int p0[4], p1[4];
+        for (int sl = 0; sl < in.n_slabs; sl += 8) {             // (six slabs at the sizes of the 1B model: one round trip)
+            int p0[8], p1[8];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
+            for (int i = 0; i < 8; i++) {
                 const bool on = sl + i < in.n_slabs;
                 p0[i] = on ? __ldcg(src + (sl + i) * in.slab_stride) : 0;
                 p1[i] = on ? __ldcg(src + (sl + i) * in.slab_stride + 32) : 0;
             }
-            a0 += (p0[0] + p0[1]) + (p0[2] + p0[3]);
-            a1 += (p1[0] + p1[1]) + (p1[2] + p1[3]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) { a0 += p0[i]; a1 += p1[i]; }
         }
     }
     for (int i = tid; i < npages; i += NT) pt_sm[i] = page_table[(long)b * max_pages + i];
@@ -591,10 +594,10 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     ATT_TS(1);
     // ---- A. prepare: warps 0..3 the query heads, warp 4 the key head, warp 5 the value head
     int8_t new_a = 0, new_b = 0; float new_s = 0.0f;                  // warps 4 / 5: the new token's quantised head, for the staging patch
-    if (w < 6) {
+    if (w < G || w == 4 || w == 5) {
         const long pg = page_table[(long)b * max_pages + pos / PAGE];
         const int slot = pos % PAGE;
-        const int h = w < 4 ? hkv * G + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
+        const int h = w < 4 ? hq0 + w : (w == 4 ? HQ + hkv : HQ + HKV + hkv);
         const float stk = __ldcg(in.tok_scale + b);
         const float x0 = ((float)a0 * stk) * in.ch_scale[h * 64 + lane];
         const float x1 = ((float)a1 * stk) * in.ch_scale[h * 64 + lane + 32];
@@ -664,7 +667,7 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         bq[ks][1] = gi < G ? *reinterpret_cast<const int*>(&q_sm[gi][ks * 32 + 16 + ti * 4]) : 0;
     }
     // lanes ti < 2 receive the sums of heads 2 ti and 2 ti + 1 for the keys gi and gi + 8 of the block
-    const float qs0 = q_scale[(2 * ti) & 3], qs1 = q_scale[(2 * ti + 1) & 3];
+    const float qs0 = q_scale[ONE ? 0 : (2 * ti) & 3], qs1 = q_scale[ONE ? 0 : (2 * ti + 1) & 3];
     float mx0 = -1e32f, mx1 = -1e32f;
     const int nblk = (nk + 15) >> 4;
     for (int blk = w; blk < nblk; blk += NT / 32) {
@@ -682,16 +685,16 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         const int kA = blk * 16 + gi, kB = kA + 8;
         const float ksA = sc[kA < nk ? kA : nk - 1], ksB = sc[kB < nk ? kB : nk - 1];
         __syncwarp();                            // every lane has read its keys' scales before row 0 is overwritten below
-        if (ti < 2) {
+        if (ti < (ONE ? 1 : 2)) {
             const int h0 = 2 * ti, h1 = h0 + 1;
             if (kA < nk) {
                 const float x0 = (((float)d[0] * qs0) * ksA) * 0.125f, x1 = (((float)d[1] * qs1) * ksA) * 0.125f;
-                sc[h0 * cs + kA] = x0; sc[h1 * cs + kA] = x1;
+                sc[h0 * cs + kA] = x0; if (!ONE) sc[h1 * cs + kA] = x1;
                 mx0 = x0 > mx0 ? x0 : mx0; mx1 = x1 > mx1 ? x1 : mx1;
             }
             if (kB < nk) {
                 const float x0 = (((float)d[2] * qs0) * ksB) * 0.125f, x1 = (((float)d[3] * qs1) * ksB) * 0.125f;
-                sc[h0 * cs + kB] = x0; sc[h1 * cs + kB] = x1;
+                sc[h0 * cs + kB] = x0; if (!ONE) sc[h1 * cs + kB] = x1;
                 mx0 = x0 > mx0 ? x0 : mx0; mx1 = x1 > mx1 ? x1 : mx1;
             }
         }
@@ -703,7 +706,7 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
     }
-    if (lane < 2) { red[2 * lane][w] = mx0; red[2 * lane + 1][w] = mx1; }
+    if (lane < (ONE ? 1 : 2)) { red[2 * lane][w] = mx0; if (!ONE) red[2 * lane + 1][w] = mx1; }
     tc::fence_proxy_async_smem();               // this thread's reads / writes of the staging area, before the V copies overwrite it
     named_sync_id<NT>(bar);
     // warp 7: the V^T pages into the staging area
@@ -732,7 +735,15 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
     // ---- D. e = exp(x - max), in place: the four heads of a key together (four independent evaluations in flight)
     //         (The warp-wide form was slower here, on a peaked softmax, where most values take the scalar form's early exit: 1.303
     //         instead of 1.276 ms a step of 32 sequences, and on a spread one: 114.8 instead of 113.6 ms for 32 x (256 + 96) tokens.)
-    {
+    if constexpr (ONE) {
+        const float m0 = row_max[0];
+        for (int key = tid; key < nk; key += 2 * NT) {                  // two evaluations in flight
+            const bool two = key + NT < nk;
+            const float e0 = ref_expf(sc[key] - m0), e1 = ref_expf(two ? sc[key + NT] - m0 : -200.0f);
+            sc[key] = e0;
+            if (two) sc[key + NT] = e1;
+        }
+    } else {
         const float m0 = row_max[0], m1 = row_max[1], m2 = row_max[2], m3 = row_max[3];
         for (int key = tid; key < nk; key += NT) {
             const float x0 = sc[key] - m0, x1 = sc[cs + key] - m1, x2 = sc[2 * cs + key] - m2, x3 = sc[3 * cs + key] - m3;
@@ -776,7 +787,7 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         bool ok_g[G];
 #pragma unroll
         for (int g = 0; g < G; g++) {
-            rinv_g[g] = row_rinv[g]; as_g[g] = a_s[hkv * G + g];
+            rinv_g[g] = row_rinv[g]; as_g[g] = a_s[hq0 + g];
             c_g[g] = dec_u8_factor(rinv_g[g], as_g[g], ok_g[g]);
         }
 #pragma unroll
@@ -814,7 +825,7 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         int d[4] = {0, 0, 0, 0};
         for (int p = pset; p < npages; p += NPS) {
             const uint8_t* rows = st.kv + (size_t)p * 4096 + (size_t)(dblk * 16 + gi) * PAGE + ti * 4;
-            const uint8_t* ucol = u_sm + (gi & 3) * cs + p * PAGE + ti * 4;
+            const uint8_t* ucol = u_sm + (ONE ? 0 : gi & 3) * cs + p * PAGE + ti * 4;
 #pragma unroll
             for (int ks = 0; ks < 2; ks++) {
                 int af[4], bu[2];
@@ -832,20 +843,21 @@ __device__ __forceinline__ bool dec_attn_staged_body(const DecAttnIn& in, const 
         // 3 KB of the item's scratch, which holds at least 4 KB)
         int* pv_sm = reinterpret_cast<int*>(dsm);
         named_sync_id<NT>(bar);
-        if (pset > 0 && ti < 2) {
+        if (pset > 0 && ti < (ONE ? 1 : 2)) {
             int* dst = pv_sm + (pset - 1) * (G * 64);
-            dst[(2 * ti) * 64 + dblk * 16 + gi] = d[0]; dst[(2 * ti + 1) * 64 + dblk * 16 + gi] = d[1];
-            dst[(2 * ti) * 64 + dblk * 16 + gi + 8] = d[2]; dst[(2 * ti + 1) * 64 + dblk * 16 + gi + 8] = d[3];
+            dst[(2 * ti) * 64 + dblk * 16 + gi] = d[0];
+            dst[(2 * ti) * 64 + dblk * 16 + gi + 8] = d[2];
+            if (!ONE) { dst[(2 * ti + 1) * 64 + dblk * 16 + gi] = d[1]; dst[(2 * ti + 1) * 64 + dblk * 16 + gi + 8] = d[3]; }
         }
         named_sync_id<NT>(bar);
-        if (pset == 0 && ti < 2) {
+        if (pset == 0 && ti < (ONE ? 1 : 2)) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
+            for (int i = 0; i < 4; i += ONE ? 2 : 1) {
                 const int hd = 2 * ti + (i & 1), dim = dblk * 16 + gi + (i >> 1) * 8;
                 int tot = d[i];
 #pragma unroll
                 for (int ps = 0; ps < NPS - 1; ps++) tot += pv_sm[ps * (G * 64) + hd * 64 + dim];
-                const int hq = hkv * G + hd;
+                const int hq = hq0 + hd;
                 out[((long)b * HQ + hq) * 64 + dim] = (float)tot * a_s[hq];
             }
         }

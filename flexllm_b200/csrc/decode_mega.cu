@@ -276,12 +276,12 @@ __device__ __forceinline__ void mega_row_norm(const MegaArgs& a, int row, const 
 // Attention output row b -> int8 (Modules/quant.h:349-430), by the 256 threads of the half whose item arrived
 // last on the sequence's counter. Arrival: acq_rel atomic by one thread after the half's barrier (orders the
 // half's stores before it; the last arriver sees every other item's stores after it).
-__device__ __forceinline__ void mega_att_row_quant(const MegaArgs& a, int b, DecAttnSmem& sm, int t, int bar) {
+__device__ __forceinline__ void mega_att_row_quant(const MegaArgs& a, int b, DecAttnSmem& sm, int t, int bar, int items) {      // items of a sequence
     named_sync_id<256>(bar);
     if (t == 0) {
         int old;
         asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(a.att_cnt + b), "r"(1) : "memory");
-        sm.last = old == a.HKV - 1;
+        sm.last = old == items - 1;
         if (sm.last) a.att_cnt[b] = 0;          // next use: the next layer's attention phase, grid barriers away
     }
     named_sync_id<256>(bar);
@@ -525,6 +525,16 @@ __device__ __noinline__ void mega_row_sample(const MegaArgs& a, int row, int col
     }
 }
 
+// Asks L2 for a layer's scales and gains (108 KB at the sizes of the 1B model): thread `t` of `n`. In the phases that use them they would each
+// be a round trip to memory on the critical path.
+__device__ __forceinline__ void mega_prefetch_params(const MegaArgs& a, const MegaLayer& L, int t, int n) {
+    auto ask = [&](const float* p, int floats) {
+        for (int i = t * 32; i < floats; i += n * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+    };
+    ask(L.sqkv, (a.HQ + 2 * a.HKV) * 64); ask(L.so, a.D); ask(L.sgu, 2 * a.F); ask(L.sd, a.D);
+    ask(L.g0, a.D); ask(L.g1, a.D); ask(L.a_s, a.HQ);
+}
+
 // ---- the kernel -----------------------------------------------------------------------------------
 // ATT selects which attention bodies are compiled in. The whole kernel is several hundred KB of instructions and a
 // latency-bound step pays for every instruction-cache miss, so the host launches the leanest variant that covers the
@@ -532,6 +542,8 @@ __device__ __noinline__ void mega_row_sample(const MegaArgs& a, int row, int col
 //   0  every body: both item layouts, the staged copies and the per-thread-load body for contexts beyond the staging area
 //   1  two items per CTA, staged copies only (more items than CTAs, every context fits half of the operand ring)
 //   2  one item per CTA on all 512 threads, staged copies only (no more items than CTAs, every context fits the ring)
+//   3  one query head of an item per CTA, likewise (four times the items are no more than the CTAs): the pages are read by four CTAs, but the
+//      exponentials, the quantiser and the outputs of a head have all threads
 // A variant that meets a context it was not built for raises the device-data error bit and skips the item.
 template <int BN, int ATT>
 __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid_constant__ MegaArgs a) {
@@ -751,7 +763,8 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                 // idle CTAs of the FHT phase, or from all CTAs at its start -- the page-table look-ups are a chain of
                 // latencies that then sits on that phase's critical path.)
                 const MegaLayer& nx = a.layers[p == 0 ? 0 : l + 1];
-                if (ATT == 2 || (ATT == 0 && a.B * a.HKV <= G)) {
+                mega_prefetch_params(a, nx, (cta - a.B) * MG_WORKERS + tid, (G - a.B) * MG_WORKERS);
+                if (ATT >= 2 || (ATT == 0 && a.B * a.HKV <= G)) {
                     // few items (at most one per CTA): groups of 128 threads with one dependent load per thread
                     // (measured: 1.5 % off the step at 16 sequences; at 32 sequences the plain form below was 0.7 % faster)
                     const int grp = tid >> 7, stride = G - a.B;
@@ -782,11 +795,12 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
             stg.cap_pages = half_bytes / 4096 < 20 ? half_bytes / 4096 : 20;
             stg.abort_flag = abort_flag;
             if (is_tma) prefetch_weights_l2(mega_job(a, l, 1));
-            if (ATT != 1 && (ATT == 2 || a.B * a.HKV <= G)) {
+            if (ATT != 1 && (ATT >= 2 || a.B * a.HKV <= G)) {
                 // no more items than CTAs: one item per CTA, worked on by all 512 threads (an item is a chain of dependent
                 // stages; twice the threads shorten the stages that scale -- scores, exponentials, quantiser, P.V)
-                if (cta < a.B * a.HKV) {
-                    const int b = cta / a.HKV;
+                constexpr int PER = ATT == 3 ? 4 : 1;            // CTAs of an item
+                if (cta < a.B * a.HKV * PER) {
+                    const int item = cta / PER, b = item / a.HKV, hkv = item % a.HKV, part = cta % PER;
                     const int pos = dec_guarded_pos(a.ctx, b, a.max_ctx, a.error_flag);
                     uint8_t* dsm1 = scratch;
                     DecAttnSmem& sm1 = *reinterpret_cast<DecAttnSmem*>(dsm1 + a.attn_bytes - sizeof(DecAttnSmem));
@@ -799,20 +813,20 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                     if (pos / PAGE + 1 <= st1.cap_pages) {
                         st1.parity = att_uses & 1u;
                         att_uses++;
-                        ok1 = dec_attn_staged_body<512>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.HQ, a.HKV, a.cs, a.att,
-                                                        cta % a.HKV, b, pos, dsm1, sm1, st1, tid, MG_BAR_WORK);
+                        ok1 = dec_attn_staged_body<512, 4 / PER>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.HQ, a.HKV, a.cs, a.att,
+                                                                 hkv, b, pos, dsm1, sm1, st1, tid, MG_BAR_WORK, hkv * 4 + part);
                     } else if (ATT == 0) {
                         dec_attn_fused_body<2, 512>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.ctx, a.HQ, a.HKV, a.cs,
-                                                    a.att, nullptr, cta % a.HKV, b, dsm1, sm1, tid, MG_BAR_WORK);
+                                                    a.att, nullptr, hkv, b, dsm1, sm1, tid, MG_BAR_WORK);
                     } else if (tid == 0) {
                         atomicOr(a.error_flag, 2);
                     }
                     if (ok1) {
                         named_sync<MG_BAR_WORK, MG_WORKERS>();
-                        if (tid < 256) mega_att_row_quant(a, b, sm1, tid, MG_BAR_HALF0);
+                        if (tid < 256) mega_att_row_quant(a, b, sm1, tid, MG_BAR_HALF0, a.HKV * PER);
                     }
                 }
-            } else if (ATT != 2) {
+            } else if (ATT < 2) {
                 // items spread over the CTAs first (item i on CTA i mod G)
                 for (int idx = cta + half * G; idx < a.B * a.HKV; idx += 2 * G) {
                     const int b = idx / a.HKV;
@@ -820,8 +834,8 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                     if (pos / PAGE + 1 <= stg.cap_pages) {
                         stg.parity = att_uses & 1u;
                         att_uses++;
-                        if (!dec_attn_staged_body<256>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.HQ, a.HKV, a.cs, a.att,
-                                                       idx % a.HKV, b, pos, dsm, sm, stg, tid & 255, MG_BAR_HALF0 + half))
+                        if (!dec_attn_staged_body<256, 4>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.HQ, a.HKV, a.cs, a.att,
+                                                          idx % a.HKV, b, pos, dsm, sm, stg, tid & 255, MG_BAR_HALF0 + half, idx % a.HKV * 4))
                             break;
                     } else if (ATT == 0) {     // contexts beyond the staging area: per-thread global loads
                         dec_attn_fused_body<2, 256>(in, a.cos_t, a.sin_t, ly.a_s, ly.kv, a.page_table, a.max_pages, a.ctx, a.HQ, a.HKV, a.cs,
@@ -831,7 +845,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) decode_mega_kernel(const __grid
                     }
                     // the item that completes its sequence's attention row (the last of its HKV items to arrive)
                     // quantises the row for the o projection -- no separate phase, no extra grid barrier
-                    mega_att_row_quant(a, b, sm, tid & 255, MG_BAR_HALF0 + half);
+                    mega_att_row_quant(a, b, sm, tid & 255, MG_BAR_HALF0 + half, a.HKV);
                 }
             }
             // both halves are done with the ring (each thread has fenced its accesses): the o projection's weights may come in
@@ -931,9 +945,9 @@ int mega_create(const MegaModelView& v, MegaPlan** out) {
     if (v.max_batch > G) return FLEXLLM_ENOTSUP;
     const int bn = v.max_batch <= 32 ? 32 : 64;
     if (bn == 32 && G < 4 * 32) return FLEXLLM_ENOTSUP;     // the 32-sequence kernel always splits an FFN row over four CTAs
-    const void* kerns[3];
-    if (bn == 32) { kerns[0] = (const void*)decode_mega_kernel<32, 0>; kerns[1] = (const void*)decode_mega_kernel<32, 1>; kerns[2] = (const void*)decode_mega_kernel<32, 2>; }
-    else { kerns[0] = (const void*)decode_mega_kernel<64, 0>; kerns[1] = (const void*)decode_mega_kernel<64, 1>; kerns[2] = (const void*)decode_mega_kernel<64, 2>; }
+    const void* kerns[4];
+    if (bn == 32) { kerns[0] = (const void*)decode_mega_kernel<32, 0>; kerns[1] = (const void*)decode_mega_kernel<32, 1>; kerns[2] = (const void*)decode_mega_kernel<32, 2>; kerns[3] = (const void*)decode_mega_kernel<32, 3>; }
+    else { kerns[0] = (const void*)decode_mega_kernel<64, 0>; kerns[1] = (const void*)decode_mega_kernel<64, 1>; kerns[2] = (const void*)decode_mega_kernel<64, 2>; kerns[3] = (const void*)decode_mega_kernel<64, 3>; }
     const void* kern = kerns[0];
     cudaFuncAttributes fa;
     FLEXLLM_CHECK_CUDA(cudaFuncGetAttributes(&fa, kern));
@@ -949,7 +963,7 @@ int mega_create(const MegaModelView& v, MegaPlan** out) {
     if (stages > MG_MAX_STAGES) stages = MG_MAX_STAGES;
     if (stages < 3) return FLEXLLM_ENOTSUP;      // long contexts: the per-operator kernels take over
     const size_t smem = 1024 + (size_t)stages * stage_bytes + scratch + 256;
-    for (int i = 0; i < 3; i++) {
+    for (int i = 0; i < 4; i++) {
         FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kerns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         FLEXLLM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], MG_THREADS, smem));
@@ -1052,13 +1066,13 @@ static std::atomic<int> g_hook_barrier_extra{0};
 // The leanest kernel variant that covers a launch of B sequences whose positions stay <= max_pos.
 int mega_variant(const MegaPlan* p, int B, int max_pos) {
     const int pages = max_pos / PAGE + 1;
-    if (B * p->args.HKV <= p->grid) return pages <= p->cap_single ? 2 : 0;
+    if (B * p->args.HKV <= p->grid) return pages > p->cap_single ? 0 : 4 * B * p->args.HKV <= p->grid ? 3 : 2;
     return pages <= p->cap_pair ? 1 : 0;
 }
 
 int mega_launch(MegaPlan* p, int B, int variant, cudaStream_t st) {
-    if (B < 1 || B > p->bn || variant < 0 || variant > 2) return FLEXLLM_EINVAL;
-    if (variant == 2 && B * p->args.HKV > p->grid) return FLEXLLM_EINVAL;
+    if (B < 1 || B > p->bn || variant < 0 || variant > 3) return FLEXLLM_EINVAL;
+    if (variant >= 2 && B * p->args.HKV * (variant == 3 ? 4 : 1) > p->grid) return FLEXLLM_EINVAL;
     if (variant == 1 && B * p->args.HKV <= p->grid) return FLEXLLM_EINVAL;
     p->args.B = B;
     const long long lim = g_hook_wait_limit_ns.load();
@@ -1073,11 +1087,13 @@ int mega_launch(MegaPlan* p, int B, int variant, cudaStream_t st) {
     if (p->bn == 32) {
         if (variant == 0) cudaLaunchKernelEx(&cfg, decode_mega_kernel<32, 0>, p->args);
         else if (variant == 1) cudaLaunchKernelEx(&cfg, decode_mega_kernel<32, 1>, p->args);
-        else cudaLaunchKernelEx(&cfg, decode_mega_kernel<32, 2>, p->args);
+        else if (variant == 2) cudaLaunchKernelEx(&cfg, decode_mega_kernel<32, 2>, p->args);
+        else cudaLaunchKernelEx(&cfg, decode_mega_kernel<32, 3>, p->args);
     } else {
         if (variant == 0) cudaLaunchKernelEx(&cfg, decode_mega_kernel<64, 0>, p->args);
         else if (variant == 1) cudaLaunchKernelEx(&cfg, decode_mega_kernel<64, 1>, p->args);
-        else cudaLaunchKernelEx(&cfg, decode_mega_kernel<64, 2>, p->args);
+        else if (variant == 2) cudaLaunchKernelEx(&cfg, decode_mega_kernel<64, 2>, p->args);
+        else cudaLaunchKernelEx(&cfg, decode_mega_kernel<64, 3>, p->args);
     }
     return launch_status();
 }
