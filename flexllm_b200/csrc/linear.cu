@@ -40,7 +40,12 @@ static int linear_decode(const int8_t* a, const float* s_tok, const int8_t* w, c
     if (M == 0) return FLEXLLM_OK;
     if (M > 64) return FLEXLLM_ENOTSUP;
     cudaStream_t st = (cudaStream_t)stream;
-    if (M <= 8) return gemv_i8(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
+    // Up to eight tokens: the GEMV, whose dot products bind it from three tokens on, or the tensor-core form, which costs a few microseconds whatever
+    // the tokens (us, GEMV / tensor cores: 3072x2048 4.2 / 6.9 for 3 tokens, 5.5 / 7.0 for 8; 4096x4096 8.9 / 8.9, 9.6 / 8.9; 16384x2048 10.6 / 10.9,
+    // 14.7 / 11.0; 2048x8192 10.4 / 10.3, 13.5 / 10.4; 128256x2048 50 / 46, 81 / 47; 2 tokens 44.6 / 45.8 there). Behind other kernels of a chain
+    // it has its weights early: MLP block of 3 tokens 22.4 / 17.9, of 8 32.4 / 18.7, of 2 17.5 / 17.9.
+    const bool large = (long)N * K >= 12L << 20;
+    if (M <= (large ? (g_pdl ? 2 : 3) : 8)) return gemv_i8(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
     return gemm_i8_decode(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
 }
 

@@ -386,6 +386,20 @@ def test_linear_decode_tcgen05(F, M, N, K):
     assert_same(to_np(y2), y_o, "y (scratch)")
 
 
+@pytest.mark.parametrize("M", [2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("N,K", [(6136, 2048), (6144, 2048), (2048, 8192), (6000, 2800)])
+def test_linear_decode_few_tokens_of_large_matrices(F, M, N, K):
+    """Both sides of the line between the GEMV and the tensor-core form, with and without K split over a cluster, accumulators and residual."""
+    a, st, w, sc = lin_inputs(M, N, K, 25)
+    acc_o, y_o = oracle.linear_i8(a, st, w, sc)
+    t = [dev(x) for x in (a, st, w, sc)]
+    acc, y = F.dec_Linear_Layer_i8xi8(*t, want_acc=True)
+    assert_same(to_np(acc), acc_o, "acc"); assert_same(to_np(y), y_o, "y")
+    res = np.random.default_rng(M).standard_normal((M, N)).astype(np.float32)
+    _, out = F.dec_Linear_Layer_i8xi8(*t, residual=dev(res))
+    assert_same(to_np(out), oracle.residual(res, y_o), "residual")
+
+
 def test_linear_decode_streams_at_once(F):
     """The layer keeps nothing between calls: launches that overlap on several streams do not touch one another's sums."""
     M, N, K = 40, 2048, 8192
