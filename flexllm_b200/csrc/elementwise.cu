@@ -4,6 +4,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace flexllm {
 
@@ -397,50 +398,71 @@ __global__ void softmax_kernel(const float* __restrict__ x, long rows, int len, 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Greedy argmax, ties to the lowest index (Logits.h:13-17 strict '>'). One CTA per row.
+// Greedy argmax, ties to the lowest index (Logits.h:13-17 strict '>'). One CTA of 1024 threads per row, or, few long rows, a cluster of eight
+// CTAs with an eighth of the row each: one SM takes 12 us for a row of 128256 (it reads 43 GB/s), which a decode step waits for; eight take 4.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ logits, long V, int32_t* __restrict__ idx) {
+constexpr int ARGMAX_CL = 8;
+template <int CL, int NT>
+__global__ void __launch_bounds__(NT) argmax_kernel(const float* __restrict__ logits, long V, int32_t* __restrict__ idx) {
     __shared__ float sv[32];
     __shared__ int si[32];
+    __shared__ float cv[CL];
+    __shared__ int ci[CL];
+    if (CL > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // the first CTA's slots may be written once all have started
     pdl_sync();
-    const float* l = logits + (long)blockIdx.x * V;
+    const int part = blockIdx.x % CL;
+    const long row = blockIdx.x / CL, v1 = V * (part + 1) / CL;
+    const float* l = logits + row * V;
     float best = -INFINITY;
     int bi = 0x7fffffff;
     // strided scan in increasing v; eight loads in flight
-    long v = threadIdx.x;
-    for (; v + 7L * blockDim.x < V; v += 8L * blockDim.x) {
+    long v = V * part / CL + threadIdx.x;
+    for (; v + 7L * NT < v1; v += 8L * NT) {
         float t[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) t[i] = l[v + (long)i * blockDim.x];
+        for (int i = 0; i < 8; i++) t[i] = l[v + (long)i * NT];
 #pragma unroll
         for (int i = 0; i < 8; i++)
-            if (t[i] > best || bi == 0x7fffffff) { best = t[i]; bi = (int)(v + (long)i * blockDim.x); }
+            if (t[i] > best || bi == 0x7fffffff) { best = t[i]; bi = (int)(v + (long)i * NT); }
     }
-    for (; v < V; v += blockDim.x) {
+    for (; v < v1; v += NT) {
         const float t = l[v];
         if (t > best || bi == 0x7fffffff) { best = t; bi = (int)v; }
     }
     auto better = [](float a, int ai, float b, int bi2) { return a > b || (a == b && ai < bi2); };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-    }
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { sv[w] = best; si[w] = bi; }
-    __syncthreads();
-    if (w == 0) {
-        const int nw = blockDim.x >> 5;
-        best = lane < nw ? sv[lane] : -INFINITY;
-        bi = lane < nw ? si[lane] : 0x7fffffff;
+    auto warp_best = [&]() {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             float ob = __shfl_xor_sync(0xffffffffu, best, o);
             int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
         }
-        if (lane == 0) idx[blockIdx.x] = bi;
+    };
+    warp_best();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (CL > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    if (lane == 0) { sv[w] = best; si[w] = bi; }
+    __syncthreads();
+    if (w == 0) {
+        best = lane < NT / 32 ? sv[lane] : -INFINITY;
+        bi = lane < NT / 32 ? si[lane] : 0x7fffffff;
+        warp_best();
+        if (CL == 1) {
+            if (lane == 0) idx[row] = bi;
+        } else if (lane == 0) {
+            const uint32_t av = tc::cluster_addr(tc::smem_u32(cv + part), 0), ai = tc::cluster_addr(tc::smem_u32(ci + part), 0);
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(av), "f"(best) : "memory");
+            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ai), "r"(bi) : "memory");
+        }
+    }
+    if (CL > 1) {
+        tc::cluster_sync();
+        if (part == 0 && w == 0) {
+            best = lane < CL ? cv[lane % CL] : -INFINITY;
+            bi = lane < CL ? ci[lane % CL] : 0x7fffffff;
+            warp_best();
+            if (lane == 0) idx[row] = bi;
+        }
     }
 }
 
@@ -637,6 +659,10 @@ extern "C" int flexllm_softmax(const float* x, long rows, int len, const int32_t
 extern "C" int flexllm_logits_argmax(const float* logits, int B, long V, int32_t* idx, void* stream) {
     FLEXLLM_REQUIRE(logits && idx && B >= 0 && V > 0);
     if (B == 0) return FLEXLLM_OK;
-    launch_k(argmax_kernel, dim3(B), dim3(1024), 0, (cudaStream_t)stream, logits, V, idx);
+    // clusters while all of them run at once, and where an eighth is more than a few loads a thread
+    if (B <= 64 && V >= 8192)
+        launch_cluster(argmax_kernel<ARGMAX_CL, 256>, dim3(B * ARGMAX_CL), dim3(256), ARGMAX_CL, 0, (cudaStream_t)stream, logits, V, idx);
+    else
+        launch_k(argmax_kernel<1, 1024>, dim3(B), dim3(1024), 0, (cudaStream_t)stream, logits, V, idx);
     return launch_status();
 }

@@ -319,6 +319,19 @@ def test_argmax(F):
     assert idx[1] == 77 and idx[2] == 0 and idx[3] == 128255
 
 
+@pytest.mark.parametrize("B,V", [(1, 8191), (1, 8192), (3, 8197), (64, 9000), (65, 9000), (4, 128256)])
+def test_argmax_long_rows(F, B, V):
+    """Rows of one CTA and rows of a cluster: ties across and inside the eighths, the largest value first and last, rows of -inf alone."""
+    l = rng(16).standard_normal((B, V)).astype(np.float32)
+    for b in range(B):
+        at = [(b * 977) % V, V - 1 - (b * 31) % 50, V // 8 * (b % 8)]
+        l[b, at[: 1 + b % 3]] = 9.0
+    l[0, [0, V - 1]] = 9.0
+    l[B // 2] = -np.inf
+    assert_same(to_np(F.dec_Logits_argmax(dev(l))), oracle.argmax(l))
+
+
+
 # ------------------------------------------------------------------------------ linear layers
 def lin_inputs(M, N, K, seed):
     g = rng(seed)
