@@ -11,6 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libflexllm_b200.so")
+FRONT_END = os.path.join(HERE, "_front_end.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -90,9 +91,30 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_front_end(force=False):
+    """The Python extension of csrc/front_end.cpp (host code against torch's headers)."""
+    src = os.path.join(CSRC, "front_end.cpp")
+    header = os.path.join(HERE, "..", "include", "flexllm_b200.h")
+    if not force and os.path.exists(FRONT_END) and os.path.getmtime(FRONT_END) > max(os.path.getmtime(src), os.path.getmtime(header)):
+        return FRONT_END
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")), "..", "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(root, "include"),
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I", cuda, src, "-o", FRONT_END,
+           "-L", os.path.join(root, "lib"), "-lc10", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed on front_end.cpp:\n" + r.stdout + r.stderr)
+    return FRONT_END
+
+
 def build(force=False, verbose=False, ptxas_info=False):
     if not os.path.exists(os.path.join(CSRC, "exp_constants.inc")):
         gen_exp_constants()
+    build_front_end(force)
     if not force and not needs_build():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -5,6 +5,7 @@ token-parallel (prefill) operators, ``dec_*`` for the single-token (decode) ones
 takes CUDA tensors, allocates its outputs with torch, and launches on the current torch stream.
 """
 import ctypes as C
+import importlib
 
 import torch
 
@@ -29,10 +30,39 @@ def _call(name, *args):
     _check(name, getattr(lib(), name)(*args, _stream()))
 
 
+# The extension that runs the plain form of the smallest calls without the interpreter's share (csrc/front_end.cpp): it returns the output, a
+# status, or None for arguments that the general path below has to look at.
+_front = None
+
+
+def _bind_front_end():
+    global _front
+    if _front is None:
+        try:
+            m = importlib.import_module("._front_end", __package__)
+        except ImportError:             # not built for this interpreter: the general path does the same
+            _front = False
+        else:
+            m.bind(*(C.cast(getattr(lib(), f), C.c_void_p).value for f in (
+                "flexllm_linear_prefill_i8", "flexllm_linear_decode_i8", "flexllm_mlp_block_workspace", "flexllm_mlp_block_decode")))
+            _front = m
+    return _front
+
+
+def _out(name, r):
+    if type(r) is int:
+        _check(name, r)
+    return r
+
+
 # ------------------------------------------------------------------------------ linear layers
 def pref_Linear_Layer_i8xi8(a, s_tok, w, s_ch, want_acc=False, want_y=True, residual=None):
     """Prefill W8A8 linear layer. a [M,K] int8, w [N,K] int8. Returns (acc int32 | None, y fp32 | None).
     With residual [M,N] the following Residual_Layer is fused: y = residual + dequant."""
+    if want_y and not want_acc and residual is None and (_front or _bind_front_end()):
+        y = _front.linear(False, a, s_tok, w, s_ch)
+        if y is not None:
+            return None, _out("flexllm_linear_prefill_i8", y)
     M, K = a.shape; N = w.shape[0]
     if residual is not None:
         y = torch.empty((M, N), dtype=torch.float32, device=a.device)
@@ -46,6 +76,10 @@ def pref_Linear_Layer_i8xi8(a, s_tok, w, s_ch, want_acc=False, want_y=True, resi
 
 def dec_Linear_Layer_i8xi8(a, s_tok, w, s_ch, want_acc=False, want_y=True, residual=None):
     """Decode W8A8 linear layer, M <= 64 tokens (optionally fused with the residual add)."""
+    if want_y and not want_acc and residual is None and (_front or _bind_front_end()):
+        y = _front.linear(True, a, s_tok, w, s_ch)
+        if y is not None:
+            return None, _out("flexllm_linear_decode_i8", y)
     M, K = a.shape; N = w.shape[0]
     if residual is not None:
         y = torch.empty((M, N), dtype=torch.float32, device=a.device)
@@ -354,6 +388,10 @@ def MHA_i8xi8_Prefilling(q, qs, k, ks, v, vs, cos_t, sin_t, a_s, want_oacc=False
 def dec_MLP_block(x, gamma, w_gu, s_gu, w_d, s_d, eps=1e-5, order=8, fht_scale=90.50966799, out=None, workspace=None):
     """Decode MLP block in one call: RMSNorm + quant -> gate|up -> SiLU * up -> FHT-8192 -> quant -> down + residual.
     x [M,D] fp32; w_gu [2F,D] int8 (gate rows, then up rows); w_d [D,F]. Returns y [M,D] fp32."""
+    if out is None and workspace is None and (_front or _bind_front_end()):
+        y = _front.mlp_block(x, gamma, w_gu, s_gu, w_d, s_d, eps, order, fht_scale)
+        if y is not None:
+            return _out("flexllm_mlp_block_decode", y)
     M, D = x.shape
     Fd = w_d.shape[1]
     nbytes = lib().flexllm_mlp_block_workspace(M, D, Fd)

@@ -545,3 +545,38 @@ def test_asymmetric_4bit_linear(F, M, N, K, decode):
     acco = oracle.gemm_s8s8(qo.astype(np.int8), w)
     assert_same(to_np(acc), acco, "integer sums")
     assert_same(to_np(y), oracle.dequant_asym(acco, so, bo, sc, wsum), "dequantised output")
+
+
+def test_front_end_general_path(F, monkeypatch):
+    """The extension's calls against the general path's: the same outputs, the same refusals, and whatever it does not take goes there."""
+    from flexllm_b200 import ops
+    assert ops._bind_front_end(), "the extension is built beside the library"
+    a, st, w, sc = [dev(x) for x in lin_inputs(5, 256, 512, 30)]
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(3, 2048, device="cuda", generator=g)
+    s8 = lambda *n: torch.randint(-127, 128, n, dtype=torch.int8, device="cuda", generator=g)
+    u = lambda *n: torch.rand(n, device="cuda", generator=g) * 1e-2
+    mlp = (x, 1 + u(2048), s8(16384, 2048), u(16384), s8(2048, 8192), u(2048))
+
+    def results():
+        out = [F.dec_Linear_Layer_i8xi8(a, st, w, sc)[1], F.pref_Linear_Layer_i8xi8(a, st, w, sc)[1], F.dec_MLP_block(*mlp),
+               F.dec_MLP_block(*mlp, eps=1e-3),
+               F.dec_Linear_Layer_i8xi8(a, st.view(5, 1), w, sc.view(-1, 1))[1]]                          # shapes that only the general path takes
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            out.append(F.dec_Linear_Layer_i8xi8(a, st, w, sc)[1])
+        side.synchronize()
+        for bad in (lambda: F.dec_Linear_Layer_i8xi8(a.cpu(), st, w, sc), lambda: F.dec_Linear_Layer_i8xi8(a[:0], st[:0], w, sc), lambda: F.pref_Linear_Layer_i8xi8(a, st, w.t(), sc),
+                    lambda: F.dec_MLP_block(x.t(), *mlp[1:]), lambda: F.dec_Linear_Layer_i8xi8(a[:, :504].contiguous(), st, w, sc),
+                    lambda: F.dec_MLP_block(x, mlp[1], mlp[2], mlp[3], s8(2048, 4096), mlp[5])):
+            with pytest.raises((AssertionError, ops.FlexLLMError)) as e:
+                bad()
+            out.append(e.type)
+        return out
+    with_it = results()
+    monkeypatch.setattr(ops, "_front", False)
+    monkeypatch.setattr(ops, "_bind_front_end", lambda: False)
+    for p, q in zip(with_it, results()):
+        assert p is q if isinstance(p, type) else torch.equal(p, q) and p.dtype == q.dtype
+
