@@ -83,27 +83,44 @@ __device__ __forceinline__ float head8_quant(const float (&x)[8], uint32_t& lo, 
     return sc;
 }
 
-// Q and K of the stand-alone operator: dequant -> RoPE -> FHT-64/8 -> per-head int8 quant (same arithmetic as
+// 32 tokens of one value head: V [B][S][HKV][64] -> V^T [B][HKV][64][S] (keys contiguous, the K-major operand of P.V) and
+// vs [B][S][HKV] -> [B][HKV][S]. S is a multiple of 16, v 4-byte aligned.
+__device__ __forceinline__ void v_transpose_tile(const int8_t* __restrict__ v, const float* __restrict__ vs, int S, int HKV, int h,
+                                                 int8_t* __restrict__ vT, float* __restrict__ vsT) {
+    __shared__ int8_t tile[32][64 + 4];
+    const int b = blockIdx.z, s0 = blockIdx.y * 32, tid = threadIdx.x;
+    for (int i = tid; i < 32 * 16; i += 256) {
+        const int r = i >> 4, c4 = i & 15;                             // token, group of 4 dims
+        if (s0 + r < S) *reinterpret_cast<int*>(&tile[r][c4 * 4]) = *reinterpret_cast<const int*>(v + (((long)b * S + s0 + r) * HKV + h) * 64 + c4 * 4);
+    }
+    if (tid < 32 && s0 + tid < S) vsT[((long)b * HKV + h) * S + s0 + tid] = vs[((long)b * S + s0 + tid) * HKV + h];
+    __syncthreads();
+    for (int i = tid; i < 64 * 8; i += 256) {
+        const int d = i >> 3, r = (i & 7) * 4;                         // dim, group of 4 tokens
+        if (s0 + r < S)
+            *reinterpret_cast<char4*>(vT + (((long)b * HKV + h) * 64 + d) * S + s0 + r) = make_char4(tile[r][d], tile[r + 1][d], tile[r + 2][d], tile[r + 3][d]);
+    }
+}
+
+// Q and K of the stand-alone operator (and, in the last HKV columns of the grid, V): dequant -> RoPE -> FHT-64/8 -> per-head int8 quant (same arithmetic as
 // qk_prepare_kernel), written head-major [B][H][S][64] with scales [B][H][S] so that one head's rows are contiguous.
 // VEC: q and k are 4-byte and the tables 16-byte aligned (else the same values are fetched one by one).
+// Grid (head, 32 tokens, sequence), so that nothing has to be divided to find a thread's head and token: with a flat index the four 64-bit
+// divisions were most of the kernel (4 x 1024 tokens, 32 + 8 heads: 21.0 -> XXX us).
 template <bool VEC>
 __global__ void __launch_bounds__(256) attn_qk_prepare_kernel(const int8_t* __restrict__ q, const float* __restrict__ qs,
                                                               const int8_t* __restrict__ k, const float* __restrict__ ks,
                                                               const float* __restrict__ cos_t, const float* __restrict__ sin_t, int B, int S,
                                                               int HQ, int HKV, int8_t* __restrict__ q_out, float* __restrict__ qs_out,
-                                                              int8_t* __restrict__ k_out, float* __restrict__ ks_out) {
-    const long total = (long)B * S * (HQ + HKV);
-    long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int l8 = threadIdx.x & 7;
-    const bool live = w < total;
-    if (!live) w = total - 1;                                          // the shuffles below take whole warps
-    const long nq = (long)B * S * HQ;
-    const bool is_q = w < nq;
-    const long i = is_q ? w : w - nq;
-    const int H = is_q ? HQ : HKV;
-    const int h = (int)(i % H);
-    const long bt = i / H;
-    const int t = (int)(bt % S), b = (int)(bt / S);
+                                                              int8_t* __restrict__ k_out, float* __restrict__ ks_out, const int8_t* __restrict__ v,
+                                                              const float* __restrict__ vs, int8_t* __restrict__ vT, float* __restrict__ vsT) {
+    if ((int)blockIdx.x >= HQ + HKV) { v_transpose_tile(v, vs, S, HKV, (int)blockIdx.x - HQ - HKV, vT, vsT); return; }
+    const int l8 = threadIdx.x & 7, b = blockIdx.z, t_mine = blockIdx.y * 32 + (threadIdx.x >> 3);
+    const bool live = t_mine < S;
+    const int t = live ? t_mine : S - 1;                               // the shuffles below take whole warps
+    const bool is_q = (int)blockIdx.x < HQ;
+    const int H = is_q ? HQ : HKV, h = is_q ? blockIdx.x : blockIdx.x - HQ;
+    const long i = ((long)b * S + t) * H + h;
     const float sc_in = (is_q ? qs : ks)[i];
     const int8_t* src = (is_q ? q : k) + i * 64;
     auto four = [&](const int8_t* p) { return VEC ? *reinterpret_cast<const char4*>(p) : make_char4(p[0], p[1], p[2], p[3]); };
@@ -120,28 +137,6 @@ __global__ void __launch_bounds__(256) attn_qk_prepare_kernel(const int8_t* __re
     uint32_t* dst = reinterpret_cast<uint32_t*>((is_q ? q_out : k_out) + o * 64);
     dst[l8] = lo;
     dst[8 + l8] = hi;
-}
-
-// V [B][S][HKV][64] -> V^T [B][HKV][64][S] (keys contiguous, the K-major operand of P.V) and
-// vs [B][S][HKV] -> [B][HKV][S].
-__global__ void __launch_bounds__(256) attn_v_transpose_kernel(const int8_t* __restrict__ v, const float* __restrict__ vs,
-                                                               int B, int S, int HKV, int8_t* __restrict__ vT,
-                                                               float* __restrict__ vsT) {
-    __shared__ int8_t tile[64][64 + 4];
-    const int s0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-        const int r = i >> 4, c4 = i & 15;   // r: token in tile, c4: group of 4 dims
-        int val = 0;
-        if (s0 + r < S) val = *reinterpret_cast<const int*>(v + (((long)b * S + s0 + r) * HKV + h) * 64 + c4 * 4);
-        *reinterpret_cast<int*>(&tile[r][c4 * 4]) = val;
-    }
-    if (threadIdx.x < 64 && s0 + threadIdx.x < S)
-        vsT[((long)b * HKV + h) * S + s0 + threadIdx.x] = vs[((long)b * S + s0 + threadIdx.x) * HKV + h];
-    __syncthreads();
-    for (int i = threadIdx.x; i < 64 * 64; i += 256) {
-        const int d = i >> 6, r = i & 63;
-        if (s0 + r < S) vT[(((long)b * HKV + h) * 64 + d) * S + s0 + r] = tile[r][d];
-    }
 }
 
 // ------------------------------------------------------------------ main kernel
@@ -263,6 +258,7 @@ __global__ void __launch_bounds__(192, 4) attn_prefill_kernel(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();                                                    // barriers and TMEM are ready before the kernel in front has finished
     const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 64;
 
     if (warp == 4) {
@@ -885,33 +881,27 @@ int* device_error_flag();
 // attention kernel's Q tiles. Key heads: the same arithmetic, written straight into the KV cache's pages (row = token).
 // Value heads: per-head int8 quant (quant.h:527-650), token-major into a scratch that attn_v_to_pages_kernel transposes
 // into the cache's V^T pages.
+// Grid (head, 32 tokens, sequence): see attn_qk_prepare_kernel. Bound by memory: 32768 tokens of 32 + 2 x 8 heads 160 -> XXX us (502 MB, 77 us at the
+// copy rate).
 __global__ void __launch_bounds__(256) attn_qkv_prepare_f32_kernel(const float* __restrict__ qkv, const float* __restrict__ cos_t,
                                                                    const float* __restrict__ sin_t, int B, int Sq, int q_off, int HQ, int HKV,
                                                                    int8_t* __restrict__ q2, float* __restrict__ qs2,
                                                                    int8_t* __restrict__ k_pool, float* __restrict__ ks_pool,
                                                                    const int32_t* __restrict__ page_table, int max_pages,
                                                                    int8_t* __restrict__ v2, float* __restrict__ vs2) {
-    const int heads = HQ + 2 * HKV;
-    const long total = (long)B * Sq * heads;
-    long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
-    const int l8 = threadIdx.x & 7;
-    const bool live = w < total;
-    if (!live) w = total - 1;                                          // the shuffles below take whole warps
-    const long bt = w / heads;
-    const int h = (int)(w - bt * heads);
-    const int b = (int)(bt / Sq), t = (int)(bt - (long)b * Sq);
+    const int l8 = threadIdx.x & 7, h = blockIdx.x, b = blockIdx.z, t_mine = blockIdx.y * 32 + (threadIdx.x >> 3);
+    const bool live = t_mine < Sq;
+    const int t = live ? t_mine : Sq - 1;                              // the shuffles below take whole warps
     const int pos = q_off + t;
+    const long bt = (long)b * Sq + t, w = bt * (HQ + 2 * HKV) + h;
     const float4* src = reinterpret_cast<const float4*>(qkv + w * 64);
     const float4 a = src[l8], c = src[8 + l8];
     const float raw[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
     float x[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) x[i] = raw[i];
-    head8_rotate_fht(x, reinterpret_cast<const float4*>(cos_t + (long)pos * 32)[l8], reinterpret_cast<const float4*>(sin_t + (long)pos * 32)[l8], l8);
-    if (h >= HQ + HKV) {                                               // value heads are quantised as they are
-#pragma unroll
-        for (int i = 0; i < 8; i++) x[i] = raw[i];
-    }
+    if (h < HQ + HKV)                                                  // value heads are quantised as they are
+        head8_rotate_fht(x, reinterpret_cast<const float4*>(cos_t + (long)pos * 32)[l8], reinterpret_cast<const float4*>(sin_t + (long)pos * 32)[l8], l8);
     uint32_t lo, hi;
     const float sc = head8_quant(x, lo, hi);
     if (!live) return;
@@ -1021,7 +1011,8 @@ static int mha_prefill_core(AttnArgs a, const int8_t* q2, const int8_t* kmat, ui
         attn_prefill_online_kernel<<<(unsigned)grid, 192, ATO_SMEM, st>>>(tq, tk, tv, a);
         return launch_status();
     }
-    attn_prefill_kernel<<<(unsigned)grid, 192, ATT_SMEM, st>>>(tq, tk, tv, a);
+    struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    launch_k(attn_prefill_kernel, dim3((unsigned)grid), dim3(192), (size_t)ATT_SMEM, st, tq, tk, tv, a);
     return launch_status();
 }
 
@@ -1040,7 +1031,7 @@ int mha_prefill_paged(const float* qkv, const float* cos_t, const float* sin_t, 
     PagedWs ws(workspace, B, max_prefill, HQ, HKV);
     int8_t* k_pool = c->k + (size_t)layer * c->page_bytes; int8_t* v_pool = c->v + (size_t)layer * c->page_bytes;
     float* ks_pool = c->ks + (size_t)layer * (c->scale_bytes / 4); float* vs_pool = c->vs + (size_t)layer * (c->scale_bytes / 4);
-    attn_qkv_prepare_f32_kernel<<<(unsigned)(((long)B * Sq * (HQ + 2 * HKV) + 31) / 32), 256, 0, st>>>(qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2, k_pool,
+    attn_qkv_prepare_f32_kernel<<<dim3(HQ + 2 * HKV, (Sq + 31) / 32, B), 256, 0, st>>>(qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2, k_pool,
                                                                             ks_pool, page_table, max_pages, ws.v2, ws.vs2);
     dim3 g((Sq + 63) / 64, HKV, B);
     attn_v_to_pages_kernel<<<g, 256, 0, st>>>(ws.v2, ws.vs2, Sq, q_off, HKV, page_table, max_pages, v_pool, vs_pool);
@@ -1078,10 +1069,8 @@ static int mha_prefill_contiguous(bool online, const int8_t* q, const float* qs,
     cudaStream_t st = (cudaStream_t)stream;
     PrefillWs ws(workspace, B, S, HQ, HKV);
     auto* prepare = aligned(q, 4) && aligned(k, 4) && aligned(cos_t, 16) && aligned(sin_t, 16) ? attn_qk_prepare_kernel<true> : attn_qk_prepare_kernel<false>;
-    prepare<<<(unsigned)(((long)B * S * (HQ + HKV) + 31) / 32), 256, 0, st>>>(q, qs, k, ks, cos_t, sin_t, B, S, HQ, HKV, ws.q2, ws.qs2, ws.k2, ws.ks2);
-    dim3 g((S + 63) / 64, HKV, B);
-    attn_v_transpose_kernel<<<g, 256, 0, st>>>(v, vs, B, S, HKV, ws.vT, ws.vsT);
-    int rc = launch_status(2);
+    prepare<<<dim3(HQ + 2 * HKV, (S + 31) / 32, B), 256, 0, st>>>(q, qs, k, ks, cos_t, sin_t, B, S, HQ, HKV, ws.q2, ws.qs2, ws.k2, ws.ks2, v, vs, ws.vT, ws.vsT);
+    int rc = launch_status();
     if (rc != FLEXLLM_OK) return rc;
     AttnArgs a;
     a.B = B; a.HQ = HQ; a.HKV = HKV; a.Sq = S; a.q_off = 0; a.Sk = S;
