@@ -78,6 +78,15 @@ inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cl
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// Launches in its scope carry the attribute also outside a chain. For kernels that read nothing before their wait: these may be set up (barriers,
+// TMEM, descriptors) under the tail of whatever is in front. A kernel that holds TMEM lets others start only once it has taken its columns. Product of
+// 128 x 2048 x 2048, calls in a row: 8.2 -> 6.7 us; 9 to 8192 rows of nine matrices 1.06 times as fast, of the small ones up to 1.19.
+struct SetUpEarly {
+    const bool set = g_pdl == 0;
+    SetUpEarly() { if (set) g_pdl = 1; }
+    ~SetUpEarly() { if (set) g_pdl = 0; }
+};
+
 #define FLEXLLM_CHECK_CUDA(expr)                                   \
     do {                                                           \
         int _st = ::flexllm::cuda_status((expr));                  \

@@ -614,7 +614,6 @@ __global__ void __launch_bounds__(GpCfg<SWIGLU>::THREADS, 1) gemm_i8_pair_kernel
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
     float* stg_all = reinterpret_cast<float*>(ring_ptr + GP_STAGES * GP_STAGE_BYTES + 256);
 
-    pdl_sync();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int num_kb = (args.K + 127) >> 7;
@@ -636,6 +635,7 @@ __global__ void __launch_bounds__(GpCfg<SWIGLU>::THREADS, 1) gemm_i8_pair_kernel
     cluster_sync();                                              // the other CTA's barriers exist before anything arrives on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_slot;
+    pdl_sync();                                                  // with this CTA's columns taken: a kernel that starts early cannot take them
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer, one per CTA
@@ -871,6 +871,7 @@ static TileCosts tile_costs(int M, int N) {
 }
 int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
                     int32_t* acc, float* y, cudaStream_t st, const float* residual) {
+    const SetUpEarly early;
     const TileCosts t = tile_costs(M, N);
     const long c256 = t.c256, c128 = t.c128, c64 = t.c64, c32 = t.c32;
     if (t.pair) return launch_gemm_pair(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
@@ -888,6 +889,7 @@ int gemm_i8_prefill(const int8_t* a, const float* s_tok, const int8_t* w, const 
 // anyway (more than 128 rows); elsewhere FLEXLLM_ENOTSUP and nothing is launched.
 int gemm_i8_prefill_swiglu(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int F, int K, float* h, cudaStream_t st) {
     if (F % 128 != 0 || !tile_costs(M, 2 * F).pair) return FLEXLLM_ENOTSUP;
+    const SetUpEarly early;
     return launch_gemm_pair<true>(a, s_tok, w, s_ch, M, 2 * F, K, nullptr, h, st, nullptr);
 }
 

@@ -378,6 +378,21 @@ def test_linear_prefill_tile_choice(F, M, N, K):
     assert F.lib().flexllm_device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(128, 2048, 256), (1500, 1024, 128), (1990, 4104, 144), (100, 264, 144)])
+def test_linear_prefill_set_up_early(F, M, N, K):
+    """Products in a row, each adding to the one before: every one is set up while its predecessor still writes."""
+    a, st, w, sc = lin_inputs(M, N, K, 26)
+    t = [dev(v) for v in (a, st, w, sc)]
+    x = rng(27).standard_normal((M, N)).astype(np.float32)
+    want, got = x, dev(x)
+    y_o = oracle.linear_i8(a, st, w, sc)[1]
+    for _ in range(12):
+        _, got = F.pref_Linear_Layer_i8xi8(*t, residual=got)
+        want = oracle.residual(want, y_o)
+    assert_same(to_np(got), want, "sum")
+    assert F.lib().flexllm_device_status() == 0
+
+
 def test_linear_prefill_extremes(F):
     """Largest accumulator magnitude the path can see: |a|=|w|=128... here -128 * -128 * 8192."""
     M, N, K = 128, 128, 8192
