@@ -889,6 +889,7 @@ __global__ void __launch_bounds__(256) attn_qkv_prepare_f32_kernel(const float* 
                                                                    int8_t* __restrict__ k_pool, float* __restrict__ ks_pool,
                                                                    const int32_t* __restrict__ page_table, int max_pages,
                                                                    int8_t* __restrict__ v2, float* __restrict__ vs2) {
+    pdl_sync();
     const int l8 = threadIdx.x & 7, h = blockIdx.x, b = blockIdx.z, t_mine = blockIdx.y * 32 + (threadIdx.x >> 3);
     const bool live = t_mine < Sq;
     const int t = live ? t_mine : Sq - 1;                              // the shuffles below take whole warps
@@ -921,6 +922,7 @@ __global__ void __launch_bounds__(256) attn_qkv_prepare_f32_kernel(const float* 
 __global__ void __launch_bounds__(256) attn_v_to_pages_kernel(const int8_t* __restrict__ v, const float* __restrict__ vs, int Sq, int q_off,
                                                               int HKV, const int32_t* __restrict__ page_table, int max_pages,
                                                               int8_t* __restrict__ v_pool, float* __restrict__ vs_pool) {
+    pdl_sync();
     __shared__ int8_t tile[64][64 + 4];
     const int s0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
     const long prow = ((long)page_table[(long)b * max_pages + (q_off + s0) / 64] * HKV + h) * 64;
@@ -1011,7 +1013,7 @@ static int mha_prefill_core(AttnArgs a, const int8_t* q2, const int8_t* kmat, ui
         attn_prefill_online_kernel<<<(unsigned)grid, 192, ATO_SMEM, st>>>(tq, tk, tv, a);
         return launch_status();
     }
-    struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    const SetUpEarly early;
     launch_k(attn_prefill_kernel, dim3((unsigned)grid), dim3(192), (size_t)ATT_SMEM, st, tq, tk, tv, a);
     return launch_status();
 }
@@ -1031,10 +1033,11 @@ int mha_prefill_paged(const float* qkv, const float* cos_t, const float* sin_t, 
     PagedWs ws(workspace, B, max_prefill, HQ, HKV);
     int8_t* k_pool = c->k + (size_t)layer * c->page_bytes; int8_t* v_pool = c->v + (size_t)layer * c->page_bytes;
     float* ks_pool = c->ks + (size_t)layer * (c->scale_bytes / 4); float* vs_pool = c->vs + (size_t)layer * (c->scale_bytes / 4);
-    attn_qkv_prepare_f32_kernel<<<dim3(HQ + 2 * HKV, (Sq + 31) / 32, B), 256, 0, st>>>(qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2, k_pool,
-                                                                            ks_pool, page_table, max_pages, ws.v2, ws.vs2);
+    const SetUpEarly early;
+    launch_k(attn_qkv_prepare_f32_kernel, dim3(HQ + 2 * HKV, (Sq + 31) / 32, B), dim3(256), 0, st, qkv, cos_t, sin_t, B, Sq, q_off, HQ, HKV, ws.q2, ws.qs2,
+             k_pool, ks_pool, page_table, max_pages, ws.v2, ws.vs2);
     dim3 g((Sq + 63) / 64, HKV, B);
-    attn_v_to_pages_kernel<<<g, 256, 0, st>>>(ws.v2, ws.vs2, Sq, q_off, HKV, page_table, max_pages, v_pool, vs_pool);
+    launch_k(attn_v_to_pages_kernel, g, dim3(256), 0, st, ws.v2, ws.vs2, Sq, q_off, HKV, page_table, max_pages, v_pool, vs_pool);
     int rc = launch_status(2);
     if (rc != FLEXLLM_OK) return rc;
     AttnArgs a;

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
                                                                          int M, int D, float eps, float* __restrict__ y,
                                                                          int8_t* __restrict__ q, float* __restrict__ s) {
     extern __shared__ __align__(16) float rows_sm[];          // [8][D + 4], then rinv[8]
+    pdl_sync();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ld = D + 4, nv = D >> 2;
     const long row0 = (long)blockIdx.x * RMSP_ROWS;
@@ -589,7 +590,7 @@ extern "C" int flexllm_rmsnorm_quant(const float* x, const float* gamma, int M, 
             FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_prefill_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
             attr_done[dev].store(1, std::memory_order_release);
         }
-        rmsnorm_prefill_kernel<<<grid, RMSP_ROWS * 32, smem, st>>>(x, gamma, M, D, eps, y, q, s);
+        launch_k(rmsnorm_prefill_kernel, dim3(grid), dim3(RMSP_ROWS * 32), smem, st, x, gamma, M, D, eps, y, q, s);
     } else {
         const size_t smem = (size_t)(D + 4 * order) * sizeof(float);
         launch_k(D <= 2048 ? rmsnorm_decode_kernel<2> : rmsnorm_decode_kernel<4>, dim3(M), dim3(256), smem, st, x, gamma, D, eps, order, y, q, s);

@@ -444,6 +444,9 @@ static int prefill_chunk(flexllm_model* m, const int32_t* tokens, const float* e
     const int QKV = (HQ + 2 * HKV) * 64;
     const int M = B * Sc;
     const int g = m->g, r = m->r, Dl = m->Dl, Fl = m->Fl;
+    // Nothing below reads ahead of its wait: every kernel's launch and set-up under the one before. 1 x 32 tokens 1.95 -> 1.64 ms, 4 x 256 3.49 -> 3.21,
+    // 4 x 1024 10.26 -> 9.99; longer batches the same.
+    const SetUpEarly early;
     if (embeds) {       // rows given as vectors (not token ids): sequence b's chunk is contiguous in embeds [B][S][D]
         for (int b = 0; b < B; b++)
             TRY(copy_any(m->x + (size_t)b * Sc * D, embeds + ((size_t)b * S + c0) * D, (size_t)Sc * D * 4, st));
@@ -676,13 +679,15 @@ static int mega_prepare(flexllm_model* m) {
     return FLEXLLM_OK;
 }
 
+bool flexllm::programmatic_chains() {
+    static const bool on = [] { const char* e = getenv("FLEXLLM_PDL"); return e ? atoi(e) != 0 : true; }();
+    return on;
+}
 static int decode_step_body(flexllm_model* m, cudaStream_t st);
 static int decode_step(flexllm_model* m, cudaStream_t st) {
     TRY(mega_prepare(m));
     if (m->mega_state == 1) return mega_launch(m->mega, m->B, m->mega_variant, st);
-    static int use_pdl = -1;
-    if (use_pdl < 0) { const char* e = getenv("FLEXLLM_PDL"); use_pdl = e ? atoi(e) : 1; }
-    g_pdl = use_pdl ? 2 : 0;             // the kernels of a step read the contexts, page tables and older cache entries ahead of their wait
+    g_pdl = programmatic_chains() ? 2 : 0;             // the kernels of a step read the contexts, page tables and older cache entries ahead of their wait
     const int rc = decode_step_body(m, st);
     g_pdl = 0;
     return rc;
