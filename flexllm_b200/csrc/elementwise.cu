@@ -151,20 +151,32 @@ __global__ void static_quant_kernel(const float* __restrict__ x, long rows, int 
 // ---------------------------------------------------------------------------------------------
 constexpr int RMS_PIECE = 128;           // floats per row per staging step
 
-// Prefill order: a CTA of 8 warps takes 8 consecutive rows. All threads bring the rows into shared memory (coalesced
-// 128-bit loads, all in flight at once); warp 0 then runs the 32 chains (4 per row) over them; afterwards every warp
-// normalises and quantises one row straight from shared memory -- each row is read from global memory once. Row stride
-// D + 4 floats: the 32 chains' reads (row rr, element 4k + j) fall into 32 different banks. Requires D % 128 == 0.
-constexpr int RMSP_ROWS = 8;
+// Prefill order: a CTA of 4 warps takes 4 consecutive rows. Each warp brings one into shared memory (coalesced 128-bit loads, all in flight at
+// once); warp 0 then runs the 16 chains (4 per row) over them; afterwards every thread normalises and quantises the same columns of all four rows, whose
+// gains it has held since the start -- each row is read from global memory once. Row stride D + 4 floats: the chains' reads (row rr, element
+// 4k + j) fall into different banks. Requires D % 128 == 0. COLS: groups of four columns a thread.
+// Bound by the ordered sums and the phases around them, which six CTAs an SM take turns in: 32768 rows of 2048 98 us (353 MB: 54 us at the copy rate), 32 rows
+// 6.7 us. A warp per row in the last phase, eight rows a CTA, waited for the gains at every step: 124 and 8.5 us (rows of 4096: 493 and 15.5 us, now
+// 298 and 12.1); eight rows a CTA by columns 102 and 7.0 us; four and two rows by rows 118 and 113 us.
+constexpr int RMSP_ROWS = 4;
+template <int COLS>
 __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                                                          int M, int D, float eps, float* __restrict__ y,
                                                                          int8_t* __restrict__ q, float* __restrict__ s) {
-    extern __shared__ __align__(16) float rows_sm[];          // [8][D + 4], then rinv[8]
-    pdl_sync();
+    extern __shared__ __align__(16) float rows_sm[];          // [rows][D + 4], then rinv[rows]
+    __shared__ uint32_t amax_sm[RMSP_ROWS][RMSP_ROWS], nan_sm[RMSP_ROWS];      // per warp: the largest magnitude of each row, rows with a NaN
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ld = D + 4, nv = D >> 2;
     const long row0 = (long)blockIdx.x * RMSP_ROWS;
     float* rinv_sm = rows_sm + RMSP_ROWS * ld;
+    pdl_wait();            // before the kernels after this one may start: see rmsnorm_decode_kernel
+    pdl_launch();
+    float4 gm[COLS];                                          // this thread's columns of every row
+#pragma unroll
+    for (int i = 0; i < COLS; i++) {
+        const int c = threadIdx.x + i * RMSP_ROWS * 32;
+        gm[i] = c < nv ? reinterpret_cast<const float4*>(gamma)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     {   // warp w brings in row w
         const bool in = row0 + w < M;
         const float4* src = reinterpret_cast<const float4*>(x + (row0 + w) * D);
@@ -175,7 +187,7 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
     __syncthreads();
     if (w == 0) {
         const int rr = lane >> 2, j = lane & 3;      // chain (row rr, residue j)
-        const float* src = rows_sm + rr * ld + j;
+        const float* src = rows_sm + min(rr, RMSP_ROWS - 1) * ld + j;
         float ss = 0.0f;
         // blocks of 16 elements, the next block's loads under way while this one is added: a step then costs the
         // addition's latency alone
@@ -202,46 +214,63 @@ __global__ void __launch_bounds__(RMSP_ROWS * 32) rmsnorm_prefill_kernel(const f
         const float p0 = __shfl_sync(0xffffffffu, ss, base), p1 = __shfl_sync(0xffffffffu, ss, base + 1);
         const float p2 = __shfl_sync(0xffffffffu, ss, base + 2), p3 = __shfl_sync(0xffffffffu, ss, base + 3);
         const float tot = (p0 + p1) + (p2 + p3);
-        if (j == 0) rinv_sm[rr] = 1.0f / sqrtf(tot / (float)D + eps);
+        if (j == 0 && rr < RMSP_ROWS) rinv_sm[rr] = 1.0f / sqrtf(tot / (float)D + eps);
     }
     __syncthreads();
-    const long row = row0 + w;
-    if (row >= M) return;
-    const float r = rinv_sm[w];
-    const float4* xr = reinterpret_cast<const float4*>(rows_sm + w * ld);
-    const float4* g4 = reinterpret_cast<const float4*>(gamma);
-    float4* yr = y ? reinterpret_cast<float4*>(y + row * D) : nullptr;
-    // first pass: the normalised row's largest magnitude (max(|max|, |min|) of the row = max of |.|), fp32 output if asked for;
-    // second pass: the same products again (same bits) and the quantiser -- nothing of the row is held in registers
-    float amax = 0.0f, nan = 0.0f;
-    const f32x2 r2 = pack2(r, r);
-    auto normed = [&](int c, float (&o)[4]) {
-        const float4 v = xr[c], g = g4[c];
+    // first pass: every row's largest magnitude (max(|max|, |min|) of the row = max of |.|), fp32 output if asked for; second pass: the same products
+    // again (same bits) and the quantiser
+    const int rows = (int)(M - row0 < RMSP_ROWS ? M - row0 : RMSP_ROWS);
+    auto normed = [&](int rr, int i, float (&o)[4]) {
+        const float4 v = reinterpret_cast<const float4*>(rows_sm + rr * ld)[threadIdx.x + i * RMSP_ROWS * 32], g = gm[i];
+        const float r = rinv_sm[rr];
+        const f32x2 r2 = pack2(r, r);
         unpack2(mul2(mul2(pack2(v.x, v.y), r2), pack2(g.x, g.y)), o[0], o[1]);
         unpack2(mul2(mul2(pack2(v.z, v.w), r2), pack2(g.z, g.w)), o[2], o[3]);
     };
-#pragma unroll 4
-    for (int c = lane; c < nv; c += 32) {
-        float o[4];
-        normed(c, o);
-        if (yr) yr[c] = make_float4(o[0], o[1], o[2], o[3]);
-        amax = max3(max3(amax, fabsf(o[0]), fabsf(o[1])), fabsf(o[2]), fabsf(o[3]));
-        nan = max3_nan(max3_nan(nan, o[0], o[1]), o[2], o[3]);
+    uint32_t nan_rows = 0;
+#pragma unroll
+    for (int rr = 0; rr < RMSP_ROWS; rr++) {
+        float amax = 0.0f, nan = 0.0f;
+#pragma unroll
+        for (int i = 0; i < COLS; i++) {
+            const int c = threadIdx.x + i * RMSP_ROWS * 32;
+            if (c >= nv) continue;
+            float o[4];
+            normed(rr, i, o);
+            if (y && rr < rows) reinterpret_cast<float4*>(y + (row0 + rr) * D)[c] = make_float4(o[0], o[1], o[2], o[3]);
+            amax = max3(max3(amax, fabsf(o[0]), fabsf(o[1])), fabsf(o[2]), fabsf(o[3]));
+            nan = max3_nan(max3_nan(nan, o[0], o[1]), o[2], o[3]);
+        }
+        const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));      // not negative, not NaN: ordered as its bits
+        if (lane == 0) amax_sm[w][rr] = m;
+        nan_rows |= (uint32_t)(nan != nan) << rr;
     }
-    if (q) {
-        amax = warp_max(amax);
-        const float sc = sym_scale_from(amax, -amax);
-        const bool ok = __all_sync(0xffffffffu, nan == nan) && sc >= 0x1p-60f && sc <= 0x1p60f;
-        const float w8 = 1.0f / sc;         // one reciprocal per row
-        if (lane == 0) s[row] = sc;
-        uint32_t* qr = reinterpret_cast<uint32_t*>(q + row * D);
-#pragma unroll 4
-        for (int c = lane; c < nv; c += 32) {
+    if (!q) return;
+    nan_rows = __reduce_or_sync(0xffffffffu, nan_rows);
+    if (lane == 0) nan_sm[w] = nan_rows;
+    __syncthreads();
+    // lane rr, rr + RMSP_ROWS, ...: the scale of row rr
+    const int mine = lane % RMSP_ROWS;
+    uint32_t m = 0, bad = 0;
+#pragma unroll
+    for (int k = 0; k < RMSP_ROWS; k++) { m = max(m, amax_sm[k][mine]); bad |= nan_sm[k]; }
+    const float sc_mine = sym_scale_from(__uint_as_float(m), -__uint_as_float(m)), w8_mine = 1.0f / sc_mine;         // one reciprocal per row
+    const uint32_t ok_rows = __ballot_sync(0xffffffffu, !(bad >> mine & 1) && sc_mine >= 0x1p-60f && sc_mine <= 0x1p60f);
+    if (w == 0 && lane < rows) s[row0 + lane] = sc_mine;
+#pragma unroll
+    for (int rr = 0; rr < RMSP_ROWS; rr++) {
+        const float sc = __shfl_sync(0xffffffffu, sc_mine, rr), w8 = __shfl_sync(0xffffffffu, w8_mine, rr);
+        const bool ok = ok_rows >> rr & 1;
+        if (rr >= rows) break;
+#pragma unroll
+        for (int i = 0; i < COLS; i++) {
+            const int c = threadIdx.x + i * RMSP_ROWS * 32;
+            if (c >= nv) continue;
             float o[4];
             uint32_t b[4];
-            normed(c, o);
+            normed(rr, i, o);
             q8_short(o, w8, ok, b, [&](float t) { return q8_exact(t, sc); });
-            qr[c] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+            reinterpret_cast<uint32_t*>(q + (row0 + rr) * D)[c] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
         }
     }
 }
@@ -584,13 +613,15 @@ extern "C" int flexllm_rmsnorm_quant(const float* x, const float* gamma, int M, 
         const int dev = current_device();
         if (dev < 0) return FLEXLLM_ECUDA;
         if (!attr_done[dev].load(std::memory_order_acquire)) {
-            FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                    (int)(((size_t)RMSP_ROWS * (4096 + 4) + RMSP_ROWS) * sizeof(float))));
-            // three 66 KB CTAs per SM need the largest shared-memory carve-out
-            FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(rmsnorm_prefill_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+            for (auto kern : {rmsnorm_prefill_kernel<16 / RMSP_ROWS>, rmsnorm_prefill_kernel<32 / RMSP_ROWS>}) {
+                FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)(((size_t)RMSP_ROWS * (4096 + 4) + RMSP_ROWS) * sizeof(float))));
+                // six 33 KB CTAs per SM need the largest shared-memory carve-out
+                FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+            }
             attr_done[dev].store(1, std::memory_order_release);
         }
-        launch_k(rmsnorm_prefill_kernel, dim3(grid), dim3(RMSP_ROWS * 32), smem, st, x, gamma, M, D, eps, y, q, s);
+        launch_k(D <= 2048 ? rmsnorm_prefill_kernel<16 / RMSP_ROWS> : rmsnorm_prefill_kernel<32 / RMSP_ROWS>, dim3(grid), dim3(RMSP_ROWS * 32), smem, st, x, gamma, M, D, eps, y, q, s);
     } else {
         const size_t smem = (size_t)(D + 4 * order) * sizeof(float);
         launch_k(D <= 2048 ? rmsnorm_decode_kernel<2> : rmsnorm_decode_kernel<4>, dim3(M), dim3(256), smem, st, x, gamma, D, eps, order, y, q, s);

@@ -257,6 +257,23 @@ def test_rmsnorm_row_of_nan(F, order, D):
     assert_same(to_np(s), so, "scale"); assert not to_np(q)[1].any()
 
 
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 9])
+@pytest.mark.parametrize("D", [128, 384, 1920, 2048, 2176, 4096])
+def test_rmsnorm_prompt_rows_by_columns(F, M, D):
+    """Row counts around a CTA's four, widths that leave threads without a column; a row of zeros, one with a NaN, one with an infinity."""
+    g = rng(92)
+    x = g.standard_normal((M, D)).astype(np.float32); gamma = (1 + 0.1 * g.standard_normal(D)).astype(np.float32)
+    if M > 1: x[1] = 0
+    if M > 2: x[2, D // 2] = np.nan
+    if M > 4: x[4, D - 1] = np.inf
+    y, q, s = F.pref_Layer_Norm(dev(x), dev(gamma), 1e-5, 0, quant=True)
+    yo = oracle.rmsnorm(x, gamma, 1e-5, 0)
+    qo, so = oracle.quant_per_token(yo)
+    odd = ~np.isfinite(yo).all(1)
+    assert (np.isnan(to_np(y)) == np.isnan(yo)).all() and not to_np(q)[odd].any()
+    assert_same(to_np(y)[~odd], yo[~odd], "y"); assert_same(to_np(s)[~odd], so[~odd], "scale"); assert_same(to_np(q)[~odd], qo[~odd], "q")
+
+
 @pytest.mark.parametrize("order", [0, 4, 8])
 @pytest.mark.parametrize("M", [1, 64, 130])
 def test_rmsnorm_quant(F, order, M):
