@@ -895,7 +895,8 @@ int gemm_i8_prefill_swiglu(const int8_t* a, const float* s_tok, const int8_t* w,
 
 // Decode orientation: weights on the 128-row side, M <= 64 tokens on the N side. K is split over clusters of up to four CTAs as
 // long as the tiles leave half the SMs idle and every split keeps two 128-byte blocks. (64 tokens of 2048 x 8192: 23.5 / 19.8 /
-// 14.0 / 18.3 us with clusters of 1 / 2 / 4 / 8, of 2048 x 2048: 13.3 / 14.4 / 10.4 / 15.4 us: larger clusters start and meet later.)
+// 14.0 / 18.3 us with clusters of 1 / 2 / 4 / 8, of 2048 x 2048: 13.3 / 14.4 / 10.4 / 15.4 us: larger clusters start and meet later. Those were taken
+// with an epilogue that loaded value by value; with its loads in flight together the clusters of four take 12 and 8 us.)
 int gemm_i8_decode(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
                    int32_t* acc, float* y, cudaStream_t st, const float* residual) {
     if (M > 64) return FLEXLLM_ENOTSUP;
