@@ -331,7 +331,7 @@ static int launch_dec_fused(bool in_f32, const int8_t* q, const float* qs, const
                             cudaStream_t st) {
     const size_t smem = dec_attn_smem_bytes<G>(cs);
     auto kern = in_f32 ? dec_attn_fused_kernel<true, 512, G> : dec_attn_fused_kernel<false, 512, G>;
-    if (smem > 40 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));   // 48 KB with the static part
+    TRY_RC(allow_shared(kern, smem));
     launch_k(kern, dim3(4 / G * HKV, B), dim3(512), smem, st, q, qs, k, ks, v, vs, qkv_f32, cos_t, sin_t, a_s, L, page_table, max_pages, ctx,
              HQ, HKV, cs, out, oacc, max_ctx, err);
     return launch_status(1);
@@ -655,7 +655,7 @@ static int launch_dec_cluster(bool in_f32, const DecAttnIn& in, const float* cos
                               int32_t* oacc, cudaStream_t st) {
     const size_t smem = dec_cluster_smem_bytes(pages);
     auto kern = in_f32 ? dec_attn_cluster_kernel<true> : dec_attn_cluster_kernel<false>;
-    FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TRY_RC(allow_shared(kern, smem));
     launch_cluster(kern, dim3(DEC_CL * HKV, B), dim3(DEC_CL_NT), DEC_CL, smem, st, in, cos_t, sin_t, a_s, L, page_table, max_pages, ctx, HQ, HKV,
                    pages, rank ? 1 : 0, out, oacc);
     return launch_status(1);

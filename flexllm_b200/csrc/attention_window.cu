@@ -1038,16 +1038,12 @@ __global__ void __launch_bounds__(192, 2) attn_window_prefill_kernel(const __gri
     if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem_base, a.tmem_cols); }
 }
 
-int set_smem(const void* kern, size_t bytes) {
-    return bytes > 48 * 1024 ? cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) : FLEXLLM_OK;
-}
-
 template <class T, int RC, bool FUSED, bool WIDE> int launch_row(const AttnCall& c, int splits, int L, cudaStream_t st) {
     const int R = c.s.H / c.s.G;
     const size_t smem = (size_t)row_smem(R, c.s.dkp, c.s.dv).total * 4;
     if (smem > 220 * 1024) return FLEXLLM_ENOTSUP;
     auto kern = attn_row_kernel<T, RC, FUSED, WIDE>;
-    TRY_RC(set_smem((const void*)kern, smem));
+    TRY_RC(allow_shared(kern, smem));
     launch_k(kern, dim3(splits, c.s.G, c.B * c.Sc), dim3(256), smem, st, c, L, device_error_flag());
     return launch_status();
 }
@@ -1092,7 +1088,7 @@ template <bool ONLINE, int DKC, int KS, int MPW> int launch_decode(DecodeArgs& a
     const size_t smem = decode_smem(c.s.dkp, c.s.dv, KS, a.tiles_max);
     auto kern = attn_decode_mma_kernel<ONLINE, DKC, KS, MPW>;
     if (smem > 200 * 1024) return FLEXLLM_ENOTSUP;
-    TRY_RC(set_smem((const void*)kern, smem));
+    TRY_RC(allow_shared(kern, smem));
     launch_k(kern, dim3(splits, c.s.G, c.B), dim3(256), smem, st, a);
     return launch_status();
 }
@@ -1163,7 +1159,7 @@ int run_prefill(const PrefillArgs& a, cudaStream_t st) {
     TRY_RC(cached_tmap_u8(&tv, c.v_pool, (uint64_t)c.n_pages * s.G * s.dv, PG * 2, (uint32_t)a.vrows, 0));
     const size_t smem = prefill_smem(a.kc, a.vrows, a.R, a.TQ, a.p_bufs, a.online).total;
     auto kern = a.online ? attn_window_prefill_kernel<true> : attn_window_prefill_kernel<false>;
-    TRY_RC(set_smem((const void*)kern, smem));
+    TRY_RC(allow_shared(kern, smem));
     launch_k(kern, dim3(a.n_qt, s.G, c.B), dim3(192), smem, st, tq, tk, tv, a);
     return launch_status();
 }

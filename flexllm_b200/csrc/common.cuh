@@ -31,6 +31,12 @@ inline int cuda_status(cudaError_t e) {
     g_last_cuda_error = (int)e;
     return FLEXLLM_ECUDA;
 }
+// Lets launches of `kern` ask for `bytes` of dynamic shared memory. A function's limit belongs to the (function, device) and so to every host thread
+// and every model of the process: it is raised once, to the most that the device has, and never set to the size of one call, which would lower it
+// between another thread's setting and its launch, or under a plan made earlier. Up to 40 KB need nothing (48 KB with the static part).
+int raise_shared_limit(const void* kern, size_t bytes);
+template <class K> inline int allow_shared(K kern, size_t bytes) { return bytes <= 40 * 1024 ? FLEXLLM_OK : raise_shared_limit((const void*)kern, bytes); }
+
 // status of the `n` launches that have just been issued
 inline int launch_status(int n = 1) { note_launches(n); return cuda_status(cudaGetLastError()); }
 

@@ -964,7 +964,7 @@ int mega_create(const MegaModelView& v, MegaPlan** out) {
     if (stages < 3) return FLEXLLM_ENOTSUP;      // long contexts: the per-operator kernels take over
     const size_t smem = 1024 + (size_t)stages * stage_bytes + scratch + 256;
     for (int i = 0; i < 4; i++) {
-        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kerns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        TRY_RC(allow_shared(kerns[i], smem));
         int per_sm = 0;
         FLEXLLM_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], MG_THREADS, smem));
         if (per_sm < 1) return FLEXLLM_ENOTSUP;

@@ -2,6 +2,8 @@
 // static quantisation, RMSNorm(+quant), SiLU, gate, residual, RoPE, softmax, greedy argmax.
 // All are HBM-bound: one pass over the data with 128-bit accesses where the layout allows.
 #include <atomic>
+#include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "tc_common.cuh"
@@ -11,6 +13,25 @@ namespace flexllm {
 thread_local int g_last_cuda_error = 0;
 thread_local int g_pdl = 0;
 std::atomic<unsigned long long> g_launch_count{0};
+
+int raise_shared_limit(const void* kern, size_t bytes) {
+    static std::mutex lock;
+    static std::unordered_map<const void*, size_t> limits[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0) return FLEXLLM_ECUDA;
+    std::lock_guard<std::mutex> hold(lock);
+    auto it = limits[dev].find(kern);
+    if (it == limits[dev].end()) {
+        int most = 0;
+        cudaFuncAttributes fa;
+        FLEXLLM_CHECK_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        FLEXLLM_CHECK_CUDA(cudaFuncGetAttributes(&fa, kern));
+        most -= (int)fa.sharedSizeBytes;
+        FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        it = limits[dev].emplace(kern, (size_t)most).first;
+    }
+    return bytes <= it->second ? FLEXLLM_OK : cuda_status(cudaErrorInvalidValue);
+}
 
 // ---------------------------------------------------------------------------------------------
 // Per-token symmetric int8 quantisation (Modules/quant.h:6-112, symmetric branch).

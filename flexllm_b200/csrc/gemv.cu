@@ -146,7 +146,7 @@ static int launch_gemv_as(const int8_t* a, const float* s_tok, const int8_t* w, 
                           int32_t* acc, float* y, const float* residual, cudaStream_t st) {
     const size_t smem = (size_t)BT * K + (KS == 4 ? (size_t)4 * R * BT * sizeof(int) : 0);
     auto kern = gemv_i8_kernel<BT, R, KS>;
-    if (smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TRY_RC(allow_shared(kern, smem));
     const int grid = KS == 1 ? (N + 4 * R - 1) / (4 * R) : (N + R - 1) / R;
     launch_k(kern, dim3(grid), dim3(128), smem, st, a, s_tok, w, s_ch, M, N, K, acc, y, residual);
     return launch_status();

@@ -374,7 +374,7 @@ int launch_gemv(const T* a, long lda, const bf16* w, long ldw, const float* bias
     const size_t smem = (size_t)BT * kv * 8 * sizeof(T);
     auto kern = gemv_float_kernel<T, BT, R, KS, GLU>;
     if (smem > 220 * 1024) return FLEXLLM_ENOTSUP;
-    if (smem > 48 * 1024) FLEXLLM_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TRY_RC(allow_shared(kern, smem));
     const int n_out = GLU ? N / 2 : N, out = GLU ? R / 2 : R;
     const int per_cta = KS == 1 ? 4 * out : out;
     launch_k(kern, dim3((n_out + per_cta - 1) / per_cta), dim3(128), smem, st, a, lda, w, ldw, bias, M, n_out, kv, relu2, y.f32, (T*)y.t, y.ld);

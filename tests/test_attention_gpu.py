@@ -341,3 +341,36 @@ def test_decode_cluster(F, ctx, HKV, what):
     """The form with a cluster of four CTAs per item: lengths around its lines, sequences of fewer pages than CTAs, page and quarter
     edges, few and many KV heads, two steps (the second reads what the first appended)."""
     decode_case(F, len(ctx), ctx, HQ=4 * HKV, HKV=HKV, seed=70 + len(ctx), steps=2 if ctx[0] < 5000 else 1, **what)
+
+
+def test_decode_from_several_threads(F):
+    """Calls whose shared-memory needs are far apart, from host threads on streams of their own: none takes the room of another away."""
+    import threading
+    lib, r = F.lib(), {}
+
+    def work(name, max_ctx):
+        g = torch.Generator(device="cuda").manual_seed(max_ctx)
+        s8 = lambda *s: torch.randint(-127, 128, s, dtype=torch.int8, device="cuda", generator=g)
+        u = lambda *s: torch.rand(s, device="cuda", generator=g) * 0.05
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            cache = F.KVCache(1, 2, 1)
+            a = [s8(1, 4, 64), u(1, 4), s8(1, 1, 64), u(1, 1), s8(1, 1, 64), u(1, 1), u(41, 32), u(41, 32), u(4)]
+            table = torch.zeros(1, max_ctx // 64 + 1, dtype=torch.int32, device="cuda")
+            ctx, out = torch.tensor([40], dtype=torch.int32, device="cuda"), torch.empty(1, 256, device="cuda")
+            nbytes = lib.flexllm_mha_decode_workspace(1, 4, max_ctx)
+            ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+            args = [cache._h, 0, *[t.data_ptr() for t in a], table.data_ptr(), table.shape[1], ctx.data_ptr(), max_ctx, 1, 4, out.data_ptr(), None,
+                    ws.data_ptr(), nbytes, stream.cuda_stream]
+            call = lib.flexllm_mha_i8xi8_decode
+            call(*args)
+            first = out.clone()
+            refused = sum(call(*args) != 0 for _ in range(20000))
+            stream.synchronize()
+            r[name] = refused, torch.equal(first, out)
+            cache.close()
+
+    threads = [threading.Thread(target=work, args=a) for a in (("long", 32000), ("short", 600), ("middle", 9000))]
+    for t in threads: t.start()
+    for t in threads: t.join()
+    assert r == {k: (0, True) for k in ("long", "short", "middle")}

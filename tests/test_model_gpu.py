@@ -81,6 +81,21 @@ def test_model_swiglu_in_the_product(F, B, S):
     run_case(F, 1, 256, 4, 1, 512, B, S, 1, seed=70 + S, use_graph=False)
 
 
+def test_model_of_longer_contexts_beside_another(F):
+    """A model whose decode step needs more shared memory than that of one made after it: both go on giving their tokens."""
+    from flexllm_b200 import synthetic
+    W = synthetic.numpy_weights(1, 256, 4, 1, 8192, 512, 2112, seed=91)
+    tok = torch.randint(0, 512, (2, 32), dtype=torch.int32, generator=torch.Generator().manual_seed(4))
+    models = []
+    for max_ctx in (2112, 68):
+        models.append(F.Model(1, 256, 4, 1, 8192, 512, max_batch=2, max_prefill=64, max_ctx=max_ctx))
+        synthetic.load_numpy_weights(models[-1], W)
+    want = models[0].generate_host(tok, 4, use_graph=False).numpy()
+    for m in models[::-1] + models:
+        assert np.array_equal(m.generate_host(tok, 4, use_graph=False).numpy(), want)
+    for m in models: m.close()
+
+
 def test_model_batch_over_8(F):
     """More than 8 sequences sends the decode linear layers down the tensor-core split-K path."""
     run_case(F, layers=2, hidden=512, hq=8, hkv=2, vocab=1000, B=12, S=16, n_new=4, seed=53, use_graph=True)
