@@ -14,6 +14,7 @@
 #include <ATen/ops/empty.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/flexllm_b200.h"
@@ -40,11 +41,12 @@ bool modes() { return c10::impl::dispatch_mode_enabled() || at::impl::torch_func
 PyObject* result(int status, at::Tensor&& y) { return status != 0 ? PyLong_FromLong(status) : THPVariable_Wrap(std::move(y)); }
 bool fits(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 
-template <class F> PyObject* guarded(F f) {          // C++ exceptions (out of memory, a CUDA error) as Python ones
+template <class F> PyObject* guarded(F f) {          // C++ exceptions as torch's own functions raise them (torch.OutOfMemoryError, torch.AcceleratorError, ...)
     try {
         return f();
-    } catch (const std::exception& e) {
-        return PyErr_Format(PyExc_RuntimeError, "%s", e.what());
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
     }
 }
 

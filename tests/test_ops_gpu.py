@@ -612,3 +612,22 @@ def test_front_end_general_path(F, monkeypatch):
     for p, q in zip(with_it, results()):
         assert p is q if isinstance(p, type) else torch.equal(p, q) and p.dtype == q.dtype
 
+
+def test_front_end_out_of_memory(F, monkeypatch):
+    """Outputs and workspaces larger than the device: torch's own exception, whichever path allocates."""
+    from flexllm_b200 import ops
+    i8 = lambda *n: torch.zeros(n, dtype=torch.int8, device="cuda")
+    f32 = lambda *n: torch.zeros(n, device="cuda")
+    M, N = 400000, 200000                                   # fp32 output of 320 GB
+    linear = (i8(M, 16), f32(M), i8(N, 16), f32(N))
+    mlp = (f32(8 * M, 16), f32(16), i8(16384, 16), f32(16384), i8(16, 8192), f32(16))
+
+    def refused():
+        for call in (lambda: F.pref_Linear_Layer_i8xi8(*linear), lambda: F.dec_Linear_Layer_i8xi8(*linear), lambda: F.dec_MLP_block(*mlp)):
+            with pytest.raises(torch.OutOfMemoryError):
+                call()
+    assert ops._bind_front_end()
+    refused()
+    monkeypatch.setattr(ops, "_front", False)
+    monkeypatch.setattr(ops, "_bind_front_end", lambda: False)
+    refused()
