@@ -33,7 +33,7 @@ def main(argv=None):
             print("%s (%s): %s" % (n, ", ".join(e.dtypes), " ".join(e.__doc__.split())))
         return 0
     from . import build
-    build.build()
+    build.build_library()
     prompts = [[int(t) for t in p.split(",")] for p in a.prompt]
     B, n = len(prompts), len(prompts[0])
     m = models.load(a.model, max_batch=B, max_prefill=a.max_prefill, max_ctx=n + a.n_new, dtype=a.dtype)

@@ -7,11 +7,11 @@ import glob
 import os
 import subprocess
 import sys
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libflexllm_b200.so")
-FRONT_END = os.path.join(HERE, "_front_end.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -91,30 +91,40 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def front_end_path():
+    """File of the Python extension of csrc/front_end.cpp. It is compiled against the layouts of one interpreter and one torch, so its name
+    says which: another torch or Python does not find it and gets one of its own."""
+    import sysconfig
+    import torch
+    return os.path.join(HERE, "_front_end.torch-%s%s" % (torch.__version__, sysconfig.get_config_var("EXT_SUFFIX")))
+
+
 def build_front_end(force=False):
-    """The Python extension of csrc/front_end.cpp (host code against torch's headers)."""
+    """Builds that extension (host code against torch's headers)."""
+    out = front_end_path()
     src = os.path.join(CSRC, "front_end.cpp")
     header = os.path.join(HERE, "..", "include", "flexllm_b200.h")
-    if not force and os.path.exists(FRONT_END) and os.path.getmtime(FRONT_END) > max(os.path.getmtime(src), os.path.getmtime(header)):
-        return FRONT_END
+    if not force and os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(src), os.path.getmtime(header)):
+        return out
     import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.join(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")), "..", "include")
+    part = "%s.%d.part" % (out, os.getpid())                  # never half a file under the name that is loaded
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
            "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(root, "include"),
-           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I", cuda, src, "-o", FRONT_END,
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I", cuda, src, "-o", part,
            "-L", os.path.join(root, "lib"), "-lc10", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("g++ failed on front_end.cpp:\n" + r.stdout + r.stderr)
-    return FRONT_END
+    os.replace(part, out)
+    return out
 
 
-def build(force=False, verbose=False, ptxas_info=False):
+def build_library(force=False, verbose=False, ptxas_info=False):
     if not os.path.exists(os.path.join(CSRC, "exp_constants.inc")):
         gen_exp_constants()
-    build_front_end(force)
     if not force and not needs_build():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
@@ -138,6 +148,16 @@ def build(force=False, verbose=False, ptxas_info=False):
         raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
     if verbose or ptxas_info:
         print("\n".join(log))
+    return LIB
+
+
+def build(force=False, verbose=False, ptxas_info=False):
+    """The library, and the extension where it can be built: without it the calls that it serves take the general path in Python."""
+    build_library(force, verbose, ptxas_info)
+    try:
+        build_front_end(force)
+    except (ImportError, OSError, RuntimeError) as e:       # no torch, no compiler, no headers
+        warnings.warn("flexllm_b200: the native front end was not built, its calls go through Python: %s" % e)
     return LIB
 
 

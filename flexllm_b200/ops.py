@@ -5,7 +5,8 @@ token-parallel (prefill) operators, ``dec_*`` for the single-token (decode) ones
 takes CUDA tensors, allocates its outputs with torch, and launches on the current torch stream.
 """
 import ctypes as C
-import importlib
+import importlib.machinery
+import importlib.util
 
 import torch
 
@@ -38,9 +39,13 @@ _front = None
 def _bind_front_end():
     global _front
     if _front is None:
+        from .build import front_end_path
         try:
-            m = importlib.import_module("._front_end", __package__)
-        except ImportError:             # not built for this interpreter: the general path does the same
+            name, path = __package__ + "._front_end", front_end_path()
+            loader = importlib.machinery.ExtensionFileLoader(name, path)
+            m = importlib.util.module_from_spec(importlib.util.spec_from_loader(name, loader))
+            loader.exec_module(m)
+        except ImportError:             # not built for this interpreter and torch: the general path does the same
             _front = False
         else:
             m.bind(*(C.cast(getattr(lib(), f), C.c_void_p).value for f in (

@@ -49,7 +49,7 @@ def main(argv=None):
     ap.add_argument("--max-tokens", type=int, required=True)
     a = ap.parse_args(argv)
     from . import build
-    build.build()
+    build.build_library()
     n = max(1, a.max_tokens)
     try:
         model = models.load(a.model, max_batch=1, max_prefill=min(n, MAX_CHUNK), max_ctx=n, dtype=a.dtype)
