@@ -49,6 +49,7 @@ inline int launch_status(int n = 1) { note_launches(n); return cuda_status(cudaG
 // completed, and the kernels behind it start after it: between the two halves (pdl_launch, pdl_wait) these may read whatever no kernel
 // of the same sequence of launches writes. Weights may be read there in any case.
 extern thread_local int g_pdl;
+bool programmatic_launches();          // FLEXLLM_PDL=0 in the environment: every kernel starts behind the whole one before
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { pdl_launch(); pdl_wait(); }
@@ -88,7 +89,7 @@ inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cl
 // TMEM, descriptors) under the tail of whatever is in front. A kernel that holds TMEM lets others start only once it has taken its columns. Product of
 // 128 x 2048 x 2048, calls in a row: 8.2 -> 6.7 us; 9 to 8192 rows of nine matrices 1.06 times as fast, of the small ones up to 1.19.
 struct SetUpEarly {
-    const bool set = g_pdl == 0;
+    const bool set = g_pdl == 0 && programmatic_launches();
     SetUpEarly() { if (set) g_pdl = 1; }
     ~SetUpEarly() { if (set) g_pdl = 0; }
 };

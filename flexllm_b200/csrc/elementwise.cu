@@ -1,6 +1,8 @@
 // Row-wise and elementwise operators of the quantized Llama path: per-token quantisation, dequant,
 // static quantisation, RMSNorm(+quant), SiLU, gate, residual, RoPE, softmax, greedy argmax.
 // All are HBM-bound: one pass over the data with 128-bit accesses where the layout allows.
+#include <stdlib.h>
+
 #include <atomic>
 #include <mutex>
 #include <unordered_map>
@@ -12,6 +14,10 @@ namespace flexllm {
 
 thread_local int g_last_cuda_error = 0;
 thread_local int g_pdl = 0;
+bool programmatic_launches() {
+    static const bool on = [] { const char* e = getenv("FLEXLLM_PDL"); return e ? atoi(e) != 0 : true; }();
+    return on;
+}
 std::atomic<unsigned long long> g_launch_count{0};
 
 int raise_shared_limit(const void* kern, size_t bytes) {

@@ -101,7 +101,7 @@ extern "C" int flexllm_mlp_block_decode(const float* x, const float* gamma, cons
     cudaStream_t st = (cudaStream_t)stream;
     // The products ask for their weights without waiting, and a caller's kernel may have written those just before: the first
     // kernel therefore lets the others start only when everything before it in the stream has completed.
-    struct PdlScope { int before; PdlScope() : before(g_pdl) { g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    struct PdlScope { int before; PdlScope() : before(g_pdl) { if (programmatic_launches()) g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
     TRY_RC(flexllm_rmsnorm_quant(x, gamma, M, D, eps, order, nullptr, xq, xs, st));
     TRY_RC(linear_decode(xq, xs, w_gu, s_gu, M, 2 * F, D, nullptr, gu, nullptr, st));
     TRY_RC(swiglu_fht_quant_strided(gu, gu + F, 2L * F, M, fht_scale, hq, hs, st));

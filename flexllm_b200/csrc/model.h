@@ -12,7 +12,6 @@ struct flexllm_tp;
 struct flexllm_model;
 
 namespace flexllm {
-bool programmatic_chains();                                    // FLEXLLM_PDL: 0 launches every kernel of a step behind the whole one before
 struct ModelFamily {
     virtual ~ModelFamily() {}
     // One weight tensor by its name in the checkpoint (host or device memory). Unknown names: FLEXLLM_EINVAL.
