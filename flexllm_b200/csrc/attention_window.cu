@@ -1229,6 +1229,7 @@ void attn_bias_table(const AttnShape& s, const float* table, int rows, int bias_
 template <class T> int attn_window(const AttnCall& c, cudaStream_t st) {
     TRY_RC(check_call(c));
     if (c.Sc == 1) {
+        const ReadsAhead keys;
         const int rc = run_tensor_decode<T>(c, st);
         return rc == FLEXLLM_ENOTSUP ? run_row<T, true>(c, st) : rc;
     }

@@ -8,6 +8,7 @@
 #include <atomic>
 
 #include "../../include/flexllm_b200.h"
+#include "launch_mode.h"
 
 namespace flexllm {
 
@@ -40,16 +41,7 @@ template <class K> inline int allow_shared(K kern, size_t bytes) { return bytes 
 // status of the `n` launches that have just been issued
 inline int launch_status(int n = 1) { note_launches(n); return cuda_status(cudaGetLastError()); }
 
-// Programmatic dependent launch (decode path): when g_pdl is set by the model runner, kernels are
-// launched with the stream-serialization attribute relaxed, so the next kernel's launch and CTA
-// scheduling overlap the tail of the previous one. Every kernel launched this way calls pdl_sync()
-// before it touches memory: it first lets its own dependents start launching, then waits until the
-// kernel before it has completed and flushed (so data hazards are exactly those of an ordinary stream).
-// g_pdl = 2: the next kernel is launched without the attribute and sets g_pdl to 1. It starts when everything before it in the stream has
-// completed, and the kernels behind it start after it: between the two halves (pdl_launch, pdl_wait) these may read whatever no kernel
-// of the same sequence of launches writes. Weights may be read there in any case.
-extern thread_local int g_pdl;
-bool programmatic_launches();          // FLEXLLM_PDL=0 in the environment: every kernel starts behind the whole one before
+// the two halves of a kernel's side of programmatic launches (launch_mode.h)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_sync() { pdl_launch(); pdl_wait(); }
@@ -58,12 +50,12 @@ inline void launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute at[1];
-    if (g_pdl == 1) {
+    if (programmatic_next()) {
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
     }
-    if (g_pdl) g_pdl = 1;
+    launched();
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
@@ -76,23 +68,14 @@ inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cl
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cluster; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    if (g_pdl == 1) {
+    if (programmatic_next()) {
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    if (g_pdl) g_pdl = 1;
+    launched();
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
-
-// Launches in its scope carry the attribute also outside a chain. For kernels that read nothing before their wait: these may be set up (barriers,
-// TMEM, descriptors) under the tail of whatever is in front. A kernel that holds TMEM lets others start only once it has taken its columns. Product of
-// 128 x 2048 x 2048, calls in a row: 8.2 -> 6.7 us; 9 to 8192 rows of nine matrices 1.06 times as fast, of the small ones up to 1.19.
-struct SetUpEarly {
-    const bool set = g_pdl == 0 && programmatic_launches();
-    SetUpEarly() { if (set) g_pdl = 1; }
-    ~SetUpEarly() { if (set) g_pdl = 0; }
-};
 
 #define FLEXLLM_CHECK_CUDA(expr)                                   \
     do {                                                           \

@@ -13,7 +13,7 @@
 namespace flexllm {
 
 thread_local int g_last_cuda_error = 0;
-thread_local int g_pdl = 0;
+thread_local LaunchMode g_pdl = kWhole;
 bool programmatic_launches() {
     static const bool on = [] { const char* e = getenv("FLEXLLM_PDL"); return e ? atoi(e) != 0 : true; }();
     return on;

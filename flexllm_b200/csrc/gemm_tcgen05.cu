@@ -805,7 +805,7 @@ static int launch_gemm(const int8_t* A, int rowsA, const int8_t* B, int rowsB, i
     g.rowsA = rowsA; g.rowsB = rowsB; g.K = K;
     g.tilesA = (rowsA + 127) / 128; g.tilesB = (rowsB + BN - 1) / BN; g.ksplit = ksplit;
     g.ldo = ldo; g.acc = acc; g.y = y; g.sA = sA; g.sB = sB; g.error_flag = device_error_flag();
-    g.residual = residual; g.cluster = SWAP && ksplit > 1; g.ahead = g_pdl == 1;
+    g.residual = residual; g.cluster = SWAP && ksplit > 1; g.ahead = may_read_ahead();
     auto kern = gemm_i8_tcgen05_kernel<BN, SWAP, KCH>;
     // the attribute belongs to (function, device): once per device, not once per process
     static std::atomic<bool> attr_set[kMaxDevices];

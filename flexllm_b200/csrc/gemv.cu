@@ -167,6 +167,7 @@ static int launch_gemv(const int8_t* a, const float* s_tok, const int8_t* w, con
 int gemv_i8(const int8_t* a, const float* s_tok, const int8_t* w, const float* s_ch, int M, int N, int K,
             int32_t* acc, float* y, const float* residual, cudaStream_t st) {
     if (M > 8) return FLEXLLM_ENOTSUP;
+    const ReadsAhead weights;
     if (M <= 1) return launch_gemv<1>(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
     if (M <= 2) return launch_gemv<2>(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
     if (M <= 4) return launch_gemv<4>(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);

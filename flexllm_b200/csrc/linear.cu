@@ -45,7 +45,7 @@ static int linear_decode(const int8_t* a, const float* s_tok, const int8_t* w, c
     // 14.7 / 11.0; 2048x8192 10.4 / 10.3, 13.5 / 10.4; 128256x2048 50 / 46, 81 / 47; 2 tokens 44.6 / 45.8 there). Behind other kernels of a chain
     // it has its weights early: MLP block of 3 tokens 22.4 / 17.9, of 8 32.4 / 18.7, of 2 17.5 / 17.9.
     const bool large = (long)N * K >= 12L << 20;
-    if (M <= (large ? (g_pdl ? 2 : 3) : 8)) return gemv_i8(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
+    if (M <= (large ? (in_chain() ? 2 : 3) : 8)) return gemv_i8(a, s_tok, w, s_ch, M, N, K, acc, y, residual, st);
     return gemm_i8_decode(a, s_tok, w, s_ch, M, N, K, acc, y, st, residual);
 }
 
@@ -101,7 +101,7 @@ extern "C" int flexllm_mlp_block_decode(const float* x, const float* gamma, cons
     cudaStream_t st = (cudaStream_t)stream;
     // The products ask for their weights without waiting, and a caller's kernel may have written those just before: the first
     // kernel therefore lets the others start only when everything before it in the stream has completed.
-    struct PdlScope { int before; PdlScope() : before(g_pdl) { if (programmatic_launches()) g_pdl = 1; } ~PdlScope() { g_pdl = before; } } pdl;
+    struct PdlScope { LaunchMode before; PdlScope() : before(g_pdl) { if (programmatic_launches()) g_pdl = kChain; } ~PdlScope() { g_pdl = before; } } pdl;
     TRY_RC(flexllm_rmsnorm_quant(x, gamma, M, D, eps, order, nullptr, xq, xs, st));
     TRY_RC(linear_decode(xq, xs, w_gu, s_gu, M, 2 * F, D, nullptr, gu, nullptr, st));
     TRY_RC(swiglu_fht_quant_strided(gu, gu + F, 2L * F, M, fht_scale, hq, hs, st));

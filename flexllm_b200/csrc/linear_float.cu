@@ -468,6 +468,7 @@ int check(const void* a, long lda, const void* w, long ldw, int M, int N, int K,
 int linear_bf16(const bf16* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     TRY_RC(check(a, lda, w, ldw, M, N, K, act, y));
     if (M == 0) return FLEXLLM_OK;
+    const ReadsAhead weights;
     // Measured on the layer shapes of 1B to 8B models (us; GEMV / warp-MMA / tensor-core form):
     //   1 token : 5120x2048 5.8 / 7.1 / 9.5, 16384x2048 13.7 / 14.7 / 14.5; long rows 2048x8192 9.6 / 7.6 / 18.6
     //   2 to 8  : 5120x2048 8.0 / 7.1 / 9.5, 16384x2048 15.5 / 14.7 / 14.6, head 128256x2048 92 / 77 / 80
@@ -487,6 +488,7 @@ int linear_bf16(const bf16* a, long lda, const bf16* w, long ldw, const float* b
 int linear_f32(const float* a, long lda, const bf16* w, long ldw, const float* bias, int M, int N, int K, int act, LinearOut y, cudaStream_t st) {
     TRY_RC(check(a, lda, w, ldw, M, N, K, act, y));
     if (M == 0) return FLEXLLM_OK;
+    const ReadsAhead weights;
     if (M <= 4) {
         const int rc = gemv_any<float>(a, lda, w, ldw, bias, M, N, K, act, y, st);
         if (rc != FLEXLLM_ENOTSUP) return rc;

@@ -683,9 +683,9 @@ static int decode_step_body(flexllm_model* m, cudaStream_t st);
 static int decode_step(flexllm_model* m, cudaStream_t st) {
     TRY(mega_prepare(m));
     if (m->mega_state == 1) return mega_launch(m->mega, m->B, m->mega_variant, st);
-    g_pdl = programmatic_launches() ? 2 : 0;             // the kernels of a step read the contexts, page tables and older cache entries ahead of their wait
+    g_pdl = programmatic_launches() ? kChainStart : kWhole;             // the kernels of a step read the contexts, page tables and older cache entries ahead of their wait
     const int rc = decode_step_body(m, st);
-    g_pdl = 0;
+    g_pdl = kWhole;
     return rc;
 }
 static int decode_step_body(flexllm_model* m, cudaStream_t st) {

@@ -530,9 +530,9 @@ class DecoderFamily : public ModelFamily {
         // Pibidra of 16 layers, 2048 channels: 1 x 40 tokens 1.85 -> 1.61 ms, 4 x 40 2.26 -> 2.11, 4 x 500 5.55 -> 5.35; Sabisun 1.80 -> 1.64, 2.34 -> 2.27,
         // 5.67 -> 5.55; from 4000 tokens on the same.
         struct Chain {
-            const bool set = g_pdl == 0 && programmatic_launches();
-            Chain() { if (set) g_pdl = 2; }
-            ~Chain() { if (set) g_pdl = 0; }
+            const bool set = g_pdl == kWhole && programmatic_launches();
+            Chain() { if (set) g_pdl = kChainStart; }
+            ~Chain() { if (set) g_pdl = kWhole; }
         } chain;
         return cfg.dtype == FLEXLLM_BF16 ? step<bf16>(m, tok, B, S, c0, Sc, st) : step<float>(m, tok, B, S, c0, Sc, st);
     }

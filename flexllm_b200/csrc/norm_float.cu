@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(NT) hyper_norm_kernel(const HyperNormArgs a) {
 template <class T, int NS> int launch_hyper(const HyperNormArgs& a, int rows, cudaStream_t st) {
     const int nv = (a.D + 3) / 4;
     const bool ahead = rows <= kAheadRows;
+    const ReadsAhead gains;
 #define FLEXLLM_HYPER(NT_, VPT_) launch_k(ahead ? hyper_norm_kernel<T, NS, NT_, VPT_, true> : hyper_norm_kernel<T, NS, NT_, VPT_, false>, dim3(rows), dim3(NT_), 0, st, a)
     if (nv <= 128) FLEXLLM_HYPER(128, 1);
     else if (nv <= 256) FLEXLLM_HYPER(256, 1);
@@ -269,6 +270,7 @@ template <class T> int res_norm(const ResNormArgs& a, int rows, cudaStream_t st)
     if (rows == 0) return FLEXLLM_OK;
     const int nv = (a.D + 3) / 4;
     const bool ahead = rows <= kAheadRows;
+    const ReadsAhead gains;
 #define FLEXLLM_RES(NT_, VPT_) launch_k(ahead ? res_norm_kernel<T, NT_, VPT_, true> : res_norm_kernel<T, NT_, VPT_, false>, dim3(rows), dim3(NT_), 0, st, a)
     if (nv <= 128) FLEXLLM_RES(128, 1);
     else if (nv <= 256) FLEXLLM_RES(256, 1);

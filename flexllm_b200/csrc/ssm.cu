@@ -610,6 +610,7 @@ template <class T> int ssm_mixer(const SsmCall& c, cudaStream_t st) {
     FLEXLLM_REQUIRE(c.proj && c.conv_w && c.conv_b && c.dt_bias && c.A && c.D && c.gain && c.state && c.conv_state && c.ctx && c.y && c.out);
     FLEXLLM_REQUIRE(c.B > 0 && c.Sc > 0 && c.xbc);
     if (!ssm_supported(s) || c.B > 65535 || c.Sc > 65535 * kConvTokens) return FLEXLLM_ENOTSUP;
+    const ReadsAhead states;
     TRY_RC(run_conv<T>(c, st));
     int rc = c.Sc == 1 ? run_scan<T, 1>(c, st) : run_chunks<T>(c, st);
     if (rc == FLEXLLM_ENOTSUP) rc = run_scan<T, kScanTile>(c, st);
