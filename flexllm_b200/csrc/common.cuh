@@ -77,6 +77,28 @@ inline void launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, int cl
     cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
 
+// Greedy token of a row, scanned by many threads: the largest value, the lowest index among equals (Logits.h:13-17). A NaN exceeds nothing and nothing
+// exceeds it, so a scan from index 0 by '>' takes a NaN at index 0 and no other. Every thread looks at its elements in increasing order.
+struct GreedyToken {
+    float v = -INFINITY;
+    int i = 0x7fffffff;
+    __device__ __forceinline__ GreedyToken() {}
+    __device__ __forceinline__ GreedyToken(float v_, int i_) : v(v_), i(i_) {}
+    // begin: the thread's first index, below the row's end or not (-inf there: right for that value, and for a NaN less than any index before it)
+    __device__ __forceinline__ void begin(long first, long end) { if (first < end) i = (int)first; }
+    __device__ __forceinline__ void take(float t, long at) { if (t > v) { v = t; i = (int)at; } }
+    __device__ __forceinline__ void first_of_row(float t) { if (t != t) { v = INFINITY; i = 0; } }      // index 0, after the thread's scan
+    __device__ __forceinline__ void merge(float ov, int oi) { if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; } }
+    __device__ __forceinline__ void merge_warp() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+            merge(ov, oi);
+        }
+    }
+};
+
 #define FLEXLLM_CHECK_CUDA(expr)                                   \
     do {                                                           \
         int _st = ::flexllm::cuda_status((expr));                  \

@@ -481,33 +481,20 @@ __device__ __forceinline__ void mega_row_fht4(const MegaArgs& a, const MegaLayer
 __device__ __forceinline__ void mega_row_argmax(const MegaArgs& a, int row, int col, int n_cols, float* sv, int* si) {
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const float* l = a.logits + (long)row * a.V;
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int v = tid; v < a.V; v += MG_WORKERS) {
-        const float t = __ldcg(l + v);
-        if (t > best || bi == 0x7fffffff) { best = t; bi = v; }
-    }
-    auto better = [](float x, int xi, float y, int yi) { return x > y || (x == y && xi < yi); };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-    }
-    if (lane == 0) { sv[w] = best; si[w] = bi; }
+    const float first = __ldcg(l);
+    GreedyToken g;
+    g.begin(tid, a.V);
+    for (int v = tid; v < a.V; v += MG_WORKERS) g.take(__ldcg(l + v), v);
+    if (tid == 0) g.first_of_row(first);
+    g.merge_warp();
+    if (lane == 0) { sv[w] = g.v; si[w] = g.i; }
     named_sync<MG_BAR_WORK, MG_WORKERS>();
     if (w == 0) {
-        best = lane < MG_WORKERS / 32 ? sv[lane] : -INFINITY;
-        bi = lane < MG_WORKERS / 32 ? si[lane] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-        }
+        g = lane < MG_WORKERS / 32 ? GreedyToken(sv[lane], si[lane]) : GreedyToken();
+        g.merge_warp();
         if (lane == 0) {
-            a.next[row] = bi;
-            if (col < n_cols) a.out_tokens[(long)row * n_cols + col] = bi;
+            a.next[row] = g.i;
+            if (col < n_cols) a.out_tokens[(long)row * n_cols + col] = g.i;
             a.ctx[row] += 1;
         }
     }

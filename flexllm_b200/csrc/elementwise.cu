@@ -470,55 +470,43 @@ __global__ void __launch_bounds__(NT) argmax_kernel(const float* __restrict__ lo
     const int part = blockIdx.x % CL;
     const long row = blockIdx.x / CL, v1 = V * (part + 1) / CL;
     const float* l = logits + row * V;
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
+    const float first = l[0];
+    GreedyToken g;
     // strided scan in increasing v; eight loads in flight
     long v = V * part / CL + threadIdx.x;
+    const bool has_first = v == 0;
+    g.begin(v, v1);
     for (; v + 7L * NT < v1; v += 8L * NT) {
         float t[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) t[i] = l[v + (long)i * NT];
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (t[i] > best || bi == 0x7fffffff) { best = t[i]; bi = (int)(v + (long)i * NT); }
+        for (int i = 0; i < 8; i++) g.take(t[i], v + (long)i * NT);
     }
-    for (; v < v1; v += NT) {
-        const float t = l[v];
-        if (t > best || bi == 0x7fffffff) { best = t; bi = (int)v; }
-    }
-    auto better = [](float a, int ai, float b, int bi2) { return a > b || (a == b && ai < bi2); };
-    auto warp_best = [&]() {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-        }
-    };
-    warp_best();
+    for (; v < v1; v += NT) g.take(l[v], v);
+    if (has_first) g.first_of_row(first);
+    g.merge_warp();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (CL > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-    if (lane == 0) { sv[w] = best; si[w] = bi; }
+    if (lane == 0) { sv[w] = g.v; si[w] = g.i; }
     __syncthreads();
     if (w == 0) {
-        best = lane < NT / 32 ? sv[lane] : -INFINITY;
-        bi = lane < NT / 32 ? si[lane] : 0x7fffffff;
-        warp_best();
+        g = lane < NT / 32 ? GreedyToken(sv[lane], si[lane]) : GreedyToken();
+        g.merge_warp();
         if (CL == 1) {
-            if (lane == 0) idx[row] = bi;
+            if (lane == 0) idx[row] = g.i;
         } else if (lane == 0) {
             const uint32_t av = tc::cluster_addr(tc::smem_u32(cv + part), 0), ai = tc::cluster_addr(tc::smem_u32(ci + part), 0);
-            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(av), "f"(best) : "memory");
-            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ai), "r"(bi) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(av), "f"(g.v) : "memory");
+            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(ai), "r"(g.i) : "memory");
         }
     }
     if (CL > 1) {
         tc::cluster_sync();
         if (part == 0 && w == 0) {
-            best = lane < CL ? cv[lane % CL] : -INFINITY;
-            bi = lane < CL ? ci[lane % CL] : 0x7fffffff;
-            warp_best();
-            if (lane == 0) idx[row] = bi;
+            g = lane < CL ? GreedyToken(cv[lane % CL], ci[lane % CL]) : GreedyToken();
+            g.merge_warp();
+            if (lane == 0) idx[row] = g.i;
         }
     }
 }

@@ -88,33 +88,20 @@ __global__ void __launch_bounds__(1024) argmax_pair_kernel(const float* __restri
     __shared__ int si[32];
     pdl_sync();
     const float* l = logits + (long)blockIdx.x * V;
-    float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (long v = threadIdx.x; v < V; v += blockDim.x) {
-        const float t = l[v];
-        if (t > best || bi == 0x7fffffff) { best = t; bi = (int)v; }
-    }
-    auto better = [](float a, int ai, float b, int bi2) { return a > b || (a == b && ai < bi2); };
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-    }
+    const float first = l[0];
+    GreedyToken g;
+    g.begin(threadIdx.x, V);
+    for (long v = threadIdx.x; v < V; v += blockDim.x) g.take(l[v], v);
+    if (threadIdx.x == 0 && offset == 0) g.first_of_row(first);          // the first slice has the row's index 0
+    g.merge_warp();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { sv[w] = best; si[w] = bi; }
+    if (lane == 0) { sv[w] = g.v; si[w] = g.i; }
     __syncthreads();
     if (w == 0) {
         const int nw = blockDim.x >> 5;
-        best = lane < nw ? sv[lane] : -INFINITY;
-        bi = lane < nw ? si[lane] : 0x7fffffff;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (better(ob, oi, best, bi)) { best = ob; bi = oi; }
-        }
-        if (lane == 0) { out[blockIdx.x].val = best; out[blockIdx.x].idx = bi + offset; }
+        g = lane < nw ? GreedyToken(sv[lane], si[lane]) : GreedyToken();
+        g.merge_warp();
+        if (lane == 0) { out[blockIdx.x].val = g.v; out[blockIdx.x].idx = g.i + offset; }
     }
 }
 // pairs [g][B] -> idx [B]

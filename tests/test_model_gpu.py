@@ -96,6 +96,21 @@ def test_model_of_longer_contexts_beside_another(F):
     for m in models: m.close()
 
 
+@pytest.mark.parametrize("mega", ["1", "0"])
+def test_greedy_token_beside_nan_logits(F, monkeypatch, mega):
+    """Logits that are NaN (here by their scale) are never the token and hide no other, in the prompt and on either decode path."""
+    from flexllm_b200 import synthetic
+    monkeypatch.setenv("FLEXLLM_MEGA", mega)
+    W = synthetic.numpy_weights(1, 256, 4, 1, 8192, 9000, 48, seed=92)
+    W["lm_s"][1:900] = np.nan
+    tokens = np.random.default_rng(93).integers(900, 9000, (8, 32)).astype(np.int32)
+    m = F.Model(1, 256, 4, 1, 8192, 9000, max_batch=8, max_prefill=32, max_ctx=48)
+    synthetic.load_numpy_weights(m, W)
+    out = m.generate_host(torch.from_numpy(tokens), 12, use_graph=False)
+    m.close()
+    assert np.array_equal(out.numpy(), oracle.model_generate(W, tokens, 12)["tokens"])
+
+
 def test_model_batch_over_8(F):
     """More than 8 sequences sends the decode linear layers down the tensor-core split-K path."""
     run_case(F, layers=2, hidden=512, hq=8, hkv=2, vocab=1000, B=12, S=16, n_new=4, seed=53, use_graph=True)

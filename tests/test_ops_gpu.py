@@ -348,6 +348,19 @@ def test_argmax_long_rows(F, B, V):
     assert_same(to_np(F.dec_Logits_argmax(dev(l))), oracle.argmax(l))
 
 
+@pytest.mark.parametrize("B,V", [(4, 1000), (4, 8191), (4, 8192), (64, 9000), (65, 9000), (4, 128256)])
+def test_argmax_nan(F, B, V):
+    """A NaN is the token at index 0 and nowhere else, and hides no other element: NaN at index 0, in the first element of many threads of either
+    form, all over."""
+    l = rng(17).standard_normal((B, V)).astype(np.float32)
+    l[0, 0] = np.nan
+    l[1, 1:900] = np.nan
+    for p in range(8): l[2, V * p // 8 + (p == 0):V * p // 8 + 100] = np.nan
+    l[3, 1:] = np.nan
+    l[3, 0] = -np.inf
+    if B > 4: l[4] = np.nan; l[5, 0] = np.nan; l[5, V // 2] = np.inf
+    assert_same(to_np(F.dec_Logits_argmax(dev(l))), oracle.argmax(l))
+
 
 # ------------------------------------------------------------------------------ linear layers
 def lin_inputs(M, N, K, seed):

@@ -131,6 +131,31 @@ def test_tp_ranks_sharing_one_gpu_match_oracle(world, cfg, mode, monkeypatch):
     assert np.array_equal(ret["hidden"].view(np.uint32), ref["hidden"].view(np.uint32))
 
 
+def test_tp_greedy_token_beside_nan_logits(monkeypatch):
+    """NaN logits at the start of both slices of the vocabulary, index 0 apart: never the token, and they hide no other."""
+    import threading
+    import oracle
+    import flexllm_b200 as F
+    from flexllm_b200 import synthetic
+    monkeypatch.setenv("FLEXLLM_TP_MODE", "allgather")
+    cfg = (1, 512, 8, 2, 8000, 4, 32, 6, 94)
+    layers, hidden, hq, hkv, vocab, B, S, n_new, seed = cfg
+    W = synthetic.numpy_weights(layers, hidden, hq, hkv, 8192, vocab, S + n_new, seed=seed)
+    W["lm_s"][1:900] = np.nan
+    W["lm_s"][4000:4900] = np.nan
+    tokens = np.random.default_rng(seed + 1).integers(5000, vocab, (B, S)).astype(np.int32)
+    group, ret = F.TensorParallel.local_group(2), {}
+    threads = [threading.Thread(target=_shared_device_rank, args=(tp, cfg, W, tokens, ret)) for tp in group]
+    for t in threads: t.start()
+    for t in threads: t.join()
+    for tp in group: tp.close()
+    assert not [k for k in ret if k.startswith("error")], ret
+    with oracle.exp_mode(oracle.EXP_CORRECTLY_ROUNDED):
+        want = oracle.model_generate(W, tokens, n_new)["tokens"]
+    for rank in range(2):
+        assert np.array_equal(ret[f"tokens{rank}"], want)
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_collectives_of_ranks_sharing_one_gpu(world):
     """Every collective of the device-sharing group against numpy: all-reduce (sum, max), reduce-scatter, all-gather,
