@@ -331,7 +331,7 @@ def test_kv_append_alone(F):
 
 
 @pytest.mark.parametrize("ctx,HKV,what", [
-    ([512, 0, 63, 64, 65, 127, 128, 191, 192, 256], 8, {}), ([511, 510, 100], 8, {}),                # one side and the other of the first length
+    ([512, 0, 63, 64, 65, 127, 128, 191, 192, 256], 8, {}), ([511, 510, 100], 8, {}), ([510, 500, 100], 8, {}),     # the first length's line is 512
     ([3000, 0, 63, 64, 255, 256, 257, 3000, 1023, 1024], 2, {}), ([3000, 2999, 31], 1, dict(q_gain=20.0)),
     ([1700] + [130] * 9 + [1700] * 9 + [0], 8, {}), ([1662] + [40] * 18, 8, {}), ([1664, 1663] + [40] * 17, 8, dict(a_gain=0.01)),       # by length, with equal ones
     ([2000] + [300] * 16, 8, {}), ([2000] + [300] * 17, 8, {}),                                      # all clusters at once, and not quite

@@ -108,3 +108,35 @@ def test_full_model_two_decode_paths(F, monkeypatch, layers, B, S, n_new, what):
     assert_same(res["1"][2], res["0"][2], "logits of the last decode step")
     # not a degenerate run: the sequences do not all emit one token
     assert len(np.unique(res["1"][0])) > min(B, 8)
+
+
+@pytest.mark.parametrize("B,S,n_new,max_ctx,variant", [
+    (1, 1024, 3, 1026, 3), (4, 1040, 3, 1042, 3), (4, 208, 3, 210, 3),          # a query head per CTA: one to four sequences
+    (4, 1904, 16, 2112, 3), (4, 1904, 17, 2112, 0),                             # the longest call whose pages fit the operand ring, and one more step
+    (5, 1040, 3, 1042, 2), (18, 1040, 3, 1042, 2), (19, 304, 3, 306, 1),        # an item per CTA, and two
+])
+def test_variant_of_the_persistent_step(F, monkeypatch, B, S, n_new, max_ctx, variant):
+    """Which attention variant a decode step launches on either side of each line of the rule, at full width in two layers, and the same tokens,
+    residual stream and logits as the kernel-per-operator path."""
+    from torch.profiler import ProfilerActivity, profile
+    from flexllm_b200 import synthetic
+    cfg = dict(synthetic.LLAMA32_1B)
+    cfg["layers"] = 2
+    tok = torch.randint(0, cfg["vocab"], (B, S), dtype=torch.int32, generator=torch.Generator().manual_seed(78))
+    res = {}
+    for mega in ("1", "0"):
+        monkeypatch.setenv("FLEXLLM_MEGA", mega)
+        m = F.Model(max_batch=32, max_prefill=S, max_ctx=max_ctx, **cfg)
+        synthetic.load_random_weights(m, max_ctx=max_ctx, seed=6, **cfg)
+        with profile(activities=[ProfilerActivity.CUDA]) as seen:
+            out = m.generate_host(tok, n_new, use_graph=False)
+        names = {e.key.split("(")[0].split("::")[-1] for e in seen.key_averages() if "decode_mega" in e.key}
+        assert names == ({"decode_mega_kernel<32, %d>" % variant} if mega == "1" else set())
+        assert F.lib().flexllm_device_status() == 0
+        res[mega] = (out.numpy().copy(), to_np(m.buffer(0, (B, cfg["hidden"]), torch.float32)), to_np(m.buffer(1, (B, cfg["vocab"]), torch.float32)))
+        m.close()
+        del m
+        torch.cuda.empty_cache()
+    assert np.array_equal(res["1"][0], res["0"][0])
+    assert_same(res["1"][1], res["0"][1], "residual stream of the last decode step")
+    assert_same(res["1"][2], res["0"][2], "logits of the last decode step")

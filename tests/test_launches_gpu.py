@@ -69,3 +69,61 @@ def test_programmatic_launches_can_be_switched_off(pdl):
     assert set(found) == {"products", "attention", "mlp", "prompt"}
     for name, (programmatic, n) in found.items():
         assert n > 0 and (programmatic > 0 if pdl == "1" else programmatic == 0), (name, programmatic, n)
+
+
+def chain(F, seed):
+    """Inputs and the launches of a prompt's operators one after another, each on the output of the one before."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    s8 = lambda *n: torch.randint(-127, 128, n, dtype=torch.int8, device="cuda", generator=gen)
+    u = lambda *n: torch.rand(n, device="cuda", generator=gen) * 1e-2
+    a, w, sc = s8(256, 1024), [s8(1024, 1024) for _ in range(3)], u(1024)
+    q, k, v, cos, sin, a_s = s8(2, 128, 16, 64), s8(2, 128, 4, 64), s8(2, 128, 4, 64), u(128, 32), u(128, 32), u(16)
+    qs, ks, s0 = u(2, 128, 16), u(2, 128, 4), u(256)
+
+    def work():
+        y = F.pref_Linear_Layer_i8xi8(a, s0, w[0], sc)[1]
+        for m in w[1:]:
+            x, s = F.pref_quant_layer_fp32_qint(y)
+            y = F.pref_Linear_Layer_i8xi8(x, s, m, sc, residual=y)[1]
+        x, s = F.pref_quant_layer_fp32_qint(y)
+        out = F.MHA_i8xi8_Prefilling(x.view(2, 128, 16, 64), qs, k, ks, v, ks, cos, sin, a_s)[0]
+        return y, out, F.MHA_i8xi8_Prefilling(q, qs, k, ks, v, ks, cos, sin, a_s)[0]
+    return (a, k), work
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_prompt_operators_behind_another_stream(captured):
+    """Inputs written late on another stream, which the first product follows through an event alone; eagerly and as a graph that is replayed
+    on inputs it was not captured with."""
+    import flexllm_b200 as F
+    (a, k), work = chain(F, 5)
+    new = [torch.randint(-127, 128, t.shape, dtype=torch.int8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i, t in enumerate((a, k))]
+    old = [a.clone(), k.clone()]
+    for t, n in zip((a, k), new): t.copy_(n)
+    want = [t.clone() for t in work()]
+    for t, n in zip((a, k), old): t.copy_(n)
+    main, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def forked():
+        other.wait_stream(main)
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(2_000_000)              # a millisecond: the products would be long over
+            for t, n in zip((a, k), new): t.copy_(n)
+        main.wait_stream(other)
+        return work()
+    with torch.cuda.stream(main):
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            g.capture_begin()
+            got = forked()
+            g.capture_end()
+            for _ in range(3):
+                for t, n in zip((a, k), old): t.copy_(n)
+                g.replay()
+        else:
+            got = forked()
+    torch.cuda.synchronize()
+    for x, y in zip(got, want):
+        assert torch.equal(x, y)
+    assert F.lib().flexllm_device_status() == 0

@@ -81,6 +81,40 @@ def test_model_swiglu_in_the_product(F, B, S):
     run_case(F, 1, 256, 4, 1, 512, B, S, 1, seed=70 + S, use_graph=False)
 
 
+@pytest.mark.parametrize("what", ["infinite_gate", "nan_up", "nan_channel_scale", "large", "tiny", "zero", "rows"])
+def test_model_swiglu_in_the_product_out_of_range(F, what):
+    """Infinities, NaN and scales beyond the short quantiser's range through the product that forms silu(gate) * up (256 rows) and the rest of the
+    transform: what the plain product and the whole transform (128 rows) give for each sequence alone; the oracle's bits where it has numbers."""
+    from flexllm_b200 import synthetic
+    B, S, D, V = 2, 128, 256, 512
+    W = synthetic.numpy_weights(1, D, 4, 1, 8192, V, S + 1, seed=95)
+    tokens = np.random.default_rng(96).integers(8, V, (B, S)).astype(np.int32)
+    if what == "infinite_gate": W["sg"][0][[7, 4100]] = 3e38           # +-inf, or finite where the sum is small; silu(-inf) * up is NaN
+    if what == "nan_up": W["su"][0][9] = np.nan
+    if what == "nan_channel_scale": W["sg"][0][8191] = np.nan
+    if what == "large": W["sg"][0][:] *= 1e12; W["su"][0][:] *= 1e12
+    if what == "tiny": W["su"][0][:] *= 1e-25
+    if what == "zero": W["su"][0][:] = 0
+    if what == "rows":                                                  # rows of their own, late in a sequence: a NaN spreads to the ones behind it
+        W["lm_s"][:3] = [np.inf, np.nan, 1e36]
+        tokens[0, [100, 120]] = [2, 0]; tokens[1, 127] = 1
+    m = F.Model(1, D, 4, 1, 8192, V, max_batch=B, max_prefill=S, max_ctx=S + 1)
+    synthetic.load_numpy_weights(m, W)
+    def hidden(t):
+        m.prefill(torch.from_numpy(t).cuda())
+        torch.cuda.synchronize()
+        return to_np(m.buffer(0, (len(t) * S, D), torch.float32)).copy()
+    got = hidden(tokens)
+    want = np.concatenate([hidden(tokens[b:b + 1]) for b in range(B)])
+    m.close()
+    nan = np.isnan(want)
+    assert (np.isnan(got) == nan).all()
+    assert np.array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32))
+    if what in ("large", "tiny", "zero"):
+        assert not nan.any()
+        assert np.array_equal(got.view(np.uint32), oracle.model_generate(W, tokens, 1, want_hidden=True)["hidden"].view(np.uint32))
+
+
 def test_model_of_longer_contexts_beside_another(F):
     """A model whose decode step needs more shared memory than that of one made after it: both go on giving their tokens."""
     from flexllm_b200 import synthetic
