@@ -345,7 +345,8 @@ static int launch_dec_fused(bool in_f32, const int8_t* q, const float* qs, const
 // bytes of a row are its four operand words. A CTA needs 5 bytes per key, so four share an SM (64 registers a thread): while one waits for its
 // pages, its peers or the ordered sums, the others have work.
 // Bound by that chain of phases (64 x 8100 keys, one generation of CTAs: 46 us, of which the scores 11, ordered sums 8, P.V 5) and by memory:
-// 64 sequences of 512 to 8192 keys (47 us at the copy rate) 98 us, 125 before with every page read by two SMs.
+// 64 sequences of 512 to 8192 keys (47 us at the copy rate), calls one after another: 99 to 116 us by the draw of the lengths, 122 to 146 with every
+// page read by two SMs.
 constexpr int DEC_FUSED_KEYS = 10240;      // most keys of the forms with an item per CTA
 constexpr int DEC_CL = 4, DEC_CL_NT = 256, DEC_CL_PAGES = 512;       // CTAs of a cluster (one per query head), threads, most pages of a sequence
 struct DecClusterSmem {
@@ -858,9 +859,11 @@ int flexllm::mha_decode_run(flexllm_kv_cache* c, int layer, const int8_t* q, con
     // Three forms. us, 8 KV heads: one or two CTAs per (sequence, head) / a cluster of four: 1 x 400 keys 8.0 / 8.2, 1 x 513 9.0 / 7.9,
     // 1 x 2000 13.3 / 9.6; 16 x 400 9.4 / 10.3, 16 x 513 11.6 / 10.6, 16 x 8100 66.6 / 43.2; 18 x 2000 20.3 / 21.7; 32 x 1400 22.8 / 25.5,
     // 32 x 1700 27.6 / 27.2, 32 x 8100 132 / 93.5; 64 x 300 19.2 / 33.3, 64 x 1700 57.7 / 56.1, 64 x 4096 120 / 102, 64 x 8100 245 / 170, 64 of 512 to
-    // 8192 125 / 98. So clusters from 513 keys where they all run at once (25 for every 24 SMs do not: their CTAs share a part of the
-    // chip), from 1665 where they follow one another, and where the second wave would be nearly empty not at all.
-    // Kernel per phase / cluster, the only choices for longer contexts: 1 x 10500 65 / 25, 16 x 32000 449 / 346, 64 x 14000 535 / 335.
+    // 8192 (five draws of the lengths) 122 to 146 / 99 to 116. So clusters from 513 keys where they all run at once (25 for every 24 SMs do
+    // not: their CTAs share a part of the chip), from 1665 where they follow one another, and where the second wave would be nearly empty not at all.
+    // Kernel per phase / cluster, the only choices for contexts above DEC_FUSED_KEYS: 1 x 10500 65 / 25, 16 x 32000 449 / 346, 64 x 14000 535 / 335.
+    // at_once counts four CTAs an SM, which their shared memory allows up to about 10600 keys. Beyond that they may follow one another also
+    // where it holds; they then run in the order of the sequences and not by length.
     const int sms = gemm_sm_count(), items = B * HKV;
     const bool at_once = items * 25 <= sms * 24;
     if (max_ctx > (at_once ? 512 : 1664) && ctx_stride <= DEC_CL_PAGES * PAGE && (at_once || items > sms || ctx_stride > DEC_FUSED_KEYS)) {

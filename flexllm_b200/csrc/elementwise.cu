@@ -182,7 +182,7 @@ constexpr int RMS_PIECE = 128;           // floats per row per staging step
 // once); warp 0 then runs the 16 chains (4 per row) over them; afterwards every thread normalises and quantises the same columns of all four rows, whose
 // gains it has held since the start -- each row is read from global memory once. Row stride D + 4 floats: the chains' reads (row rr, element
 // 4k + j) fall into different banks. Requires D % 128 == 0. COLS: groups of four columns a thread.
-// Bound by the ordered sums and the phases around them, which six CTAs an SM take turns in: 32768 rows of 2048 98 us (353 MB: 54 us at the copy rate), 32 rows
+// Bound by the ordered sums and the phases around them, which six CTAs an SM take turns in: 32768 rows of 2048 98 us (336 MB: 51 us at the copy rate), 32 rows
 // 6.7 us. A warp per row in the last phase, eight rows a CTA, waited for the gains at every step: 124 and 8.5 us (rows of 4096: 493 and 15.5 us, now
 // 298 and 12.1); eight rows a CTA by columns 102 and 7.0 us; four and two rows by rows 118 and 113 us.
 constexpr int RMSP_ROWS = 4;
