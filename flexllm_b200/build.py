@@ -115,10 +115,14 @@ def build_front_end(force=False):
            "-I", sysconfig.get_paths()["include"], "-isystem", os.path.join(root, "include"),
            "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"), "-I", cuda, src, "-o", part,
            "-L", os.path.join(root, "lib"), "-lc10", "-ltorch_cpu", "-ltorch_python", "-lc10_cuda"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("g++ failed on front_end.cpp:\n" + r.stdout + r.stderr)
-    os.replace(part, out)
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("g++ failed on front_end.cpp:\n" + r.stdout + r.stderr)
+        os.replace(part, out)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
     return out
 
 
